@@ -70,7 +70,7 @@ def build(ref: bool = True, ref_root: Optional[str] = None) -> None:
     names an existing reference source tree, the reference library."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
     root = ref_root or REF_ROOT
-    if ref and root and os.path.isdir(root):
+    if ref and root and os.path.isdir(os.path.join(root, "db")):
         subprocess.run(["make", "-s", "-j8", "-C", HERE, "ref", f"REF_ROOT={root}"],
                        check=True)
         # the compiled drop-in and its CPU twin (needs the engine library built)
