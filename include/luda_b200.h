@@ -298,8 +298,7 @@ lc_status lc_build_table(lc_engine* e, const lc_table_options* opt, int64_t n,
  * (table/table_builder.cc:186-189) and that ReadBlock's verify_checksums path
  * checks (table/format.cc:87-94).  Computed on the engine's device over many
  * CTAs; data is host memory (copied in) or, with on_device, device memory.
- * The result is written to *masked_crc (host memory).  Scratch comes from the
- * engine's device memory pool. */
+ * The result is written to *masked_crc (host memory). */
 lc_status lc_crc32c(lc_engine* e, const uint8_t* data, uint64_t n, int32_t on_device,
                     uint32_t* masked_crc);
 
@@ -312,16 +311,16 @@ lc_status lc_crc32c(lc_engine* e, const uint8_t* data, uint64_t n, int32_t on_de
  * bytes; d_masked_crc: 4 output bytes), runs on `stream` (a cudaStream_t, or
  * NULL for the default stream) and returns without waiting for the GPU.
  *
- * Scratch is one fixed static device array (about 64 KiB, held by every
- * device that loads the library until the process exits), so n is limited to
- * 1 GiB; larger buffers are rejected with LC_ERR_UNSUPPORTED before anything
- * is launched.  Null pointers give LC_ERR_INVALID_ARG, runtime failures
+ * Scratch is one fixed static device array (a few words, held by every device
+ * that loads the library until the process exits).  n is limited to 1 GiB;
+ * larger buffers are rejected with LC_ERR_UNSUPPORTED before anything is
+ * launched.  Null pointers give LC_ERR_INVALID_ARG, runtime failures
  * LC_ERR_CUDA; each failure also sets lc_last_error().  The first call on a
  * device looks up the array's device address (cudaGetSymbolAddress) with that
  * device current and keeps it; make that first call before any stream capture,
  * and do not use the entry point across a cudaDeviceReset (the kept address
- * belongs to the context that was reset).  Every call clears the part of the array that must
- * start at zero, but all calls share the array: calls that overlap on the GPU
+ * belongs to the context that was reset).  Every call clears the array first,
+ * but all calls share it: calls that overlap on the GPU
  * (on different streams, or from different threads) race, so serialise them,
  * e.g. on one stream. */
 lc_status lc_crc32c_noalloc(const uint8_t* d_data, uint64_t n, uint32_t* d_masked_crc,

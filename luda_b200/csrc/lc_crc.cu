@@ -1,5 +1,5 @@
 // Chunked masked CRC32C of one buffer (see lc_crc_chunks.cuh), with scratch
-// (per-chunk registers and a ticket counter) supplied by the caller.
+// (the accumulator and a ticket counter) supplied by the caller.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -9,18 +9,16 @@
 namespace lc {
 
 namespace {
-__global__ void __launch_bounds__(kCrcChunkThreads)
-    k_crc32c_chunks(const uint8_t* data, uint64_t n, uint32_t* partials, uint32_t* counter,
-                    uint32_t* out) {
-  crc32c_chunks_body(data, n, partials, counter, out);
+__global__ void __launch_bounds__(kCrcChunkThreads, 2)
+    k_crc32c_chunks(const uint8_t* data, uint64_t n, uint32_t* scratch, uint32_t* out) {
+  crc32c_chunks_body(data, n, scratch, out);
 }
 }  // namespace
 
-void launch_crc32c_chunks(const uint8_t* data, uint64_t n, uint32_t* partials,
-                          uint32_t* counter, uint32_t* out, cudaStream_t st) {
+void launch_crc32c_chunks(const uint8_t* data, uint64_t n, uint32_t* scratch, uint32_t* out,
+                          cudaStream_t st) {
   note_launch();
-  k_crc32c_chunks<<<crc32c_chunk_count(n), kCrcChunkThreads, 0, st>>>(data, n, partials, counter,
-                                                                        out);
+  k_crc32c_chunks<<<crc32c_chunk_ctas(n), kCrcChunkThreads, 0, st>>>(data, n, scratch, out);
 }
 
 }  // namespace lc

@@ -45,7 +45,7 @@ struct Batch {
   uint32_t B = 0;
   // maxima over the batch, for grid sizes
   uint32_t max_tables = 0, max_gp = 0, max_cap_triggers = 0, max_cap_files = 0;
-  uint64_t max_blocks_in = 0, max_entries = 0;
+  uint64_t max_blocks_in = 0, max_entries = 0, max_cap_wide = 0;
   uint32_t merge_rounds = 0;
   uint32_t max_runs = 1;
   uint32_t chunk = 4096;
@@ -75,9 +75,10 @@ enum ScanSel : int {
 void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_cap, cudaStream_t st);
 uint64_t scan_scratch_elems(uint64_t n_cap);
 
-// lc_crc.cu -- masked CRC32C of one buffer; `counter` must be zero at launch
-void launch_crc32c_chunks(const uint8_t* data, uint64_t n, uint32_t* partials, uint32_t* counter,
-                          uint32_t* out, cudaStream_t st);
+// lc_crc.cu -- masked CRC32C of one buffer; the kCrcScratchWords words of
+// `scratch` must be zero at launch and are zero again when the kernel is done
+void launch_crc32c_chunks(const uint8_t* data, uint64_t n, uint32_t* scratch, uint32_t* out,
+                          cudaStream_t st);
 
 // lc_decode.cu -- input tables -> decoded entries
 void launch_table_index_count(const Batch& bt, cudaStream_t st);

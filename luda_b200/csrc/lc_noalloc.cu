@@ -1,11 +1,9 @@
 // Allocation-free masked CRC32C: lc_crc32c_noalloc (include/luda_b200.h).
 //
-// Same computation as lc_crc32c (chunk registers combined by the last CTA,
-// lc_crc_chunks.cuh), but the scratch lives in a fixed file-scope device
-// array instead of the engine's memory pool, so the call allocates nothing.
-// The array is part of the loaded module: every device that loads this
-// library holds it (kNoAllocCrcMaxChunks + 1 words, about 64 KiB) until the
-// process exits.
+// Same computation as lc_crc32c (lc_crc_chunks.cuh), but the scratch words
+// live in a fixed file-scope device array instead of the engine's memory, so
+// the call allocates nothing.  The array is part of the loaded module: every
+// device that loads this library holds it until the process exits.
 //
 // Host code must not use the array's name as a device address (in host code
 // it is only a stand-in), so the first call on each device looks the address
@@ -25,21 +23,18 @@
 
 namespace {
 
-// Largest buffer: kNoAllocCrcMaxChunks chunks of kCrcChunkBytes = 1 GiB.
-constexpr uint32_t kNoAllocCrcMaxChunks = 16384;
-constexpr uint64_t kNoAllocCrcMaxBytes = (uint64_t)kNoAllocCrcMaxChunks * lc::kCrcChunkBytes;
+constexpr uint64_t kNoAllocCrcMaxBytes = 1ull << 30;  // largest buffer of one call
 constexpr int kMaxDevices = 64;
 
-// [0, kNoAllocCrcMaxChunks): per-chunk CRC registers; [kNoAllocCrcMaxChunks]:
-// the ticket counter, cleared before every launch.
-__device__ __align__(256) uint32_t g_noalloc_crc_scratch[kNoAllocCrcMaxChunks + 1];
+// The accumulator and the ticket counter, cleared before every launch.
+__device__ __align__(256) uint32_t g_noalloc_crc_scratch[lc::kCrcScratchWords];
 
 std::mutex g_setup_mu;
 uint32_t* g_scratch_addr[kMaxDevices] = {};
 
-__global__ void __launch_bounds__(lc::kCrcChunkThreads)
+__global__ void __launch_bounds__(lc::kCrcChunkThreads, 2)
     k_crc32c_chunks_static(const uint8_t* data, uint64_t n, uint32_t* scratch, uint32_t* out) {
-  lc::crc32c_chunks_body(data, n, scratch, scratch + kNoAllocCrcMaxChunks, out);
+  lc::crc32c_chunks_body(data, n, scratch, out);
 }
 
 // Records the failing step (and the CUDA error, if any) as the calling
@@ -61,7 +56,7 @@ lc_status lc_crc32c_noalloc(const uint8_t* d_data, uint64_t n, uint32_t* d_maske
     return noalloc_fail(LC_ERR_INVALID_ARG, "lc_crc32c_noalloc: null device pointer");
   if (n > kNoAllocCrcMaxBytes)
     return noalloc_fail(LC_ERR_UNSUPPORTED,
-                        "lc_crc32c_noalloc: buffer larger than the 1 GiB static scratch limit");
+                        "lc_crc32c_noalloc: buffer larger than the 1 GiB limit of one call");
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return noalloc_fail(LC_ERR_CUDA, "lc_crc32c_noalloc: cudaGetDevice", e);
@@ -81,10 +76,10 @@ lc_status lc_crc32c_noalloc(const uint8_t* d_data, uint64_t n, uint32_t* d_maske
     scratch = g_scratch_addr[dev];
   }
   cudaStream_t st = (cudaStream_t)stream;
-  // the ticket counter must start at zero; the registers are overwritten
-  e = cudaMemsetAsync(scratch + kNoAllocCrcMaxChunks, 0, sizeof(uint32_t), st);
-  if (e != cudaSuccess) return noalloc_fail(LC_ERR_CUDA, "lc_crc32c_noalloc: clear counter", e);
-  k_crc32c_chunks_static<<<lc::crc32c_chunk_count(n), lc::kCrcChunkThreads, 0, st>>>(
+  // both words must start at zero (an overlapping call may have left them set)
+  e = cudaMemsetAsync(scratch, 0, lc::kCrcScratchWords * sizeof(uint32_t), st);
+  if (e != cudaSuccess) return noalloc_fail(LC_ERR_CUDA, "lc_crc32c_noalloc: clear scratch", e);
+  k_crc32c_chunks_static<<<lc::crc32c_chunk_ctas(n), lc::kCrcChunkThreads, 0, st>>>(
       d_data, n, scratch, d_masked_crc);
   e = cudaGetLastError();
   if (e != cudaSuccess) return noalloc_fail(LC_ERR_CUDA, "lc_crc32c_noalloc: launch", e);
