@@ -20,7 +20,8 @@
 // in flight while the four before them are looked up.  64 MiB in device
 // memory on B200: the bytewise form this replaces took 290 us (0.23 TB/s, one
 // 256-byte run per thread, uncoalesced byte loads); warps with runs of their
-// own 42 us (seven serial products per warp at the end); this form @@ us.
+// own 42 us (seven serial products per warp at the end); this form
+// 32 us (2.1 TB/s).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

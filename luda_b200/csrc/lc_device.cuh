@@ -199,24 +199,6 @@ struct FastMod {
 // ---------------------------------------------------------------------------
 // CRC32C
 
-// Fills a 256-entry byte table in shared memory (call with all threads, then
-// __syncthreads()).
-__device__ __forceinline__ void crc_table_init(uint32_t* tab) {
-  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
-    uint32_t c = i;
-#pragma unroll
-    for (int k = 0; k < 8; k++) c = (c & 1) ? (c >> 1) ^ kCrcPoly : (c >> 1);
-    tab[i] = c;
-  }
-}
-
-// Raw CRC register update (no inversion) over n bytes.
-__device__ __forceinline__ uint32_t crc_raw(const uint32_t* tab, uint32_t c, const uint8_t* p,
-                                            uint32_t n) {
-  for (uint32_t i = 0; i < n; i++) c = tab[(c ^ p[i]) & 0xff] ^ (c >> 8);
-  return c;
-}
-
 // a * b mod P with the byte table tab (tab[i] = register after byte i from
 // 0, that is i * x^32 mod P): a's four bytes by Horner, the byte groups of
 // b x^j (j < 8) by their bits, and each step of x^8 as one zero byte fed to
@@ -284,33 +266,6 @@ __device__ __forceinline__ uint32_t crc_shift_tab(const JobDev& J, const uint32_
   uint32_t m = __ldg(J.crc_xpow + lo);
   if (hi) m = gf2_mulmod_tab(tab, m, __ldg(J.crc_xpow_hi + hi));
   return gf2_mulmod_tab(tab, c, m);
-}
-
-// Masked CRC32C of contents followed by the type byte: the block trailer of
-// table/table_builder.cc:186-189, computed cooperatively by one warp over `n`
-// bytes at `p` (the type byte, 0 for an uncompressed block, is appended
-// implicitly).
-__device__ __forceinline__ uint32_t warp_block_crc(const JobDev& J, const uint32_t* tab,
-                                                   const uint8_t* p, uint32_t n,
-                                                   uint8_t type = 0) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t total = n + 1;  // contents + type byte
-  uint32_t seg = (total + 31) / 32;
-  uint32_t b = lane * seg;
-  uint32_t e = min(total, b + seg);
-  uint32_t c = 0;
-  for (uint32_t i = b; i < e; i++) {
-    uint8_t byte = i < n ? p[i] : type;
-    c = tab[(c ^ byte) & 0xff] ^ (c >> 8);
-  }
-  // shift each lane's raw CRC by the bytes after its segment, xor together
-  uint32_t after = total > e ? total - e : 0;
-  uint32_t v = (b < total) ? crc_shift(J, c, after) : 0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v ^= __shfl_xor_sync(0xffffffffu, v, o);
-  // init 0xffffffff contributes shift(~0, total); final inversion
-  uint32_t full = v ^ crc_shift(J, 0xffffffffu, total) ^ 0xffffffffu;
-  return ((full >> 15) | (full << 17)) + 0xa282ead8u;  // crc32c::Mask
 }
 
 // Up to kMax (a multiple of 4, at most 32) bytes from src (any alignment) to
@@ -407,45 +362,36 @@ __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) 
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
 }
+// *p |= v, p in shared memory (word aligned), without the old value.
+__device__ __forceinline__ void smem_or(void* p, uint32_t v) {
+  asm volatile("red.shared.or.b32 [%0], %1;\n" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v)
+               : "memory");
+}
+
+// One bulk copy (TMA, untiled) from shared to global memory: both addresses
+// 16-byte aligned, n a multiple of 16.  The issuing thread waits for its
+// copies' reads of shared memory with bulk_wait_read; the writers of the
+// source bytes fence (fence_proxy_async_smem) and synchronise before it.
+__device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uint32_t n) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem_src);
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n"
+               "cp.async.bulk.commit_group;\n" ::"l"(gdst), "r"(s), "r"(n) : "memory");
+}
+// The lines of [p, p + n) into L2 with one instruction (the 16-byte pieces
+// that hold them).
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t n) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p), q = a & ~uintptr_t(15);
+  const uint32_t m = (uint32_t)(a + n - q + 15) & ~15u;
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(q), "r"(m) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+}
+__device__ __forceinline__ void fence_proxy_async_smem() {
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
-// Slicing-by-4 CRC32C tables in shared memory: tab4[k][x] is the register
-// update for byte x followed by k zero bytes (tab4[0] is the byte table).
-__device__ __forceinline__ void crc_tables4_init(uint32_t* tab4) {
-  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
-    uint32_t c = i;
-#pragma unroll
-    for (int k = 0; k < 8; k++) c = (c & 1) ? (c >> 1) ^ kCrcPoly : (c >> 1);
-    tab4[i] = c;
-  }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
-    uint32_t c = tab4[i];
-    for (int k = 1; k < 4; k++) {
-      c = (c >> 8) ^ tab4[c & 0xff];
-      tab4[256 * k + i] = c;
-    }
-  }
-}
-
-// Raw CRC register update over [p, p+n) in shared memory, four bytes per
-// step once p is word aligned.
-__device__ __forceinline__ uint32_t crc_raw4(const uint32_t* tab4, uint32_t c, const uint8_t* p,
-                                             uint32_t n) {
-  uint32_t i = 0;
-  while (i < n && (reinterpret_cast<uintptr_t>(p + i) & 3)) {
-    c = tab4[(c ^ p[i]) & 0xff] ^ (c >> 8);
-    i++;
-  }
-  for (; i + 4 <= n; i += 4) {
-    c ^= *reinterpret_cast<const uint32_t*>(p + i);
-    c = tab4[768 + (c & 0xff)] ^ tab4[512 + ((c >> 8) & 0xff)] ^ tab4[256 + ((c >> 16) & 0xff)] ^
-        tab4[c >> 24];
-  }
-  for (; i < n; i++) c = tab4[(c ^ p[i]) & 0xff] ^ (c >> 8);
-  return c;
 }
 
 // ---------------------------------------------------------------------------
@@ -494,6 +440,50 @@ __device__ __forceinline__ uint32_t crc_h5(const uint32_t* __restrict__ h5, uint
     r ^= *reinterpret_cast<const uint32_t*>(t + 4 * kCrcFieldEntries * i + f4);
   }
   return r;
+}
+
+// ---------------------------------------------------------------------------
+// CRC32C of consecutive words by folding.  x^209 = x^144 + x^54 + x^39 + x^14
+// + 1 mod P (found by a search over the 6-term multiples of P: the one of
+// least degree whose two highest terms lie 32 or more apart), so a message bit
+// may be moved 65, 155, 170, 195 and 209 bits towards the message's end
+// instead of being divided: word t of the message takes those shifts of the
+// words 2 to 7 before it, which no longer count.  (The scheme of sparse
+// multiples of the generator polynomial, as in Russell, "Chorba: a novel CRC32
+// implementation", 2024, with a multiple of CRC32C's polynomial.)
+//
+// What word t = 8k + i (v: ring of the last eight folded words, word t at t %
+// 8) receives from the words before it; kLast: words 8k.. are the message's
+// last eight, which are not folded further, so only words before 8k count.
+template <bool kLast>
+__device__ __forceinline__ uint32_t crc_fold_word(const uint32_t (&v)[8], uint32_t i) {
+  const auto at = [&](uint32_t back) -> uint32_t {  // word t - back
+    return kLast && back <= i ? 0u : v[(i - back) & 7];
+  };
+  return __funnelshift_l(at(3), at(2), 1) ^ __funnelshift_l(at(5), at(4), 27) ^
+         __funnelshift_l(at(6), at(5), 10) ^ __funnelshift_l(at(7), at(6), 3) ^
+         __funnelshift_l(at(7), at(6), 17);
+}
+
+// The raw register (from zero) after the 32 bytes r: one lookup per 5-bit
+// field, conflict-free as in crc_h5.
+constexpr uint32_t kCrcH8Fields = (256 + kCrcFieldBits - 1) / kCrcFieldBits;
+constexpr uint32_t kCrcH8Words = kCrcH8Fields * kCrcFieldEntries;
+__device__ __forceinline__ uint32_t crc_h8(const uint32_t* __restrict__ h8, const uint32_t (&r)[8]) {
+  constexpr uint32_t mask = (kCrcFieldEntries - 1) << 2;
+  const uint8_t* t = reinterpret_cast<const uint8_t*>(h8);
+  uint32_t u = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < kCrcH8Fields; i++) {
+    const uint32_t s = kCrcFieldBits * i, q = s >> 5, o = s & 31;
+    uint32_t f4;
+    if (o + kCrcFieldBits <= 32 || q == 7)
+      f4 = (o >= 2 ? (r[q] >> (o - 2)) : (r[q] << (2 - o))) & mask;
+    else
+      f4 = __funnelshift_r(r[q], r[q + 1], o - 2) & mask;
+    u ^= *reinterpret_cast<const uint32_t*>(t + 4 * kCrcFieldEntries * i + f4);
+  }
+  return u;
 }
 
 // The bytes of word x at grid position pos that belong to the message
@@ -549,25 +539,6 @@ __device__ __forceinline__ uint32_t crc_rows_finish(const uint32_t* __restrict__
                                                     uint32_t last, uint32_t m1) {
   const uint32_t full = crc_rows_raw(xinv, tab8, u, last, m1) ^ 0xffffffffu;
   return ((full >> 15) | (full << 17)) + 0xa282ead8u;  // crc32c::Mask
-}
-
-// Masked block trailer CRC of the block [p, p + n) plus the zero type byte at
-// p[n], read from memory in 16-byte chunks by one warp (p - (p & 15) is the
-// grid origin; bytes of the chunks outside the block are read and ignored).
-__device__ __forceinline__ uint32_t warp_block_crc_rows(const uint32_t* __restrict__ h5,
-                                                        const uint32_t* __restrict__ xinv,
-                                                        const uint32_t* __restrict__ tab8,
-                                                        const uint8_t* p, uint32_t n) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t m0 = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 15), m1 = m0 + n + 1;
-  const uint8_t* g = p - m0;
-  uint32_t u = 0, last = 0xffffffffu;
-  for (uint32_t q = 16 * lane; q < m1; q += kCrcRowBytes) {
-    const uint4 x = __ldcg(reinterpret_cast<const uint4*>(g + q));  // the warp's own stores, via L2
-    u = crc_chunk_step(h5, u, q, m0, m1, x.x, x.y, x.z, x.w);
-    last = q;
-  }
-  return crc_rows_finish(xinv, tab8, u, last, m1);
 }
 
 }  // namespace lc

@@ -40,6 +40,10 @@ namespace lc {
 namespace {
 
 constexpr uint32_t kNoSep = 0xffffffffu;
+constexpr uint32_t kEncWarps = 16;
+constexpr uint32_t kEncAhead = 32;  // entries of the next block copied ahead
+constexpr uint32_t kEncLong = 33;   // values at least this long: by lane groups
+
 __constant__ char kFilterName[] = "filter.leveldb.BuiltinBloomFilter2";
 constexpr uint32_t kFilterNameLen = 34;
 
@@ -551,6 +555,13 @@ __device__ void block_layout_one(const JobDev& J, uint64_t b) {
   const uint64_t off = J.b_cum[b] - base;
   J.b_file[b] = f;
   J.b_off[b] = off;
+  if (J.b_size[b] > kEncNarrow) {  // windows for the longest 16-byte phase
+    const uint32_t n = (15 + J.b_size[b] + 1 + kEncWindow - 1) / kEncWindow;
+    const uint32_t at = atomicAdd(&J.ctr->n_wide, n);
+    // (past the capacity: the files outgrow the output, an error of the file layout)
+    for (uint32_t i = 0; i < n && at + i < J.cap_wide; i++) J.wide[at + i] = make_uint2((uint32_t)b, i);
+    J.b_crc[b] = 0;
+  }
   // filter group: blocks of this file whose start offsets share off >> 11
   uint32_t gbytes = 0, gkeys = 0;
   if (J.bits_per_key > 0) {
@@ -650,233 +661,88 @@ __global__ void k_file_layout(const JobDev* __restrict__ jobs) {
   }
 }
 
-// One warp per output data block, assembled around the warp's shared-memory
-// stage, which has the block's own 16-byte phase in global memory: stage
-// position p is global byte dst - ph + p, ph = dst & 15.  Three steps:
-//  1. Entries in rounds of 32, one lane per entry: entry sizes and output
-//     offsets by a warp scan.  A key delta or value of at least kEncLong
-//     bytes lists its whole 16-byte chunks in the warp's list of long
-//     stretches (at most kEncMaxLong; a lane stages the chunks of a stretch
-//     past the list itself).  Once the list is complete (the last round), the
-//     listed chunks of the first two chunk rows are loaded, and while they
-//     are in flight the lanes write entry headers, restart words, short
-//     stretches whole and the unaligned heads and tails of long ones to the
-//     stage.
-//  2. The block's 16-byte chunks, lane l taking chunks l, l + 32, ..., each
-//     loaded two chunks ahead of its use: a chunk inside a listed stretch is
-//     read from global memory (five 4-byte loads and four funnel shifts at
-//     any source alignment), any other from the stage.  A chunk wholly
-//     inside the block and its type byte goes out with one 16-byte store,
-//     and every chunk feeds the lane's share of the block CRC (crc_h5).  The
-//     stage's first and last chunks are cleared before step 1, so the grid
-//     bytes outside the message are zero and every chunk takes the same CRC
-//     step; the initial all-ones register enters at the end, as its register
-//     carried over the message's length (crc_ones).
-//  3. The lanes' CRC shares combined, the trailer (type byte and CRC) into
-//     the stage, and the partial chunks at both ends from the stage with byte
-//     stores.
-// A block that does not fit the stage takes the direct path.
-constexpr uint32_t kEncWarps = 8;
-constexpr uint32_t kEncStage = 6144;  // block + 5-byte trailer + 16-byte phase + read slack
-constexpr uint32_t kEncLong = 33;     // stretches at least this long are read by chunks
-constexpr uint32_t kEncMaxLong = 64;  // listed long stretches per block
-constexpr uint32_t kEncFromInput = 0x80000000u;
+// Data blocks, assembled in shared memory: one warp per block of at most
+// kEncNarrow bytes, and one per window of kEncWindow bytes of a wider block
+// (k_block_layout lists those).  The warp's stage has the block's own 16-byte
+// phase in global memory: stage position p is global byte dst - ph + p0 + p,
+// ph = dst & 15, p0 the window's first grid position (0 for a narrow block).
+//  1. The stage is cleared, then the entries are taken in rounds of 32, one
+//     lane per entry: sizes and places by a warp scan, entry headers and
+//     restart words with byte stores, key deltas and short values (up to 32
+//     bytes) lane by lane in words, longer values by groups of 8 or 32 lanes
+//     in words (coalesced loads; source and destination alignments differ, so
+//     every word is two source words and a funnel shift).  A word shared with
+//     a neighbouring piece is ored into the cleared stage, all others are
+//     stored, so no byte is stored twice and nothing is written bytewise but
+//     headers.
+//  2. The whole 16-byte chunks go out with one bulk copy from shared memory,
+//     and meanwhile every lane feeds its chunks (l, l + 32, ...) to the row
+//     CRC (crc_h5).  The grid bytes outside the message are zero, so every
+//     chunk takes the same step; the initial all-ones register enters at the
+//     end, as its register carried over the message's length (crc_ones).
+//  3. The lanes' registers combined, the trailer, and the partial chunks at
+//     both ends with byte stores.  A window's register is moved over the
+//     bytes after it and xored into its block's (k_meta_trailers finishes
+//     wide blocks).
+//
+// Bound by its serial chain per block (about 2000 instructions and six waits
+// on memory) at the warps an SM holds: 32 of them (64 registers, 5.8 KB of
+// shared memory each) where 24 warps with a 6 KB stage took a third longer.
+// Measured on B200, one launch: 1 GiB of 1 KiB values 866 -> 623 us, 480 MiB of
+// 32-byte values 712 -> 447 us, 66 MiB of lognormal values 224 -> 98 us (before:
+// values as 16-byte chunks straight from global to global memory through the
+// row CRC, short pieces bytewise into the stage); 200 MiB in 16 KiB blocks 2753
+// -> 282 us and 240 MiB of 4-64 KiB values 6759 -> 229 us (before: a lane per
+// entry, byte by byte, for any block beyond the stage).
 struct EncWarp {
-  uint32_t ls_c0[kEncMaxLong];   // first whole chunk (stage grid) | kEncFromInput
-  uint32_t ls_n[kEncMaxLong];    // whole chunks
-  uint32_t ls_src[kEncMaxLong];  // source offset of the first chunk (key arena or input)
-  uint32_t ahead[5][32];         // next block: lane j's entry (key length, shared, value
-                                 // length, key offset, value offset), copied ahead
+  uint32_t ahead[5][kEncAhead];  // next block's entries: key length, shared, value length, key
+                                 // offset, value offset
   __align__(16) uint8_t stage[kEncStage];
 };
+static_assert(kEncAhead % 32 == 0, "whole rounds of entries are copied ahead");
 constexpr size_t kEncSmem = (size_t)kEncWarps * sizeof(EncWarp);
 
-// 16 bytes from src at any alignment: the five words holding them (the fifth
-// only when src is not word aligned) and four funnel shifts.
-__device__ __forceinline__ void load16(const uint8_t* src, uint32_t (&w)[4]) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-  const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
-  const uint32_t sh = 8 * (uint32_t)(a & 3);
-  uint32_t x[5];
+// Up to 4 kW bytes (len >= 1) from src (any alignment) to the cleared stage
+// at p (any alignment), by one lane: all loads first; whole words stored,
+// words shared with neighbours ored.  Only source words that hold a needed
+// byte are loaded.
+template <uint32_t kW>
+__device__ __forceinline__ void enc_piece(uint8_t* p, const uint8_t* src, uint32_t len) {
+  const uint32_t da = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
+  const uintptr_t s = reinterpret_cast<uintptr_t>(src), s0 = s - da;  // stage word q: source s0 + 4q
+  const uintptr_t b0 = s0 & ~uintptr_t(3);
+  const uint32_t sh = 8 * (uint32_t)(s0 & 3);
+  const uint32_t first = (uint32_t)(s - b0), end = first + len;  // needed bytes from b0
+  const uint32_t* base = reinterpret_cast<const uint32_t*>(b0);
+  uint32_t w[kW + 2];
 #pragma unroll
-  for (int i = 0; i < 4; i++) x[i] = __ldg(q + i);
-  x[4] = sh ? __ldg(q + 4) : 0u;
+  for (uint32_t i = 0; i < kW + 2; i++)
+    w[i] = (4 * i + 4 > first && 4 * i < end) ? __ldg(base + i) : 0u;
+  uint32_t* dw = reinterpret_cast<uint32_t*>(p - da);
+  const uint32_t dend = da + len;
 #pragma unroll
-  for (int i = 0; i < 4; i++) w[i] = __funnelshift_r(x[i], x[i + 1], sh);
-}
-
-// The direct path: entries written straight to global memory, one lane per
-// entry, then the CRC read back from there.
-__device__ __forceinline__ void enc_direct(const JobDev& J, const uint32_t* h5,
-                                           const uint32_t* xinv, const uint32_t* tab8, uint64_t b,
-                                           uint8_t* dst, uint32_t lane) {
-  const uint64_t s = J.b_first[b], n = J.b_first[b + 1] - s;
-  const uint32_t R = J.restart_interval;
-  const uint32_t bsz = J.b_size[b];
-  const uint64_t nrest = (n + R - 1) / R;
-  uint8_t* ra = dst + bsz - 4 * nrest - 4;
-  uint64_t carry = 0;
-  for (uint64_t j0 = 0; j0 < n; j0 += 32) {
-    const uint64_t j = j0 + lane;
-    const bool valid = j < n;
-    const bool restart = (j % R) == 0;
-    const uint64_t k = s + j;
-    const uint64_t size = valid ? (restart ? J.k_a[k] : J.k_b[k]) : 0;
-    uint64_t tot;
-    const uint64_t ex = warp_excl<uint64_t>(size, &tot) + carry;
-    carry += tot;
-    if (valid) {
-      const uint32_t kl = J.k_klen[k], vl = J.k_vlen[k];
-      const uint8_t* key = J.keys + J.k_koff[k];
-      const uint8_t* val = J.in + J.k_voff[k];
-      const uint32_t sh = restart ? 0 : J.k_shared[k];
-      uint8_t* p = dst + ex;
-      p = put_varint(p, sh);
-      p = put_varint(p, kl - sh);
-      p = put_varint(p, vl);
-      if (J.dec_vpos)  // the value's place in its file, for the decoded form
-        J.dec_vpos[k] = (uint32_t)(J.b_off[b] + (uint64_t)(p - dst) + (kl - sh));
-      for (uint32_t i = sh; i < kl; i++) *p++ = key[i];
-      for (uint32_t i = 0; i < vl; i++) *p++ = val[i];
-      if (restart) {
-        const uint64_t rem = n - j;
-        const uint32_t cnt = (uint32_t)(rem < R ? rem : R);
-        st_le32(ra + 4 * (j / R), ((uint32_t)ex << 8) | cnt);
-      }
-    }
-  }
-  if (lane == 0) {
-    st_le32(dst + bsz - 4, (uint32_t)nrest);
-    dst[bsz] = 0;
-  }
-  __syncwarp();
-  const uint32_t crc = warp_block_crc_rows(h5, xinv, tab8, dst, bsz);
-  if (lane == 0) st_le32(dst + bsz + 1, crc);
-}
-
-// A key delta or value of `len` bytes at stage position pos, from base +
-// off.  A stretch shorter than kEncLong is staged whole; a longer one lists
-// its whole 16-byte chunks in slot li while the list has room, and stages only
-// its unaligned head and tail.  enc_list records the slot (li advances past
-// every long stretch); enc_stage writes the staged bytes, and the chunks of a
-// long stretch that found the list full.
-__device__ __forceinline__ void enc_list(EncWarp& W, uint32_t pos, uint32_t len, uint32_t off,
-                                         uint32_t from, uint32_t& li) {
-  if (len < kEncLong) return;
-  if (li < kEncMaxLong) {
-    const uint32_t first = (pos + 15) & ~15u, last = (pos + len) & ~15u;
-    W.ls_c0[li] = (first >> 4) | from;
-    W.ls_n[li] = (last - first) >> 4;
-    W.ls_src[li] = off + (first - pos);
-  }
-  li++;
-}
-
-__device__ __forceinline__ void enc_stage(uint8_t* st, uint32_t pos, uint32_t len,
-                                          const uint8_t* src, bool listed) {
-  if (len < kEncLong) {
-    // the 16-byte form when every lane here has at most 16 bytes (a lane
-    // that takes the 32-byte form is right for any length below kEncLong)
-    if (__all_sync(__activemask(), len <= 16))
-      copy_small<16>(st + pos, src, len);
-    else
-      copy_small<32>(st + pos, src, len);
-    return;
-  }
-  const uint32_t first = (pos + 15) & ~15u, last = (pos + len) & ~15u;
-  copy_small<16>(st + pos, src, first - pos);
-  copy_small<16>(st + last, src + (last - pos), pos + len - last);
-  if (!listed) {
-    const uint32_t nq = (last - first) >> 4;
-    for (uint32_t q = 0; q < nq; q++) {
-      uint32_t w[4];
-      load16(src + (first - pos) + 16 * q, w);
-      *reinterpret_cast<uint4*>(st + first + 16 * q) = make_uint4(w[0], w[1], w[2], w[3]);
+  for (uint32_t q = 0; q < kW + 1; q++) {
+    if (4 * q >= dend) break;
+    uint32_t v = __funnelshift_r(w[q], w[q + 1], sh);
+    if (4 * q >= da && 4 * q + 4 <= dend) {
+      dw[q] = v;
+    } else {
+      if (q == 0) v &= 0xffffffffu << (8 * da);
+      if (4 * q + 4 > dend) v &= 0xffffffffu >> (8 * (4 * q + 4 - dend));
+      smem_or(dw + q, v);
     }
   }
 }
 
-// A chunk slot: the five words holding a chunk's 16 bytes as loaded, and
-// the right shift (bits) that aligns them.  Loads fill the slot; the shift is
-// applied only where the chunk is used, so a slot loaded ahead does not hold
-// up the warp until then.
-struct EncSlot {
-  uint32_t x[5];
-  uint32_t sh;
-};
-
-__device__ __forceinline__ void enc_slot_load(const uint8_t* src, EncSlot& s) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(src);
-  const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
-  s.sh = 8 * (uint32_t)(a & 3);
-#pragma unroll
-  for (int i = 0; i < 4; i++) s.x[i] = __ldg(q + i);
-  s.x[4] = s.sh ? __ldg(q + 4) : 0u;
-}
-
-// Chunk c of the stage grid from its source when it lies in listed stretch
-// *k (k advances along the list); false when it is a stage chunk.
-__device__ __forceinline__ bool enc_fetch_listed(const JobDev& J, const EncWarp& W, uint32_t nls,
-                                                 uint32_t c, uint32_t& k, EncSlot& s) {
-  while (k < nls && c >= (W.ls_c0[k] & ~kEncFromInput) + W.ls_n[k]) k++;
-  const uint32_t c0 = k < nls ? W.ls_c0[k] : 0xffffffffu;
-  if (c0 != 0xffffffffu && c >= (c0 & ~kEncFromInput)) {
-    const uint8_t* base = (c0 & kEncFromInput) ? J.in : J.keys;
-    enc_slot_load(base + W.ls_src[k] + 16 * (c - (c0 & ~kEncFromInput)), s);
-    return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void enc_fetch_stage(const uint8_t* st, uint32_t c, EncSlot& s) {
-  const uint4 v = *reinterpret_cast<const uint4*>(st + 16 * c);
-  s.x[0] = v.x, s.x[1] = v.y, s.x[2] = v.z, s.x[3] = v.w, s.x[4] = 0u;
-  s.sh = 0u;
-}
-
-__device__ __forceinline__ void enc_fetch(const JobDev& J, const EncWarp& W, const uint8_t* st,
-                                          uint32_t nls, uint32_t c, uint32_t& k, EncSlot& s) {
-  if (!enc_fetch_listed(J, W, nls, c, k, s)) enc_fetch_stage(st, c, s);
-}
-
-// Chunk at stage position p out to global memory when it lies wholly inside
-// the message [m0, m1) (block and type byte), and into the lane's CRC share.
-// The grid bytes outside the message are zero in every chunk (the stage's
-// edges are cleared), so every chunk takes the same step; the CRC's initial
-// register is added at the end.
-__device__ __forceinline__ void enc_chunk_out(const uint32_t* h5, uint8_t* gbase, uint32_t p,
-                                              uint32_t m0, uint32_t m1, const EncSlot& s,
-                                              uint32_t& u, uint32_t& last) {
-  uint32_t w[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) w[i] = __funnelshift_r(s.x[i], s.x[i + 1], s.sh);
-  if (p >= m0 && p + 16 <= m1)
-    *reinterpret_cast<uint4*>(gbase + p) = make_uint4(w[0], w[1], w[2], w[3]);
-  u = crc_h5(h5, w[0] ^ u, w[1], w[2], w[3]);
-  last = p;
-}
-
-// A block's place and entry range, loaded one block ahead; lane j's entry of
-// its first 32 is copied to the warp's `ahead` area (cp.async, no registers
-// held) while the current block is encoded, so that the next block's first
-// steps do not wait on two rounds of dependent loads.
-struct EncAhead {
-  uint8_t* dst;
-  uint32_t bsz, n;
-  uint32_t s;
-};
-
-__device__ __forceinline__ void enc_ahead_entries(const JobDev& J, EncWarp& W, const EncAhead& A,
-                                                  uint32_t lane) {
-  cp_async_wait_all();  // no copy into the area is still in flight
-  if (lane < A.n) {
-    const uint32_t k = A.s + lane;
-    cp_async4(&W.ahead[0][lane], J.k_klen + k);
-    cp_async4(&W.ahead[1][lane], J.k_shared + k);
-    cp_async4(&W.ahead[2][lane], J.k_vlen + k);
-    cp_async4(&W.ahead[3][lane], J.k_koff + k);
-    cp_async4(&W.ahead[4][lane], J.k_voff + k);
-  }
+// The word at src (any alignment); bytes at or past end are zero.
+__device__ __forceinline__ uint32_t enc_word(const uint8_t* src, const uint8_t* end) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(src), q = a & ~uintptr_t(3);
+  const uint32_t lo = __ldg(reinterpret_cast<const uint32_t*>(q));
+  const uint32_t hi = ((a & 3) && q + 4 < reinterpret_cast<uintptr_t>(end))
+                          ? __ldg(reinterpret_cast<const uint32_t*>(q + 4)) : 0u;
+  const uint32_t v = __funnelshift_r(lo, hi, 8 * (uint32_t)(a & 3));
+  const uint32_t n = (uint32_t)(end - src);
+  return n >= 4 ? v : v & ((1u << (8 * n)) - 1u);
 }
 
 // x / R for the restart interval R: a shift when R is a power of two (the
@@ -897,18 +763,342 @@ struct RestartDiv {
       q = x / R;
     return q;
   }
-  __device__ __forceinline__ bool starts_run(uint32_t x) const { return x - div(x) * R == 0u; }
 };
 
-__global__ void __launch_bounds__(kEncWarps * 32, 3) k_encode_blocks(const JobDev* __restrict__ jobs) {
-  __shared__ uint32_t s_h5[kCrcH5Words];
+// A block's place and entry range, loaded one block ahead.
+struct EncBlock {
+  uint8_t* dst;
+  uint32_t bsz, n, s;
+  uint32_t off;  // in its file
+};
+
+// The block's first kEncAhead entries into the warp's `ahead` area, by cp.async
+// (no registers held) while the block before it is still encoded; then
+// enc_prefetch brings the lines that their keys and values lie in into L2.
+__device__ __forceinline__ void enc_ahead_entries(const JobDev& J, EncWarp& W, const EncBlock& A,
+                                                  uint32_t lane) {
+#pragma unroll
+  for (uint32_t j = lane; j < kEncAhead; j += 32) {
+    if (j < A.n) {
+      const uint32_t k = A.s + j;
+      cp_async4(&W.ahead[0][j], J.k_klen + k);
+      cp_async4(&W.ahead[1][j], J.k_shared + k);
+      cp_async4(&W.ahead[2][j], J.k_vlen + k);
+      cp_async4(&W.ahead[3][j], J.k_koff + k);
+      cp_async4(&W.ahead[4][j], J.k_voff + k);
+    }
+  }
+}
+__device__ __forceinline__ void enc_prefetch(const JobDev& J, const EncWarp& W, uint32_t n,
+                                             uint32_t lane) {
+  for (uint32_t j = lane; j < min(n, kEncAhead); j += 32) {
+    const uint32_t kl = W.ahead[0][j], vl = W.ahead[2][j];
+    const uint32_t ko = W.ahead[3][j], vo = W.ahead[4][j];
+    prefetch_l2(J.keys + ko);
+    prefetch_l2(J.keys + ko + kl - 1);
+    if (vl >= 256) {
+      bulk_prefetch_l2(J.in + vo, vl);
+    } else if (vl) {
+      prefetch_l2(J.in + vo);
+      prefetch_l2(J.in + vo + vl - 1);
+    }
+  }
+}
+
+// Where in its block (bytes from the block's start) the round of 32 entries
+// that holds block byte `at` starts, and that round: the prefix sums k_pb
+// give an entry's place but for the restarts before it, whose extra bytes are
+// summed here, a lane per round.
+__device__ __forceinline__ void enc_seek(const JobDev& J, const EncBlock& B, uint32_t R, uint32_t at,
+                                         uint32_t lane, uint32_t* j0, uint32_t* pos) {
+  const uint64_t pb0 = J.k_pb[B.s];
+  uint32_t extra0 = 0;  // extra bytes of the restarts before the group of 32 rounds
+  *j0 = 0, *pos = 0;
+  for (uint32_t g = 0; g < B.n; g += 1024) {
+    const uint32_t a = g + 32 * lane, z = min(a + 32, B.n);  // the lane's round
+    uint32_t x = 0;
+    for (uint32_t j = (a + R - 1) / R * R; j < z; j += R) x += J.k_a[B.s + j] - J.k_b[B.s + j];
+    uint32_t tot;
+    const uint32_t before = warp_excl<uint32_t>(x, &tot) + extra0;
+    extra0 += tot;
+    const uint32_t p = a < B.n ? (uint32_t)(J.k_pb[B.s + a] - pb0) + before : 0xffffffffu;
+    const unsigned m = __ballot_sync(0xffffffffu, p <= at);
+    if (!m) return;  // the group starts past `at`: the last round of the one before
+    const int l = 31 - __clz(m);
+    *j0 = g + 32 * l;
+    *pos = __shfl_sync(0xffffffffu, p, l);
+    if (l < 31) return;
+  }
+}
+
+// Grid positions [p0, p1) of the block into the warp's stage (kWide: a
+// window; else the whole block, p0 = 0).
+template <bool kWide>
+__device__ __forceinline__ void enc_assemble(const JobDev& J, EncWarp& W, const EncBlock& B,
+                                             const RestartDiv& rd, uint32_t ph, uint32_t p0,
+                                             uint32_t p1, uint32_t lane) {
+  uint8_t* st = W.stage;
+  const uint32_t n = B.n, R = rd.R;
+  const uint32_t nrest = rd.div(n + R - 1);
+  const uint32_t rbase = ph + B.bsz - 4 * nrest - 4;  // grid position of the restart array
+  for (uint32_t q = 16 * lane; q < p1 - p0; q += 512)
+    *reinterpret_cast<uint4*>(st + q) = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  uint32_t carry = 0, j0 = 0;
+  if (kWide) {
+    if (p1 > rbase) {  // the window's restart words, a lane per run
+      const uint64_t pb0 = J.k_pb[B.s];
+      uint32_t extra = 0;
+      for (uint32_t r0 = 0; r0 < nrest; r0 += 32) {
+        const uint32_t r = r0 + lane, k = B.s + r * R;
+        const bool on = r < nrest;
+        uint32_t tot;
+        const uint32_t before = warp_excl<uint32_t>(on ? J.k_a[k] - J.k_b[k] : 0u, &tot) + extra;
+        extra += tot;
+        if (on) {
+          const uint32_t ex = (uint32_t)(J.k_pb[k] - pb0) + before;
+          const uint32_t word = (ex << 8) | min(n - r * R, R), rp = rbase + 4 * r - p0;
+#pragma unroll
+          for (uint32_t i = 0; i < 4; i++)
+            if (rp + i < p1 - p0) st[rp + i] = (uint8_t)(word >> (8 * i));
+        }
+      }
+    }
+    if (p0 && n > 32) enc_seek(J, B, R, p0 - ph, lane, &j0, &carry);
+  }
+  for (; j0 < n; j0 += 32) {
+    if (kWide && ph + carry >= p1) break;
+    const uint32_t j = j0 + lane, k = B.s + j;
+    const bool valid = j < n;
+    uint32_t kd = 0, vl = 0, sh = 0, koff = 0, voff = 0, hl = 0, run = 0;
+    bool restart = false;
+    if (valid) {
+      uint32_t kl;
+      if (!kWide && j0 < kEncAhead) {
+        kl = W.ahead[0][j], sh = W.ahead[1][j], vl = W.ahead[2][j];
+        koff = W.ahead[3][j], voff = W.ahead[4][j];
+      } else {
+        kl = J.k_klen[k], sh = J.k_shared[k], vl = J.k_vlen[k];
+        koff = J.k_koff[k], voff = J.k_voff[k];
+      }
+      run = rd.div(j);
+      restart = run * R == j;
+      if (restart) sh = 0;
+      kd = kl - sh;
+      hl = varint_len32(sh) + varint_len32(kd) + varint_len32(vl);
+    }
+    uint32_t tot;
+    const uint32_t ex = warp_excl<uint32_t>(hl + kd + vl, &tot) + carry;
+    const uint32_t hpos = ph + ex;
+    const bool outside = kWide && (ph + carry + tot <= p0 || ph + carry >= p1);
+    carry += tot;
+    uint32_t kpos = hpos + hl, vpos = kpos + kd;
+    if (valid) {
+      // restart word and header bytes
+      if (!kWide && restart) st_le32(st + rbase + 4 * run, (ex << 8) | min(n - j, R));
+      if (!outside) {
+        uint32_t q = hpos - p0;
+        const auto put = [&](uint32_t v) {
+          while (v >= 128) {
+            if (!kWide || q < p1 - p0) st[q] = (uint8_t)(v | 128);
+            q++;
+            v >>= 7;
+          }
+          if (!kWide || q < p1 - p0) st[q] = (uint8_t)v;
+          q++;
+        };
+        put(sh);
+        put(kd);
+        put(vl);
+        // the value's place in its file, for the decoded form
+        if (J.dec_vpos && (!kWide || (hpos >= p0 && hpos < p1)))
+          J.dec_vpos[k] = B.off + ex + hl + kd;
+      }
+    }
+    if (outside) continue;
+    const uint8_t* key = J.keys + (koff + sh);
+    const uint8_t* val = J.in + voff;
+    if (kWide) {  // the pieces' parts inside the window
+      const uint32_t ka = min(max(kpos, p0), p1), kz = min(max(vpos, p0), p1);
+      const uint32_t ve = min(max(vpos + vl, p0), p1);
+      key += ka - kpos, val += kz > vpos ? kz - vpos : 0;
+      const uint32_t va = kz;
+      kd = kz - ka, vl = ve - va;
+      kpos = ka, vpos = va;
+    }
+    kpos -= p0, vpos -= p0;  // stage positions
+    __syncwarp();  // every header of the round is written: the words may be ored now
+    const bool lng = vl >= kEncLong;
+    const bool any_lng = __any_sync(0xffffffffu, lng);
+    // a long value's partial words at both ends: loaded before the key's bytes
+    // are, so that one wait covers both
+    const uint32_t head = (0u - vpos) & 3, tail = (vpos + vl) & 3;
+    uint32_t hw = 0, tw = 0;
+    if (any_lng) {
+      if (lng && head) hw = enc_word(val, val + head) << (8 * (4 - head));
+      if (lng && tail) tw = enc_word(val + vl - tail, val + vl);
+    }
+    if (__any_sync(0xffffffffu, kd > 16)) {
+      for (uint32_t t = 0; t < kd; t += 32) enc_piece<8>(st + kpos + t, key + t, min(32u, kd - t));
+    } else if (kd) {
+      enc_piece<4>(st + kpos, key, kd);
+    }
+    if (vl && !lng) enc_piece<8>(st + vpos, val, vl);
+    if (any_lng) {
+      if (lng) {
+        if (head) smem_or(st + (vpos & ~3u), hw);
+        if (tail) smem_or(st + ((vpos + vl) & ~3u), tw);
+      }
+      const uint32_t w0 = (vpos + head) >> 2;                   // first whole word,
+      const uint32_t fw = lng ? ((vpos + vl) >> 2) - w0 : 0u;   // their count,
+      const uint32_t so = (uint32_t)(val - J.in) + head;        // their source
+      // the long values average 512 bytes or more: one after the other, all
+      // lanes, 1 KiB in flight (a lane's higher source word is its neighbour's
+      // lower one); else four at a time, 8 lanes each (a 100-byte value is
+      // three steps)
+      unsigned m = __ballot_sync(0xffffffffu, lng);
+      if (__reduce_add_sync(0xffffffffu, lng ? vl : 0u) >= 512 * __popc(m)) {
+        for (; m; m &= m - 1) {
+          const int e = __ffs(m) - 1;
+          const uint32_t efw = __shfl_sync(0xffffffffu, fw, e);
+          const uintptr_t a = reinterpret_cast<uintptr_t>(J.in + __shfl_sync(0xffffffffu, so, e));
+          const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3)) + lane;
+          const uint32_t fsh = 8 * (uint32_t)(a & 3);
+          const uint32_t lim = efw + (fsh ? 1 : 0);  // source words
+          uint32_t* d = reinterpret_cast<uint32_t*>(st) + __shfl_sync(0xffffffffu, w0, e) + lane;
+          constexpr uint32_t kU = 8;
+          for (uint32_t i = lane; i - lane < efw; i += 32 * kU, q += 32 * kU, d += 32 * kU) {
+            uint32_t lo[kU + 1];
+#pragma unroll
+            for (uint32_t x = 0; x <= kU; x++)
+              lo[x] = (i + 32 * x < lim && (x < kU || lane == 0)) ? __ldg(q + 32 * x) : 0u;
+#pragma unroll
+            for (uint32_t x = 0; x < kU; x++) {
+              const uint32_t hi =
+                  __shfl_sync(0xffffffffu, lane == 0 ? lo[x + 1] : lo[x], (lane + 1) & 31);
+              if (i + 32 * x < efw) d[32 * x] = __funnelshift_r(lo[x], hi, fsh);
+            }
+          }
+        }
+      } else {
+        const uint32_t li = lane & 7, cnt = min(32u, n - j0);
+        for (uint32_t e0 = 0; e0 < cnt; e0 += 4) {
+          const uint32_t e = e0 + (lane >> 3);
+          const uint32_t ew0 = __shfl_sync(0xffffffffu, w0, e);
+          const uint32_t efw = __shfl_sync(0xffffffffu, fw, e);
+          const uint32_t eso = __shfl_sync(0xffffffffu, so, e);
+          const uintptr_t a = reinterpret_cast<uintptr_t>(J.in + eso);
+          const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3)) + li;
+          const uint32_t fsh = 8 * (uint32_t)(a & 3);
+          uint32_t* d = reinterpret_cast<uint32_t*>(st) + ew0 + li;
+          constexpr uint32_t kU = 4;
+          for (uint32_t i = li; i < efw; i += 8 * kU, q += 8 * kU, d += 8 * kU) {
+            uint32_t lo[kU], hi[kU];
+#pragma unroll
+            for (uint32_t x = 0; x < kU; x++) {
+              const bool on = i + x * 8 < efw;
+              lo[x] = on ? __ldg(q + x * 8) : 0u;
+              hi[x] = on && fsh ? __ldg(q + x * 8 + 1) : 0u;
+            }
+#pragma unroll
+            for (uint32_t x = 0; x < kU; x++)
+              if (i + x * 8 < efw) d[x * 8] = __funnelshift_r(lo[x], hi[x], fsh);
+          }
+        }
+      }
+    }
+    __syncwarp();  // the words are written before the next round's header bytes
+  }
+  if (lane == 0) {  // the restart count (and the type byte, 0: the stage is clear)
+    const uint32_t rp = ph + B.bsz - 4 - p0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+      if (!kWide || rp + i < p1 - p0) st[rp + i] = (uint8_t)(nrest >> (8 * i));
+  }
+}
+
+// The assembled stage out: the whole 16-byte chunks inside [m0, m1) with one
+// bulk copy, every byte into the CRC.  Returns the raw register at m1 (from a
+// zero register), the same in every lane.  The copy still reads the stage when
+// this returns (enc_drain).
+//
+// The CRC: lane l takes q consecutive chunks (q odd, so the lanes' 16-byte
+// reads, 16 q bytes apart, fall on different banks), and folds them into its
+// last two with crc_fold_word, integer shifts and xors only; those 256 bits
+// are looked up (crc_h8), and the register is moved to m1 by one product.  A
+// lookup per 5 bits of every chunk, as in the row CRC, costs 26 lookups and 82
+// integer instructions per chunk and lane; folding costs 40.
+__device__ __forceinline__ uint32_t enc_out(const JobDev& J, const uint32_t* h8,
+                                            const uint32_t* xinv, const uint32_t* tab8,
+                                            uint8_t* gbase, const uint8_t* st, uint32_t m0,
+                                            uint32_t m1, uint32_t lane) {
+  const uint32_t nch = (m1 + 15) >> 4;
+  const uint32_t q = max(((nch + 31) >> 5) | 1u, 3u);
+  // the shift from the lane's last chunk's end to m1 (backwards for the lane
+  // that holds m1, whose last chunks lie past it; lanes past that hold nothing)
+  const int32_t n = (int32_t)m1 - (int32_t)(16 * q * (lane + 1));
+  const uint32_t f = n >= 0 ? __ldg(J.crc_xpow + n)
+                            : (n > -(int32_t)(16 * q) ? xinv[xinv_slot((uint32_t)-n)] : 0u);
+  fence_proxy_async_smem();  // the lanes' stage writes, before the bulk copy's reads
+  __syncwarp();
+  const uint32_t c0 = (m0 + 15) >> 4, c1 = m1 >> 4;
+  if (lane == 0 && c1 > c0) bulk_store(gbase + 16 * c0, st + 16 * c0, 16 * (c1 - c0));
+  uint32_t c = lane * q;
+  const uint32_t cz = c + q;
+  const auto load = [&](uint32_t x) -> uint4 {
+    return x < nch ? *reinterpret_cast<const uint4*>(st + 16 * x) : make_uint4(0u, 0u, 0u, 0u);
+  };
+  uint32_t v[8] = {};  // the folded words, a ring of the last eight
+  {
+    const uint4 x = load(c++);
+    v[4] = x.x, v[5] = x.y, v[6] = x.z, v[7] = x.w;
+    v[6] ^= v[4] << 1;
+    v[7] ^= __funnelshift_l(v[4], v[5], 1);
+  }
+  for (; c + 2 < cz; c += 2) {
+    const uint4 x = load(c), y = load(c + 1);
+    const uint32_t m[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) v[i] = m[i] ^ crc_fold_word<false>(v, i);
+  }
+  const uint4 x = load(c), y = load(c + 1);
+  uint32_t r[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+  for (uint32_t i = 0; i < 8; i++) r[i] ^= crc_fold_word<true>(v, i);
+  uint32_t u = gf2_mulmod_tab(tab8, crc_h8(h8, r), f);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) u ^= __shfl_xor_sync(0xffffffffu, u, o);
+  return u;
+}
+
+// The partial chunks' bytes in [a, m1) at both ends (the message's first
+// bytes, and those after its last whole chunk).
+__device__ __forceinline__ void enc_ends(uint8_t* gbase, const uint8_t* st, uint32_t m0, uint32_t m1,
+                                         uint32_t end, uint32_t lane) {
+  const uint32_t cf0 = (m0 + 15) >> 4, cf1 = m1 >> 4;  // whole chunks [cf0, cf1) went out
+  uint32_t h1 = 16 * cf0, t0 = 16 * cf1;
+  if (cf1 < cf0) h1 = t0 = m0;  // the message lies inside one chunk
+  const uint32_t nh = h1 - m0, nt = end - t0;
+  for (uint32_t x = lane; x < nh + nt; x += 32) {
+    const uint32_t q = x < nh ? m0 + x : t0 + (x - nh);
+    gbase[q] = st[q];
+  }
+}
+
+__device__ __forceinline__ void enc_drain(uint32_t lane) {
+  if (lane == 0) bulk_wait_read();
+  __syncwarp();
+}
+
+__global__ void __launch_bounds__(kEncWarps * 32, 2) k_encode_blocks(const JobDev* __restrict__ jobs) {
+  __shared__ uint32_t s_h8[kCrcH8Words];
   __shared__ uint32_t s_xinv[kCrcXinvSmem];
   __shared__ uint32_t s_tab8[256];
   __shared__ JobDev s_job;  // the job's descriptor, read from here in every step
   extern __shared__ __align__(16) uint8_t enc_smem[];
   copy_job(jobs + blockIdx.y, &s_job);
   const JobDev& G = jobs[blockIdx.y];
-  for (uint32_t i = threadIdx.x; i < kCrcH5Words; i += blockDim.x) s_h5[i] = G.crc_h5[i];
+  for (uint32_t i = threadIdx.x; i < kCrcH8Words; i += blockDim.x) s_h8[i] = G.crc_h8[i];
   for (uint32_t i = threadIdx.x; i < kCrcXinvN; i += blockDim.x) s_xinv[xinv_slot(i)] = G.crc_xinv[i];
   for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab8[i] = G.crc_byte[i];
   __syncthreads();
@@ -917,23 +1107,23 @@ __global__ void __launch_bounds__(kEncWarps * 32, 3) k_encode_blocks(const JobDe
   EncWarp& W = reinterpret_cast<EncWarp*>(enc_smem)[warp];
   if (J.ctr->error) return;
   const uint32_t nb = (uint32_t)J.ctr->n_blocks_out;  // block and survivor indices fit 32 bits
-  const uint32_t R = J.restart_interval;
-  const RestartDiv rd(R);
+  const RestartDiv rd(J.restart_interval);
   const uint32_t stride = gridDim.x * kEncWarps;
   uint8_t* st = W.stage;
   uint32_t b = blockIdx.x * kEncWarps + warp;
-  EncAhead cur{};
+  EncBlock cur{};
   if (b < nb) {
+    cur.off = (uint32_t)J.b_off[b];
     cur.dst = J.out + J.files[J.b_file[b]].out_off + J.b_off[b];
     cur.bsz = J.b_size[b];
     cur.s = J.b_first[b];
-    cur.n = (uint32_t)(J.b_first[b + 1] - cur.s);
+    cur.n = J.b_first[b + 1] - cur.s;
     enc_ahead_entries(J, W, cur, lane);
   }
   for (; b < nb; b += stride) {
-    // the next block's place and range (its entries follow after step 2)
+    // the next block's place and range
     const uint32_t bn = b + stride;
-    EncAhead nxt{};
+    EncBlock nxt{};
     uint32_t n_file = 0;
     uint64_t n_off = 0;
     if (bn < nb) {
@@ -941,146 +1131,65 @@ __global__ void __launch_bounds__(kEncWarps * 32, 3) k_encode_blocks(const JobDe
       n_off = J.b_off[bn];
       nxt.bsz = J.b_size[bn];
       nxt.s = J.b_first[bn];
-      nxt.n = (uint32_t)(J.b_first[bn + 1] - nxt.s);
+      nxt.n = J.b_first[bn + 1];  // (less nxt.s, below: not waited for here)
     }
-    uint8_t* dst = cur.dst;
-    const uint32_t bsz = cur.bsz, n = cur.n;
-    const uint32_t s = cur.s;
-    const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 15);
-    if (ph + bsz + kTrailer + 16 > kEncStage) {
-      enc_direct(J, s_h5, s_xinv, s_tab8, b, dst, lane);
-    } else {
-      const uint32_t nrest = rd.div(n + R - 1);
-      const uint32_t rbase = ph + bsz - 4 * nrest - 4;  // stage position of the restart array
-      const uint32_t m0 = ph, m1 = ph + bsz + 1;        // the message: block and type byte
-      // the initial register's share of the CRC, and zeros in the stage's
-      // first and last chunks (grid bytes outside the message)
-      const uint32_t ones = __ldg(J.crc_ones + (m1 - m0));
-      if (lane == 0) *reinterpret_cast<uint4*>(st) = make_uint4(0u, 0u, 0u, 0u);
-      if (lane == 1) *reinterpret_cast<uint4*>(st + ((m1 - 1) & ~15u)) = make_uint4(0u, 0u, 0u, 0u);
-      __syncwarp();
-      // 1. entries: the long stretches listed first; once the list is
-      // complete (last round) the first two chunk rows' listed chunks are
-      // loaded while the lanes write headers, restart words, short stretches
-      // and cut edges to the stage
-      uint32_t carry = 0, lcarry = 0, nls = 0, k = 0;
-      EncSlot sa{}, sb{};
-      bool ga = false, gb = false;  // sa / sb came from a listed stretch
-      for (uint32_t j0 = 0; j0 < n; j0 += 32) {
-        const uint32_t j = j0 + lane;
-        uint32_t size = 0, hl = 0, kd = 0, vl = 0, sh = 0, koff = 0, voff = 0;
-        if (j < n) {
-          uint32_t kl;
-          if (j0 == 0) {
-            cp_async_wait_all();  // this lane's own copies
-            kl = W.ahead[0][lane], sh = W.ahead[1][lane], vl = W.ahead[2][lane];
-            koff = W.ahead[3][lane], voff = W.ahead[4][lane];
-          } else {
-            const uint32_t e = s + j;
-            kl = J.k_klen[e], sh = J.k_shared[e], vl = J.k_vlen[e];
-            koff = J.k_koff[e], voff = J.k_voff[e];
-          }
-          if (rd.starts_run(j)) sh = 0;
-          kd = kl - sh;
-          koff += sh;
-          hl = varint_len32(sh) + varint_len32(kd) + varint_len32(vl);
-          size = hl + kd + vl;
-        }
-        uint32_t tot, ltot;
-        const uint32_t ex = warp_excl<uint32_t>(size, &tot) + carry;
-        const uint32_t nl = j < n ? (uint32_t)(kd >= kEncLong) + (uint32_t)(vl >= kEncLong) : 0u;
-        uint32_t li = warp_excl<uint32_t>(nl, &ltot) + lcarry;
-        carry += tot;
-        lcarry += ltot;
-        const uint32_t kpos = ph + ex + hl;
-        const uint32_t lik = li;
-        if (j < n) enc_list(W, kpos, kd, koff, 0u, li);
-        const uint32_t liv = li;
-        if (j < n) enc_list(W, kpos + kd, vl, voff, kEncFromInput, li);
-        if (j0 + 32 >= n) {
-          __syncwarp();
-          nls = min(lcarry, kEncMaxLong);
-          if (16 * lane < m1) ga = enc_fetch_listed(J, W, nls, lane, k, sa);
-          if (16 * (lane + 32) < m1) gb = enc_fetch_listed(J, W, nls, lane + 32, k, sb);
-        }
-        if (j < n) {
-          uint8_t* p = st + ph + ex;
-          p = put_varint32(p, sh);
-          p = put_varint32(p, kd);
-          put_varint32(p, vl);
-          const uint32_t run = rd.div(j);
-          if (j == run * R) {
-            const uint32_t rem = n - j;
-            st_le32(st + rbase + 4 * run, (ex << 8) | (rem < R ? rem : R));
-          }
-          if (J.dec_vpos)  // the value's place in its file, for the decoded form
-            J.dec_vpos[s + j] = (uint32_t)(J.b_off[b] + ex + hl + kd);
-          enc_stage(st, kpos, kd, J.keys + koff, lik < kEncMaxLong);
-          enc_stage(st, kpos + kd, vl, J.in + voff, liv < kEncMaxLong);
-        }
-      }
-      if (lane == 0) {
-        st_le32(st + ph + bsz - 4, nrest);
-        st[ph + bsz] = 0;  // kNoCompression
-      }
-      __syncwarp();
-      // 2. chunks: out to global memory and into the CRC; each chunk's loads
-      // are issued two chunks ahead of its use (three rotating slots)
-      uint8_t* gbase = dst - ph;
-      uint32_t u = 0, last = 0xffffffffu;
-      EncSlot sc;
-      bool vb = 16 * (lane + 32) < m1;
-      if (16 * lane < m1 && !ga) enc_fetch_stage(st, lane, sa);
-      if (vb && !gb) enc_fetch_stage(st, lane + 32, sb);
-      if (bn < nb) {  // the next block's place and entries, in flight meanwhile
-        nxt.dst = J.out + J.files[n_file].out_off + n_off;
-        enc_ahead_entries(J, W, nxt, lane);
-      }
-      for (uint32_t c = lane; 16 * c < m1; c += 96) {
-        const bool vc = 16 * (c + 64) < m1;
-        if (vc) enc_fetch(J, W, st, nls, c + 64, k, sc);
-        enc_chunk_out(s_h5, gbase, 16 * c, m0, m1, sa, u, last);
-        if (16 * (c + 96) < m1) enc_fetch(J, W, st, nls, c + 96, k, sa);
-        if (vb) enc_chunk_out(s_h5, gbase, 16 * (c + 32), m0, m1, sb, u, last);
-        const bool ve = 16 * (c + 128) < m1;
-        if (ve) enc_fetch(J, W, st, nls, c + 128, k, sb);
-        if (vc) enc_chunk_out(s_h5, gbase, 16 * (c + 64), m0, m1, sc, u, last);
-        vb = ve;
-      }
-      // the lines the next block's entry pass copies bytes from (its keys,
-      // its values' first and last bytes) into L2 while this block finishes
-      if (bn < nb && lane < nxt.n) {
-        cp_async_wait_all();
-        const uint32_t pkl = W.ahead[0][lane], pvl = W.ahead[2][lane];
-        const uint32_t pko = W.ahead[3][lane], pvo = W.ahead[4][lane];
-        prefetch_l2(J.keys + pko);
-        prefetch_l2(J.keys + pko + pkl - 1);
-        prefetch_l2(J.in + pvo);
-        if (pvl) prefetch_l2(J.in + pvo + pvl - 1);
-      }
-      // 3. CRC (with the initial register's share), trailer, partial chunks
-      // at both ends
-      const uint32_t full = crc_rows_raw(s_xinv, s_tab8, u, last, m1) ^ ones ^ 0xffffffffu;
+    const bool narrow = cur.bsz <= kEncNarrow;  // wide blocks: by their windows, below
+    const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(cur.dst) & 15);
+    const uint32_t m0 = ph, m1 = ph + cur.bsz + 1;  // the message: block and type byte
+    cp_async_wait_all();  // this lane's entries of the block
+    uint32_t ones = 0;
+    if (narrow) {
+      ones = __ldg(J.crc_ones + (m1 - m0));
+      enc_drain(lane);
+      enc_assemble<false>(J, W, cur, rd, ph, 0, m1, lane);
+    }
+    if (bn < nb) {  // the next block's place and entries, in flight meanwhile
+      nxt.n -= nxt.s;
+      nxt.off = (uint32_t)n_off;
+      nxt.dst = J.out + J.files[n_file].out_off + n_off;
+      enc_ahead_entries(J, W, nxt, lane);  // each lane's own slots
+    }
+    if (narrow) {
+      uint8_t* gbase = cur.dst - ph;
+      const uint32_t full =
+          enc_out(J, s_h8, s_xinv, s_tab8, gbase, st, m0, m1, lane) ^ ones ^ 0xffffffffu;
       const uint32_t crc = ((full >> 15) | (full << 17)) + 0xa282ead8u;  // crc32c::Mask
+      if (bn < nb && nxt.bsz <= kEncNarrow) {
+        cp_async_wait_all();
+        enc_prefetch(J, W, nxt.n, lane);
+      }
       if (lane == 0) st_le32(st + m1, crc);
       __syncwarp();
-      const uint32_t cf0 = (m0 + 15) >> 4, cf1 = m1 >> 4;  // whole chunks [cf0, cf1) went out
-      uint32_t h1 = 16 * cf0, t0 = 16 * cf1;
-      if (cf1 < cf0) h1 = t0 = m0;  // the message lies inside one chunk
-      const uint32_t nh = h1 - m0, nt = m1 + 4 - t0;
-      for (uint32_t x = lane; x < nh + nt; x += 32) {
-        const uint32_t q = x < nh ? m0 + x : t0 + (x - nh);
-        gbase[q] = st[q];
-      }
+      enc_ends(gbase, st, m0, m1, m1 + 4, lane);
       __syncwarp();
-    }
-    if (bn < nb && nxt.dst == nullptr) {  // the direct path
-      nxt.dst = J.out + J.files[n_file].out_off + n_off;
-      enc_ahead_entries(J, W, nxt, lane);
     }
     cur = nxt;
   }
-  cp_async_wait_all();  // a direct-path last block never waited for its entries' copies
+  // windows of the wide blocks
+  const uint32_t nw = min(J.ctr->n_wide, J.cap_wide);
+  for (uint32_t x = blockIdx.x * kEncWarps + warp; x < nw; x += stride) {
+    const uint2 un = J.wide[x];  // block, window
+    EncBlock B;
+    B.off = (uint32_t)J.b_off[un.x];
+    B.dst = J.out + J.files[J.b_file[un.x]].out_off + J.b_off[un.x];
+    B.bsz = J.b_size[un.x];
+    B.s = J.b_first[un.x];
+    B.n = J.b_first[un.x + 1] - B.s;
+    const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(B.dst) & 15);
+    const uint32_t end = ph + B.bsz + 1;  // the message's end
+    const uint32_t p0 = un.y * kEncWindow, p1 = min(end, p0 + kEncWindow);
+    if (p0 >= end) continue;  // the layout counted the longest phase
+    enc_drain(lane);
+    enc_assemble<true>(J, W, B, rd, ph, p0, p1, lane);
+    uint8_t* gbase = B.dst - ph + p0;
+    const uint32_t m0 = p0 ? 0 : ph, m1 = p1 - p0;
+    const uint32_t raw = enc_out(J, s_h8, s_xinv, s_tab8, gbase, st, m0, m1, lane);
+    if (lane == 0) atomicXor(J.b_crc + un.x, crc_shift_tab(J, s_tab8, raw, end - p1));
+    enc_ends(gbase, st, m0, m1, m1, lane);
+    __syncwarp();
+  }
+  cp_async_wait_all();
+  enc_drain(lane);
 }
 
 // The survivors' decoded form for later jobs (keep_decoded): key bytes at
@@ -1422,20 +1531,41 @@ __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ job
   }
 }
 
+// The register after n zero bytes from all ones.
+__device__ __forceinline__ uint32_t crc_ones_after(const JobDev& J, uint64_t n) {
+  const uint64_t N = J.crc_xpow_n;
+  if (n < N) return J.crc_ones[n];
+  if (n >= N * N) return crc_shift(J, 0xffffffffu, n);
+  return gf2_mulmod(J.crc_ones[n % N], J.crc_xpow_hi[n / N]);
+}
+
+__device__ __forceinline__ void put_trailer(uint8_t* p, uint32_t raw) {
+  const uint32_t full = raw ^ 0xffffffffu;
+  p[0] = 0;  // kNoCompression
+  st_le32(p + 1, ((full >> 15) | (full << 17)) + 0xa282ead8u);  // crc32c::Mask
+}
+
+// The trailers of the filter, metaindex and index blocks, and of the data
+// blocks that were written in windows.
 __global__ void k_meta_trailers(const JobDev* __restrict__ jobs) {
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;
-  const uint32_t nf = J.ctr->n_files;
-  for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < 3 * nf; x += gridDim.x * blockDim.x) {
+  const uint32_t nf = J.ctr->n_files, nw = min(J.ctr->n_wide, J.cap_wide);
+  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (uint32_t x = t0; x < 3 * nf; x += stride) {
     const uint32_t f = x / 3, r = x % 3;
     if (r == 0 && J.bits_per_key <= 0) continue;
     const FileOut& F = J.files[f];
     uint64_t off, len;
     meta_region(F, r, &off, &len);
-    uint8_t* p = J.out + F.out_off + off + len;
-    const uint32_t full = F.crc_acc[r] ^ 0xffffffffu;
-    p[0] = 0;  // kNoCompression
-    st_le32(p + 1, ((full >> 15) | (full << 17)) + 0xa282ead8u);  // crc32c::Mask
+    put_trailer(J.out + F.out_off + off + len, F.crc_acc[r]);
+  }
+  for (uint32_t x = t0; x < nw; x += stride) {
+    const uint2 un = J.wide[x];
+    if (un.y != 0) continue;  // once per block
+    const uint32_t b = un.x, size = J.b_size[b];
+    put_trailer(J.out + J.files[J.b_file[b]].out_off + J.b_off[b] + size,
+                J.b_crc[b] ^ crc_ones_after(J, (uint64_t)size + 1));
   }
 }
 
@@ -1487,9 +1617,11 @@ void encode_kernel_attributes() {
 }
 
 void launch_encode_blocks(const Batch& bt, cudaStream_t st) {
-  // grid-stride over the device-side block count: 3 CTAs per SM x 4 waves,
-  // shared out among the jobs
-  note_launch(), k_encode_blocks<<<dim3(grid_x(bt.max_entries, kEncWarps, per_job(bt, 148 * 3 * 4)),
+  // grid-stride over the device-side counts of blocks and windows: 3 CTAs per
+  // SM x 4 waves, shared out among the jobs (a job of few entries may have as
+  // many windows as its output bytes allow)
+  note_launch(), k_encode_blocks<<<dim3(grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide),
+                                               kEncWarps, per_job(bt, 148 * 2 * 4)),
                                         bt.B), kEncWarps * 32, kEncSmem, st>>>(bt.d);
 }
 void launch_emit_decoded(const Batch& bt, cudaStream_t st) {
@@ -1514,7 +1646,10 @@ void launch_encode_meta(const Batch& bt, cudaStream_t st) {
     per_file *= 2;
   note_launch(), k_meta_crc<<<dim3(per_file, std::min<uint32_t>(bt.max_cap_files, 65535), bt.B),
                               256, 0, st>>>(bt.d);
-  note_launch(), k_meta_trailers<<<dim3((3 * bt.max_cap_files + 255) / 256, bt.B), 256, 0, st>>>(bt.d);
+  // (the wide blocks are at most the entries)
+  note_launch(), k_meta_trailers<<<dim3(std::max((3 * bt.max_cap_files + 255) / 256,
+                                                 grid_x(bt.max_entries, 2048, per_job(bt, 148 * 2))),
+                                        bt.B), 256, 0, st>>>(bt.d);
 }
 
 }  // namespace lc

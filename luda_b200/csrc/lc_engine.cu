@@ -528,6 +528,7 @@ void fill_common(JobDev& J, const lc_job* j, lc_engine* e) {
   J.crc_byte = J.crc_xinv + kCrcXinvN;
   J.crc_ones = J.crc_byte + 256;
   J.crc_xpow_hi = J.crc_ones + kCrcXpowN;
+  J.crc_h8 = J.crc_xpow_hi + kCrcXpowN;
   J.chunk = kChunk;
   J.chain_smem_words = 11 * 1024;  // 44 KiB (static shared memory takes the rest of 48)
 }
@@ -710,6 +711,9 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
     J.cap_out = r.in_bytes + 3 * J.cap_key_bytes + N * (80 + (bpk + 7) / 8) +
                 (uint64_t)J.cap_files * 256 + (r.in_bytes + J.cap_key_bytes) / 256 + 65536;
   }
+  J.cap_wide = (uint32_t)std::min<uint64_t>(J.cap_out / (kEncNarrow / 2) + 16, 0xffffffffu);
+  J.wide = A.get<uint2>(J.cap_wide);
+  J.b_crc = J.k_block;
   J.out = A.output(J.cap_out, r.j->outputs_on_device == 1 || r.j->outputs_on_device == 2);
   if (r.j->keep_decoded && !r.failed) {
     // the survivors' decoded form, kept with the outputs: keys (at most the
@@ -742,6 +746,7 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
 struct lc_slot {
   cudaStream_t st = nullptr;
   JobDev* d_jobs = nullptr;
+  uint32_t* d_crc = nullptr;  // lc_crc32c: scratch words (zero between calls), one result word
   uint32_t cap = 0;
   struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
@@ -794,6 +799,8 @@ struct lc_slot {
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     cap = capacity;
     CK(cudaMalloc(&d_jobs, sizeof(JobDev) * cap));
+    CK(cudaMalloc(&d_crc, 4 * (kCrcScratchWords + 1)));
+    CK(cudaMemsetAsync(d_crc, 0, 4 * (kCrcScratchWords + 1), st));
   }
   void destroy() {
     for (auto& g : graphs) {
@@ -808,8 +815,10 @@ struct lc_slot {
     pin_dev = nullptr;
     pin_cap = 0;
     if (d_jobs) cudaFree(d_jobs);
+    if (d_crc) cudaFree(d_crc);
     if (st) cudaStreamDestroy(st);
     d_jobs = nullptr;
+    d_crc = nullptr;
     st = nullptr;
   }
   std::map<std::string, uint32_t> seen;  // shape keys met without a graph
@@ -825,10 +834,10 @@ struct lc_slot {
       return 0;
     }
     char key[256];
-    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
+    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%llu|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
              (int)decode_merge, bt.B, bt.max_tables, bt.max_gp, bt.max_cap_triggers,
              bt.max_cap_files, (unsigned long long)bt.max_blocks_in,
-             (unsigned long long)bt.max_entries, bt.merge_rounds, bt.chunk, bt.ctas_per_job,
+             (unsigned long long)bt.max_entries, (unsigned long long)bt.max_cap_wide, bt.merge_rounds, bt.chunk, bt.ctas_per_job,
              bt.merge_items, bt.merge_threads, bt.max_runs,
              (int)bt.any_keep_decoded);
     auto it = graphs.find(key);
@@ -1220,6 +1229,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       }
       max_runs = std::max<uint32_t>(max_runs, r.J.n_runs);
       bt.max_entries = std::max<uint64_t>(bt.max_entries, r.N);
+      bt.max_cap_wide = std::max<uint64_t>(bt.max_cap_wide, r.J.cap_wide);
       bt.max_gp = std::max<uint32_t>(bt.max_gp, r.J.n_gp);
       bt.max_cap_triggers = std::max<uint32_t>(bt.max_cap_triggers, r.J.cap_triggers);
       bt.max_cap_files = std::max<uint32_t>(bt.max_cap_files, r.J.cap_files);
@@ -1230,6 +1240,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     // grid shapes in powers of two, so that batches of similar size share a
     // captured graph (the kernels loop over whatever the grid leaves)
     bt.max_entries = pow2_at_least(std::max<uint64_t>(bt.max_entries, 1));
+    bt.max_cap_wide = pow2_at_least(bt.max_cap_wide);
     bt.max_blocks_in = pow2_at_least(bt.max_blocks_in);  // decode grid size only
     bt.max_cap_files = (uint32_t)pow2_at_least(bt.max_cap_files);
     bt.max_cap_triggers = (uint32_t)pow2_at_least(bt.max_cap_triggers);
@@ -1512,6 +1523,7 @@ void run_build(lc_job* j, lc_slot& slot) {
     bt.d = slot.d_jobs;
     bt.B = 1;
     bt.max_entries = std::max<uint64_t>(N, 1);
+    bt.max_cap_wide = J.cap_wide;
     bt.max_cap_files = J.cap_files;
     bt.max_cap_triggers = J.cap_triggers;
     T.mark(kUpload);
@@ -1772,7 +1784,7 @@ void fill_out(lc_job* j, lc_job_out* o) {
 }
 
 // The engine's CRC tables, one device array: [x^(8n) | row fields | x^(-8n) |
-// byte table | all-ones shifts | long shifts].
+// byte table | all-ones shifts | long shifts | 32-byte fields].
 //  * x^(8n) mod P for n < kCrcXpowN (register shifts by n zero bytes);
 //  * for the row CRC: entry kCrcFieldEntries i + v is the register after 16
 //    bytes holding v at bits [W i, W i + W) (W = kCrcFieldBits) and zero
@@ -1782,7 +1794,9 @@ void fill_out(lc_job* j, lc_job_out* o) {
 //  * for n < kCrcXpowN, the register after n zero bytes from all ones (the
 //    CRC's initial register carried to the end of an n-byte message);
 //  * x^(8 kCrcXpowN h) mod P for h < kCrcXpowN: with the first table, any
-//    shift below kCrcXpowN^2 bytes is one product of two entries.
+//    shift below kCrcXpowN^2 bytes is one product of two entries;
+//  * for crc_h8: entry kCrcFieldEntries i + v is the register after 32 bytes
+//    holding v at bits [W i, W i + W) and zero elsewhere, from register 0.
 // Registers are reflected (bit 31 is x^0), as in util/crc32c.cc.
 uint32_t host_crc_byte(uint32_t c, uint8_t b) {
   c ^= b;
@@ -1791,7 +1805,7 @@ uint32_t host_crc_byte(uint32_t c, uint8_t b) {
 }
 
 void host_crc_tables(std::vector<uint32_t>& t) {
-  t.assign(kCrcXpowN + kCrcH5Words + kCrcXinvN + 256 + 2 * kCrcXpowN, 0);
+  t.assign(kCrcXpowN + kCrcH5Words + kCrcXinvN + 256 + 2 * kCrcXpowN + kCrcH8Words, 0);
   uint32_t c = 0x80000000u;  // x^0
   for (uint32_t m = 0; m < kCrcXpowN; m++) {
     t[m] = c;
@@ -1837,6 +1851,20 @@ void host_crc_tables(std::vector<uint32_t>& t) {
     hi[h] = c;
     c = gf2_mulmod(c, step);
   }
+  uint32_t* h8 = hi + kCrcXpowN;
+  for (uint32_t i = 0; i < kCrcH8Fields; i++)
+    for (uint32_t v = 0; v < kCrcFieldEntries; v++) {
+      uint32_t r = 0;
+      for (uint32_t k = 0; k < 32; k++) {
+        uint8_t x = 0;
+        for (uint32_t bit = 0; bit < kCrcFieldBits; bit++) {
+          const uint32_t at = kCrcFieldBits * i + bit;
+          if (((v >> bit) & 1) && at >> 3 == k) x |= (uint8_t)(1u << (at & 7));
+        }
+        r = host_crc_byte(r, x);
+      }
+      h8[kCrcFieldEntries * i + v] = r;
+    }
 }
 
 }  // namespace
@@ -2336,7 +2364,6 @@ lc_status lc_crc32c(lc_engine* e, const uint8_t* data, uint64_t n, int32_t on_de
     slot = e->take_slot();
     st = slot->st;
     const uint8_t* d_data = data;
-    const uint32_t chunks = crc32c_chunk_count(n);
     void* p = nullptr;
     if (!on_device && n) {
       CK(cudaMallocAsync(&p, n, st));
@@ -2344,20 +2371,18 @@ lc_status lc_crc32c(lc_engine* e, const uint8_t* data, uint64_t n, int32_t on_de
       CK(cudaMemcpyAsync(p, data, n, cudaMemcpyHostToDevice, st));
       d_data = (const uint8_t*)p;
     }
-    // scratch: one register per chunk, the ticket counter, the result
-    CK(cudaMallocAsync(&p, ((size_t)chunks + 2) * sizeof(uint32_t), st));
-    ptrs.push_back(p);
-    uint32_t* partials = (uint32_t*)p;
-    uint32_t* counter = partials + chunks;
-    uint32_t* d_out = counter + 1;
-    CK(cudaMemsetAsync(counter, 0, sizeof(uint32_t), st));
-    launch_crc32c_chunks(d_data, n, partials, counter, d_out, st);
+    // the kernel stores the result into the slot's mapped staging buffer
+    uint32_t* h_out = reinterpret_cast<uint32_t*>(slot->pinned(16));
+    uint32_t* d_out = slot->pin_dev ? reinterpret_cast<uint32_t*>(slot->pin_dev)
+                                    : slot->d_crc + kCrcScratchWords;
+    launch_crc32c_chunks(d_data, n, slot->d_crc, d_out, st);
     CK(cudaGetLastError());
-    uint32_t h = 0;
-    CK(cudaMemcpyAsync(&h, d_out, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    if (!slot->pin_dev)
+      CK(cudaMemcpyAsync(h_out, d_out, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     for (void* q : ptrs) CK(cudaFreeAsync(q, st));
     ptrs.clear();
     CK(cudaStreamSynchronize(st));
+    const uint32_t h = *reinterpret_cast<volatile uint32_t*>(h_out);
     e->put_slot(slot);
     *masked_crc = h;
     return LC_OK;

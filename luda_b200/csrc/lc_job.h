@@ -48,7 +48,7 @@ struct Counters {
   uint64_t bytes_out;
   uint32_t n_triggers;
   uint32_t n_files;
-  uint32_t n_groups;
+  uint32_t n_wide;  // windows of the output blocks too wide for the encoder's stage
   uint32_t pad;
   uint64_t kept_key_bytes;    // internal-key bytes of the survivors
   uint64_t kept_value_bytes;  // value bytes of the survivors
@@ -232,6 +232,10 @@ struct JobDev {
   uint32_t* t_blocks;        // output block starting at each grandparent cut
   uint32_t* t_kept;          // survivor position of each grandparent cut (ascending)
   uint64_t* k_pb;            // n_kept + 1: prefix sums of k_b (block size estimates)
+  uint2* wide;               // (block, window) of the wide blocks, n_wide of them
+  uint32_t cap_wide;
+  uint32_t* b_crc;           // wide blocks: raw CRC32C registers xored from their windows
+                             // (k_block's memory, which the layout no longer needs)
   uint64_t cap_blocks_out;
 
   // files
@@ -256,6 +260,7 @@ struct JobDev {
   const uint32_t* crc_xpow;
   uint32_t crc_xpow_n;
   const uint32_t* crc_h5;     // kCrcH5Words: the field tables of the row CRC
+  const uint32_t* crc_h8;     // kCrcH8Words: the field tables of 32 bytes (crc_h8)
   const uint32_t* crc_xinv;   // kCrcXinvN: x^(-8n) mod P, back shifts by n bytes
   const uint32_t* crc_byte;   // 256: the byte table (register after byte i, from 0)
   const uint32_t* crc_ones;   // crc_xpow_n: the register after n zero bytes from all ones

@@ -33,6 +33,13 @@ void merge_kernel_attributes();
 // Chunks per group in the block-chain resolution.
 constexpr uint32_t kChainGroup = 64;
 
+// Block encoder (k_encode_blocks): a warp's shared-memory stage, the widest
+// block assembled whole in it, and the windows of wider ones.  A block of z >
+// kEncNarrow bytes has at most z / (kEncNarrow / 2) windows.
+constexpr uint32_t kEncStage = 5120;
+constexpr uint32_t kEncNarrow = kEncStage - 64;
+constexpr uint32_t kEncWindow = 4608;  // 9 full CRC rows
+
 // Largest merge tile (threads x items) and the shared memory the tile takes
 // per position.
 constexpr uint32_t kMergeMaxTile = 4096;
