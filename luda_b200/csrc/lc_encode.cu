@@ -1456,8 +1456,9 @@ __global__ void __launch_bounds__(256) k_encode_meta(const JobDev* __restrict__ 
 // piece's 16-byte chunks); a piece's raw register, moved to the region's end
 // past its type byte, is xored into the file's accumulator (the xor of every
 // byte's share is the register of the whole), and k_meta_trailers writes the
-// finished CRCs.  CTAs per file: from the entries per file (the filter and
-// index blocks grow with them), 4 to 32.
+// finished CRCs.  The grid follows the job's entries (the filter and index
+// blocks grow with them); a grid of CTAs per file and file slot spent 446 us of
+// a 32-job batch on CTAs that loaded their tables and had no file.
 constexpr uint32_t kMetaPiece = 4096;
 
 __device__ __forceinline__ void meta_region(const FileOut& F, uint32_t r, uint64_t* off,
@@ -1475,20 +1476,20 @@ __device__ __forceinline__ void meta_region(const FileOut& F, uint32_t r, uint64
 }
 
 __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ jobs) {
-  const JobDev& J = jobs[blockIdx.z];
+  const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_h5[kCrcH5Words];
   __shared__ uint32_t s_xinv[kCrcXinvSmem];
   __shared__ uint32_t s_tab8[256];
-  __shared__ uint32_t s_skip;
-  if (threadIdx.x == 0) s_skip = J.ctr->error || blockIdx.y >= J.ctr->n_files;
+  if (J.ctr->error) return;
   for (uint32_t i = threadIdx.x; i < kCrcH5Words; i += blockDim.x) s_h5[i] = J.crc_h5[i];
   for (uint32_t i = threadIdx.x; i < kCrcXinvN; i += blockDim.x) s_xinv[xinv_slot(i)] = J.crc_xinv[i];
   for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab8[i] = J.crc_byte[i];
   __syncthreads();
-  if (s_skip) return;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t nf = J.ctr->n_files;
-  for (uint32_t f = blockIdx.y; f < nf; f += gridDim.y) {
+  const uint32_t lane = threadIdx.x & 31, nf = J.ctr->n_files;
+  // the pieces of all files are dealt to the job's warps in turn
+  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
+  uint64_t turn = (uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  for (uint32_t f = 0; f < nf; f++) {
     const FileOut& F = J.files[f];
     uint64_t off[3], len[3], np[3];
     for (uint32_t r = 0; r < 3; r++) {
@@ -1497,10 +1498,9 @@ __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ job
     }
     const uint8_t* fbase = J.out + F.out_off;
     const uint64_t total = np[0] + np[1] + np[2];
-    for (uint64_t p = (uint64_t)blockIdx.x * (blockDim.x / 32) + warp; p < total;
-         p += (uint64_t)gridDim.x * (blockDim.x / 32)) {
+    for (; turn < total; turn += warps) {
       uint32_t r = 0;
-      uint64_t q = p;
+      uint64_t q = turn;
       while (q >= np[r]) q -= np[r++];
       const uint64_t a = q * kMetaPiece, e = min(len[r], a + kMetaPiece);
       const uint8_t* pa = fbase + off[r] + a;
@@ -1528,6 +1528,7 @@ __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ job
       if (lane == 0)
         atomicXor(&J.files[f].crc_acc[r], crc_shift_tab(J, s_tab8, raw, len[r] + 1 - e));
     }
+    turn -= total;
   }
 }
 
@@ -1566,6 +1567,33 @@ __global__ void k_meta_trailers(const JobDev* __restrict__ jobs) {
     const uint32_t b = un.x, size = J.b_size[b];
     put_trailer(J.out + J.files[J.b_file[b]].out_off + J.b_off[b] + size,
                 J.b_crc[b] ^ crc_ones_after(J, (uint64_t)size + 1));
+  }
+}
+
+// The job's counters and its files' descriptions and boundary keys straight
+// into mapped pinned host memory, as many as there are: how many is known only
+// here, and a copy of the arrays' capacity (hundreds of files a job) took the
+// link 69 us and the host's reading of it 1.3 ms for a batch of 32 jobs.  One
+// warp per file; the last kernel of a batch.
+__global__ void __launch_bounds__(256) k_results(const JobDev* __restrict__ jobs) {
+  const JobDev& J = jobs[blockIdx.y];
+  if (!J.res_ctr) return;
+  const uint32_t lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const auto copy = [&](void* dst, const void* src, uint32_t n) {  // n: a multiple of 8
+    for (uint32_t i = lane; i < n / 8; i += 32)
+      reinterpret_cast<uint64_t*>(dst)[i] = reinterpret_cast<const uint64_t*>(src)[i];
+  };
+  if (w == 0) copy(J.res_ctr, J.ctr, sizeof(Counters));
+  if (J.ctr->error) return;
+  const uint32_t nf = J.ctr->n_files;
+  for (uint32_t f = w; f < nf; f += (gridDim.x * blockDim.x) >> 5) {
+    copy(J.res_files + f, J.files + f, sizeof(FileOut));
+    const uint32_t l0 = (uint32_t)J.fkoff[2 * f], l1 = (uint32_t)J.fkoff[2 * f + 1];
+    if (lane < 2) J.res_klen[2 * f + lane] = lane ? l1 : l0;
+    const uint64_t at = 2ull * f * J.fkey_stride;
+    for (uint32_t i = lane; i < l0; i += 32) J.res_keys[at + i] = J.fkeys[at + i];
+    for (uint32_t i = lane; i < l1; i += 32)
+      J.res_keys[at + J.fkey_stride + i] = J.fkeys[at + J.fkey_stride + i];
   }
 }
 
@@ -1640,16 +1668,16 @@ void launch_encode_index(const Batch& bt, cudaStream_t st) {
 }
 void launch_encode_meta(const Batch& bt, cudaStream_t st) {
   note_launch(), k_encode_meta<<<dim3(bt.max_cap_files, bt.B), 256, 0, st>>>(bt.d);
-  uint32_t per_file = 4;
-  while (per_file < 32 && (uint64_t)per_file * 8192 * std::max<uint32_t>(bt.max_cap_files, 1) <
-                              bt.max_entries)
-    per_file *= 2;
-  note_launch(), k_meta_crc<<<dim3(per_file, std::min<uint32_t>(bt.max_cap_files, 65535), bt.B),
-                              256, 0, st>>>(bt.d);
+  note_launch(), k_meta_crc<<<dim3(grid_x(bt.max_entries, 4096, per_job(bt, 148 * 4)), bt.B), 256, 0,
+                              st>>>(bt.d);
   // (the wide blocks are at most the entries)
   note_launch(), k_meta_trailers<<<dim3(std::max((3 * bt.max_cap_files + 255) / 256,
                                                  grid_x(bt.max_entries, 2048, per_job(bt, 148 * 2))),
                                         bt.B), 256, 0, st>>>(bt.d);
+}
+
+void launch_results(const Batch& bt, cudaStream_t st) {
+  note_launch(), k_results<<<dim3(grid_x(bt.max_cap_files, 8, 16), bt.B), 256, 0, st>>>(bt.d);
 }
 
 }  // namespace lc

@@ -556,7 +556,8 @@ struct JobRun {
   bool failed = false;
   Counters hc{};
   std::vector<FileOut> files;
-  std::vector<uint64_t> koff;
+  std::vector<uint32_t> klen;  // lengths of the files' smallest and largest keys
+  std::vector<uint64_t> koff;  // (run_build: the same, as copied from the device)
   uint8_t* dec_block = nullptr;  // keep_decoded: the decoded buffer (device output slab)
   uint64_t dec_cap = 0;
 };
@@ -621,6 +622,7 @@ void launch_tail(const Batch& bt, bool decode_merge, cudaStream_t st, PhaseTimer
   launch_encode_filters(bt, st);
   launch_encode_index(bt, st);
   launch_encode_meta(bt, st);
+  if (decode_merge) launch_results(bt, st);
   T.mark(kEncodeMeta);
 }
 
@@ -1247,30 +1249,39 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     bt.max_gp = bt.max_gp ? (uint32_t)pow2_at_least(bt.max_gp + 1) - 1 : 0;
     bt.merge_rounds = ceil_log2(max_runs);
     bt.max_runs = max_runs;
-    // every job's per-file results in one device region, read back with one
-    // copy: [files | key offsets | keys] per job
+    // every job's per-file arrays in one device region, [files | key lengths |
+    // keys] per job, and a region of the same layout in pinned memory
+    // (k_results fills it with the files there are)
     std::vector<size_t> res_off(B + 1, 0);
+    const auto res_at = [&](uint32_t i, size_t* klen, size_t* keys) {
+      const size_t cap = runs[i].J.cap_files;
+      *klen = res_off[i] + ((sizeof(FileOut) * cap + 15) & ~size_t(15));
+      *keys = *klen + ((8 * (2 * cap + 1) + 15) & ~size_t(15));
+      return *keys + ((2 * cap * runs[i].max_klen + 1 + 15) & ~size_t(15));
+    };
     for (uint32_t i = 0; i < B; i++) {
-      const JobDev& J = runs[i].J;
-      const size_t sz = ((sizeof(FileOut) * J.cap_files + 15) & ~size_t(15)) +
-                        ((8 * (2ull * J.cap_files + 1) + 15) & ~size_t(15)) +
-                        ((2ull * J.cap_files * runs[i].max_klen + 1 + 15) & ~size_t(15));
-      res_off[i + 1] = res_off[i] + sz;
+      size_t klen, keys;
+      res_off[i + 1] = res_at(i, &klen, &keys);
     }
     uint8_t* d_res = A.get<uint8_t>(res_off[B]);
-    for (uint32_t i = 0; i < B; i++) {
-      JobDev& J = runs[i].J;
-      uint8_t* q = d_res + res_off[i];
-      J.files = reinterpret_cast<FileOut*>(q);
-      q += (sizeof(FileOut) * J.cap_files + 15) & ~size_t(15);
-      J.fkoff = reinterpret_cast<uint64_t*>(q);
-      q += (8 * (2ull * J.cap_files + 1) + 15) & ~size_t(15);
-      J.fkeys = q;
-    }
     // pinned staging after the first sync: [counters | descriptors | results]
     const size_t p_hj = (sizeof(Counters) * B + 255) & ~size_t(255);
     const size_t p_res = p_hj + ((sizeof(JobDev) * B + 255) & ~size_t(255));
     uint8_t* pin2 = slot.pinned(p_res + res_off[B]);
+    for (uint32_t i = 0; i < B; i++) {
+      JobDev& J = runs[i].J;
+      size_t klen, keys;
+      res_at(i, &klen, &keys);
+      J.files = reinterpret_cast<FileOut*>(d_res + res_off[i]);
+      J.fkoff = reinterpret_cast<uint64_t*>(d_res + klen);
+      J.fkeys = d_res + keys;
+      if (uint8_t* m = slot.pin_dev) {
+        J.res_ctr = reinterpret_cast<Counters*>(m) + i;
+        J.res_files = reinterpret_cast<FileOut*>(m + p_res + res_off[i]);
+        J.res_klen = reinterpret_cast<uint32_t*>(m + p_res + klen);
+        J.res_keys = m + p_res + keys;
+      }
+    }
     if (any_zeroed) {
       memcpy(pin2, hc.data(), sizeof(Counters) * B);
       slot.to_device(d_ctr, pin2, sizeof(Counters) * B);
@@ -1284,25 +1295,31 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     (how == 0 ? e->n_direct : how == 1 ? e->n_captures : e->n_replays)++;
     e->n_batches++;
     e->n_jobs += B;
-    // ---- per-job results: two transfers into pinned memory, one sync
-    slot.to_host(pin2 + p_res, d_res, res_off[B]);
-    slot.to_host(pin2, d_ctr, sizeof(Counters) * B);
+    // ---- per-job results: in pinned memory after the batch's last kernel
+    // (without mapped memory, copied there), one sync
+    if (!slot.pin_dev) {
+      slot.to_host(pin2 + p_res, d_res, res_off[B]);
+      slot.to_host(pin2, d_ctr, sizeof(Counters) * B);
+    }
     CK(cudaStreamSynchronize(st));
     memcpy(hc.data(), pin2, sizeof(Counters) * B);
     for (uint32_t i = 0; i < B; i++) {
       JobRun& r = runs[i];
-      const uint8_t* q = pin2 + p_res + res_off[i];
-      r.files.resize(r.J.cap_files);
-      r.koff.resize(2ull * r.J.cap_files + 1);
-      r.j->key_bytes.resize(2ull * r.J.cap_files * r.max_klen + 1);
-      const uint32_t nf = std::min<uint32_t>(hc[i].n_files, r.J.cap_files);
-      memcpy(r.files.data(), q, sizeof(FileOut) * nf);
-      q += (sizeof(FileOut) * r.J.cap_files + 15) & ~size_t(15);
-      memcpy(r.koff.data(), q, 8 * (2ull * nf + 1));
-      q += (8 * (2ull * r.J.cap_files + 1) + 15) & ~size_t(15);
-      // keys in fixed slots of max_klen bytes, their lengths in koff
-      const uint64_t kb = 2ull * nf * r.max_klen;
-      memcpy(r.j->key_bytes.data(), q, std::min<uint64_t>(kb, r.j->key_bytes.size()));
+      size_t klen, keys;
+      res_at(i, &klen, &keys);
+      const uint32_t nf = hc[i].error ? 0 : std::min<uint32_t>(hc[i].n_files, r.J.cap_files);
+      const FileOut* hf = reinterpret_cast<const FileOut*>(pin2 + p_res + res_off[i]);
+      r.files.assign(hf, hf + nf);
+      r.klen.resize(2ull * nf);
+      for (uint32_t x = 0; x < 2 * nf; x++)
+        r.klen[x] = slot.pin_dev ? reinterpret_cast<const uint32_t*>(pin2 + p_res + klen)[x]
+                                 : (uint32_t)reinterpret_cast<const uint64_t*>(pin2 + p_res + klen)[x];
+      // keys in fixed slots of max_klen bytes
+      r.j->key_bytes.resize(2ull * nf * r.max_klen + 1);
+      for (uint32_t x = 0; x < 2 * nf; x++)
+        memcpy(r.j->key_bytes.data() + (uint64_t)x * r.max_klen,
+               pin2 + p_res + keys + (uint64_t)x * r.max_klen,
+               std::min<uint32_t>(r.klen[x], r.max_klen));
     }
     std::vector<lc_job*> retry;  // single-pass jobs whose key arena was too small
     // downloads of this batch after the previous batch's (CopyLane)
@@ -1354,9 +1371,9 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
         j->file_size[f] = F.size;
         j->file_entries[f] = F.end_kept - F.first_kept;
         j->small_off[f] = 2ull * f * r.max_klen;
-        j->small_len[f] = (uint32_t)r.koff[2 * f];
+        j->small_len[f] = r.klen[2 * f];
         j->large_off[f] = (2ull * f + 1) * r.max_klen;
-        j->large_len[f] = (uint32_t)r.koff[2 * f + 1];
+        j->large_len[f] = r.klen[2 * f + 1];
       }
       j->bytes_out = nbytes;
       j->entries_out = hc[i].n_kept;

@@ -251,6 +251,10 @@ struct JobDev {
                              // of fkey_stride bytes each
   uint64_t* fkoff;           // their lengths (2 * cap_files)
   uint32_t fkey_stride;      // longest internal key the job can hold
+  Counters* res_ctr;         // mapped pinned host memory the job's results go to (k_results):
+  FileOut* res_files;        //   counters; then, n_files of each, files,
+  uint32_t* res_klen;        //   lengths of their smallest and largest keys (pairs),
+  uint8_t* res_keys;         //   the keys in slots of fkey_stride bytes.  Null: no such memory
   const uint64_t* src_koffs; // flush encoder: key offsets (n + 1)
   const uint64_t* src_voffs; // flush encoder: value offsets (n + 1)
   uint64_t* scan_scratch;    // tile sums of the prefix sums

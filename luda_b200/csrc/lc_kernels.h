@@ -127,6 +127,8 @@ void launch_emit_decoded(const Batch& bt, cudaStream_t st);
 void launch_encode_index(const Batch& bt, cudaStream_t st);
 // metaindex, footer, filter tails and the trailers of filter/meta/index
 void launch_encode_meta(const Batch& bt, cudaStream_t st);
+// counters and per-file results to the jobs' host buffers (JobDev::res_*)
+void launch_results(const Batch& bt, cudaStream_t st);
 
 // grid x for a kernel over up to `items` items per job, `per` items per CTA,
 // capped at `cap` CTAs (the kernel loops over the rest)
