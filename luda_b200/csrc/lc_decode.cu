@@ -81,6 +81,7 @@ __device__ __forceinline__ const uint8_t* entry_header(const uint8_t* p, const u
 }
 
 __global__ void k_table_index_count(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   const uint32_t t = blockIdx.x;
   if (t >= J.n_tables) return;
@@ -148,6 +149,7 @@ __global__ void k_table_index_count(const JobDev* __restrict__ jobs) {
 constexpr uint32_t kIdxSplit = 16;
 
 __global__ void k_table_index_entries(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   const uint32_t t = blockIdx.x / kIdxSplit, part = blockIdx.x % kIdxSplit;
   if (t >= J.n_tables) return;
@@ -404,6 +406,7 @@ __device__ void block_count_one(const JobDev& J, uint64_t b, uint32_t lane, cons
 }
 
 __global__ void __launch_bounds__(kDecWarps * 32) k_block_count(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   extern __shared__ __align__(16) uint8_t dec_smem[];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -438,6 +441,7 @@ __global__ void __launch_bounds__(kDecWarps * 32) k_block_count(const JobDev* __
 // holds the entry count of its run): one thread per block.  The run byte
 // ranges are checked here; the entries themselves when they are decoded.
 __global__ void k_block_restarts(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // after a footer or index error some handles are unset
   const uint64_t nblk = min(J.ctr->n_blocks_in, J.cap_blocks_in);
@@ -483,6 +487,7 @@ __global__ void k_block_restarts(const JobDev* __restrict__ jobs) {
 // with one byte run per lane (a table lookup and a byte load per byte), 12.2
 // us so.
 __global__ void __launch_bounds__(256) k_verify_blocks(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_h5[kCrcH5Words];
   __shared__ uint32_t s_xinv[kCrcXinvSmem];
@@ -537,6 +542,7 @@ __global__ void __launch_bounds__(256) k_verify_blocks(const JobDev* __restrict_
 // Entries of merge child r start at the first block of its first table: one
 // thread per table, the first table of each run writes the run's start.
 __global__ void k_run_bounds(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   const bool bad = J.ctr->error != 0;  // the job fails; keep every read in bounds
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < J.n_tables;
@@ -586,6 +592,7 @@ __device__ __forceinline__ uint4 dec_record(uint32_t src, uint32_t sh, uint32_t 
 }
 
 __global__ void __launch_bounds__(256) k_decode_walk(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   __shared__ JobDev s_job;
   copy_job(jobs + blockIdx.y, &s_job);
   __syncthreads();
@@ -706,6 +713,7 @@ __global__ void __launch_bounds__(256) k_decode_walk(const JobDev* __restrict__ 
 
 // The arena holds every key (k_decode_keys checks it before writing any).
 __global__ void k_decode_fit(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (threadIdx.x == 0 && !J.ctr->error && J.ctr->key_total > J.cap_key_bytes)
     set_error(J.ctr, J.reserve_keys ? kErrRetryExact : kErrArenaOverflow, 5);
@@ -742,6 +750,7 @@ __device__ __forceinline__ uint64_t dec_unit_start(const JobDev& J, uint64_t e, 
 }
 
 __global__ void __launch_bounds__(256) k_decode_keys(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   __shared__ JobDev s_job;
   copy_job(jobs + blockIdx.y, &s_job);
   __syncthreads();
@@ -877,6 +886,7 @@ __global__ void __launch_bounds__(256) k_decode_keys(const JobDev* __restrict__ 
 }
 
 __global__ void k_entries_from_offsets(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   const uint64_t n = J.cap_entries;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -902,10 +912,10 @@ __global__ void k_entries_from_offsets(const JobDev* __restrict__ jobs) {
 }  // namespace
 
 void launch_table_index_count(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_table_index_count<<<dim3(bt.max_tables, bt.B), 1024, 0, st>>>(bt.d);
+  launch(k_table_index_count, dim3(bt.max_tables, bt.B), 1024, 0, st, bt.d);
 }
 void launch_table_index_entries(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_table_index_entries<<<dim3(bt.max_tables * kIdxSplit, bt.B), 1024, 0, st>>>(bt.d);
+  launch(k_table_index_entries, dim3(bt.max_tables * kIdxSplit, bt.B), 1024, 0, st, bt.d);
 }
 
 static void dec_smem_attr(const void* fn) {
@@ -923,36 +933,30 @@ static unsigned dec_ctas(const Batch& bt) {
 void decode_kernel_attributes() { dec_smem_attr((const void*)k_block_count); }
 
 void launch_block_count(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_block_count<<<dim3(dec_ctas(bt), bt.B), kDecWarps * 32,
-                                 kDecWarps * sizeof(DecWarpSmem), st>>>(bt.d);
+  launch(k_block_count, dim3(dec_ctas(bt), bt.B), kDecWarps * 32, kDecWarps * sizeof(DecWarpSmem), st, bt.d);
 }
 void launch_block_restarts(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_block_restarts<<<dim3(grid_x(bt.max_blocks_in, 256, 148 * 8), bt.B), 256, 0, st>>>(
-      bt.d);
+  launch(k_block_restarts, dim3(grid_x(bt.max_blocks_in, 256, 148 * 8), bt.B), 256, 0, st, bt.d);
 }
 void launch_verify_blocks(const Batch& bt, cudaStream_t st) {
   if (!bt.any_verify) return;
-  note_launch(), k_verify_blocks<<<dim3(grid_x(bt.max_blocks_in, 8, 148 * 4), bt.B), 256, 0, st>>>(
-      bt.d);
+  launch(k_verify_blocks, dim3(grid_x(bt.max_blocks_in, 8, 148 * 4), bt.B), 256, 0, st, bt.d);
 }
 void launch_run_bounds(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_run_bounds<<<dim3((bt.max_tables + 127) / 128 + 1, bt.B), 128, 0, st>>>(bt.d);
+  launch(k_run_bounds, dim3((bt.max_tables + 127) / 128 + 1, bt.B), 128, 0, st, bt.d);
 }
 void launch_block_decode(const Batch& bt, cudaStream_t st) {
   // pass 1: one warp per group of 8 or 32 blocks; pass 2: one warp per unit
   // of kDecUnit entries; 8 warps per CTA, at most 8 CTAs per SM over the batch
   const uint64_t cap = std::max<uint64_t>(1, bt.ctas_per_job ? bt.ctas_per_job : 148 * 8 / bt.B);
   const uint64_t walk = (bt.max_blocks_in + 63) / 64, keys = (bt.max_entries + 8 * kDecUnit - 1) / (8 * kDecUnit);
-  note_launch(), k_decode_walk<<<dim3((unsigned)std::max<uint64_t>(1, std::min(walk, cap)), bt.B), 256, 0,
-                                 st>>>(bt.d);
+  launch(k_decode_walk, dim3((unsigned)std::max<uint64_t>(1, std::min(walk, cap)), bt.B), 256, 0, st, bt.d);
   scan_batch(kScanDecKlen, bt, bt.max_entries, st);
-  note_launch(), k_decode_fit<<<dim3(1, bt.B), 32, 0, st>>>(bt.d);
-  note_launch(), k_decode_keys<<<dim3((unsigned)std::max<uint64_t>(1, std::min(keys, cap)), bt.B), 256, 0,
-                                 st>>>(bt.d);
+  launch(k_decode_fit, dim3(1, bt.B), 32, 0, st, bt.d);
+  launch(k_decode_keys, dim3((unsigned)std::max<uint64_t>(1, std::min(keys, cap)), bt.B), 256, 0, st, bt.d);
 }
 void launch_entries_from_offsets(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_entries_from_offsets<<<dim3(grid_x(bt.max_entries, 256, 148 * 8), bt.B), 256, 0,
-                                          st>>>(bt.d);
+  launch(k_entries_from_offsets, dim3(grid_x(bt.max_entries, 256, 148 * 8), bt.B), 256, 0, st, bt.d);
 }
 
 }  // namespace lc

@@ -21,6 +21,13 @@ constexpr uint32_t kFilterBaseLg = 11;                             // table/filt
 constexpr uint32_t kTrailer = 5;                                   // type byte + crc
 constexpr uint32_t kFooter = 48;                                   // table/format.h:61
 
+// First statement of every kernel launched with launch(): waits until the
+// kernel before it in the stream has completed (its writes are visible), then
+// lets the one after it be set up while this one runs.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t ld_le32(const uint8_t* p) {
   return (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
 }

@@ -75,6 +75,7 @@ __device__ __forceinline__ const uint8_t* kept_key(const JobDev& J, uint64_t k, 
 // (k_b), the shared prefix with the previous survivor, survivor byte totals;
 // also clears the block-start flags (n + 1 of them) for the chain.
 __global__ void k_sizes(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t n = J.ctr->n_kept;
@@ -157,6 +158,7 @@ __device__ __forceinline__ uint64_t next_of(const JobDev& J, uint64_t s, uint64_
 }
 
 __global__ void k_next(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t n = J.ctr->n_kept;
@@ -197,6 +199,7 @@ __device__ __forceinline__ uint64_t chain_sub_walk(const uint32_t* s_next, uint6
 }
 
 __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
@@ -246,6 +249,7 @@ __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
 // tables (one thread per entry point).  Only when the chunk tables do not fit
 // the resolving CTA's shared memory.
 __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t n = J.ctr->n_kept;
@@ -271,6 +275,7 @@ __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
 // fit), then one thread per group walks its chunks from the group's entry
 // point.
 __global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
@@ -339,6 +344,7 @@ __global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
 // (recomputed as k_chain_tables does) and every sub-chunk is walked by its
 // own thread.
 __global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
@@ -398,6 +404,7 @@ __global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
 // Output blocks: first survivor of each block, and the block's size (the
 // block that starts at k ends where the chain says the next one starts).
 __global__ void k_block_list(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t n = J.ctr->n_kept;
@@ -427,6 +434,7 @@ __global__ void k_block_list(const JobDev* __restrict__ jobs) {
 
 // t_blocks[i] = output block that starts at grandparent cut i (ascending).
 __global__ void k_forced_blocks(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -436,6 +444,7 @@ __global__ void k_forced_blocks(const JobDev* __restrict__ jobs) {
 }
 
 __global__ void k_file_next(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t nb = J.ctr->n_blocks_out;
@@ -479,6 +488,7 @@ __global__ void k_file_next(const JobDev* __restrict__ jobs) {
 constexpr uint32_t kFileTile = 4096;
 constexpr uint32_t kFileThreads = kFileTile / 4;
 __global__ void k_files(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
@@ -538,6 +548,7 @@ __device__ __forceinline__ uint32_t file_of_block(const JobDev& J, uint64_t b) {
 __device__ void block_layout_one(const JobDev& J, uint64_t b);
 
 __global__ void k_block_layout(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t nb = J.ctr->n_blocks_out;
@@ -611,6 +622,7 @@ __device__ void block_layout_one(const JobDev& J, uint64_t b) {
 }
 
 __global__ void k_file_layout(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
@@ -1091,6 +1103,7 @@ __device__ __forceinline__ void enc_drain(uint32_t lane) {
 }
 
 __global__ void __launch_bounds__(kEncWarps * 32, 2) k_encode_blocks(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   __shared__ uint32_t s_h8[kCrcH8Words];
   __shared__ uint32_t s_xinv[kCrcXinvSmem];
   __shared__ uint32_t s_tab8[256];
@@ -1197,6 +1210,7 @@ __global__ void __launch_bounds__(kEncWarps * 32, 2) k_encode_blocks(const JobDe
 // value places were written by k_encode_blocks.  One warp per 32 survivors,
 // lanes over the group's key bytes.
 __global__ void k_emit_decoded(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error || !J.dec_keys) return;
   const uint64_t n = J.ctr->n_kept;
@@ -1324,6 +1338,7 @@ __device__ __forceinline__ void filter_group_thread(const JobDev& J, uint64_t b,
 // Filter groups (at their first blocks): groups of a few keys one per thread,
 // larger ones one per warp (bits in the warp's shared memory, or in place).
 __global__ void k_encode_filters(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_filter[8][kFilterSmem / 4];  // blockDim 256: 8 warps
   const uint32_t lane = threadIdx.x & 31;
@@ -1383,6 +1398,7 @@ __device__ __forceinline__ void encode_index_entry(const JobDev& J, uint64_t b) 
 }
 
 __global__ void k_encode_index(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;
   const uint64_t nb = J.ctr->n_blocks_out;
@@ -1395,6 +1411,7 @@ __global__ void k_encode_index(const JobDev* __restrict__ jobs) {
 // 0), then the trailers of the filter, metaindex and index blocks, each a
 // CRC32C over the whole CTA: one CTA per output file.
 __global__ void __launch_bounds__(256) k_encode_meta(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_skip;
   if (threadIdx.x == 0) s_skip = J.ctr->error || blockIdx.x >= J.ctr->n_files;
@@ -1476,6 +1493,7 @@ __device__ __forceinline__ void meta_region(const FileOut& F, uint32_t r, uint64
 }
 
 __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_h5[kCrcH5Words];
   __shared__ uint32_t s_xinv[kCrcXinvSmem];
@@ -1549,6 +1567,7 @@ __device__ __forceinline__ void put_trailer(uint8_t* p, uint32_t raw) {
 // The trailers of the filter, metaindex and index blocks, and of the data
 // blocks that were written in windows.
 __global__ void k_meta_trailers(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;
   const uint32_t nf = J.ctr->n_files, nw = min(J.ctr->n_wide, J.cap_wide);
@@ -1576,6 +1595,7 @@ __global__ void k_meta_trailers(const JobDev* __restrict__ jobs) {
 // link 69 us and the host's reading of it 1.3 ms for a batch of 32 jobs.  One
 // warp per file; the last kernel of a batch.
 __global__ void __launch_bounds__(256) k_results(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (!J.res_ctr) return;
   const uint32_t lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1604,41 +1624,35 @@ inline unsigned per_job(const Batch& bt, unsigned total) {
 }  // namespace
 
 void launch_sizes(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_sizes<<<dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0,
-                           st>>>(bt.d);
+  launch(k_sizes, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_next(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_next<<<dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0,
-                          st>>>(bt.d);
+  launch(k_next, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_chain(const Batch& bt, cudaStream_t st) {
   const uint64_t chunks = (bt.max_entries + bt.chunk - 1) / bt.chunk + 1;
   // next() values, sub-chunk exits (windows up to kChainSub) and entry points
   const size_t smem = ((size_t)bt.chunk + (bt.chunk / kChainSub) * (kChainSub + 1)) * sizeof(uint32_t);
   const unsigned g = (unsigned)std::min<uint64_t>(chunks, per_job(bt, 148 * 4));
-  note_launch(), k_chain_tables<<<dim3(g, bt.B), 256, smem, st>>>(bt.d);
+  launch(k_chain_tables, dim3(g, bt.B), 256, smem, st, bt.d);
   if (chunks > kChainGroup)
-    note_launch(), k_chain_groups<<<dim3(grid_x(chunks / kChainGroup * bt.chunk, 256, 148 * 4), bt.B),
-                                    256, 0, st>>>(bt.d);
-  note_launch(), k_chain_resolve<<<dim3(1, bt.B), 1024, (size_t)bt.chain_smem_words * 4, st>>>(bt.d);
-  note_launch(), k_chain_mark<<<dim3(g, bt.B), 128, smem, st>>>(bt.d);
+    launch(k_chain_groups, dim3(grid_x(chunks / kChainGroup * bt.chunk, 256, 148 * 4), bt.B), 256, 0, st, bt.d);
+  launch(k_chain_resolve, dim3(1, bt.B), 1024, (size_t)bt.chain_smem_words * 4, st, bt.d);
+  launch(k_chain_mark, dim3(g, bt.B), 128, smem, st, bt.d);
 }
 void launch_block_list(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_block_list<<<dim3(grid_x(bt.max_entries + 1, 256, per_job(bt, 148 * 8)), bt.B), 256,
-                                0, st>>>(bt.d);
+  launch(k_block_list, dim3(grid_x(bt.max_entries + 1, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_files(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_forced_blocks<<<dim3((bt.max_cap_triggers + 255) / 256, bt.B), 256, 0, st>>>(bt.d);
-  note_launch(), k_file_next<<<dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0,
-                               st>>>(bt.d);
-  note_launch(), k_files<<<dim3(1, bt.B), kFileThreads, 0, st>>>(bt.d);
+  launch(k_forced_blocks, dim3((bt.max_cap_triggers + 255) / 256, bt.B), 256, 0, st, bt.d);
+  launch(k_file_next, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_files, dim3(1, bt.B), kFileThreads, 0, st, bt.d);
 }
 void launch_block_layout(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_block_layout<<<dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256,
-                                  0, st>>>(bt.d);
+  launch(k_block_layout, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_file_layout(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_file_layout<<<dim3(1, bt.B), 256, 0, st>>>(bt.d);
+  launch(k_file_layout, dim3(1, bt.B), 256, 0, st, bt.d);
 }
 void encode_kernel_attributes() {
   cudaFuncSetAttribute(k_encode_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEncSmem);
@@ -1648,36 +1662,28 @@ void launch_encode_blocks(const Batch& bt, cudaStream_t st) {
   // grid-stride over the device-side counts of blocks and windows: 3 CTAs per
   // SM x 4 waves, shared out among the jobs (a job of few entries may have as
   // many windows as its output bytes allow)
-  note_launch(), k_encode_blocks<<<dim3(grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide),
-                                               kEncWarps, per_job(bt, 148 * 2 * 4)),
-                                        bt.B), kEncWarps * 32, kEncSmem, st>>>(bt.d);
+  launch(k_encode_blocks, dim3(grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide), kEncWarps, per_job(bt, 148 * 2 * 4)), bt.B), kEncWarps * 32, kEncSmem, st, bt.d);
 }
 void launch_emit_decoded(const Batch& bt, cudaStream_t st) {
   if (!bt.any_keep_decoded) return;
   scan_batch(kScanDecKey, bt, bt.max_entries, st);
-  note_launch(), k_emit_decoded<<<dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256,
-                                  0, st>>>(bt.d);
+  launch(k_emit_decoded, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_encode_filters(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_encode_filters<<<dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B),
-                                    256, 0, st>>>(bt.d);
+  launch(k_encode_filters, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_encode_index(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_encode_index<<<dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 16)), bt.B), 256,
-                                  0, st>>>(bt.d);
+  launch(k_encode_index, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 16)), bt.B), 256, 0, st, bt.d);
 }
 void launch_encode_meta(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_encode_meta<<<dim3(bt.max_cap_files, bt.B), 256, 0, st>>>(bt.d);
-  note_launch(), k_meta_crc<<<dim3(grid_x(bt.max_entries, 4096, per_job(bt, 148 * 4)), bt.B), 256, 0,
-                              st>>>(bt.d);
+  launch(k_encode_meta, dim3(bt.max_cap_files, bt.B), 256, 0, st, bt.d);
+  launch(k_meta_crc, dim3(grid_x(bt.max_entries, 4096, per_job(bt, 148 * 4)), bt.B), 256, 0, st, bt.d);
   // (the wide blocks are at most the entries)
-  note_launch(), k_meta_trailers<<<dim3(std::max((3 * bt.max_cap_files + 255) / 256,
-                                                 grid_x(bt.max_entries, 2048, per_job(bt, 148 * 2))),
-                                        bt.B), 256, 0, st>>>(bt.d);
+  launch(k_meta_trailers, dim3(std::max((3 * bt.max_cap_files + 255) / 256, grid_x(bt.max_entries, 2048, per_job(bt, 148 * 2))), bt.B), 256, 0, st, bt.d);
 }
 
 void launch_results(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_results<<<dim3(grid_x(bt.max_cap_files, 8, 16), bt.B), 256, 0, st>>>(bt.d);
+  launch(k_results, dim3(grid_x(bt.max_cap_files, 8, 16), bt.B), 256, 0, st, bt.d);
 }
 
 }  // namespace lc

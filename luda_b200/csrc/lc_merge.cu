@@ -39,6 +39,7 @@ namespace {
 // Then, per grandparent, its prefix after those bytes, or where it sorts
 // against every entry when it does not share them.  One CTA per job.
 __global__ void k_key_skip(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed, s_skip;
   if (threadIdx.x == 0) {
@@ -106,6 +107,7 @@ __device__ __forceinline__ bool run_first(const JobDev& J, uint64_t e) {
 // out of order fails the job here (kErrUnsorted) rather than reaching the
 // merge path, whose cuts assume sorted children.
 __global__ void k_prefix(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;
   const uint32_t L = J.ctr->key_skip;
@@ -141,6 +143,7 @@ __global__ void k_prefix(const JobDev* __restrict__ jobs) {
 
 // A single merge child (no round): the merged order is the input order.
 __global__ void k_merge_single(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t n = J.ctr->n_entries_in;
@@ -220,6 +223,7 @@ __device__ __forceinline__ uint32_t src_id(const MergeRound& m, uint64_t i) {
 // tile.
 __global__ void k_merge_partition(const JobDev* __restrict__ jobs, uint32_t r, uint32_t rounds,
                                   uint32_t tile) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const MergeRound m = merge_round(J, r, rounds);
@@ -246,6 +250,7 @@ __global__ void k_merge_partition(const JobDev* __restrict__ jobs, uint32_t r, u
 // (two ascending streams).  Only equal prefixes read key bytes.
 __global__ void __launch_bounds__(1024) k_merge_tile(const JobDev* __restrict__ jobs, uint32_t r,
                                                      uint32_t rounds, uint32_t items) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
@@ -383,6 +388,7 @@ __device__ __forceinline__ void drop_one(const JobDev& J, const uint32_t* __rest
 }
 
 __global__ void k_drop(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t n = J.ctr->n_entries_in;
@@ -394,6 +400,7 @@ __global__ void k_drop(const JobDev* __restrict__ jobs) {
 // gp_first[g] = first merged position whose grandparent count reaches g
 // (gp_idx is non-decreasing along the merge order).
 __global__ void k_gp_first(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   uint32_t* gp_first = J.gp_first;
@@ -415,6 +422,7 @@ __global__ void k_gp_first(const JobDev* __restrict__ jobs) {
 // prefix[g] - prefix[gp_idx[t]] > limit.  Few cuts; one thread walks them
 // over shared-memory copies of the prefix and first-position arrays.
 __global__ void k_triggers(const JobDev* __restrict__ jobs, bool in_smem) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
@@ -464,6 +472,7 @@ __global__ void k_triggers(const JobDev* __restrict__ jobs, bool in_smem) {
 }
 
 __global__ void k_kept_compact(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint32_t* __restrict__ ids = J.m_ids;
@@ -483,6 +492,7 @@ __global__ void k_kept_compact(const JobDev* __restrict__ jobs) {
 }
 
 __global__ void k_forced(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -522,14 +532,13 @@ uint64_t merge_tile_capacity(uint64_t entries, uint32_t runs) {
 }
 
 void launch_key_skip(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_key_skip<<<dim3(1, bt.B), 256, 0, st>>>(bt.d);
-  note_launch(), k_prefix<<<dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st>>>(bt.d);
+  launch(k_key_skip, dim3(1, bt.B), 256, 0, st, bt.d);
+  launch(k_prefix, dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st, bt.d);
 }
 
 void launch_merge(const Batch& bt, cudaStream_t st) {
   if (bt.merge_rounds == 0) {
-    note_launch(), k_merge_single<<<dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st>>>(
-        bt.d);
+    launch(k_merge_single, dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st, bt.d);
     return;
   }
   const uint32_t items = merge_items_of(bt);
@@ -537,29 +546,26 @@ void launch_merge(const Batch& bt, cudaStream_t st) {
   const uint32_t tile = threads * items;
   const uint64_t tiles = bt.max_entries / tile + bt.max_runs + 1;
   for (uint32_t r = 0; r < bt.merge_rounds; r++) {
-    note_launch(), k_merge_partition<<<dim3(grid_x(tiles, 128, 148 * 16), bt.B), 128, 0, st>>>(
-        bt.d, r, bt.merge_rounds, tile);
-    note_launch(), k_merge_tile<<<dim3(flat_ctas(bt, tiles, 1), bt.B), threads,
-                                  kMergeSmemPerPos * (size_t)tile, st>>>(bt.d, r, bt.merge_rounds,
-                                                                         items);
+    launch(k_merge_partition, dim3(grid_x(tiles, 128, 148 * 16), bt.B), 128, 0, st, bt.d, r, bt.merge_rounds, tile);
+    launch(k_merge_tile, dim3(flat_ctas(bt, tiles, 1), bt.B), threads, kMergeSmemPerPos * (size_t)tile, st, bt.d, r, bt.merge_rounds, items);
   }
 }
 
 void launch_drop(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_drop<<<dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st>>>(bt.d);
+  launch(k_drop, dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st, bt.d);
 }
 
 void launch_triggers(const Batch& bt, cudaStream_t st) {
   if (bt.max_gp)
-    note_launch(), k_gp_first<<<dim3((bt.max_gp + 1 + 255) / 256, bt.B), 256, 0, st>>>(bt.d);
+    launch(k_gp_first, dim3((bt.max_gp + 1 + 255) / 256, bt.B), 256, 0, st, bt.d);
   const size_t smem = (size_t)(bt.max_gp + 1) * 12;
   const bool in_smem = smem + 64 <= 48 * 1024;  // with the kernel's static shared memory
-  note_launch(), k_triggers<<<dim3(1, bt.B), 256, in_smem ? smem : 0, st>>>(bt.d, in_smem);
+  launch(k_triggers, dim3(1, bt.B), 256, in_smem ? smem : 0, st, bt.d, in_smem);
 }
 
 void launch_kept_compact(const Batch& bt, cudaStream_t st) {
-  note_launch(), k_kept_compact<<<dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st>>>(bt.d);
-  note_launch(), k_forced<<<dim3((bt.max_cap_triggers + 255) / 256 + 1, bt.B), 256, 0, st>>>(bt.d);
+  launch(k_kept_compact, dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st, bt.d);
+  launch(k_forced, dim3((bt.max_cap_triggers + 255) / 256 + 1, bt.B), 256, 0, st, bt.d);
 }
 
 }  // namespace lc

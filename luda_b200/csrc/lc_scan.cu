@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <stdint.h>
 
+#include "lc_device.cuh"
 #include "lc_kernels.h"
 
 namespace lc {
@@ -176,6 +177,7 @@ __device__ __forceinline__ T block_excl_scan(T v, T* total) {
 
 template <int S>
 __global__ void k_tile_reduce(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   using SP = ScanOf<S>;
   using TO = typename SP::TO;
   const JobDev& J = jobs[blockIdx.y];
@@ -211,6 +213,7 @@ __device__ __forceinline__ T block_sum(const T* a, uint64_t lo, uint64_t hi) {
 
 template <int S>
 __global__ void k_tile_scan(const JobDev* __restrict__ jobs) {
+  pdl_begin();
   using SP = ScanOf<S>;
   using TO = typename SP::TO;
   const JobDev& J = jobs[blockIdx.y];
@@ -262,9 +265,8 @@ void scan_sel(const Batch& bt, uint64_t n_cap, cudaStream_t st) {
   // one tile (n + 1 <= kTile for every job of the batch): no tile sums to
   // add, so the scan pass alone does it
   const bool one_tile = n_cap + 1 <= kTile;
-  note_launch(one_tile ? 1 : 2);
-  if (!one_tile) k_tile_reduce<S><<<dim3(tiles, bt.B), kScanThreads, 0, st>>>(bt.d);
-  k_tile_scan<S><<<dim3(tiles, bt.B), kScanThreads, 0, st>>>(bt.d);
+  if (!one_tile) launch(k_tile_reduce<S>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
+  launch(k_tile_scan<S>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
 }
 
 }  // namespace
@@ -297,6 +299,7 @@ namespace {
 // few-KB cudaMemcpyAsync waited behind megabytes of them and held up its
 // job's next kernels.  16-byte words, then the last bytes.
 __global__ void k_xfer(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, uint64_t n) {
+  pdl_begin();
   const uint64_t n16 = n / 16;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -312,8 +315,7 @@ bool launch_xfer(void* dst, const void* src, uint64_t n, cudaStream_t st) {
   if (!n) return true;
   const uint64_t words = n / 16 + 1;
   const unsigned grid = (unsigned)std::min<uint64_t>((words + 255) / 256, 148);
-  note_launch(1);
-  k_xfer<<<grid, 256, 0, st>>>((uint8_t*)dst, (const uint8_t*)src, n);
+  launch(k_xfer, dim3(grid), 256, 0, st, (uint8_t*)dst, (const uint8_t*)src, n);
   return true;
 }
 
