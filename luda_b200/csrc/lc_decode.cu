@@ -559,7 +559,7 @@ __global__ void k_run_bounds(const JobDev* __restrict__ jobs) {
 // Decode of the data blocks into the entry arrays, in two passes.
 //
 // Pass 1 (k_decode_walk): one warp per group of dec_group consecutive data
-// blocks (32, or 8 for blocks of many entries).  The group's restart runs,
+// blocks (as many as have 32 restart runs, at most 32).  The group's restart runs,
 // one lane per run in rounds of 32, walk their entry headers straight from
 // global memory (the lines a run's headers lie in are read once, through L1)
 // with the checks of the counting walk, and write one 16-byte record per
@@ -571,7 +571,7 @@ __global__ void k_run_bounds(const JobDev* __restrict__ jobs) {
 // A scan of the key lengths gives every key its place in the arena (keys in
 // entry order).
 //
-// Pass 2 (k_decode_keys): one warp per unit of about kDecUnit entries, cut
+// Pass 2 (k_decode_keys): one warp per unit of about dec_unit entries, cut
 // at entries without a shared prefix (every restart has none), in rounds of
 // 32, one lane per entry: each lane copies its key delta into the warp's key
 // buffer at the key's place; the shared prefixes then follow in entry order
@@ -581,7 +581,6 @@ __global__ void k_run_bounds(const JobDev* __restrict__ jobs) {
 // a round whose keys do not fit the buffer is built in the arena directly.
 constexpr uint32_t kDecGroupMax = 32;   // data blocks per warp in pass 1
 constexpr uint32_t kDecRunSlice = 16;   // pseudo-block entries per lane
-constexpr uint32_t kDecUnit = 256;      // entries per warp in pass 2
 constexpr uint32_t kDecPseudo = 0xffffu;  // shared length of a pseudo entry's record
 
 // Record of entry e: x key delta offset in `in` (a pseudo entry: its block),
@@ -591,9 +590,13 @@ __device__ __forceinline__ uint4 dec_record(uint32_t src, uint32_t sh, uint32_t 
   return make_uint4(src, sh | (kl << 16), vl, voff);
 }
 
-__global__ void __launch_bounds__(256) k_decode_walk(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* __restrict__ jobs) {
   pdl_begin();
   __shared__ JobDev s_job;
+  {  // the surplus CTAs of a small job leave at once
+    const JobDev& G = jobs[blockIdx.y];
+    if (blockIdx.x * 8ull * G.dec_group >= G.ctr->n_blocks_in) return;
+  }
   copy_job(jobs + blockIdx.y, &s_job);
   __syncthreads();
   const JobDev& J = s_job;
@@ -749,9 +752,13 @@ __device__ __forceinline__ uint64_t dec_unit_start(const JobDev& J, uint64_t e, 
   return n;
 }
 
-__global__ void __launch_bounds__(256) k_decode_keys(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict__ jobs) {
   pdl_begin();
   __shared__ JobDev s_job;
+  {
+    const JobDev& G = jobs[blockIdx.y];
+    if (blockIdx.x * 8ull * G.dec_unit >= G.ctr->n_entries_in) return;
+  }
   copy_job(jobs + blockIdx.y, &s_job);
   __syncthreads();
   const JobDev& J = s_job;
@@ -760,10 +767,10 @@ __global__ void __launch_bounds__(256) k_decode_keys(const JobDev* __restrict__ 
   DecKeysSmem& W = s_w[warp];
   if (J.ctr->error) return;
   const uint64_t n = J.ctr->n_entries_in;
-  const uint64_t nunits = (n + kDecUnit - 1) / kDecUnit;
+  const uint64_t unit = J.dec_unit, nunits = (n + unit - 1) / unit;
   for (uint64_t u = (uint64_t)blockIdx.x * 8 + warp; u < nunits; u += (uint64_t)gridDim.x * 8) {
-    const uint64_t e0 = u == 0 ? 0 : dec_unit_start(J, u * kDecUnit, n, lane);
-    const uint64_t e1 = dec_unit_start(J, (u + 1) * kDecUnit, n, lane);
+    const uint64_t e0 = u == 0 ? 0 : dec_unit_start(J, u * unit, n, lane);
+    const uint64_t e1 = dec_unit_start(J, (u + 1) * unit, n, lane);
     bool last_staged = true;  // the previous key is in W.last (not needed at a unit start)
     uint64_t last_at = 0;     // else its arena offset
     for (uint64_t r0 = e0; r0 < e1; r0 += 32) {
@@ -915,7 +922,7 @@ void launch_table_index_count(const Batch& bt, cudaStream_t st) {
   launch(k_table_index_count, dim3(bt.max_tables, bt.B), 1024, 0, st, bt.d);
 }
 void launch_table_index_entries(const Batch& bt, cudaStream_t st) {
-  launch(k_table_index_entries, dim3(bt.max_tables * kIdxSplit, bt.B), 1024, 0, st, bt.d);
+  launch(k_table_index_entries, dim3(bt.max_tables * kIdxSplit, bt.B), 256, 0, st, bt.d);
 }
 
 static void dec_smem_attr(const void* fn) {
@@ -926,8 +933,7 @@ static void dec_smem_attr(const void* fn) {
 static unsigned dec_ctas(const Batch& bt) {
   // grid-stride over the device-side block count: 3 CTAs per SM x 8 waves in
   // total, shared out among the jobs of the batch
-  const uint64_t cap = std::max<uint64_t>(1, bt.ctas_per_job ? bt.ctas_per_job : 148 * 3 * 8 / bt.B);
-  return grid_x(bt.max_blocks_in, kDecWarps, cap);
+  return grid_x(bt.max_blocks_in, kDecWarps, bt.per_job(148 * 3 * 8));
 }
 
 void decode_kernel_attributes() { dec_smem_attr((const void*)k_block_count); }
@@ -936,24 +942,23 @@ void launch_block_count(const Batch& bt, cudaStream_t st) {
   launch(k_block_count, dim3(dec_ctas(bt), bt.B), kDecWarps * 32, kDecWarps * sizeof(DecWarpSmem), st, bt.d);
 }
 void launch_block_restarts(const Batch& bt, cudaStream_t st) {
-  launch(k_block_restarts, dim3(grid_x(bt.max_blocks_in, 256, 148 * 8), bt.B), 256, 0, st, bt.d);
+  launch(k_block_restarts, dim3(grid_x(bt.max_blocks_in, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_verify_blocks(const Batch& bt, cudaStream_t st) {
   if (!bt.any_verify) return;
-  launch(k_verify_blocks, dim3(grid_x(bt.max_blocks_in, 8, 148 * 4), bt.B), 256, 0, st, bt.d);
+  launch(k_verify_blocks, dim3(grid_x(bt.max_blocks_in, 8, bt.per_job(148 * 4)), bt.B), 256, 0, st, bt.d);
 }
 void launch_run_bounds(const Batch& bt, cudaStream_t st) {
   launch(k_run_bounds, dim3((bt.max_tables + 127) / 128 + 1, bt.B), 128, 0, st, bt.d);
 }
 void launch_block_decode(const Batch& bt, cudaStream_t st) {
-  // pass 1: one warp per group of 8 or 32 blocks; pass 2: one warp per unit
-  // of kDecUnit entries; 8 warps per CTA, at most 8 CTAs per SM over the batch
-  const uint64_t cap = std::max<uint64_t>(1, bt.ctas_per_job ? bt.ctas_per_job : 148 * 8 / bt.B);
-  const uint64_t walk = (bt.max_blocks_in + 63) / 64, keys = (bt.max_entries + 8 * kDecUnit - 1) / (8 * kDecUnit);
-  launch(k_decode_walk, dim3((unsigned)std::max<uint64_t>(1, std::min(walk, cap)), bt.B), 256, 0, st, bt.d);
+  // pass 1: one warp per group of blocks; pass 2: one warp per unit of
+  // entries, as many CTAs as the SMs hold at once (5 and 4 each); 8 warps per
+  // CTA
+  launch(k_decode_walk, dim3(grid_x(bt.max_dec_groups, 8, bt.per_job(148 * 5)), bt.B), 256, 0, st, bt.d);
   scan_batch(kScanDecKlen, bt, bt.max_entries, st);
   launch(k_decode_fit, dim3(1, bt.B), 32, 0, st, bt.d);
-  launch(k_decode_keys, dim3((unsigned)std::max<uint64_t>(1, std::min(keys, cap)), bt.B), 256, 0, st, bt.d);
+  launch(k_decode_keys, dim3(grid_x(bt.max_dec_units, 8, bt.per_job(148 * 4)), bt.B), 256, 0, st, bt.d);
 }
 void launch_entries_from_offsets(const Batch& bt, cudaStream_t st) {
   launch(k_entries_from_offsets, dim3(grid_x(bt.max_entries, 256, 148 * 8), bt.B), 256, 0, st, bt.d);

@@ -74,7 +74,7 @@ __device__ __forceinline__ const uint8_t* kept_key(const JobDev& J, uint64_t k, 
 // Entry sizes as a restart entry (k_a) and as a prefix-compressed entry
 // (k_b), the shared prefix with the previous survivor, survivor byte totals;
 // also clears the block-start flags (n + 1 of them) for the chain.
-__global__ void k_sizes(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 8) k_sizes(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
@@ -157,7 +157,7 @@ __device__ __forceinline__ uint64_t next_of(const JobDev& J, uint64_t s, uint64_
   }
 }
 
-__global__ void k_next(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 6) k_next(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
@@ -547,7 +547,7 @@ __device__ __forceinline__ uint32_t file_of_block(const JobDev& J, uint64_t b) {
 
 __device__ void block_layout_one(const JobDev& J, uint64_t b);
 
-__global__ void k_block_layout(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 6) k_block_layout(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
@@ -1109,8 +1109,10 @@ __global__ void __launch_bounds__(kEncWarps * 32, 2) k_encode_blocks(const JobDe
   __shared__ uint32_t s_tab8[256];
   __shared__ JobDev s_job;  // the job's descriptor, read from here in every step
   extern __shared__ __align__(16) uint8_t enc_smem[];
-  copy_job(jobs + blockIdx.y, &s_job);
   const JobDev& G = jobs[blockIdx.y];
+  // the surplus CTAs of a small job leave before they load any table
+  if (G.ctr->error || blockIdx.x * kEncWarps >= max(G.ctr->n_blocks_out, (uint64_t)G.ctr->n_wide)) return;
+  copy_job(jobs + blockIdx.y, &s_job);
   for (uint32_t i = threadIdx.x; i < kCrcH8Words; i += blockDim.x) s_h8[i] = G.crc_h8[i];
   for (uint32_t i = threadIdx.x; i < kCrcXinvN; i += blockDim.x) s_xinv[xinv_slot(i)] = G.crc_xinv[i];
   for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab8[i] = G.crc_byte[i];
@@ -1118,7 +1120,6 @@ __global__ void __launch_bounds__(kEncWarps * 32, 2) k_encode_blocks(const JobDe
   const JobDev& J = s_job;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   EncWarp& W = reinterpret_cast<EncWarp*>(enc_smem)[warp];
-  if (J.ctr->error) return;
   const uint32_t nb = (uint32_t)J.ctr->n_blocks_out;  // block and survivor indices fit 32 bits
   const RestartDiv rd(J.restart_interval);
   const uint32_t stride = gridDim.x * kEncWarps;
@@ -1499,13 +1500,15 @@ __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ job
   __shared__ uint32_t s_xinv[kCrcXinvSmem];
   __shared__ uint32_t s_tab8[256];
   if (J.ctr->error) return;
+  const uint32_t ctas = (uint32_t)min((uint64_t)gridDim.x, J.ctr->n_kept / 4096 + 1);  // at work
+  if (blockIdx.x >= ctas) return;
   for (uint32_t i = threadIdx.x; i < kCrcH5Words; i += blockDim.x) s_h5[i] = J.crc_h5[i];
   for (uint32_t i = threadIdx.x; i < kCrcXinvN; i += blockDim.x) s_xinv[xinv_slot(i)] = J.crc_xinv[i];
   for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab8[i] = J.crc_byte[i];
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31, nf = J.ctr->n_files;
   // the pieces of all files are dealt to the job's warps in turn
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
+  const uint64_t warps = (uint64_t)ctas * (blockDim.x / 32);
   uint64_t turn = (uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   for (uint32_t f = 0; f < nf; f++) {
     const FileOut& F = J.files[f];
@@ -1617,23 +1620,19 @@ __global__ void __launch_bounds__(256) k_results(const JobDev* __restrict__ jobs
   }
 }
 
-inline unsigned per_job(const Batch& bt, unsigned total) {
-  return bt.ctas_per_job ? bt.ctas_per_job : std::max<unsigned>(1, total / bt.B);
-}
-
 }  // namespace
 
 void launch_sizes(const Batch& bt, cudaStream_t st) {
-  launch(k_sizes, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_sizes, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_next(const Batch& bt, cudaStream_t st) {
-  launch(k_next, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_next, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_chain(const Batch& bt, cudaStream_t st) {
   const uint64_t chunks = (bt.max_entries + bt.chunk - 1) / bt.chunk + 1;
   // next() values, sub-chunk exits (windows up to kChainSub) and entry points
   const size_t smem = ((size_t)bt.chunk + (bt.chunk / kChainSub) * (kChainSub + 1)) * sizeof(uint32_t);
-  const unsigned g = (unsigned)std::min<uint64_t>(chunks, per_job(bt, 148 * 4));
+  const unsigned g = (unsigned)std::min<uint64_t>(chunks, bt.per_job(148 * 4));
   launch(k_chain_tables, dim3(g, bt.B), 256, smem, st, bt.d);
   if (chunks > kChainGroup)
     launch(k_chain_groups, dim3(grid_x(chunks / kChainGroup * bt.chunk, 256, 148 * 4), bt.B), 256, 0, st, bt.d);
@@ -1641,15 +1640,15 @@ void launch_chain(const Batch& bt, cudaStream_t st) {
   launch(k_chain_mark, dim3(g, bt.B), 128, smem, st, bt.d);
 }
 void launch_block_list(const Batch& bt, cudaStream_t st) {
-  launch(k_block_list, dim3(grid_x(bt.max_entries + 1, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_block_list, dim3(grid_x(bt.max_entries + 1, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_files(const Batch& bt, cudaStream_t st) {
   launch(k_forced_blocks, dim3((bt.max_cap_triggers + 255) / 256, bt.B), 256, 0, st, bt.d);
-  launch(k_file_next, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_file_next, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
   launch(k_files, dim3(1, bt.B), kFileThreads, 0, st, bt.d);
 }
 void launch_block_layout(const Batch& bt, cudaStream_t st) {
-  launch(k_block_layout, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_block_layout, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_file_layout(const Batch& bt, cudaStream_t st) {
   launch(k_file_layout, dim3(1, bt.B), 256, 0, st, bt.d);
@@ -1662,24 +1661,24 @@ void launch_encode_blocks(const Batch& bt, cudaStream_t st) {
   // grid-stride over the device-side counts of blocks and windows: 3 CTAs per
   // SM x 4 waves, shared out among the jobs (a job of few entries may have as
   // many windows as its output bytes allow)
-  launch(k_encode_blocks, dim3(grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide), kEncWarps, per_job(bt, 148 * 2 * 4)), bt.B), kEncWarps * 32, kEncSmem, st, bt.d);
+  launch(k_encode_blocks, dim3(grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide), kEncWarps, bt.per_job(148 * 2 * 4)), bt.B), kEncWarps * 32, kEncSmem, st, bt.d);
 }
 void launch_emit_decoded(const Batch& bt, cudaStream_t st) {
   if (!bt.any_keep_decoded) return;
   scan_batch(kScanDecKey, bt, bt.max_entries, st);
-  launch(k_emit_decoded, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_emit_decoded, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_encode_filters(const Batch& bt, cudaStream_t st) {
-  launch(k_encode_filters, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_encode_filters, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_encode_index(const Batch& bt, cudaStream_t st) {
-  launch(k_encode_index, dim3(grid_x(bt.max_entries, 256, per_job(bt, 148 * 16)), bt.B), 256, 0, st, bt.d);
+  launch(k_encode_index, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 16)), bt.B), 256, 0, st, bt.d);
 }
 void launch_encode_meta(const Batch& bt, cudaStream_t st) {
   launch(k_encode_meta, dim3(bt.max_cap_files, bt.B), 256, 0, st, bt.d);
-  launch(k_meta_crc, dim3(grid_x(bt.max_entries, 4096, per_job(bt, 148 * 4)), bt.B), 256, 0, st, bt.d);
+  launch(k_meta_crc, dim3(grid_x(bt.max_entries, 4096, bt.per_job(148 * 4)), bt.B), 256, 0, st, bt.d);
   // (the wide blocks are at most the entries)
-  launch(k_meta_trailers, dim3(std::max((3 * bt.max_cap_files + 255) / 256, grid_x(bt.max_entries, 2048, per_job(bt, 148 * 2))), bt.B), 256, 0, st, bt.d);
+  launch(k_meta_trailers, dim3(std::max((3 * bt.max_cap_files + 255) / 256, grid_x(bt.max_entries, 2048, bt.per_job(148 * 2))), bt.B), 256, 0, st, bt.d);
 }
 
 void launch_results(const Batch& bt, cudaStream_t st) {

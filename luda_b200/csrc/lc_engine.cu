@@ -836,11 +836,12 @@ struct lc_slot {
       return 0;
     }
     char key[256];
-    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%llu|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
+    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%llu|%llu|%u|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
              (int)decode_merge, bt.B, bt.max_tables, bt.max_gp, bt.max_cap_triggers,
-             bt.max_cap_files, (unsigned long long)bt.max_blocks_in,
+             bt.max_cap_files, (unsigned long long)bt.max_dec_groups,
+             (unsigned long long)bt.max_dec_units,
              (unsigned long long)bt.max_entries, (unsigned long long)bt.max_cap_wide, bt.merge_rounds, bt.chunk, bt.ctas_per_job,
-             bt.merge_items, bt.merge_threads, bt.max_runs,
+             bt.merge_items, bt.merge_threads, bt.max_runs, bt.jobs_of_largest,
              (int)bt.any_keep_decoded);
     auto it = graphs.find(key);
     bool fresh = false;
@@ -1149,7 +1150,8 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       bt.max_tables = std::max(bt.max_tables, J.n_tables);
       bt.any_verify = bt.any_verify || (J.verify_checksums && !r.failed);
       bt.any_keep_decoded = bt.any_keep_decoded || (j->keep_decoded && !r.failed);
-      bt.max_blocks_in = std::max(bt.max_blocks_in, cap_blk);
+      // (blocks are closed at block_size bytes; the input's block size is not known)
+      bt.max_blocks_in = std::max<uint64_t>(bt.max_blocks_in, r.in_bytes / 2048 + 1);
     }
     if (host_up) {
       CK(cudaEventRecord(e->up_lane.done, st));
@@ -1164,6 +1166,14 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     // ---- parse: index blocks, then entry counts -- exact: a walk of every
     // entry header, which also gives the key bytes; single pass: the restart
     // words alone, the decode reserving key space itself
+    {
+      uint64_t all = 0, most = 1;
+      for (auto& r : runs) {
+        all += r.in_bytes;
+        most = std::max(most, r.in_bytes);
+      }
+      bt.jobs_of_largest = (uint32_t)std::max<uint64_t>(1, (all + most / 2) / most);
+    }
     if (bt.max_tables) {
       launch_table_index_count(bt, st);
       scan_batch(kScanTblBlocks, bt, bt.max_tables, st);
@@ -1214,16 +1224,36 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       }
       r.J.reserve_keys = exact ? 0 : 1;
       r.J.max_key_len = kFastMaxKey;
-      // blocks of many entries are walked 8 to a warp (four restart runs of
-      // 16 entries each fill its lanes), blocks of few 32
-      r.J.dec_group = (!r.failed && hc[i].n_entries_in > 16 * hc[i].n_blocks_in) ? 8 : 32;
+      // pass 1 of the decode: as many blocks to a warp as have 32 restart runs
+      // (a lane each), if the input was written with the job's restart
+      // interval
+      if (!r.failed && hc[i].n_blocks_in) {
+        const uint64_t per_block = hc[i].n_entries_in / hc[i].n_blocks_in;
+        const uint64_t rpb = (per_block + r.j->opt.restart_interval) / r.j->opt.restart_interval;
+        r.J.dec_group = (uint32_t)std::max<uint64_t>(1, 32 / std::min<uint64_t>(32, rpb));
+      } else {
+        r.J.dec_group = 32;
+      }
+      bt.max_dec_groups = std::max<uint64_t>(bt.max_dec_groups, hc[i].n_blocks_in / r.J.dec_group + 1);
       r.j->entries_in = r.N;
       r.j->key_bytes_in = exact ? r.K : 0;
     }
     // (the zeroed counters are uploaded below, from pinned memory)
+    uint64_t all_n = 0, max_n = 1;
+    for (uint32_t i = 0; i < B; i++) {
+      all_n += runs[i].N;
+      max_n = std::max(max_n, runs[i].N);
+    }
+    bt.jobs_of_largest = (uint32_t)std::max<uint64_t>(1, (all_n + max_n / 2) / max_n);
+    // units of the decode's second pass: 32 entries (one round of a warp; its
+    // latency is what a small batch pays) while the SMs' 4736 resident warps do
+    // not get a dozen each, else 256 (a unit's start and end are searched for)
+    const uint32_t dec_unit = all_n < 4736ull * 32 * 12 ? 32 : 256;
     uint32_t max_runs = 1;
     for (uint32_t i = 0; i < B; i++) {
       JobRun& r = runs[i];
+      r.J.dec_unit = dec_unit;
+      bt.max_dec_units = std::max<uint64_t>(bt.max_dec_units, r.N / dec_unit + 1);
       alloc_tail(r, A, true);
       if (r.failed) {
         // run_entry_begin[0] must read 0 for the merge kernels
@@ -1243,7 +1273,8 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     // captured graph (the kernels loop over whatever the grid leaves)
     bt.max_entries = pow2_at_least(std::max<uint64_t>(bt.max_entries, 1));
     bt.max_cap_wide = pow2_at_least(bt.max_cap_wide);
-    bt.max_blocks_in = pow2_at_least(bt.max_blocks_in);  // decode grid size only
+    bt.max_dec_groups = pow2_at_least(bt.max_dec_groups);
+    bt.max_dec_units = pow2_at_least(bt.max_dec_units);
     bt.max_cap_files = (uint32_t)pow2_at_least(bt.max_cap_files);
     bt.max_cap_triggers = (uint32_t)pow2_at_least(bt.max_cap_triggers);
     bt.max_gp = bt.max_gp ? (uint32_t)pow2_at_least(bt.max_gp + 1) - 1 : 0;

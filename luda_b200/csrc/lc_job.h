@@ -158,6 +158,7 @@ struct JobDev {
   uint64_t cap_key_bytes;
   uint4* e_rec;              // per entry: decode record (pass 1 -> pass 2)
   uint32_t dec_group;        // data blocks per warp in the decode's first pass
+  uint32_t dec_unit;         // entries per warp in its second pass
   uint32_t* e_koff;
   uint32_t* e_klen;
   uint32_t* e_voff;

@@ -106,7 +106,7 @@ __device__ __forceinline__ bool run_first(const JobDev& J, uint64_t e) {
 // its child.  table/merger.cc merges children it trusts to be sorted; a child
 // out of order fails the job here (kErrUnsorted) rather than reaching the
 // merge path, whose cuts assume sorted children.
-__global__ void k_prefix(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 8) k_prefix(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;
@@ -245,10 +245,13 @@ __global__ void k_merge_partition(const JobDev* __restrict__ jobs, uint32_t r, u
 
 // One tile per CTA step: the tile's stretches of both groups (ids and
 // prefixes) are loaded into shared memory with coalesced reads, every thread
-// finds its own diagonal there and merges `items` outputs, and the tile is
-// written back with coalesced stores; the tags follow by source position
-// (two ascending streams).  Only equal prefixes read key bytes.
-__global__ void __launch_bounds__(1024) k_merge_tile(const JobDev* __restrict__ jobs, uint32_t r,
+// finds its own diagonal there and merges `items` outputs as source positions,
+// and the tile is written back with coalesced stores, ids and prefixes from
+// shared memory and the tags from memory by source position (two ascending
+// streams).  Only equal prefixes read key bytes.  Bound by the latency of the
+// serial merge: 14 bytes of shared memory a position instead of 28 and 40
+// registers give an SM 48 warps instead of 24 (8M entries on B200: 221 -> 166 us).
+__global__ void __maxnreg__(40) k_merge_tile(const JobDev* __restrict__ jobs, uint32_t r,
                                                      uint32_t rounds, uint32_t items) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
@@ -259,10 +262,9 @@ __global__ void __launch_bounds__(1024) k_merge_tile(const JobDev* __restrict__ 
   const uint32_t tile = blockDim.x * items;
   extern __shared__ __align__(16) uint8_t merge_smem[];
   uint64_t* in_pfx = reinterpret_cast<uint64_t*>(merge_smem);
-  uint64_t* out_pfx = in_pfx + tile;
-  uint32_t* in_ids = reinterpret_cast<uint32_t*>(out_pfx + tile);
-  uint32_t* out_ids = in_ids + tile;
-  uint32_t* out_src = out_ids + tile;  // source position (in the tile) of each output
+  uint32_t* in_ids = reinterpret_cast<uint32_t*>(in_pfx + tile);
+  uint16_t* out_src = reinterpret_cast<uint16_t*>(in_ids + tile);  // source position (in the
+                                                                   // tile) of each output
   const MergeRound m = merge_round(J, r, rounds);
   for (uint64_t g = blockIdx.x; g < J.cap_merge_tiles; g += gridDim.x) {
     MergeTile t;
@@ -299,18 +301,15 @@ __global__ void __launch_bounds__(1024) k_merge_tile(const JobDev* __restrict__ 
       for (uint32_t o = k; o < stop; o++) {
         const bool take_a =
             i < na && (j >= nb || entry_le(J, in_ids[i], in_pfx[i], in_ids[na + j], in_pfx[na + j]));
-        const uint32_t x = take_a ? i++ : na + j++;
-        out_ids[o] = in_ids[x];
-        out_pfx[o] = in_pfx[x];
-        out_src[o] = x;
+        out_src[o] = (uint16_t)(take_a ? i++ : na + j++);
       }
     }
     __syncthreads();
     const uint64_t o0 = t.a0 + t.d0;
     for (uint32_t x = threadIdx.x; x < len; x += blockDim.x) {
-      m.dst_ids[o0 + x] = out_ids[x];
-      m.dst_pfx[o0 + x] = out_pfx[x];
       const uint32_t y = out_src[x];
+      m.dst_ids[o0 + x] = in_ids[y];
+      m.dst_pfx[o0 + x] = in_pfx[y];
       m.dst_tag[o0 + x] = m.src_tag[y < na ? t.a0 + i0 + y : t.a0 + t.na + j0 + (y - na)];
     }
   }
@@ -387,7 +386,7 @@ __device__ __forceinline__ void drop_one(const JobDev& J, const uint32_t* __rest
   }
 }
 
-__global__ void k_drop(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 6) k_drop(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
@@ -508,16 +507,19 @@ __global__ void k_forced(const JobDev* __restrict__ jobs) {
 }  // namespace
 
 static unsigned flat_ctas(const Batch& bt, uint64_t items, unsigned per) {
-  const uint64_t cap = std::max<uint64_t>(1, bt.ctas_per_job ? bt.ctas_per_job : 148 * 8 / bt.B);
-  return grid_x(items, per, cap);
+  return grid_x(items, per, bt.per_job(148 * 8));
 }
 
-// Merge tile (threads x items, at most kMergeMaxTile) and the shared memory
-// it takes: ids and prefixes of the tile's input and output and each output's
-// source position.
+// Merge tile: threads x items, at most kMergeMaxTile (a source position in
+// the tile fits 16 bits), and no more items than leave every SM two tiles: a
+// small job is bound by one tile's serial merge, so it takes more, shorter ones
+// (80k entries in
+// two rounds on B200: 44 us with 2048-position tiles, 20 us with 512).
 static uint32_t merge_items_of(const Batch& bt) {
   uint32_t items = std::max<uint32_t>(1, bt.merge_items);
   while ((uint64_t)bt.merge_threads * items > kMergeMaxTile && items > 1) items >>= 1;
+  while (items > 1 && bt.max_entries * bt.jobs_of_largest < 2ull * 148 * bt.merge_threads * items)
+    items >>= 1;
   return items;
 }
 
@@ -546,7 +548,7 @@ void launch_merge(const Batch& bt, cudaStream_t st) {
   const uint32_t tile = threads * items;
   const uint64_t tiles = bt.max_entries / tile + bt.max_runs + 1;
   for (uint32_t r = 0; r < bt.merge_rounds; r++) {
-    launch(k_merge_partition, dim3(grid_x(tiles, 128, 148 * 16), bt.B), 128, 0, st, bt.d, r, bt.merge_rounds, tile);
+    launch(k_merge_partition, dim3(grid_x(tiles, 128, bt.per_job(148 * 16)), bt.B), 128, 0, st, bt.d, r, bt.merge_rounds, tile);
     launch(k_merge_tile, dim3(flat_ctas(bt, tiles, 1), bt.B), threads, kMergeSmemPerPos * (size_t)tile, st, bt.d, r, bt.merge_rounds, items);
   }
 }

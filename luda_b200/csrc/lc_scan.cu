@@ -1,11 +1,13 @@
-// Exclusive prefix sums of per-job arrays in two launches for a whole batch
-// (grid y = job): per-tile sums, then the scan of each tile from its offset,
-// which every CTA sums from the tile sums before it.
+// Exclusive prefix sums of per-job arrays for a whole batch (grid y = job), in
+// two launches: per-tile sums (scan_scratch; the scans of a job run one after
+// another), then the scan of each tile from its offset, which every CTA sums
+// from the tile sums before it.  Short arrays take the second launch alone,
+// the offset summed from the elements.
 //
 // The array and its length are chosen by a selector from the job descriptor;
 // the length lives in device memory, so a scan can be enqueued before the
 // producing kernel's count is known on the host.  The grid is sized from a
-// host-side capacity and tiles past the count exit early.  out has n+1
+// host-side estimate of the length; the kernels loop over the rest.  out has n+1
 // entries: out[n] is the total, optionally also stored to a counter.
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -134,12 +136,6 @@ struct ScanOf<kScanDecKlen> {
   static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->key_cursor; }
 };
 
-// Tile-sum scratch of a scan (the scans of a job run one after another).
-template <int S>
-__device__ __forceinline__ uint64_t* scan_tiles_of(const JobDev& J) {
-  return J.scan_scratch;
-}
-
 template <typename T>
 __device__ __forceinline__ T warp_incl_scan(T v) {
   const int lane = threadIdx.x & 31;
@@ -175,6 +171,46 @@ __device__ __forceinline__ T block_excl_scan(T v, T* total) {
   return res;
 }
 
+// Eight consecutive elements from i (a multiple of 8) as 16-byte loads
+// (every scanned array starts on a 256-byte boundary); elements at or past n
+// read as zero.
+template <typename TI, typename TO>
+__device__ __forceinline__ void load8(const TI* in, uint64_t i, uint64_t n, TO (&v)[8]) {
+  if (i + 8 <= n) {
+    constexpr int kB = 8 * sizeof(TI);
+    if constexpr (kB == 8) {
+      const uint64_t w = *reinterpret_cast<const uint64_t*>(in + i);
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[k] = (TO)((w >> (8 * k)) & 0xff);
+    } else {
+      alignas(16) TI x[8];
+#pragma unroll
+      for (int k = 0; k < kB / 16; k++)
+        reinterpret_cast<uint4*>(x)[k] = reinterpret_cast<const uint4*>(in + i)[k];
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[k] = (TO)x[k];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = i + k < n ? (TO)in[i + k] : TO(0);
+  }
+}
+
+// Sum of in[lo, hi) over the CTA (every thread gets it); lo a multiple of 8.
+template <typename TO, typename TI>
+__device__ __forceinline__ TO block_sum(const TI* in, uint64_t lo, uint64_t hi) {
+  TO s = 0;
+  for (uint64_t i = lo + 8 * threadIdx.x; i < hi; i += 8 * blockDim.x) {
+    TO v[8];
+    load8<TI, TO>(in, i, hi, v);
+#pragma unroll
+    for (int k = 0; k < 8; k++) s += v[k];
+  }
+  TO total;
+  block_excl_scan<TO>(s, &total);
+  return total;
+}
+
 template <int S>
 __global__ void k_tile_reduce(const JobDev* __restrict__ jobs) {
   pdl_begin();
@@ -186,104 +222,110 @@ __global__ void k_tile_reduce(const JobDev* __restrict__ jobs) {
   __syncthreads();
   if (s_failed) return;
   const uint64_t n = SP::n(J);
-  TO* tile_sums = reinterpret_cast<TO*>(scan_tiles_of<S>(J));
-  const typename SP::TI* in = SP::in(J);
+  TO* tile_sums = reinterpret_cast<TO*>(J.scan_scratch);
   for (uint64_t t = blockIdx.x; t * kTile <= n; t += gridDim.x) {
-    const uint64_t base = t * kTile;
-    TO s = 0;
-    for (int k = 0; k < kScanItems; k++) {
-      const uint64_t i = base + (uint64_t)k * kScanThreads + threadIdx.x;
-      if (i < n) s += (TO)in[i];
-    }
-    TO total;
-    block_excl_scan<TO>(s, &total);
+    const TO total = block_sum<TO>(SP::in(J), t * kTile, min(n, (t + 1) * kTile));
     if (threadIdx.x == 0) tile_sums[t] = total;
   }
 }
 
-// Sum of a[lo, hi) over the CTA (every thread gets it).
-template <typename T>
-__device__ __forceinline__ T block_sum(const T* a, uint64_t lo, uint64_t hi) {
-  T v = 0;
-  for (uint64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) v += a[i];
-  T total;
-  block_excl_scan<T>(v, &total);
-  return total;
-}
-
-template <int S>
-__global__ void k_tile_scan(const JobDev* __restrict__ jobs) {
+// kDirect: no tile sums; a CTA sums the elements before its tile itself.
+template <int S, int kThreads, bool kDirect>
+__global__ void __launch_bounds__(kThreads) k_tile_scan(const JobDev* __restrict__ jobs) {
   pdl_begin();
   using SP = ScanOf<S>;
   using TO = typename SP::TO;
+  constexpr uint64_t kT = (uint64_t)kThreads * kScanItems;
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error || SP::out(J) == nullptr;
   __syncthreads();
   if (s_failed) return;
   const uint64_t n = SP::n(J);
-  const TO* tile_sums = reinterpret_cast<const TO*>(scan_tiles_of<S>(J));
-  const uint64_t n_tiles = n / kTile + 1;
+  if (blockIdx.x * kT > n) return;
+  const TO* tile_sums = reinterpret_cast<const TO*>(J.scan_scratch);
   const typename SP::TI* in = SP::in(J);
   TO* out = SP::out(J);
   uint64_t* total_out = SP::total(J);
-  // offset of this CTA's first tile: the sums of the tiles before it; each
-  // step of the grid stride adds the sums of the tiles it skips
-  TO carry = block_sum<TO>(tile_sums, 0, (uint64_t)blockIdx.x < n_tiles ? blockIdx.x : n_tiles);
-  for (uint64_t t = blockIdx.x; t * kTile <= n; t += gridDim.x) {
-    const uint64_t base = t * kTile;
-    TO vals[kScanItems];
+  // offset of this CTA's first tile; each step of the grid stride adds the
+  // tiles it skips
+  const auto before = [&](uint64_t t0, uint64_t t1) -> TO {  // tiles [t0, t1)
+    if constexpr (kDirect) return block_sum<TO>(in, t0 * kT, min(n, t1 * kT));
+    TO x = 0, total;
+    for (uint64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) x += tile_sums[i];
+    block_excl_scan<TO>(x, &total);
+    return total;
+  };
+  TO carry = before(0, blockIdx.x);
+  for (uint64_t t = blockIdx.x; t * kT <= n; t += gridDim.x) {
+    const uint64_t tb = t * kT + (uint64_t)threadIdx.x * kScanItems;
+    alignas(16) TO v[8];
+    load8<typename SP::TI, TO>(in, tb, n, v);
     TO s = 0;
-    const uint64_t tb = base + (uint64_t)threadIdx.x * kScanItems;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-      const uint64_t i = tb + k;
-      vals[k] = i < n ? (TO)in[i] : TO(0);
-      s += vals[k];
+      const TO x = v[k];
+      v[k] = s;
+      s += x;
     }
     TO total;
-    TO ex = block_excl_scan<TO>(s, &total) + carry;
+    const TO ex = block_excl_scan<TO>(s, &total) + carry;
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-      const uint64_t i = tb + k;
-      if (i < n) {
-        out[i] = ex;
-      } else if (i == n) {
-        out[n] = ex;
-        if (total_out) *total_out = (uint64_t)ex;
-      }
-      ex += vals[k];
+    for (int k = 0; k < kScanItems; k++) v[k] += ex;
+    if (tb + kScanItems <= n) {
+#pragma unroll
+      for (int k = 0; k < (int)(kScanItems * sizeof(TO) / 16); k++)
+        reinterpret_cast<uint4*>(out + tb)[k] = reinterpret_cast<const uint4*>(v)[k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanItems; k++)
+        if (tb + k < n) out[tb + k] = v[k];
     }
-    if ((t + gridDim.x) * kTile <= n)  // another tile of this CTA follows
-      carry += block_sum<TO>(tile_sums, t, t + gridDim.x < n_tiles ? t + gridDim.x : n_tiles);
+    if (tb <= n && n < tb + kScanItems) {  // the total after the last element
+      TO all = ex + s;  // (elements past n are zero)
+      out[n] = all;
+      if (total_out) *total_out = (uint64_t)all;
+    }
+    if ((t + gridDim.x) * kT <= n) {  // another tile of this CTA follows
+      carry += before(t, t + gridDim.x);
+    }
   }
 }
 
+// Up to kDirectMax elements (by the caller's estimate; the kernel is right for
+// any count): one launch with tiles of 8192, every CTA reading the elements
+// before its tile, at most 16 tiles.  More: tile sums first.  At 80k elements
+// one launch takes 4 us, two take 7.
+constexpr uint64_t kDirectThreads = 1024;
+constexpr uint64_t kDirectMax = 16 * kDirectThreads * kScanItems;
+
 template <int S>
-void scan_sel(const Batch& bt, uint64_t n_cap, cudaStream_t st) {
-  const unsigned tiles = grid_x(n_cap + 1, kTile, 148 * 8);
-  // one tile (n + 1 <= kTile for every job of the batch): no tile sums to
-  // add, so the scan pass alone does it
-  const bool one_tile = n_cap + 1 <= kTile;
-  if (!one_tile) launch(k_tile_reduce<S>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
-  launch(k_tile_scan<S>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
+void scan_sel(const Batch& bt, uint64_t n_est, cudaStream_t st) {
+  if (n_est <= kDirectMax) {
+    launch(k_tile_scan<S, kDirectThreads, true>,
+           dim3(grid_x(n_est + 1, kDirectThreads * kScanItems, 16), bt.B), kDirectThreads, 0, st, bt.d);
+    return;
+  }
+  const unsigned tiles = grid_x(n_est + 1, kTile, bt.per_job(148 * 8));
+  launch(k_tile_reduce<S>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
+  launch(k_tile_scan<S, kScanThreads, false>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
 }
 
 }  // namespace
 
-void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_cap, cudaStream_t st) {
+void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st) {
   switch (sel) {
-    case kScanTblBlocks: scan_sel<kScanTblBlocks>(bt, n_cap, st); break;
-    case kScanBlkEnt: scan_sel<kScanBlkEnt>(bt, n_cap, st); break;
-    case kScanBlkKey: scan_sel<kScanBlkKey>(bt, n_cap, st); break;
-    case kScanKeep: scan_sel<kScanKeep>(bt, n_cap, st); break;
-    case kScanBstart: scan_sel<kScanBstart>(bt, n_cap, st); break;
-    case kScanBcum: scan_sel<kScanBcum>(bt, n_cap, st); break;
-    case kScanGcum: scan_sel<kScanGcum>(bt, n_cap, st); break;
-    case kScanIcum: scan_sel<kScanIcum>(bt, n_cap, st); break;
-    case kScanDecKey: scan_sel<kScanDecKey>(bt, n_cap, st); break;
-    case kScanKb: scan_sel<kScanKb>(bt, n_cap, st); break;
-    case kScanDecKlen: scan_sel<kScanDecKlen>(bt, n_cap, st); break;
+    case kScanTblBlocks: scan_sel<kScanTblBlocks>(bt, n_est, st); break;
+    case kScanBlkEnt: scan_sel<kScanBlkEnt>(bt, n_est, st); break;
+    case kScanBlkKey: scan_sel<kScanBlkKey>(bt, n_est, st); break;
+    case kScanKeep: scan_sel<kScanKeep>(bt, n_est, st); break;
+    case kScanBstart: scan_sel<kScanBstart>(bt, n_est, st); break;
+    case kScanBcum: scan_sel<kScanBcum>(bt, n_est, st); break;
+    case kScanGcum: scan_sel<kScanGcum>(bt, n_est, st); break;
+    case kScanIcum: scan_sel<kScanIcum>(bt, n_est, st); break;
+    case kScanDecKey: scan_sel<kScanDecKey>(bt, n_est, st); break;
+    case kScanKb: scan_sel<kScanKb>(bt, n_est, st); break;
+    case kScanDecKlen: scan_sel<kScanDecKlen>(bt, n_est, st); break;
   }
 }
 
