@@ -860,6 +860,7 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
           J.e_vlen[e] = rec.z;
           J.e_pfx[e] = user_prefix(kb + ko, kl);
           J.e_tag[e] = ld_le64(kb + ko + kl - 8);
+          if (J.bits_per_key > 0) J.e_hash[e] = bloom_hash(kb + ko, kl);
         }
       } else {
         // long keys: built in the arena, one key at a time, the lanes over
@@ -885,6 +886,7 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
           J.e_vlen[e] = rec.z;
           J.e_pfx[e] = user_prefix(gdst + ko, kl);
           J.e_tag[e] = ld_le64(gdst + ko + kl - 8);
+          if (J.bits_per_key > 0) J.e_hash[e] = bloom_hash(gdst + ko, kl);
         }
       }
       __syncwarp();
@@ -913,6 +915,7 @@ __global__ void k_entries_from_offsets(const JobDev* __restrict__ jobs) {
     J.k_klen[i] = (uint32_t)kl;
     J.k_voff[i] = (uint32_t)J.src_voffs[i];
     J.k_vlen[i] = (uint32_t)(J.src_voffs[i + 1] - J.src_voffs[i]);
+    if (J.bits_per_key > 0) J.k_hash[i] = bloom_hash(J.keys + ko, (uint32_t)kl);
   }
 }
 

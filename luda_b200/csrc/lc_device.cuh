@@ -141,25 +141,27 @@ __device__ __forceinline__ uint64_t user_prefix_after(const uint8_t* k, uint32_t
   return v;
 }
 
+// The job's entries a and b whose prefixes are equal, by user key: below, equal
+// or above zero.  Their first key_skip + 8 bytes are equal as far as both user
+// keys have them, so that only what follows is compared.
+__device__ __forceinline__ int user_key_rest_cmp(const JobDev& J, uint32_t a, uint32_t b) {
+  const uint32_t al = J.e_klen[a] - 8, bl = J.e_klen[b] - 8, m = al < bl ? al : bl;
+  uint32_t i = J.ctr->key_skip + 8;
+  if (i < m) {
+    const uint8_t *x = J.keys + J.e_koff[a], *y = J.keys + J.e_koff[b];
+    for (; i < m; i++)
+      if (x[i] != y[i]) return x[i] < y[i] ? -1 : 1;
+  }
+  return al < bl ? -1 : (al > bl ? 1 : 0);
+}
+
 // a before b in the merge (InternalKeyComparator order), given their user-key
 // prefixes: the prefixes decide unless equal.
 __device__ __forceinline__ bool entry_le(const JobDev& J, uint32_t a, uint64_t pa, uint32_t b,
                                          uint64_t pb) {
   if (pa != pb) return pa < pb;
-  return ikey_cmp(J.keys + J.e_koff[a], J.e_klen[a], J.keys + J.e_koff[b], J.e_klen[b]) <= 0;
-}
-
-// Same user key?  (pa, pb: their user-key prefixes)
-__device__ __forceinline__ bool same_user_key(const JobDev& J, uint32_t a, uint64_t pa, uint32_t b,
-                                              uint64_t pb) {
-  if (pa != pb) return false;
-  uint32_t al = J.e_klen[a] - 8, bl = J.e_klen[b] - 8;
-  if (al != bl) return false;
-  const uint8_t* x = J.keys + J.e_koff[a];
-  const uint8_t* y = J.keys + J.e_koff[b];
-  for (uint32_t i = 0; i < al; i++)
-    if (x[i] != y[i]) return false;
-  return true;
+  const int r = user_key_rest_cmp(J, a, b);
+  return r < 0 || (r == 0 && J.e_tag[a] >= J.e_tag[b]);
 }
 
 // Hash of util/hash.cc:22-51 (the bloom filter's hash) over bytes that may
@@ -189,6 +191,11 @@ __device__ __forceinline__ uint32_t leveldb_hash_words(const uint8_t* data, uint
     h ^= (h >> 24);
   }
   return h;
+}
+
+// The bloom filter's hash of an internal key's user key (util/bloom.cc:14-16).
+__device__ __forceinline__ uint32_t bloom_hash(const uint8_t* key, uint32_t klen) {
+  return leveldb_hash_words(key, klen - 8, 0xbc9f1d34u);
 }
 
 // a % d for 32-bit a and a divisor d >= 1 fixed over many calls, from

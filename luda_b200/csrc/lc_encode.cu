@@ -25,8 +25,9 @@
 // survivor s gets next(s), the start of the following block if a block began
 // at s.  The chain from survivor 0 is resolved in three steps: per chunk of
 // survivors, a table of exits for every possible entry point (pointer chasing
-// in shared memory); one thread composing the tables across chunks; and a
-// per-chunk chase from the resolved entry point that marks block starts.
+// in shared memory), with the blocks started on the way; one thread composing
+// the tables across chunks; and a per-chunk chase from the resolved entry
+// point that writes the block starts.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -71,20 +72,18 @@ __device__ __forceinline__ const uint8_t* kept_key(const JobDev& J, uint64_t k, 
   return J.keys + J.k_koff[k];
 }
 
-// Entry sizes as a restart entry (k_a) and as a prefix-compressed entry
-// (k_b), the shared prefix with the previous survivor, survivor byte totals;
-// also clears the block-start flags (n + 1 of them) for the chain.
+// The flush encoder's entry sizes: as a restart entry (k_a) and as a
+// prefix-compressed entry (k_b), the shared prefix with the previous entry,
+// byte totals.  (k_kept_compact computes a compaction's.)
 __global__ void __launch_bounds__(256, 8) k_sizes(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
   const uint64_t n = J.ctr->n_kept;
   unsigned long long kb = 0, vb = 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) J.k_bstart[n] = 0;
   for (uint64_t k0 = (uint64_t)blockIdx.x * blockDim.x; k0 < n; k0 += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t k = k0 + threadIdx.x;
     if (k >= n) continue;
-    J.k_bstart[k] = 0;
     uint32_t kl;
     const uint8_t* key = kept_key(J, k, &kl);
     const uint32_t vl = J.k_vlen[k];
@@ -189,13 +188,22 @@ __global__ void __launch_bounds__(256, 6) k_next(const JobDev* __restrict__ jobs
 // than a sub-chunk walk the chunk directly.
 constexpr uint32_t kChainSub = 256;
 
-// Exit of sub-chunk s of a staged chunk [c0, c1) for entry point e (an
-// absolute survivor index inside the sub-chunk's first `W`).
-__device__ __forceinline__ uint64_t chain_sub_walk(const uint32_t* s_next, uint64_t c0, uint64_t c1,
-                                                   uint64_t e, uint64_t sub_end) {
-  const uint64_t end = min(c1, sub_end);
-  while (e < end) e = s_next[e - c0];
-  return e;
+// A chain table's word: how far past the (sub-)chunk's first survivor the
+// chain leaves it (below 2^14: a chunk and a window), and above bit 16 the
+// blocks started inside it.
+__device__ __forceinline__ uint32_t chain_word(uint64_t exit_rel, uint32_t blocks) {
+  return (uint32_t)exit_rel | (blocks << 16);
+}
+
+// The chain from survivor e of a staged chunk at c0 until it reaches `end`.
+__device__ __forceinline__ uint32_t chain_walk(const uint32_t* s_next, uint64_t c0, uint64_t e,
+                                               uint64_t end, uint64_t from) {
+  uint32_t blocks = 0;
+  while (e < end) {
+    e = s_next[e - c0];
+    blocks++;
+  }
+  return chain_word(e - from, blocks);
 }
 
 __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
@@ -205,13 +213,13 @@ __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
   if (threadIdx.x == 0) s_failed = J.ctr->error;
   __syncthreads();
   if (s_failed) return;
-  extern __shared__ uint32_t s_next[];  // chunk next() values, then sub-chunk exits
+  extern __shared__ uint32_t s_next[];  // chunk next() values, then sub-chunk words
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
   if (W > C) return;  // resolved sequentially instead
   const bool sub = W <= kChainSub;
-  uint32_t* s_sub = s_next + C;  // (C / kChainSub) x W sub-chunk exits
+  uint32_t* s_sub = s_next + C;  // (C / kChainSub) x W
   for (uint64_t c = blockIdx.x; c * C < n; c += gridDim.x) {
     const uint64_t c0 = c * C;
     const uint64_t c1 = min(n, c0 + C);
@@ -219,35 +227,35 @@ __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
     for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = J.k_next[c0 + i];
     __syncthreads();
     if (!sub) {
-      for (uint32_t i = threadIdx.x; i < W; i += blockDim.x) {
-        uint64_t e = c0 + i;
-        while (e < c1) e = s_next[e - c0];
-        J.chunk_table[c * C + i] = (uint32_t)e;
-      }
+      for (uint32_t i = threadIdx.x; i < W; i += blockDim.x)
+        J.chunk_table[c * C + i] = chain_walk(s_next, c0, c0 + i, c1, c0);
       continue;
     }
     const uint32_t nsub = (uint32_t)((c1 - c0 + kChainSub - 1) / kChainSub);
     for (uint32_t x = threadIdx.x; x < nsub * W; x += blockDim.x) {
       const uint32_t sb = x / W, i = x % W;
       const uint64_t s0 = c0 + (uint64_t)sb * kChainSub;
-      s_sub[x] = (uint32_t)chain_sub_walk(s_next, c0, c1, s0 + i, s0 + kChainSub);
+      s_sub[x] = chain_walk(s_next, c0, s0 + i, min(c1, s0 + kChainSub), s0);
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < W; i += blockDim.x) {
       uint64_t e = c0 + i;
+      uint32_t blocks = 0;
       for (uint32_t sb = 0; sb < nsub && e < c1; sb++) {
         const uint64_t s0 = c0 + (uint64_t)sb * kChainSub;
-        e = s_sub[sb * W + (uint32_t)(e - s0)];  // e lies in the sub-chunk's first W survivors
+        const uint32_t w = s_sub[sb * W + (uint32_t)(e - s0)];  // e: in the sub-chunk's first W
+        e = s0 + (w & 0xffff);
+        blocks += w >> 16;
       }
-      J.chunk_table[c * C + i] = (uint32_t)e;
+      J.chunk_table[c * C + i] = chain_word(e - c0, blocks);
     }
   }
 }
 
-// Exits of groups of kChainGroup chunks for every entry point in the first
-// `window` survivors of the group's first chunk, by following the chunk
-// tables (one thread per entry point).  Only when the chunk tables do not fit
-// the resolving CTA's shared memory.
+// Exits (and blocks, in the high half) of groups of kChainGroup chunks for
+// every entry point in the first `window` survivors of the group's first
+// chunk, by following the chunk tables (one thread per entry point).  Only
+// when the chunk tables do not fit the resolving CTA's shared memory.
 __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
@@ -263,17 +271,21 @@ __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
        x += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t g = x / W, i = x % W;
     const uint64_t c0 = g * kChainGroup, c1 = min(M, c0 + kChainGroup);
-    uint64_t e = c0 * C + i;
-    for (uint64_t c = c0; c < c1 && e < n; c++) e = J.chunk_table[c * C + (e - c * C)];
-    J.group_table[g * C + i] = (uint32_t)e;
+    uint64_t e = c0 * C + i, blocks = 0;
+    for (uint64_t c = c0; c < c1 && e < n; c++) {
+      const uint32_t w = J.chunk_table[c * C + (e - c * C)];
+      e = c * C + (w & 0xffff);
+      blocks += w >> 16;
+    }
+    J.group_table[g * C + i] = e | (blocks << 32);
   }
 }
 
-// Entry point of every chunk: the chain from survivor 0 through the chunk
-// tables.  Few chunks: one thread walks them over a shared-memory copy of the
-// tables.  Many: one thread walks the group tables (in shared memory when they
-// fit), then one thread per group walks its chunks from the group's entry
-// point.
+// Entry point and first block of every chunk: the chain from survivor 0
+// through the chunk tables.  Few chunks: one thread walks them over a
+// shared-memory copy of the tables.  Many: one thread walks the group tables
+// (in shared memory when they fit), then one thread per group walks its chunks
+// from the group's entry point.
 __global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
@@ -281,19 +293,27 @@ __global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
   if (threadIdx.x == 0) s_failed = J.ctr->error;
   __syncthreads();
   if (s_failed) return;
-  extern __shared__ uint32_t s_tab[];
+  extern __shared__ __align__(8) uint32_t s_tab[];
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
-  if (n == 0) return;
+  const auto finish = [&](uint64_t blocks) {
+    J.b_first[blocks] = (uint32_t)n;
+    J.ctr->n_blocks_out = blocks;
+  };
+  if (n == 0) {
+    if (threadIdx.x == 0) finish(0);
+    return;
+  }
   if (W > C) {
     // blocks longer than a chunk: walk the whole chain
     if (threadIdx.x != 0) return;
-    uint64_t e = 0;
+    uint64_t e = 0, b = 0;
     while (e < n) {
-      J.k_bstart[e] = 1;
+      J.b_first[b++] = (uint32_t)e;
       e = J.k_next[e];
     }
+    finish(b);
     return;
   }
   const uint64_t M = (n + C - 1) / C;
@@ -302,47 +322,61 @@ __global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
       s_tab[i] = J.chunk_table[(i / W) * C + (i % W)];
     __syncthreads();
     if (threadIdx.x != 0) return;
-    uint64_t e = 0;
+    uint64_t e = 0, b = 0;
     for (uint64_t c = 0; c < M; c++) {
-      J.chunk_entry[c] = (uint32_t)e;
-      if (e < n) e = s_tab[c * W + (e - c * C)];
+      J.chunk_entry[c] = make_uint2((uint32_t)e, (uint32_t)b);
+      if (e < n) {
+        const uint32_t w = s_tab[c * W + (e - c * C)];
+        e = c * C + (w & 0xffff);
+        b += w >> 16;
+      }
     }
+    finish(b);
     return;
   }
   const uint64_t G = (M + kChainGroup - 1) / kChainGroup;
-  const bool staged = G * W + G <= J.chain_smem_words;
-  const bool entries_in_smem = G <= J.chain_smem_words;
-  uint32_t* s_entry = s_tab + (staged ? G * W : 0);  // group entry points
+  const bool staged = 2 * G * W <= J.chain_smem_words;
+  uint64_t* s_grp = reinterpret_cast<uint64_t*>(s_tab);
   if (staged) {
     for (uint64_t i = threadIdx.x; i < G * W; i += blockDim.x)
-      s_tab[i] = J.group_table[(i / W) * C + (i % W)];
+      s_grp[i] = J.group_table[(i / W) * C + (i % W)];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint64_t e = 0;
+    uint64_t e = 0, b = 0;
     for (uint64_t g = 0; g < G; g++) {
       const uint64_t c0 = g * kChainGroup;
-      if (entries_in_smem) s_entry[g] = (uint32_t)e;
-      else J.chunk_entry[c0] = (uint32_t)e;
-      if (e < n)
-        e = staged ? s_tab[g * W + (e - c0 * C)] : J.group_table[g * C + (e - c0 * C)];
+      J.chunk_entry[c0] = make_uint2((uint32_t)e, (uint32_t)b);
+      if (e < n) {
+        const uint64_t w = staged ? s_grp[g * W + (e - c0 * C)] : J.group_table[g * C + (e - c0 * C)];
+        e = w & 0xffffffffu;
+        b += w >> 32;
+      }
     }
+    finish(b);
   }
   __syncthreads();
   for (uint64_t g = threadIdx.x; g < G; g += blockDim.x) {
     const uint64_t c0 = g * kChainGroup, c1 = min(M, c0 + kChainGroup);
-    uint64_t e = entries_in_smem ? s_entry[g] : J.chunk_entry[c0];
+    const uint2 at = J.chunk_entry[c0];
+    uint64_t e = at.x;
+    uint32_t b = at.y;
     for (uint64_t c = c0; c < c1; c++) {
-      J.chunk_entry[c] = (uint32_t)e;
-      if (e < n) e = J.chunk_table[c * C + (e - c * C)];
+      J.chunk_entry[c] = make_uint2((uint32_t)e, b);
+      if (e < n) {
+        const uint32_t w = J.chunk_table[c * C + (e - c * C)];
+        e = c * C + (w & 0xffff);
+        b += w >> 16;
+      }
     }
   }
 }
 
-// Block starts: each chunk's chain from its resolved entry point.  With
-// sub-chunks, one thread finds the sub-chunks' entry points from their exits
-// (recomputed as k_chain_tables does) and every sub-chunk is walked by its
-// own thread.
+// First survivor of every block: each chunk's chain from its resolved entry
+// point.  With sub-chunks, one thread finds the sub-chunks' entry points from
+// their words (recomputed as k_chain_tables does) and every sub-chunk is
+// walked by its own thread.  (The block starts used to be flags that a scan
+// over the survivors turned into block numbers: 8M survivors, 47 us more.)
 __global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
@@ -357,18 +391,20 @@ __global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
   if (W > C) return;
   const bool sub = W <= kChainSub;
   uint32_t* s_sub = s_next + C;
-  uint32_t* s_entry = s_sub + (C / kChainSub) * (sub ? W : 0);  // sub-chunk entry points
+  __shared__ uint2 s_entry[32];  // sub-chunk entry points and first blocks (C / kChainSub of them)
   for (uint64_t c = blockIdx.x; c * C < n; c += gridDim.x) {
     const uint64_t c0 = c * C;
     const uint64_t c1 = min(n, c0 + C);
+    const uint2 at = J.chunk_entry[c];
     __syncthreads();
     for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = J.k_next[c0 + i];
     __syncthreads();
     if (!sub) {
       if (threadIdx.x == 0) {
-        uint64_t e = J.chunk_entry[c];
+        uint64_t e = at.x;
+        uint32_t b = at.y;
         while (e < c1) {
-          J.k_bstart[e] = 1;
+          J.b_first[b++] = (uint32_t)e;
           e = s_next[e - c0];
         }
       }
@@ -378,52 +414,51 @@ __global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
     for (uint32_t x = threadIdx.x; x < nsub * W; x += blockDim.x) {
       const uint32_t sb = x / W, i = x % W;
       const uint64_t s0 = c0 + (uint64_t)sb * kChainSub;
-      s_sub[x] = (uint32_t)chain_sub_walk(s_next, c0, c1, s0 + i, s0 + kChainSub);
+      s_sub[x] = chain_walk(s_next, c0, s0 + i, min(c1, s0 + kChainSub), s0);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      uint64_t e = J.chunk_entry[c];
+      uint64_t e = at.x;
+      uint32_t b = at.y;
       for (uint32_t sb = 0; sb < nsub; sb++) {
-        s_entry[sb] = (uint32_t)e;
+        s_entry[sb] = make_uint2((uint32_t)e, b);
         const uint64_t s0 = c0 + (uint64_t)sb * kChainSub;
-        if (e < c1) e = s_sub[sb * W + (uint32_t)(e - s0)];
+        if (e < c1) {
+          const uint32_t w = s_sub[sb * W + (uint32_t)(e - s0)];
+          e = s0 + (w & 0xffff);
+          b += w >> 16;
+        }
       }
     }
     __syncthreads();
     for (uint32_t sb = threadIdx.x; sb < nsub; sb += blockDim.x) {
       const uint64_t s0 = c0 + (uint64_t)sb * kChainSub, send = min(c1, s0 + kChainSub);
-      uint64_t e = s_entry[sb];
+      uint64_t e = s_entry[sb].x;
+      uint32_t b = s_entry[sb].y;
       while (e < send) {
-        J.k_bstart[e] = 1;
+        J.b_first[b++] = (uint32_t)e;
         e = s_next[e - c0];
       }
     }
   }
 }
 
-// Output blocks: first survivor of each block, and the block's size (the
-// block that starts at k ends where the chain says the next one starts).
-__global__ void k_block_list(const JobDev* __restrict__ jobs) {
+// Sizes of the output blocks.
+__global__ void k_block_sizes(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
-  const uint64_t n = J.ctr->n_kept;
+  const uint64_t nb = J.ctr->n_blocks_out;
   const uint32_t R = J.restart_interval;
-  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k <= n;
-       k += (uint64_t)gridDim.x * blockDim.x) {
-    if (k == n) {
-      J.b_first[J.k_block[n]] = (uint32_t)n;
-    } else if (J.k_bstart[k]) {
-      const uint32_t b = J.k_block[k];
-      J.b_first[b] = (uint32_t)k;
-      const uint64_t e = J.k_next[k];
-      uint64_t D = 0;
-      for (uint64_t a = k; a < e; a += R) D += J.k_a[a] - J.k_b[a];
-      const uint64_t nrest = (e - k + R - 1) / R;
-      const uint32_t size = (uint32_t)(J.k_pb[e] - J.k_pb[k] + D + 4 * nrest + 4);
-      J.b_size[b] = size;
-      J.tmp32[b] = size + kTrailer;
-    }
+  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
+       b += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t k = J.b_first[b], e = J.b_first[b + 1];
+    uint64_t D = 0;
+    for (uint64_t a = k; a < e; a += R) D += J.k_a[a] - J.k_b[a];
+    const uint64_t nrest = (e - k + R - 1) / R;
+    const uint32_t size = (uint32_t)(J.k_pb[e] - J.k_pb[k] + D + 4 * nrest + 4);
+    J.b_size[b] = size;
+    J.tmp32[b] = size + kTrailer;
   }
 }
 
@@ -431,17 +466,6 @@ __global__ void k_block_list(const JobDev* __restrict__ jobs) {
 // b gets b_fnext[b], the first block of the next file if a file began at b (a
 // binary search for the size cut, and the next forced block); one thread then
 // walks the few file starts.
-
-// t_blocks[i] = output block that starts at grandparent cut i (ascending).
-__global__ void k_forced_blocks(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= J.ctr->n_triggers) return;
-  const uint64_t kp = J.kept_pos[J.triggers[i]];
-  J.t_blocks[i] = kp < J.ctr->n_kept ? J.k_block[kp] : (uint32_t)J.ctr->n_blocks_out;
-}
 
 __global__ void k_file_next(const JobDev* __restrict__ jobs) {
   pdl_begin();
@@ -451,14 +475,6 @@ __global__ void k_file_next(const JobDev* __restrict__ jobs) {
   const uint32_t nt = J.ctr->n_triggers;
   for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
        b += (uint64_t)gridDim.x * blockDim.x) {
-    // first forced block after b
-    uint32_t lo = 0, hi = nt;
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (J.t_blocks[mid] <= b) lo = mid + 1;
-      else hi = mid;
-    }
-    const uint64_t next_forced = lo < nt ? J.t_blocks[lo] : nb;
     // first block end where the file's flushed bytes reach max_file_size
     const uint64_t cum0 = J.b_cum[b];
     const uint64_t target =
@@ -475,7 +491,26 @@ __global__ void k_file_next(const JobDev* __restrict__ jobs) {
       }
       sc = l;
     }
-    J.b_fnext[b] = (uint32_t)(min(sc, next_forced - 1) + 1);
+    // or before the first grandparent cut after the block's start, which is a
+    // block's start too: the block that starts at cut survivor kp
+    uint32_t lo = 0, hi = nt;
+    const uint32_t first = J.b_first[b];
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (J.t_kept[mid] <= first) lo = mid + 1;
+      else hi = mid;
+    }
+    if (lo < nt && J.t_kept[lo] <= J.b_first[sc]) {
+      const uint32_t kp = J.t_kept[lo];
+      uint64_t l = b + 1, h = sc;
+      while (l < h) {
+        const uint64_t mid = (l + h) >> 1;
+        if (J.b_first[mid] >= kp) h = mid;
+        else l = mid + 1;
+      }
+      sc = l - 1;
+    }
+    J.b_fnext[b] = (uint32_t)(sc + 1);
   }
 }
 
@@ -1382,10 +1417,10 @@ __device__ __forceinline__ void encode_index_entry(const JobDev& J, uint64_t b) 
   p = put_varint(p, varint_len(off) + varint_len(bsz));
   uint32_t llen;
   const uint8_t* lkey = kept_key(J, J.b_first[b + 1] - 1, &llen);
-  if (sep == kNoSep) {
-    for (uint32_t i = 0; i < ilen; i++) p[i] = lkey[i];
-  } else {
-    for (uint32_t i = 0; i < sep; i++) p[i] = lkey[i];
+  // (copy_small loads a piece's bytes before it stores any)
+  const uint32_t from_key = sep == kNoSep ? ilen : sep;
+  for (uint32_t i = 0; i < from_key; i += 32) copy_small<32>(p + i, lkey + i, min(32u, from_key - i));
+  if (sep != kNoSep) {
     p[sep] = (uint8_t)(lkey[sep] + 1);
     uint64_t t = kSeekTag;
     for (int i = 0; i < 8; i++) p[sep + 1 + i] = (uint8_t)(t >> (8 * i));
@@ -1630,8 +1665,8 @@ void launch_next(const Batch& bt, cudaStream_t st) {
 }
 void launch_chain(const Batch& bt, cudaStream_t st) {
   const uint64_t chunks = (bt.max_entries + bt.chunk - 1) / bt.chunk + 1;
-  // next() values, sub-chunk exits (windows up to kChainSub) and entry points
-  const size_t smem = ((size_t)bt.chunk + (bt.chunk / kChainSub) * (kChainSub + 1)) * sizeof(uint32_t);
+  // next() values, sub-chunk words (windows up to kChainSub)
+  const size_t smem = ((size_t)bt.chunk + (bt.chunk / kChainSub) * kChainSub) * sizeof(uint32_t);
   const unsigned g = (unsigned)std::min<uint64_t>(chunks, bt.per_job(148 * 4));
   launch(k_chain_tables, dim3(g, bt.B), 256, smem, st, bt.d);
   if (chunks > kChainGroup)
@@ -1639,11 +1674,10 @@ void launch_chain(const Batch& bt, cudaStream_t st) {
   launch(k_chain_resolve, dim3(1, bt.B), 1024, (size_t)bt.chain_smem_words * 4, st, bt.d);
   launch(k_chain_mark, dim3(g, bt.B), 128, smem, st, bt.d);
 }
-void launch_block_list(const Batch& bt, cudaStream_t st) {
-  launch(k_block_list, dim3(grid_x(bt.max_entries + 1, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
+void launch_block_sizes(const Batch& bt, cudaStream_t st) {
+  launch(k_block_sizes, dim3(grid_x(bt.max_entries, 1024, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_files(const Batch& bt, cudaStream_t st) {
-  launch(k_forced_blocks, dim3((bt.max_cap_triggers + 255) / 256, bt.B), 256, 0, st, bt.d);
   launch(k_file_next, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
   launch(k_files, dim3(1, bt.B), kFileThreads, 0, st, bt.d);
 }

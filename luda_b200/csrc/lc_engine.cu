@@ -47,7 +47,11 @@ thread_local std::string g_last_error;
 
 const char* kVersion = "luda_b200 0.1 (sm_100a)";
 constexpr uint32_t kCrcXpowN = 8192;
-constexpr uint32_t kChunk = 4096;
+// Survivors per chunk of the block chain (a CTA each): short chunks for batches
+// too small to give every SM a long one, when blocks are expected (from the
+// block size and the mean entry) to hold at most a quarter as many; blocks of
+// more survivors than a chunk are resolved one after the other.
+constexpr uint32_t kChunk = 4096, kShortChunk = 1024;
 
 struct CudaError {
   cudaError_t e;
@@ -599,16 +603,15 @@ void launch_tail(const Batch& bt, bool decode_merge, cudaStream_t st, PhaseTimer
     T.mark(kMerge);
     launch_drop(bt, st);
     launch_triggers(bt, st);
-    scan_batch(kScanKeep, bt, bt.max_entries, st);
     launch_kept_compact(bt, st);
     T.mark(kDrop);
+  } else {
+    launch_sizes(bt, st);
   }
-  launch_sizes(bt, st);
   scan_batch(kScanKb, bt, bt.max_entries, st);
   launch_next(bt, st);
   launch_chain(bt, st);
-  scan_batch(kScanBstart, bt, bt.max_entries, st);
-  launch_block_list(bt, st);
+  launch_block_sizes(bt, st);
   scan_batch(kScanBcum, bt, bt.max_entries, st);
   launch_files(bt, st);
   launch_block_layout(bt, st);
@@ -642,38 +645,34 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
     J.e_vlen = A.get<uint32_t>(N);
     J.e_pfx = A.get<uint64_t>(N);
     J.e_tag = A.get<uint64_t>(N);
+    J.e_hash = A.get<uint32_t>(J.bits_per_key > 0 ? N : 1);
     J.m_ids = A.get<uint32_t>(N);
     J.m_tmp = A.get<uint32_t>(N);
     J.m_pfx = A.get<uint64_t>(N);
     J.m_pfx_tmp = A.get<uint64_t>(N);
     J.m_tag = A.get<uint64_t>(N);
     J.m_tag_tmp = A.get<uint64_t>(N);
-    J.cap_merge_tiles = (uint32_t)merge_tile_capacity(N, J.n_runs);
-    J.m_split = A.get<uint32_t>(J.cap_merge_tiles);
     J.keep = A.get<uint8_t>(N);
     J.gp_idx = A.get<uint32_t>(J.n_gp ? N : 1);
-    J.kept_pos = A.get<uint32_t>(N + 1);
     J.gp_first = A.get<uint32_t>(J.n_gp + 1);
     J.gp_upfx = A.get<uint64_t>(J.n_gp + 1);
     J.gp_mode = A.get<uint8_t>(J.n_gp + 1);
-    J.k_forced = A.get<uint8_t>(N + 1);
   }
   J.k_koff = A.get<uint32_t>(N);
   J.k_klen = A.get<uint32_t>(N);
   J.k_voff = A.get<uint32_t>(N);
   J.k_vlen = A.get<uint32_t>(N);
+  J.k_hash = A.get<uint32_t>(J.bits_per_key > 0 ? N : 1);
   J.cap_triggers = J.n_gp + 1;
   J.triggers = A.get<uint32_t>(J.cap_triggers);
   J.k_a = A.get<uint32_t>(N);
   J.k_b = A.get<uint32_t>(N);
   J.k_shared = A.get<uint32_t>(N);
   J.k_next = A.get<uint32_t>(N);
-  J.k_bstart = A.get<uint8_t>(N + 1);
-  J.k_block = A.get<uint32_t>(N + 1);
   const uint64_t chunks = (N + J.chunk - 1) / J.chunk + 1;
   J.chunk_table = A.get<uint32_t>(chunks * J.chunk);
-  J.chunk_entry = A.get<uint32_t>(chunks);
-  J.group_table = A.get<uint32_t>((chunks / kChainGroup + 1) * J.chunk);
+  J.chunk_entry = A.get<uint2>(chunks);
+  J.group_table = A.get<uint64_t>((chunks / kChainGroup + 1) * J.chunk);
   J.b_first = A.get<uint32_t>(N + 1);
   J.b_size = A.get<uint32_t>(N);
   J.tmp32 = A.get<uint32_t>(N);
@@ -683,7 +682,6 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
                  (8 * (r.in_bytes + J.cap_key_bytes) + N * 64) / std::max<uint64_t>(1, J.max_file_size));
   J.files = A.get<FileOut>(J.cap_files);
   J.b_fnext = A.get<uint32_t>(N);
-  J.t_blocks = A.get<uint32_t>(J.cap_triggers);
   J.t_kept = A.get<uint32_t>(J.cap_triggers);
   J.k_pb = A.get<uint64_t>(N + 1);
   J.b_file = A.get<uint32_t>(N);
@@ -715,7 +713,7 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
   }
   J.cap_wide = (uint32_t)std::min<uint64_t>(J.cap_out / (kEncNarrow / 2) + 16, 0xffffffffu);
   J.wide = A.get<uint2>(J.cap_wide);
-  J.b_crc = J.k_block;
+  J.b_crc = J.k_next;
   J.out = A.output(J.cap_out, r.j->outputs_on_device == 1 || r.j->outputs_on_device == 2);
   if (r.j->keep_decoded && !r.failed) {
     // the survivors' decoded form, kept with the outputs: keys (at most the
@@ -1249,9 +1247,13 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     // latency is what a small batch pays) while the SMs' 4736 resident warps do
     // not get a dozen each, else 256 (a unit's start and end are searched for)
     const uint32_t dec_unit = all_n < 4736ull * 32 * 12 ? 32 : 256;
+    bt.chunk = all_n < 148ull * kShortChunk ? kShortChunk : kChunk;
+    for (auto& r : runs)
+      if (r.N && (uint64_t)r.j->opt.block_size * r.N > (uint64_t)kShortChunk / 4 * r.in_bytes) bt.chunk = kChunk;
     uint32_t max_runs = 1;
     for (uint32_t i = 0; i < B; i++) {
       JobRun& r = runs[i];
+      r.J.chunk = bt.chunk;
       r.J.dec_unit = dec_unit;
       bt.max_dec_units = std::max<uint64_t>(bt.max_dec_units, r.N / dec_unit + 1);
       alloc_tail(r, A, true);
@@ -1560,9 +1562,6 @@ void run_build(lc_job* j, lc_slot& slot) {
     J.e_vlen = A.get<uint32_t>(N);
     J.e_pfx = A.get<uint64_t>(N);
     J.e_tag = A.get<uint64_t>(N);
-    J.k_forced = A.get<uint8_t>(N + 1);
-    CK(cudaMemsetAsync(J.k_forced, 0, N + 1, st));
-    J.kept_pos = A.get<uint32_t>(N + 1);
     r.N = N;
     r.K = kb;
     alloc_tail(r, A, false);

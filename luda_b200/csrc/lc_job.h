@@ -165,6 +165,7 @@ struct JobDev {
   uint32_t* e_vlen;
   uint64_t* e_pfx;           // 8 user-key bytes after the key_skip common bytes, big endian
   uint64_t* e_tag;           // the key's last 8 bytes: (sequence << 8) | type
+  uint32_t* e_hash;          // the bloom hash of the user key (jobs with a filter)
   uint64_t cap_entries;
 
   // merge
@@ -174,11 +175,8 @@ struct JobDev {
   uint64_t* m_pfx_tmp;       // the other buffer of the ping-pong
   uint64_t* m_tag;           // e_tag of m_ids, in merged order (result after the last round)
   uint64_t* m_tag_tmp;       // the other buffer of the ping-pong
-  uint32_t* m_split;         // per merge tile: first-group elements before the tile
-  uint32_t cap_merge_tiles;  // capacity of m_split
   uint8_t* keep;             // per merged position
   uint32_t* gp_idx;          // per merged position: grandparents passed
-  uint32_t* kept_pos;        // exclusive scan of keep (n+1)
   uint32_t* triggers;        // merged positions where ShouldStopBefore fires
   uint32_t cap_triggers;
 
@@ -186,7 +184,8 @@ struct JobDev {
   uint32_t* k_koff;          // survivors, in output order: key offset in the arena,
   uint32_t* k_klen;          // key length,
   uint32_t* k_voff;          // value offset in `in`,
-  uint32_t* k_vlen;          // value length (gathered once from the entry arrays)
+  uint32_t* k_vlen;          // value length,
+  uint32_t* k_hash;          // bloom hash (gathered once from the entry arrays)
 
   // the survivors' decoded form, kept for later jobs (keep_decoded; else null)
   uint8_t* dec_keys;         // keys in survivor order
@@ -198,16 +197,13 @@ struct JobDev {
   uint32_t* k_a;             // size as a restart entry
   uint32_t* k_b;             // size as a prefix-compressed entry
   uint32_t* k_shared;        // shared prefix with the previous kept key
-  uint8_t* k_forced;         // a block (and file) must start here
   uint32_t* k_next;          // first entry of the next block if a block starts here
-  uint8_t* k_bstart;         // block starts here
-  uint32_t* k_block;         // exclusive scan of k_bstart (n+1)
 
   // chain resolution
   uint32_t chunk;            // entries per chunk
-  uint32_t* chunk_table;     // per chunk: exit for each window entry
-  uint32_t* chunk_entry;     // per chunk: resolved entry point
-  uint32_t* group_table;     // per group of kChainGroup chunks: exit for each window entry
+  uint32_t* chunk_table;     // per chunk: exit and blocks for each window entry (chain_word)
+  uint2* chunk_entry;        // per chunk: resolved entry point, first block
+  uint64_t* group_table;     // per group of kChainGroup chunks: exit | blocks << 32
   uint32_t window;           // table width
   uint32_t chain_smem_words; // shared-memory words for staging the chunk tables
   uint32_t reserve_keys;     // 1: decode reserves key-arena space per block (single
@@ -230,13 +226,12 @@ struct JobDev {
   uint64_t* b_gcum;          // prefix of b_gbytes
   uint32_t* b_gkeys;         // keys in the group (at group starts)
   uint32_t* b_fnext;         // first block of the next file if a file starts here
-  uint32_t* t_blocks;        // output block starting at each grandparent cut
   uint32_t* t_kept;          // survivor position of each grandparent cut (ascending)
   uint64_t* k_pb;            // n_kept + 1: prefix sums of k_b (block size estimates)
   uint2* wide;               // (block, window) of the wide blocks, n_wide of them
   uint32_t cap_wide;
   uint32_t* b_crc;           // wide blocks: raw CRC32C registers xored from their windows
-                             // (k_block's memory, which the layout no longer needs)
+                             // (k_next's memory, which the layout no longer needs)
   uint64_t cap_blocks_out;
 
   // files

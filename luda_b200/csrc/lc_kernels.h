@@ -67,8 +67,6 @@ constexpr uint32_t kEncWindow = 4608;  // 9 full CRC rows
 // per position.
 constexpr uint32_t kMergeMaxTile = 4096;
 constexpr uint32_t kMergeSmemPerPos = 14;
-// Entries of m_split a job needs for `entries` entries in `runs` children.
-uint64_t merge_tile_capacity(uint64_t entries, uint32_t runs);
 
 struct Batch {
   const JobDev* d = nullptr;  // device array of B job descriptors
@@ -80,7 +78,7 @@ struct Batch {
   uint64_t max_dec_groups = 0, max_dec_units = 0;  // decode work units
   uint32_t merge_rounds = 0;
   uint32_t max_runs = 1;
-  uint32_t chunk = 4096;
+  uint32_t chunk = 4096;    // survivors per chunk of the block chain
   uint32_t chain_smem_words = 11 * 1024;
   bool any_verify = false;  // some job checks its input blocks' CRCs
   bool any_keep_decoded = false;  // some job keeps its outputs' decoded form
@@ -105,8 +103,6 @@ enum ScanSel : int {
   kScanTblBlocks = 0,  // tbl_nblocks -> tbl_block_base      (total: n_blocks_in)
   kScanBlkEnt,         // blk_nent -> blk_ent_base           (total: n_entries_in)
   kScanBlkKey,         // blk_kbytes -> blk_key_base         (total: key_bytes_in)
-  kScanKeep,           // keep -> kept_pos                   (total: n_kept)
-  kScanBstart,         // k_bstart -> k_block                (total: n_blocks_out)
   kScanBcum,           // tmp32 -> b_cum
   kScanGcum,           // b_gbytes -> b_gcum
   kScanIcum,           // b_isize -> b_icum
@@ -145,13 +141,13 @@ void launch_key_skip(const Batch& bt, cudaStream_t st);
 void launch_merge(const Batch& bt, cudaStream_t st);
 void launch_drop(const Batch& bt, cudaStream_t st);
 void launch_triggers(const Batch& bt, cudaStream_t st);
-void launch_kept_compact(const Batch& bt, cudaStream_t st);
+void launch_kept_compact(const Batch& bt, cudaStream_t st);  // survivors and their entry sizes
 
 // lc_encode.cu -- survivors -> output tables
-void launch_sizes(const Batch& bt, cudaStream_t st);       // also clears the block starts
+void launch_sizes(const Batch& bt, cudaStream_t st);       // flush encoder: entry sizes
 void launch_next(const Batch& bt, cudaStream_t st);
 void launch_chain(const Batch& bt, cudaStream_t st);
-void launch_block_list(const Batch& bt, cudaStream_t st);  // also the block sizes
+void launch_block_sizes(const Batch& bt, cudaStream_t st);
 void launch_files(const Batch& bt, cudaStream_t st);
 void launch_block_layout(const Batch& bt, cudaStream_t st);
 void launch_file_layout(const Batch& bt, cudaStream_t st);

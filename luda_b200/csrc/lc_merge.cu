@@ -3,8 +3,8 @@
 // * Merge: the reference merges its children with MergingIterator
 //   (table/merger.cc:148, linear FindSmallest; on equal keys the earlier child
 //   wins).  Here the children are merged pairwise in rounds with merge path,
-//   in tiles: one thread per tile finds the tile's split by binary search,
-//   then a CTA stages the tile's two stretches (entry ids and their 8-byte
+//   in tiles: two warps find the tile's cuts by search, then the CTA stages
+//   its two stretches (entry ids and their 8-byte
 //   user-key prefixes) in shared memory, merges them there (each thread its
 //   own diagonal) and writes ids, prefixes and tags back coalesced, so that a
 //   round reads and writes 20 bytes per entry and key bytes are read only for
@@ -217,34 +217,33 @@ __device__ __forceinline__ uint32_t src_id(const MergeRound& m, uint64_t i) {
   return m.src_ids ? m.src_ids[i] : (uint32_t)i;
 }
 
-// m_split[g]: elements of the pair's first group before tile g's first
-// diagonal (merge path: the first group wins ties, which keeps the children's
-// order for equal internal keys, as MergingIterator does).  One thread per
-// tile.
-__global__ void k_merge_partition(const JobDev* __restrict__ jobs, uint32_t r, uint32_t rounds,
-                                  uint32_t tile) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
-  const MergeRound m = merge_round(J, r, rounds);
-  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < J.cap_merge_tiles;
-       g += (uint64_t)gridDim.x * blockDim.x) {
-    MergeTile t;
-    if (!merge_tile(J, r, g, tile, &t)) break;
-    const uint64_t d = t.d0, a = t.a0, b = t.a0 + t.na;
-    uint64_t lo = d > t.nb ? d - t.nb : 0, hi = d < t.na ? d : t.na;
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi) >> 1;
+// Elements of the pair's first group before output position d (merge path:
+// the first group wins ties, which keeps the children's order for equal
+// internal keys, as MergingIterator does), by one warp: 32 places a step.
+__device__ __forceinline__ uint64_t merge_split(const JobDev& J, const MergeRound& m,
+                                                const MergeTile& t, uint64_t d) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t a = t.a0, b = t.a0 + t.na;
+  uint64_t lo = d > t.nb ? d - t.nb : 0, hi = d < t.na ? d : t.na;
+  while (lo < hi) {
+    const uint64_t step = (hi - lo + 31) / 32, mid = lo + lane * step;
+    bool le = false;
+    if (mid < hi) {
       const uint64_t ia = a + mid, ib = b + (d - 1 - mid);
-      if (entry_le(J, src_id(m, ia), m.src_pfx[ia], src_id(m, ib), m.src_pfx[ib])) lo = mid + 1;
-      else hi = mid;
+      le = entry_le(J, src_id(m, ia), m.src_pfx[ia], src_id(m, ib), m.src_pfx[ib]);
     }
-    J.m_split[g] = (uint32_t)lo;
+    const int c = __popc(__ballot_sync(0xffffffffu, le));  // true up to the split
+    if (c == 0) break;
+    hi = min(hi, lo + c * step);
+    lo = lo + (c - 1) * step + 1;
   }
+  return lo;
 }
 
-// One tile per CTA step: the tile's stretches of both groups (ids and
-// prefixes) are loaded into shared memory with coalesced reads, every thread
+// One tile per CTA step: two warps find its cuts (a kernel of its own did, one
+// thread per tile and 16 dependent steps: 21 us of an 80k-entry job's two
+// rounds on B200), the tile's stretches of both groups (ids and prefixes) are
+// loaded into shared memory with coalesced reads, every thread
 // finds its own diagonal there and merges `items` outputs as source positions,
 // and the tile is written back with coalesced stores, ids and prefixes from
 // shared memory and the tags from memory by source position (two ascending
@@ -256,6 +255,7 @@ __global__ void __maxnreg__(40) k_merge_tile(const JobDev* __restrict__ jobs, ui
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
+  __shared__ uint64_t s_cut[2];
   if (threadIdx.x == 0) s_failed = J.ctr->error;
   __syncthreads();
   if (s_failed) return;
@@ -266,11 +266,17 @@ __global__ void __maxnreg__(40) k_merge_tile(const JobDev* __restrict__ jobs, ui
   uint16_t* out_src = reinterpret_cast<uint16_t*>(in_ids + tile);  // source position (in the
                                                                    // tile) of each output
   const MergeRound m = merge_round(J, r, rounds);
-  for (uint64_t g = blockIdx.x; g < J.cap_merge_tiles; g += gridDim.x) {
+  for (uint64_t g = blockIdx.x;; g += gridDim.x) {
     MergeTile t;
     if (!merge_tile(J, r, g, tile, &t)) break;
-    const uint64_t i0 = J.m_split[g];
-    const uint64_t i1 = t.last ? t.na : J.m_split[g + 1];
+    __syncthreads();  // the previous tile's cuts have been read
+    if (threadIdx.x < 64) {  // at least two warps (lc_set_tuning)
+      const uint32_t w = threadIdx.x >> 5;
+      const uint64_t cut = w && t.last ? t.na : merge_split(J, m, t, w ? t.d1 : t.d0);
+      if ((threadIdx.x & 31) == 0) s_cut[w] = cut;
+    }
+    __syncthreads();
+    const uint64_t i0 = s_cut[0], i1 = s_cut[1];
     if (i1 < i0 || i1 - i0 > t.d1 - t.d0) {
       // cuts out of order: only children out of order give these, and the
       // order check fails such a job first; the tile is skipped, never read
@@ -334,66 +340,110 @@ __device__ __forceinline__ bool is_base_level(const JobDev& J, const uint8_t* uk
   return true;
 }
 
-__device__ __forceinline__ void drop_one(const JobDev& J, const uint32_t* __restrict__ ids,
-                                         const uint64_t* __restrict__ pfx,
-                                         const uint64_t* __restrict__ tags, uint64_t p) {
-  const uint32_t id = ids[p];
-  const uint64_t upfx = pfx[p];
-  const uint64_t tag = tags[p];
+// The drop rule for merged position p (tag, prefix), after position p - 1
+// (ptag, ppfx).
+__device__ __forceinline__ bool keep_entry(const JobDev& J, uint64_t p, uint64_t tag, uint64_t upfx,
+                                           uint64_t ptag, uint64_t ppfx) {
   const uint32_t type = (uint32_t)(tag & 0xff);
-  const uint64_t seq = tag >> 8;
-  bool drop = false;
-  if (type <= 1) {
-    bool first = true;
-    uint64_t pseq = 0;
-    if (p > 0) {
-      const uint64_t ptag = tags[p - 1];
-      if ((ptag & 0xff) <= 1 && same_user_key(J, ids[p - 1], pfx[p - 1], id, upfx)) {
-        first = false;
-        pseq = ptag >> 8;
-      }
-    }
-    if (!first && pseq <= J.smallest_snapshot) {
-      drop = true;
-    } else if (type == 0 && seq <= J.smallest_snapshot &&
-               is_base_level(J, J.keys + J.e_koff[id], J.e_klen[id] - 8)) {
-      drop = true;
-    }
+  if (type > 1) return true;
+  if (p > 0 && ppfx == upfx && (ptag & 0xff) <= 1 && (ptag >> 8) <= J.smallest_snapshot &&
+      user_key_rest_cmp(J, J.m_ids[p - 1], J.m_ids[p]) == 0)
+    return false;
+  if (type == 0 && (tag >> 8) <= J.smallest_snapshot) {
+    const uint32_t id = J.m_ids[p];
+    if (is_base_level(J, J.keys + J.e_koff[id], J.e_klen[id] - 8)) return false;
   }
-  J.keep[p] = drop ? 0 : 1;
-  if (J.n_gp) {
-    // grandparents passed: count of g with key > largest[g] (internal-key
-    // order); the user-key prefixes decide unless equal
-    uint32_t lo = 0, hi = J.n_gp;
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      const uint64_t gp = J.gp_upfx[mid];
-      const uint32_t mode = J.gp_mode[mid];
-      bool after;
-      if (mode) {  // the grandparent lies outside the keys' common prefix
-        after = mode == 1;
-      } else if (gp != upfx) {
-        after = upfx > gp;
-      } else {
-        const uint64_t go = J.gp_key_off[mid];
-        const uint32_t gl = (uint32_t)(J.gp_key_off[mid + 1] - go);
-        after = ikey_cmp(J.keys + J.e_koff[id], J.e_klen[id], J.gp_keys + go, gl) > 0;
-      }
-      if (after) lo = mid + 1;
-      else hi = mid;
-    }
-    J.gp_idx[p] = lo;
-  }
+  return true;
 }
 
-__global__ void __launch_bounds__(256, 6) k_drop(const JobDev* __restrict__ jobs) {
+// Grandparents passed at merged position p: the count of g with key >
+// largest[g] (internal-key order); the user-key prefixes decide unless equal.
+__device__ __forceinline__ uint32_t grandparents_passed(const JobDev& J, uint64_t p, uint64_t upfx) {
+  uint32_t lo = 0, hi = J.n_gp;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    const uint64_t gp = J.gp_upfx[mid];
+    const uint32_t mode = J.gp_mode[mid];
+    bool after;
+    if (mode) {  // the grandparent lies outside the keys' common prefix
+      after = mode == 1;
+    } else if (gp != upfx) {
+      after = upfx > gp;
+    } else {
+      const uint32_t id = J.m_ids[p];
+      const uint64_t go = J.gp_key_off[mid];
+      const uint32_t gl = (uint32_t)(J.gp_key_off[mid + 1] - go);
+      after = ikey_cmp(J.keys + J.e_koff[id], J.e_klen[id], J.gp_keys + go, gl) > 0;
+    }
+    if (after) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Survivors are found and gathered in tiles of kKeepTile merged positions:
+// k_drop marks them and counts each tile's, k_kept_compact gives every tile
+// its place (the counts before it) and gathers.  A warp of k_drop loads four
+// strips of its positions ahead (tag and prefix; the position before a lane's
+// is its neighbour's, by shuffle); entry ids only where two prefixes are equal.
+// Bound by the two streams' latency: with the flags' scan and the gather as
+// kernels of their own, 8M entries took 117 + 26 + 91 us on B200 and the
+// entry sizes 108 more; k_drop and k_kept_compact take 71 + 181.
+constexpr uint32_t kKeepTile = 512;
+constexpr uint32_t kKeepThreads = 128;
+constexpr uint32_t kKeepStrips = kKeepTile / kKeepThreads;
+static_assert(kKeepTile >= 512, "the counts fit scan_scratch (scan_scratch_elems)");
+
+__global__ void __launch_bounds__(kKeepThreads, 12) k_drop(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
+  __shared__ uint32_t s_failed, s_count;
+  if (threadIdx.x == 0) {
+    s_failed = J.ctr->error;
+    s_count = 0;
+  }
+  __syncthreads();
+  if (s_failed) return;
   const uint64_t n = J.ctr->n_entries_in;
-  for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (uint64_t)gridDim.x * blockDim.x)
-    drop_one(J, J.m_ids, J.m_pfx, J.m_tag, p);
+  uint32_t* counts = reinterpret_cast<uint32_t*>(J.scan_scratch);
+  const uint64_t* __restrict__ tags = J.m_tag;
+  const uint64_t* __restrict__ pfx = J.m_pfx;
+  const bool gps = J.n_gp != 0;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint64_t t = blockIdx.x; t * kKeepTile < n; t += gridDim.x) {
+    const uint64_t w0 = t * kKeepTile + 32 * kKeepStrips * warp;  // the warp's positions
+    uint64_t tg[kKeepStrips], px[kKeepStrips];
+#pragma unroll
+    for (uint32_t i = 0; i < kKeepStrips; i++) {
+      const uint64_t p = w0 + 32 * i + lane;
+      tg[i] = p < n ? tags[p] : 0xff;
+      px[i] = p < n ? pfx[p] : 0;
+    }
+    uint64_t lt = w0 > 0 && w0 < n ? tags[w0 - 1] : 0, lp = w0 > 0 && w0 < n ? pfx[w0 - 1] : 0;
+    uint32_t cnt = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kKeepStrips; i++) {
+      const uint64_t p = w0 + 32 * i + lane;
+      const uint64_t ut = __shfl_up_sync(0xffffffffu, tg[i], 1);
+      const uint64_t up = __shfl_up_sync(0xffffffffu, px[i], 1);
+      bool keep = false;
+      if (p < n) {
+        keep = keep_entry(J, p, tg[i], px[i], lane ? ut : lt, lane ? up : lp);
+        J.keep[p] = keep ? 1 : 0;
+        if (gps) J.gp_idx[p] = grandparents_passed(J, p, px[i]);
+      }
+      lt = __shfl_sync(0xffffffffu, tg[i], 31);
+      lp = __shfl_sync(0xffffffffu, px[i], 31);
+      cnt += __popc(__ballot_sync(0xffffffffu, keep));
+    }
+    if (lane == 0 && cnt) atomicAdd(&s_count, cnt);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      counts[t] = s_count;
+      s_count = 0;
+    }
+    __syncthreads();
+  }
 }
 
 // gp_first[g] = first merged position whose grandparent count reaches g
@@ -470,37 +520,188 @@ __global__ void k_triggers(const JobDev* __restrict__ jobs, bool in_smem) {
   J.ctr->n_triggers = cnt;
 }
 
-__global__ void k_kept_compact(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
-  const uint32_t* __restrict__ ids = J.m_ids;
-  const uint64_t n = J.ctr->n_entries_in;
-  for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (uint64_t)gridDim.x * blockDim.x) {
-    if (J.keep[p]) {
-      const uint32_t k = J.kept_pos[p];
-      const uint32_t id = ids[p];
-      J.k_koff[k] = J.e_koff[id];
-      J.k_klen[k] = J.e_klen[id];
-      J.k_voff[k] = J.e_voff[id];
-      J.k_vlen[k] = J.e_vlen[id];
-      J.k_forced[k] = 0;
+// Sum of v over the CTA (kKeepThreads threads); every thread gets it, and *before
+// the sum over the threads before it.
+__device__ __forceinline__ uint32_t keep_scan(uint32_t v, uint32_t* s_warp, uint32_t* before) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += u;
+  }
+  __syncthreads();  // the last call's sums have been read
+  if (lane == 31) s_warp[warp] = x;
+  __syncthreads();
+  uint32_t all = 0, b = 0;
+#pragma unroll
+  for (uint32_t w = 0; w < kKeepThreads / 32; w++) {
+    const uint32_t y = s_warp[w];
+    if (w < warp) b += y;
+    all += y;
+  }
+  *before = b + x - v;
+  return all;
+}
+
+// The last survivor before tile t (which has some before it), by one warp.
+__device__ __forceinline__ uint64_t last_kept_before(const JobDev& J, const uint32_t* counts,
+                                                     uint64_t t) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint64_t hi = t;  // the tile, from 32 at a time
+  while (true) {
+    const bool any = hi > lane && counts[hi - 1 - lane] != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, any);
+    if (m) {
+      hi = hi - 1 - (__ffs(m) - 1);
+      break;
+    }
+    hi -= 32;
+  }
+  for (int32_t w = kKeepTile / 32 - 1; w >= 0; w--) {
+    const uint64_t p = hi * kKeepTile + 32 * w + lane;
+    const unsigned m = __ballot_sync(0xffffffffu, J.keep[p] != 0);
+    if (m) return p - lane + (31 - __clz(m));
+  }
+  return 0;  // not reached
+}
+
+// The tile's survivors gather their entries and get their sizes: as a restart
+// entry (k_a), as a prefix-compressed entry (k_b), and the prefix each shares
+// with the survivor before it (its neighbour's id, key length and prefix come by
+// shuffle).  The two prefixes (the 8 user-key bytes after the job's common
+// ones) give the shared length when they differ inside both user keys; key
+// bytes are read only otherwise.  Two survivors per thread at a time, so that
+// their loads overlap.
+__device__ __forceinline__ void gather_kept(const JobDev& J, const uint16_t* s_list, uint32_t total,
+                                            uint64_t t0, uint32_t base, uint64_t prev,
+                                            unsigned long long* kb, unsigned long long* vb) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t L = J.ctr->key_skip;
+  constexpr uint32_t kTwo = 2;
+  for (uint32_t j0 = 32 * kTwo * warp; j0 < total; j0 += kTwo * kKeepThreads) {
+    uint32_t id[kTwo], koff[kTwo], kl[kTwo], voff[kTwo], vl[kTwo], hash[kTwo];
+    uint64_t px[kTwo];
+#pragma unroll
+    for (uint32_t i = 0; i < kTwo; i++) {
+      const uint32_t j = j0 + 32 * i + lane;
+      const uint64_t p = t0 + s_list[j < total ? j : 0];
+      id[i] = J.m_ids[p];
+      px[i] = J.m_pfx[p];
+    }
+    // the survivor before the warp's first
+    const bool any_prev = base + j0 != 0;
+    const uint64_t pp = j0 ? t0 + s_list[j0 - 1] : prev;
+    uint32_t lid = any_prev ? J.m_ids[pp] : 0u, lkl = any_prev ? J.e_klen[lid] : 8u;
+    uint64_t lpx = any_prev ? J.m_pfx[pp] : 0u;
+#pragma unroll
+    for (uint32_t i = 0; i < kTwo; i++) {
+      koff[i] = J.e_koff[id[i]], kl[i] = J.e_klen[id[i]];
+      voff[i] = J.e_voff[id[i]], vl[i] = J.e_vlen[id[i]];
+      hash[i] = J.bits_per_key > 0 ? J.e_hash[id[i]] : 0u;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kTwo; i++) {
+      const uint32_t j = j0 + 32 * i + lane;
+      uint32_t pid = __shfl_up_sync(0xffffffffu, id[i], 1);
+      uint32_t pl = __shfl_up_sync(0xffffffffu, kl[i], 1);
+      uint64_t ppx = __shfl_up_sync(0xffffffffu, px[i], 1);
+      if (lane == 0) pid = lid, pl = lkl, ppx = lpx;
+      lid = __shfl_sync(0xffffffffu, id[i], 31);
+      lkl = __shfl_sync(0xffffffffu, kl[i], 31);
+      lpx = __shfl_sync(0xffffffffu, px[i], 31);
+      if (j >= total) continue;
+      const uint32_t k = base + j;
+      uint32_t shared = 0;
+      if (k) {
+        const uint32_t m = min(kl[i], pl), mu = m - 8;
+        const uint64_t d = px[i] ^ ppx;
+        shared = min(L + (d ? (uint32_t)__clzll(d) >> 3 : 8u), mu);
+        if (!d || shared == mu) {
+          const uint8_t *x = J.keys + koff[i], *y = J.keys + J.e_koff[pid];
+          while (shared < m && x[shared] == y[shared]) shared++;
+        }
+      }
+      J.k_koff[k] = koff[i];
+      J.k_klen[k] = kl[i];
+      J.k_voff[k] = voff[i];
+      J.k_vlen[k] = vl[i];
+      if (J.bits_per_key > 0) J.k_hash[k] = hash[i];
+      J.k_a[k] = 1 + varint_len32(kl[i]) + varint_len32(vl[i]) + kl[i] + vl[i];
+      J.k_b[k] = varint_len32(shared) + varint_len32(kl[i] - shared) + varint_len32(vl[i]) +
+                 (kl[i] - shared) + vl[i];
+      J.k_shared[k] = shared;
+      *kb += kl[i];
+      *vb += vl[i];
     }
   }
 }
 
-__global__ void k_forced(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(kKeepThreads, 8) k_kept_compact(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t nk = J.kept_pos[J.ctr->n_entries_in];
-  if (i == 0 && nk > 0) J.k_forced[0] = 1;
-  if (i < J.ctr->n_triggers) {
-    const uint32_t kp = J.kept_pos[J.triggers[i]];
-    if (kp < nk) J.k_forced[kp] = 1;
-    J.t_kept[i] = kp;
+  __shared__ uint32_t s_failed, s_warp[kKeepThreads / 32];
+  __shared__ uint16_t s_list[kKeepTile];  // the tile's survivors
+  __shared__ uint64_t s_prev;
+  if (threadIdx.x == 0) s_failed = J.ctr->error;
+  __syncthreads();
+  if (s_failed) return;
+  const uint64_t n = J.ctr->n_entries_in;
+  if (blockIdx.x * (uint64_t)kKeepTile >= n) return;
+  const uint32_t* counts = reinterpret_cast<const uint32_t*>(J.scan_scratch);
+  const uint32_t nt = J.ctr->n_triggers;
+  const auto before = [&](uint64_t a, uint64_t z) -> uint32_t {  // survivors of tiles [a, z)
+    uint32_t x = 0, ex;
+    for (uint64_t i = a + threadIdx.x; i < z; i += kKeepThreads) x += counts[i];
+    return keep_scan(x, s_warp, &ex);
+  };
+  uint32_t base = before(0, blockIdx.x);
+  unsigned long long kb = 0, vb = 0;
+  for (uint64_t t = blockIdx.x; t * kKeepTile < n; t += gridDim.x) {
+    const uint64_t t0 = t * kKeepTile, tb = t0 + 4 * threadIdx.x;
+    uint32_t w = tb < n ? *reinterpret_cast<const uint32_t*>(J.keep + tb) : 0;  // four flags
+    if (tb < n && n - tb < 4) w &= (1u << (8 * (uint32_t)(n - tb))) - 1;
+    uint32_t at;
+    const uint32_t total = keep_scan((uint32_t)__popc(w), s_warp, &at);
+    for (uint32_t m = w; m; m &= m - 1) s_list[at++] = (uint16_t)(4 * threadIdx.x + ((__ffs(m) - 1) >> 3));
+    if (base && threadIdx.x < 32) {
+      const uint64_t x = last_kept_before(J, counts, t);
+      if (threadIdx.x == 0) s_prev = x;
+    }
+    __syncthreads();
+    gather_kept(J, s_list, total, t0, base, s_prev, &kb, &vb);
+    // the survivors before each grandparent cut in the tile
+    if (nt) {
+      uint32_t lo = 0, hi = nt;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (J.triggers[mid] < t0) lo = mid + 1;
+        else hi = mid;
+      }
+      for (uint32_t i = lo + threadIdx.x; i < nt && J.triggers[i] < t0 + kKeepTile; i += kKeepThreads) {
+        const uint32_t off = (uint32_t)(J.triggers[i] - t0);
+        uint32_t a = 0, z = total;
+        while (a < z) {
+          const uint32_t mid = (a + z) >> 1;
+          if (s_list[mid] < off) a = mid + 1;
+          else z = mid;
+        }
+        J.t_kept[i] = base + a;
+      }
+    }
+    if (t0 + kKeepTile >= n && threadIdx.x == 0) J.ctr->n_kept = base + total;
+    if ((t + gridDim.x) * kKeepTile < n) base += total + before(t + 1, t + gridDim.x);
+    __syncthreads();  // the list is rewritten
+  }
+  // survivor byte totals, one atomic per warp
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    kb += __shfl_xor_sync(0xffffffffu, kb, o);
+    vb += __shfl_xor_sync(0xffffffffu, vb, o);
+  }
+  if ((threadIdx.x & 31) == 0 && (kb | vb)) {
+    atomicAdd((unsigned long long*)&J.ctr->kept_key_bytes, kb);
+    atomicAdd((unsigned long long*)&J.ctr->kept_value_bytes, vb);
   }
 }
 
@@ -528,11 +729,6 @@ void merge_kernel_attributes() {
                        (int)(kMergeSmemPerPos * kMergeMaxTile));
 }
 
-uint64_t merge_tile_capacity(uint64_t entries, uint32_t runs) {
-  // tiles of at least 64 positions, one partial tile per pair
-  return entries / 64 + runs + 2;
-}
-
 void launch_key_skip(const Batch& bt, cudaStream_t st) {
   launch(k_key_skip, dim3(1, bt.B), 256, 0, st, bt.d);
   launch(k_prefix, dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st, bt.d);
@@ -548,13 +744,13 @@ void launch_merge(const Batch& bt, cudaStream_t st) {
   const uint32_t tile = threads * items;
   const uint64_t tiles = bt.max_entries / tile + bt.max_runs + 1;
   for (uint32_t r = 0; r < bt.merge_rounds; r++) {
-    launch(k_merge_partition, dim3(grid_x(tiles, 128, bt.per_job(148 * 16)), bt.B), 128, 0, st, bt.d, r, bt.merge_rounds, tile);
     launch(k_merge_tile, dim3(flat_ctas(bt, tiles, 1), bt.B), threads, kMergeSmemPerPos * (size_t)tile, st, bt.d, r, bt.merge_rounds, items);
   }
 }
 
 void launch_drop(const Batch& bt, cudaStream_t st) {
-  launch(k_drop, dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st, bt.d);
+  launch(k_drop, dim3(grid_x(bt.max_entries, kKeepTile, bt.per_job(148 * 12)), bt.B), kKeepThreads, 0,
+         st, bt.d);
 }
 
 void launch_triggers(const Batch& bt, cudaStream_t st) {
@@ -566,8 +762,8 @@ void launch_triggers(const Batch& bt, cudaStream_t st) {
 }
 
 void launch_kept_compact(const Batch& bt, cudaStream_t st) {
-  launch(k_kept_compact, dim3(flat_ctas(bt, bt.max_entries, 256), bt.B), 256, 0, st, bt.d);
-  launch(k_forced, dim3((bt.max_cap_triggers + 255) / 256 + 1, bt.B), 256, 0, st, bt.d);
+  launch(k_kept_compact, dim3(grid_x(bt.max_entries, kKeepTile, bt.per_job(148 * 12)), bt.B), kKeepThreads,
+         0, st, bt.d);
 }
 
 }  // namespace lc

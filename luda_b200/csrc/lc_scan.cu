@@ -61,24 +61,6 @@ struct ScanOf<kScanBlkKey> {
   static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->key_bytes_in; }
 };
 template <>
-struct ScanOf<kScanKeep> {
-  using TI = uint8_t;
-  using TO = uint32_t;
-  static __device__ const TI* in(const JobDev& J) { return J.keep; }
-  static __device__ TO* out(const JobDev& J) { return J.kept_pos; }
-  static __device__ uint64_t n(const JobDev& J) { return J.ctr->n_entries_in; }
-  static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->n_kept; }
-};
-template <>
-struct ScanOf<kScanBstart> {
-  using TI = uint8_t;
-  using TO = uint32_t;
-  static __device__ const TI* in(const JobDev& J) { return J.k_bstart; }
-  static __device__ TO* out(const JobDev& J) { return J.k_block; }
-  static __device__ uint64_t n(const JobDev& J) { return J.ctr->n_kept; }
-  static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->n_blocks_out; }
-};
-template <>
 struct ScanOf<kScanBcum> {
   using TI = uint32_t;
   using TO = uint64_t;
@@ -318,8 +300,6 @@ void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st) {
     case kScanTblBlocks: scan_sel<kScanTblBlocks>(bt, n_est, st); break;
     case kScanBlkEnt: scan_sel<kScanBlkEnt>(bt, n_est, st); break;
     case kScanBlkKey: scan_sel<kScanBlkKey>(bt, n_est, st); break;
-    case kScanKeep: scan_sel<kScanKeep>(bt, n_est, st); break;
-    case kScanBstart: scan_sel<kScanBstart>(bt, n_est, st); break;
     case kScanBcum: scan_sel<kScanBcum>(bt, n_est, st); break;
     case kScanGcum: scan_sel<kScanGcum>(bt, n_est, st); break;
     case kScanIcum: scan_sel<kScanIcum>(bt, n_est, st); break;
@@ -329,8 +309,10 @@ void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st) {
   }
 }
 
-// tile sums for arrays of up to n_cap elements (TO up to 8 bytes)
-uint64_t scan_scratch_elems(uint64_t n_cap) { return (n_cap + 1) / kTile + 2; }
+// tile sums for arrays of up to n_cap elements: 8 bytes for every kTile of them
+// here, 4 bytes for every 512 in the drop rule's counts
+uint64_t scan_scratch_elems(uint64_t n_cap) { return (n_cap + 1) / 1024 + 4; }
+static_assert(kTile >= 1024, "scan_scratch_elems");
 
 namespace {
 
