@@ -205,6 +205,7 @@ struct FastMod {
   uint64_t M;
   uint32_t d;
   __device__ __forceinline__ explicit FastMod(uint32_t div) : M(~0ull / div + 1), d(div) {}
+  __device__ __forceinline__ FastMod(uint64_t m, uint32_t div) : M(m), d(div) {}
   __device__ __forceinline__ uint32_t operator()(uint32_t a) const {
     return (uint32_t)__umul64hi(M * a, d);
   }
