@@ -568,17 +568,24 @@ __global__ void k_run_bounds(const JobDev* __restrict__ jobs) {
 // from the decoded form of an earlier output) is cut into runs of
 // kDecRunSlice entries whose records come from that form.
 //
-// A scan of the key lengths gives every key its place in the arena (keys in
-// entry order).
+// A scan of the key lengths, each rounded up to a multiple of 8, gives every
+// key its slot in the arena (in entry order).
 //
 // Pass 2 (k_decode_keys): one warp per unit of about dec_unit entries, cut
 // at entries without a shared prefix (every restart has none), in rounds of
-// 32, one lane per entry: each lane copies its key delta into the warp's key
-// buffer at the key's place; the shared prefixes then follow in entry order
-// (a key's prefix is the head of the previous key, complete by then); the
-// round's keys go out to the arena with 16-byte stores and the entry arrays
-// with coalesced stores.  The round's last key carries into the next round;
-// a round whose keys do not fit the buffer is built in the arena directly.
+// 32, one lane per entry.  A round whose keys have at most 32 bytes is decoded
+// in registers: a lane loads its key delta at the key's own byte positions,
+// and the shared prefixes come by a scan over the lanes (a key is a head of
+// the key before it and its own bytes; two such steps compose into one).
+// Rounds with longer keys go through the warp's key buffer in shared memory:
+// key deltas at the keys' places, then the shared prefixes in entry order, then
+// 16-byte stores to the arena; keys beyond that buffer are built in the arena.
+// The round's last key carries into the next round.
+//
+// Pass 1 is bound by its chain of loads (a header names the next one's place),
+// pass 2 by issue.  8M entries of 32-byte keys on B200: pass 2 took 395 us
+// (452 with the filters' hashes) when every round went through the buffer,
+// whose bytewise steps met 8-way bank conflicts at this key length, 241 so.
 constexpr uint32_t kDecGroupMax = 32;   // data blocks per warp in pass 1
 constexpr uint32_t kDecRunSlice = 16;   // pseudo-block entries per lane
 constexpr uint32_t kDecPseudo = 0xffffu;  // shared length of a pseudo entry's record
@@ -623,7 +630,8 @@ __global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* __restrict
     s_rb[warp][lane] = warp_excl<uint32_t>(nr, &nrt);
     if (lane == 0) s_rb[warp][kDecGroupMax] = nrt;
     __syncwarp();
-    uint64_t kb = 0;
+    const uint32_t pad = J.key_pad;
+    uint64_t kb = 0, kr = 0;
     uint32_t maxk = 0;
     bool bad = false, short_key = false, long_key = false;
     for (uint32_t q0 = 0; q0 < nrt; q0 += 32) {
@@ -656,6 +664,7 @@ __global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* __restrict
           J.e_rec[e] = dec_record((uint32_t)b, kDecPseudo, kl, vl, (uint32_t)(T.off + vp));
           J.e_klen[e] = kl;
           kb += kl;
+          kr += (kl + pad) & ~pad;
           maxk = max(maxk, kl);
         }
         continue;
@@ -690,6 +699,7 @@ __global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* __restrict
         rec[k] = dec_record(doff, sh, kl, vl, doff + ns);
         klen[k] = kl;
         kb += kl;
+        kr += (kl + pad) & ~pad;
         maxk = max(maxk, kl);
         prev = kl;
         qp = d + ns + vl;
@@ -700,11 +710,12 @@ __global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* __restrict
     const bool any_short = __any_sync(0xffffffffu, short_key);
     const bool any_long = __any_sync(0xffffffffu, long_key);
     kb = warp_sum(kb);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) maxk = max(maxk, __shfl_xor_sync(0xffffffffu, maxk, o));
+    kr = warp_sum(kr);
+    maxk = __reduce_max_sync(0xffffffffu, maxk);
     if (lane == 0) {
       atomicMax(&J.ctr->max_klen, maxk);
       atomicAdd((unsigned long long*)&J.ctr->key_total, (unsigned long long)kb);
+      atomicAdd((unsigned long long*)&J.ctr->key_round, (unsigned long long)kr);
       if (any_bad) set_error(J.ctr, kErrBadBlock, (uint32_t)g0);
       else if (any_short) set_error(J.ctr, kErrShortKey, (uint32_t)g0);
       else if (any_long) set_error(J.ctr, kErrLimit, 4);
@@ -714,17 +725,9 @@ __global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* __restrict
   }
 }
 
-// The arena holds every key (k_decode_keys checks it before writing any).
-__global__ void k_decode_fit(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (threadIdx.x == 0 && !J.ctr->error && J.ctr->key_total > J.cap_key_bytes)
-    set_error(J.ctr, J.reserve_keys ? kErrRetryExact : kErrArenaOverflow, 5);
-}
-
 struct DecKeysSmem {
   uint8_t buf[kDecKeyBuf];    // the round's keys, at the arena's 16-byte phase
-  uint8_t last[kDecLastKey];  // the previous round's last key
+  __align__(16) uint8_t last[kDecLastKey];  // the previous round's last key
 };
 
 // The key bytes a record points at: the key delta in `in`, or a pseudo
@@ -752,6 +755,116 @@ __device__ __forceinline__ uint64_t dec_unit_start(const JobDev& J, uint64_t e, 
   return n;
 }
 
+constexpr uint32_t kDecRegWords = 8;  // key words a lane decodes in registers
+
+// Bytes of key word q below byte s of the key.
+__device__ __forceinline__ uint32_t dec_below(uint32_t s, uint32_t q) {
+  const int32_t n = (int32_t)s - 4 * (int32_t)q;
+  return n >= 4 ? 0xffffffffu : (n <= 0 ? 0u : (1u << (8 * n)) - 1u);
+}
+
+// The shared prefixes of a round's keys w (at most 4 N bytes each, s of them
+// the lane's own): key l takes its bytes below s from the key o before it, s
+// becoming the least shared length over those o keys, until s is 0 or reaches
+// before the round (`last`).
+template <uint32_t N>
+__device__ __forceinline__ void dec_share(uint32_t (&w)[kDecRegWords], uint32_t s, const uint8_t* last,
+                                          uint32_t lane) {
+#pragma unroll
+  for (uint32_t k = 0; k < 5; k++) {
+    const uint32_t o = 1u << k;
+    const uint32_t ps = __shfl_up_sync(0xffffffffu, s, o);
+    const uint32_t take = lane >= o ? s : 0u;
+#pragma unroll
+    for (uint32_t q = 0; q < N; q++) {
+      const uint32_t pw = __shfl_up_sync(0xffffffffu, w[q], o), m = dec_below(take, q);
+      w[q] = (w[q] & ~m) | (pw & m);
+    }
+    if (lane >= o) s = min(s, ps);
+  }
+  if (!s) return;
+#pragma unroll
+  for (uint32_t q = 0; q < N; q++) {
+    const uint32_t m = dec_below(s, q);
+    w[q] = (w[q] & ~m) | (*reinterpret_cast<const uint32_t*>(last + 4 * q) & m);
+  }
+}
+
+// A round of keys of at most 4 kDecRegWords bytes, lane l's key delta at src
+// (key bytes [sh, kl)); `last`: the key before the round's first (read only
+// when that one shares a prefix), then the round's last key.
+__device__ __forceinline__ void decode_round_regs(const JobDev& J, uint8_t* last, uint64_t e,
+                                                  bool valid, uint4 rec, const uint8_t* src,
+                                                  uint32_t kl, uint32_t sh, uint32_t cnt,
+                                                  uint32_t lane) {
+  uint32_t w[kDecRegWords];
+#pragma unroll
+  for (uint32_t q = 0; q < kDecRegWords; q++) w[q] = 0u;
+  if (valid) {
+    const uintptr_t s = reinterpret_cast<uintptr_t>(src), s0 = s - sh;  // s0: the key's byte 0
+    const uintptr_t b0 = s0 & ~uintptr_t(3);
+    const uint32_t fsh = 8 * (uint32_t)(s0 & 3);
+    const uint32_t first = (uint32_t)(s - b0), end = first + (kl - sh);  // needed bytes from b0
+    uint32_t x[kDecRegWords + 1];
+#pragma unroll
+    for (uint32_t i = 0; i <= kDecRegWords; i++)
+      x[i] = (4 * i + 4 > first && 4 * i < end) ? __ldg(reinterpret_cast<const uint32_t*>(b0) + i) : 0u;
+#pragma unroll
+    for (uint32_t q = 0; q < kDecRegWords; q++) w[q] = __funnelshift_r(x[q], x[q + 1], fsh);
+  }
+  const uint32_t s = valid ? sh : 0;
+  const uint32_t smax = __reduce_max_sync(0xffffffffu, s);
+  if (smax > 16) dec_share<kDecRegWords>(w, s, last, lane);
+  else if (smax > 4) dec_share<4>(w, s, last, lane);
+  else if (smax) dec_share<1>(w, s, last, lane);
+  __syncwarp();  // the previous key has been read
+  if (lane == cnt - 1) {
+#pragma unroll
+    for (uint32_t q = 0; q < kDecRegWords; q += 4)
+      *reinterpret_cast<uint4*>(last + 4 * q) = make_uint4(w[q], w[q + 1], w[q + 2], w[q + 3]);
+  }
+  if (!valid) return;
+  uint64_t* d = reinterpret_cast<uint64_t*>(J.keys + J.e_koff[e]);  // the slot: 8-byte aligned
+#pragma unroll
+  for (uint32_t q = 0; q < kDecRegWords; q += 2)
+    if (4 * q < kl) d[q / 2] = (uint64_t)w[q] | ((uint64_t)w[q + 1] << 32);
+  const uint32_t u = kl - 8;  // user key bytes
+  // the first 8 user-key bytes, big endian, zero padded
+  uint64_t p = ((uint64_t)__byte_perm(w[0], 0, 0x0123) << 32) | __byte_perm(w[1], 0, 0x0123);
+  if (u < 8) p = u ? p & (~0ull << (64 - 8 * u)) : 0;
+  // the last 8 bytes
+  const uint32_t t = u >> 2;  // words t.. of the key, moved down by t's bits
+  uint32_t y[6], z[4];
+#pragma unroll
+  for (uint32_t q = 0; q < 6; q++) y[q] = (t & 4) ? (q + 4 < kDecRegWords ? w[(q + 4) & 7] : 0u) : w[q];
+#pragma unroll
+  for (uint32_t q = 0; q < 4; q++) z[q] = (t & 2) ? y[q + 2] : y[q];
+  const uint32_t t0 = (t & 1) ? z[1] : z[0], t1 = (t & 1) ? z[2] : z[1], t2 = (t & 1) ? z[3] : z[2];
+  const uint32_t ts = 8 * (u & 3);
+  const uint64_t tag = (uint64_t)__funnelshift_r(t0, t1, ts) | ((uint64_t)__funnelshift_r(t1, t2, ts) << 32);
+  J.e_voff[e] = rec.w;
+  J.e_vlen[e] = rec.z;
+  J.e_pfx[e] = p;
+  J.e_tag[e] = tag;
+  if (J.bits_per_key > 0) {  // bloom_hash
+    const uint32_t m = 0xc6a4a793u;
+    uint32_t h = 0xbc9f1d34u ^ (u * m);
+#pragma unroll
+    for (uint32_t q = 0; q + 2 < kDecRegWords; q++) {
+      if (4 * q + 4 <= u) {
+        h += w[q];
+        h *= m;
+        h ^= h >> 16;
+      } else if (4 * q < u) {
+        h += w[q] & ((1u << (8 * (u - 4 * q))) - 1u);
+        h *= m;
+        h ^= h >> 24;
+      }
+    }
+    J.e_hash[e] = h;
+  }
+}
+
 __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict__ jobs) {
   pdl_begin();
   __shared__ JobDev s_job;
@@ -766,6 +879,11 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   DecKeysSmem& W = s_w[warp];
   if (J.ctr->error) return;
+  if (J.ctr->key_round > J.cap_key_bytes) {  // the arena does not hold the keys
+    set_error(J.ctr, J.reserve_keys ? kErrRetryExact : kErrArenaOverflow, 5);
+    return;
+  }
+  const uint32_t pad = J.key_pad;
   const uint64_t n = J.ctr->n_entries_in;
   const uint64_t unit = J.dec_unit, nunits = (n + unit - 1) / unit;
   for (uint64_t u = (uint64_t)blockIdx.x * 8 + warp; u < nunits; u += (uint64_t)gridDim.x * 8) {
@@ -781,15 +899,19 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
       const uint32_t kl = rec.y >> 16;
       const uint32_t sh = (rec.y & 0xffff) == kDecPseudo ? 0 : (rec.y & 0xffff);
       const uint8_t* src = valid ? dec_delta(J, e, rec) : nullptr;
+      const uint32_t mk = __reduce_max_sync(0xffffffffu, kl);
+      const uint32_t sh0 = __shfl_sync(0xffffffffu, sh, 0);
+      if (mk <= 4 * kDecRegWords && pad && (sh0 == 0 || last_staged)) {
+        decode_round_regs(J, W.last, e, valid, rec, src, kl, sh, cnt, lane);
+        last_staged = true;
+        __syncwarp();
+        continue;
+      }
       const uint64_t kpos = J.e_koff[r0];  // arena offset of the round's first key
       uint32_t tot;
-      const uint32_t ko = warp_excl<uint32_t>(kl, &tot);  // offset within the round
-      uint32_t mk = kl;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mk = max(mk, __shfl_xor_sync(0xffffffffu, mk, o));
+      const uint32_t ko = warp_excl<uint32_t>((kl + pad) & ~pad, &tot);  // offset within the round
       uint8_t* gdst = J.keys + kpos;
       const uint32_t kph = (uint32_t)(reinterpret_cast<uintptr_t>(gdst) & 15);
-      const uint32_t sh0 = __shfl_sync(0xffffffffu, sh, 0);
       const uint32_t lkl = __shfl_sync(0xffffffffu, kl, cnt - 1);
       const uint32_t lko = __shfl_sync(0xffffffffu, ko, cnt - 1);
       if (tot + kph + 16 <= kDecKeyBuf && mk <= kDecLastKey && (sh0 == 0 || last_staged)) {
@@ -960,7 +1082,6 @@ void launch_block_decode(const Batch& bt, cudaStream_t st) {
   // CTA
   launch(k_decode_walk, dim3(grid_x(bt.max_dec_groups, 8, bt.per_job(148 * 5)), bt.B), 256, 0, st, bt.d);
   scan_batch(kScanDecKlen, bt, bt.max_entries, st);
-  launch(k_decode_fit, dim3(1, bt.B), 32, 0, st, bt.d);
   launch(k_decode_keys, dim3(grid_x(bt.max_dec_units, 8, bt.per_job(148 * 4)), bt.B), 256, 0, st, bt.d);
 }
 void launch_entries_from_offsets(const Batch& bt, cudaStream_t st) {

@@ -1213,13 +1213,12 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
         any_zeroed = true;
       }
       r.N = r.failed ? 0 : hc[i].n_entries_in;
-      if (exact) {
-        r.K = r.failed ? 0 : hc[i].key_bytes_in;
-        r.max_klen = std::max<uint32_t>(hc[i].max_klen, 8);
-      } else {
-        r.K = r.failed ? 0 : std::min<uint64_t>(r.in_bytes + 65536, (1ull << 32) - 1);
-        r.max_klen = kFastMaxKey;
-      }
+      // the key arena: the keys' bytes (counted, or the input's: see
+      // kFastMaxKey), and 8-byte slots while their offsets fit 32 bits
+      r.K = r.failed ? 0 : exact ? hc[i].key_bytes_in : r.in_bytes + 65536;
+      r.J.key_pad = r.K + 8 * r.N < (1ull << 32) ? 7 : 0;
+      r.K = std::min<uint64_t>(r.K + (r.J.key_pad ? 8 * r.N : 0), (1ull << 32) - 1);
+      r.max_klen = exact ? std::max<uint32_t>(hc[i].max_klen, 8) : kFastMaxKey;
       r.J.reserve_keys = exact ? 0 : 1;
       r.J.max_key_len = kFastMaxKey;
       // pass 1 of the decode: as many blocks to a warp as have 32 restart runs
@@ -1234,7 +1233,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       }
       bt.max_dec_groups = std::max<uint64_t>(bt.max_dec_groups, hc[i].n_blocks_in / r.J.dec_group + 1);
       r.j->entries_in = r.N;
-      r.j->key_bytes_in = exact ? r.K : 0;
+      r.j->key_bytes_in = exact && !r.failed ? hc[i].key_bytes_in : 0;
     }
     // (the zeroed counters are uploaded below, from pinned memory)
     uint64_t all_n = 0, max_n = 1;
@@ -1373,7 +1372,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
         r.failed = true;
         continue;
       }
-      if (!exact) r.j->key_bytes_in = hc[i].key_cursor;
+      if (!exact) r.j->key_bytes_in = hc[i].key_total;
       std::string m;
       lc_status s = counters_status(hc[i], &m);
       if (s != LC_OK) {

@@ -52,10 +52,11 @@ struct Counters {
   uint32_t pad;
   uint64_t kept_key_bytes;    // internal-key bytes of the survivors
   uint64_t kept_value_bytes;  // value bytes of the survivors
-  uint64_t key_cursor;        // key bytes of the decoded entries (the scan of their lengths)
+  uint64_t key_cursor;        // arena bytes of the decoded keys (the scan of their slots)
   uint32_t key_skip;          // user-key bytes every input key shares (prefixes start after them)
   uint32_t pad2;
   uint64_t key_total;         // decoded key bytes, summed by the decode's first pass
+  uint64_t key_round;         // the same, every key rounded up to its slot (JobDev::key_pad)
 };
 
 struct TableDesc {
@@ -156,6 +157,8 @@ struct JobDev {
   // entries (input order)
   uint8_t* keys;             // key arena
   uint64_t cap_key_bytes;
+  uint32_t key_pad;          // 7: every key starts on an 8-byte boundary of the arena; 0: keys
+                             // back to back (jobs whose slots would pass 4 GiB)
   uint4* e_rec;              // per entry: decode record (pass 1 -> pass 2)
   uint32_t dec_group;        // data blocks per warp in the decode's first pass
   uint32_t dec_unit;         // entries per warp in its second pass
