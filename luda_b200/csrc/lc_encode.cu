@@ -1137,140 +1137,6 @@ __device__ __forceinline__ void enc_drain(uint32_t lane) {
   __syncwarp();
 }
 
-__global__ void __launch_bounds__(kEncWarps * 32, 2) k_encode_blocks(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  __shared__ uint32_t s_h8[kCrcH8Words];
-  __shared__ uint32_t s_xinv[kCrcXinvSmem];
-  __shared__ uint32_t s_tab8[256];
-  __shared__ JobDev s_job;  // the job's descriptor, read from here in every step
-  extern __shared__ __align__(16) uint8_t enc_smem[];
-  const JobDev& G = jobs[blockIdx.y];
-  // the surplus CTAs of a small job leave before they load any table
-  if (G.ctr->error || blockIdx.x * kEncWarps >= max(G.ctr->n_blocks_out, (uint64_t)G.ctr->n_wide)) return;
-  copy_job(jobs + blockIdx.y, &s_job);
-  for (uint32_t i = threadIdx.x; i < kCrcH8Words; i += blockDim.x) s_h8[i] = G.crc_h8[i];
-  for (uint32_t i = threadIdx.x; i < kCrcXinvN; i += blockDim.x) s_xinv[xinv_slot(i)] = G.crc_xinv[i];
-  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab8[i] = G.crc_byte[i];
-  __syncthreads();
-  const JobDev& J = s_job;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  EncWarp& W = reinterpret_cast<EncWarp*>(enc_smem)[warp];
-  const uint32_t nb = (uint32_t)J.ctr->n_blocks_out;  // block and survivor indices fit 32 bits
-  const RestartDiv rd(J.restart_interval);
-  const uint32_t stride = gridDim.x * kEncWarps;
-  uint8_t* st = W.stage;
-  uint32_t b = blockIdx.x * kEncWarps + warp;
-  EncBlock cur{};
-  if (b < nb) {
-    cur.off = (uint32_t)J.b_off[b];
-    cur.dst = J.out + J.files[J.b_file[b]].out_off + J.b_off[b];
-    cur.bsz = J.b_size[b];
-    cur.s = J.b_first[b];
-    cur.n = J.b_first[b + 1] - cur.s;
-    enc_ahead_entries(J, W, cur, lane);
-  }
-  for (; b < nb; b += stride) {
-    // the next block's place and range
-    const uint32_t bn = b + stride;
-    EncBlock nxt{};
-    uint32_t n_file = 0;
-    uint64_t n_off = 0;
-    if (bn < nb) {
-      n_file = J.b_file[bn];
-      n_off = J.b_off[bn];
-      nxt.bsz = J.b_size[bn];
-      nxt.s = J.b_first[bn];
-      nxt.n = J.b_first[bn + 1];  // (less nxt.s, below: not waited for here)
-    }
-    const bool narrow = cur.bsz <= kEncNarrow;  // wide blocks: by their windows, below
-    const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(cur.dst) & 15);
-    const uint32_t m0 = ph, m1 = ph + cur.bsz + 1;  // the message: block and type byte
-    cp_async_wait_all();  // this lane's entries of the block
-    uint32_t ones = 0;
-    if (narrow) {
-      ones = __ldg(J.crc_ones + (m1 - m0));
-      enc_drain(lane);
-      enc_assemble<false>(J, W, cur, rd, ph, 0, m1, lane);
-    }
-    if (bn < nb) {  // the next block's place and entries, in flight meanwhile
-      nxt.n -= nxt.s;
-      nxt.off = (uint32_t)n_off;
-      nxt.dst = J.out + J.files[n_file].out_off + n_off;
-      enc_ahead_entries(J, W, nxt, lane);  // each lane's own slots
-    }
-    if (narrow) {
-      uint8_t* gbase = cur.dst - ph;
-      const uint32_t full =
-          enc_out(J, s_h8, s_xinv, s_tab8, gbase, st, m0, m1, lane) ^ ones ^ 0xffffffffu;
-      const uint32_t crc = ((full >> 15) | (full << 17)) + 0xa282ead8u;  // crc32c::Mask
-      if (bn < nb && nxt.bsz <= kEncNarrow) {
-        cp_async_wait_all();
-        enc_prefetch(J, W, nxt.n, lane);
-      }
-      if (lane == 0) st_le32(st + m1, crc);
-      __syncwarp();
-      enc_ends(gbase, st, m0, m1, m1 + 4, lane);
-      __syncwarp();
-    }
-    cur = nxt;
-  }
-  // windows of the wide blocks
-  const uint32_t nw = min(J.ctr->n_wide, J.cap_wide);
-  for (uint32_t x = blockIdx.x * kEncWarps + warp; x < nw; x += stride) {
-    const uint2 un = J.wide[x];  // block, window
-    EncBlock B;
-    B.off = (uint32_t)J.b_off[un.x];
-    B.dst = J.out + J.files[J.b_file[un.x]].out_off + J.b_off[un.x];
-    B.bsz = J.b_size[un.x];
-    B.s = J.b_first[un.x];
-    B.n = J.b_first[un.x + 1] - B.s;
-    const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(B.dst) & 15);
-    const uint32_t end = ph + B.bsz + 1;  // the message's end
-    const uint32_t p0 = un.y * kEncWindow, p1 = min(end, p0 + kEncWindow);
-    if (p0 >= end) continue;  // the layout counted the longest phase
-    enc_drain(lane);
-    enc_assemble<true>(J, W, B, rd, ph, p0, p1, lane);
-    uint8_t* gbase = B.dst - ph + p0;
-    const uint32_t m0 = p0 ? 0 : ph, m1 = p1 - p0;
-    const uint32_t raw = enc_out(J, s_h8, s_xinv, s_tab8, gbase, st, m0, m1, lane);
-    if (lane == 0) atomicXor(J.b_crc + un.x, crc_shift_tab(J, s_tab8, raw, end - p1));
-    enc_ends(gbase, st, m0, m1, m1, lane);
-    __syncwarp();
-  }
-  cp_async_wait_all();
-  enc_drain(lane);
-}
-
-// The survivors' decoded form for later jobs (keep_decoded): key bytes at
-// dec_kcum (a scan of the key lengths), value lengths, prefixes and tags; the
-// value places were written by k_encode_blocks.  One warp per 32 survivors,
-// lanes over the group's key bytes.
-__global__ void k_emit_decoded(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error || !J.dec_keys) return;
-  const uint64_t n = J.ctr->n_kept;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * 32 < n; g += warps) {
-    const uint64_t k = g * 32 + lane;
-    if (k < n) {
-      uint32_t kl;
-      const uint8_t* key = kept_key(J, k, &kl);
-      J.dec_vlen[k] = J.k_vlen[k];
-      J.dec_pfx[k] = user_prefix(key, kl);
-      J.dec_tag[k] = ld_le64(key + kl - 8);
-    }
-    const uint64_t k1 = min(n, g * 32 + 32);
-    for (uint64_t j = g * 32; j < k1; j++) {
-      uint32_t kl;
-      const uint8_t* key = kept_key(J, j, &kl);
-      uint8_t* d = J.dec_keys + J.dec_kcum[j];
-      for (uint32_t t = lane; t < kl; t += 32) d[t] = key[t];
-    }
-  }
-}
-
 // Filter groups, each at its first block: a warp takes a run of up to 32
 // blocks.  Its lanes first load everything about their own blocks' groups
 // (one chain of dependent loads for all of them), write the groups' offsets
@@ -1284,19 +1150,13 @@ __global__ void k_emit_decoded(const JobDev* __restrict__ jobs) {
 // us for 1M keys in 256k groups; this form 86 and 19 us.
 constexpr uint32_t kFilterSmem = 1024;
 constexpr uint32_t kFilterFew = 8;    // keys, and at most 16 filter bytes: by one lane
-__global__ void __launch_bounds__(256) k_encode_filters(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  __shared__ uint32_t s_filter[8][kFilterSmem / 4 + 1];  // blockDim 256: 8 warps
-  const uint32_t lane = threadIdx.x & 31;
-  if (J.bits_per_key <= 0 || J.ctr->error) return;
+__device__ __forceinline__ void encode_filters(const JobDev& J, uint32_t* sbuf, uint64_t warp,
+                                               uint64_t warps, uint32_t lane) {
+  if (J.bits_per_key <= 0) return;
   const uint64_t nb = J.ctr->n_blocks_out;
   const uint32_t K = J.bloom_k;
-  uint32_t* sbuf = s_filter[threadIdx.x >> 5];
-  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const uint64_t run = min((uint64_t)32, (nb + warps - 1) / warps);  // blocks per warp and turn
-  for (uint64_t b0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * run; b0 < nb;
-       b0 += warps * run) {
+  for (uint64_t b0 = warp * run; b0 < nb; b0 += warps * run) {
     const uint64_t b = b0 + lane;
     uint8_t* fdst = nullptr;
     uint32_t nbytes = 0, nk = 0, k0 = 0;
@@ -1408,28 +1268,10 @@ __device__ __forceinline__ void encode_index_entry(const JobDev& J, uint64_t b) 
   if (b + 1 == fb1) st_le32(ra + 4, fb1 - fb0);
 }
 
-__global__ void k_encode_index(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;
-  const uint64_t nb = J.ctr->n_blocks_out;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (uint64_t)gridDim.x * blockDim.x)
-    encode_index_entry(J, b);
-}
-
-// Metaindex, footer and the tail of the filter block's offset array (thread
-// 0), then the trailers of the filter, metaindex and index blocks, each a
-// CRC32C over the whole CTA: one CTA per output file.
-__global__ void __launch_bounds__(256) k_encode_meta(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  __shared__ uint32_t s_skip;
-  if (threadIdx.x == 0) s_skip = J.ctr->error || blockIdx.x >= J.ctr->n_files;
-  __syncthreads();
-  if (s_skip) return;
-  const uint32_t f = blockIdx.x;
-  if (threadIdx.x == 0) {
+// File f's metaindex block, footer and the tail of its filter block's offset
+// array (lane 0), and its smallest and largest keys, by one warp.
+__device__ __forceinline__ void encode_meta_file(const JobDev& J, uint32_t f, uint32_t lane) {
+  if (lane == 0) {
     const FileOut& F = J.files[f];
     uint8_t* base = J.out + F.out_off;
     if (J.bits_per_key > 0) {
@@ -1464,7 +1306,6 @@ __global__ void __launch_bounds__(256) k_encode_meta(const JobDev* __restrict__ 
     st_le32(foot + 40, 0x8b80fb57u);
     st_le32(foot + 44, 0xdb477524u);
   }
-  __syncthreads();
   const FileOut& F = J.files[f];
   // the file's smallest and largest internal keys (FileMetaData::smallest /
   // largest) into slots 2f and 2f + 1 of fkey_stride bytes, their lengths
@@ -1474,8 +1315,166 @@ __global__ void __launch_bounds__(256) k_encode_meta(const JobDev* __restrict__ 
     uint32_t l;
     const uint8_t* k = kept_key(J, which ? F.end_kept - 1 : F.first_kept, &l);
     uint8_t* d = J.fkeys + (2ull * f + which) * J.fkey_stride;
-    for (uint32_t t = threadIdx.x; t < l; t += blockDim.x) d[t] = k[t];
-    if (threadIdx.x == 0) J.fkoff[2 * f + which] = l;
+    for (uint32_t t = lane; t < l; t += 32) d[t] = k[t];
+    if (lane == 0) J.fkoff[2 * f + which] = l;
+  }
+}
+
+// Filter blocks, index blocks and the files' metadata need the layout only, not
+// the data blocks: the first `side` CTAs of k_encode_blocks write them, beside
+// the CTAs that encode (they finish early).  As three kernels after it they took
+// another 24 us of an 80k-entry job, 121 us of 8M entries and 160 us of a
+// 32-job batch on B200.
+__device__ __forceinline__ void encode_side(const JobDev& J, uint32_t* sbuf, uint32_t cta,
+                                            uint32_t ctas) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t thread = (uint64_t)cta * blockDim.x + threadIdx.x, threads = (uint64_t)ctas * blockDim.x;
+  const uint64_t warp = thread >> 5, warps = threads >> 5;
+  encode_filters(J, sbuf, warp, warps, lane);
+  const uint64_t nb = J.ctr->n_blocks_out;
+  for (uint64_t b = thread; b < nb; b += threads) encode_index_entry(J, b);
+  for (uint64_t f = warps - 1 - warp; f < J.ctr->n_files; f += warps) encode_meta_file(J, (uint32_t)f, lane);
+}
+
+__global__ void __launch_bounds__(kEncWarps * 32, 2) k_encode_blocks(const JobDev* __restrict__ jobs,
+                                                                       uint32_t side) {
+  pdl_begin();
+  __shared__ uint32_t s_h8[kCrcH8Words];
+  __shared__ uint32_t s_xinv[kCrcXinvSmem];
+  __shared__ uint32_t s_tab8[256];
+  __shared__ JobDev s_job;  // the job's descriptor, read from here in every step
+  extern __shared__ __align__(16) uint8_t enc_smem[];
+  const JobDev& G = jobs[blockIdx.y];
+  if (G.ctr->error) return;
+  if (blockIdx.x < side) {
+    encode_side(G, reinterpret_cast<uint32_t*>(enc_smem) + (threadIdx.x >> 5) * (kFilterSmem / 4 + 1),
+                blockIdx.x, side);
+    return;
+  }
+  const uint32_t cta = blockIdx.x - side, ctas = gridDim.x - side;
+  // the surplus CTAs of a small job leave before they load any table
+  if (cta * kEncWarps >= max(G.ctr->n_blocks_out, (uint64_t)G.ctr->n_wide)) return;
+  copy_job(jobs + blockIdx.y, &s_job);
+  for (uint32_t i = threadIdx.x; i < kCrcH8Words; i += blockDim.x) s_h8[i] = G.crc_h8[i];
+  for (uint32_t i = threadIdx.x; i < kCrcXinvN; i += blockDim.x) s_xinv[xinv_slot(i)] = G.crc_xinv[i];
+  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab8[i] = G.crc_byte[i];
+  __syncthreads();
+  const JobDev& J = s_job;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  EncWarp& W = reinterpret_cast<EncWarp*>(enc_smem)[warp];
+  const uint32_t nb = (uint32_t)J.ctr->n_blocks_out;  // block and survivor indices fit 32 bits
+  const RestartDiv rd(J.restart_interval);
+  const uint32_t stride = ctas * kEncWarps;
+  uint8_t* st = W.stage;
+  uint32_t b = cta * kEncWarps + warp;
+  EncBlock cur{};
+  if (b < nb) {
+    cur.off = (uint32_t)J.b_off[b];
+    cur.dst = J.out + J.files[J.b_file[b]].out_off + J.b_off[b];
+    cur.bsz = J.b_size[b];
+    cur.s = J.b_first[b];
+    cur.n = J.b_first[b + 1] - cur.s;
+    enc_ahead_entries(J, W, cur, lane);
+  }
+  for (; b < nb; b += stride) {
+    // the next block's place and range
+    const uint32_t bn = b + stride;
+    EncBlock nxt{};
+    uint32_t n_file = 0;
+    uint64_t n_off = 0;
+    if (bn < nb) {
+      n_file = J.b_file[bn];
+      n_off = J.b_off[bn];
+      nxt.bsz = J.b_size[bn];
+      nxt.s = J.b_first[bn];
+      nxt.n = J.b_first[bn + 1];  // (less nxt.s, below: not waited for here)
+    }
+    const bool narrow = cur.bsz <= kEncNarrow;  // wide blocks: by their windows, below
+    const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(cur.dst) & 15);
+    const uint32_t m0 = ph, m1 = ph + cur.bsz + 1;  // the message: block and type byte
+    cp_async_wait_all();  // this lane's entries of the block
+    uint32_t ones = 0;
+    if (narrow) {
+      ones = __ldg(J.crc_ones + (m1 - m0));
+      enc_drain(lane);
+      enc_assemble<false>(J, W, cur, rd, ph, 0, m1, lane);
+    }
+    if (bn < nb) {  // the next block's place and entries, in flight meanwhile
+      nxt.n -= nxt.s;
+      nxt.off = (uint32_t)n_off;
+      nxt.dst = J.out + J.files[n_file].out_off + n_off;
+      enc_ahead_entries(J, W, nxt, lane);  // each lane's own slots
+    }
+    if (narrow) {
+      uint8_t* gbase = cur.dst - ph;
+      const uint32_t full =
+          enc_out(J, s_h8, s_xinv, s_tab8, gbase, st, m0, m1, lane) ^ ones ^ 0xffffffffu;
+      const uint32_t crc = ((full >> 15) | (full << 17)) + 0xa282ead8u;  // crc32c::Mask
+      if (bn < nb && nxt.bsz <= kEncNarrow) {
+        cp_async_wait_all();
+        enc_prefetch(J, W, nxt.n, lane);
+      }
+      if (lane == 0) st_le32(st + m1, crc);
+      __syncwarp();
+      enc_ends(gbase, st, m0, m1, m1 + 4, lane);
+      __syncwarp();
+    }
+    cur = nxt;
+  }
+  // windows of the wide blocks
+  const uint32_t nw = min(J.ctr->n_wide, J.cap_wide);
+  for (uint32_t x = cta * kEncWarps + warp; x < nw; x += stride) {
+    const uint2 un = J.wide[x];  // block, window
+    EncBlock B;
+    B.off = (uint32_t)J.b_off[un.x];
+    B.dst = J.out + J.files[J.b_file[un.x]].out_off + J.b_off[un.x];
+    B.bsz = J.b_size[un.x];
+    B.s = J.b_first[un.x];
+    B.n = J.b_first[un.x + 1] - B.s;
+    const uint32_t ph = (uint32_t)(reinterpret_cast<uintptr_t>(B.dst) & 15);
+    const uint32_t end = ph + B.bsz + 1;  // the message's end
+    const uint32_t p0 = un.y * kEncWindow, p1 = min(end, p0 + kEncWindow);
+    if (p0 >= end) continue;  // the layout counted the longest phase
+    enc_drain(lane);
+    enc_assemble<true>(J, W, B, rd, ph, p0, p1, lane);
+    uint8_t* gbase = B.dst - ph + p0;
+    const uint32_t m0 = p0 ? 0 : ph, m1 = p1 - p0;
+    const uint32_t raw = enc_out(J, s_h8, s_xinv, s_tab8, gbase, st, m0, m1, lane);
+    if (lane == 0) atomicXor(J.b_crc + un.x, crc_shift_tab(J, s_tab8, raw, end - p1));
+    enc_ends(gbase, st, m0, m1, m1, lane);
+    __syncwarp();
+  }
+  cp_async_wait_all();
+  enc_drain(lane);
+}
+
+// The survivors' decoded form for later jobs (keep_decoded): key bytes at
+// dec_kcum (a scan of the key lengths), value lengths, prefixes and tags; the
+// value places were written by k_encode_blocks.  One warp per 32 survivors,
+// lanes over the group's key bytes.
+__global__ void k_emit_decoded(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  if (J.ctr->error || !J.dec_keys) return;
+  const uint64_t n = J.ctr->n_kept;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * 32 < n; g += warps) {
+    const uint64_t k = g * 32 + lane;
+    if (k < n) {
+      uint32_t kl;
+      const uint8_t* key = kept_key(J, k, &kl);
+      J.dec_vlen[k] = J.k_vlen[k];
+      J.dec_pfx[k] = user_prefix(key, kl);
+      J.dec_tag[k] = ld_le64(key + kl - 8);
+    }
+    const uint64_t k1 = min(n, g * 32 + 32);
+    for (uint64_t j = g * 32; j < k1; j++) {
+      uint32_t kl;
+      const uint8_t* key = kept_key(J, j, &kl);
+      uint8_t* d = J.dec_keys + J.dec_kcum[j];
+      for (uint32_t t = lane; t < kl; t += 32) d[t] = key[t];
+    }
   }
 }
 
@@ -1517,21 +1516,32 @@ __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ job
   for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_tab8[i] = J.crc_byte[i];
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31, nf = J.ctr->n_files;
-  // the pieces of all files are dealt to the job's warps in turn
+  // the pieces of all files are dealt to the job's warps in turn; the lanes
+  // look at 32 files at a time for the one that a turn falls into (one after
+  // the other, a load chain each, took 23 us with 33 files)
   const uint64_t warps = (uint64_t)ctas * (blockDim.x / 32);
   uint64_t turn = (uint64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  for (uint32_t f = 0; f < nf; f++) {
-    const FileOut& F = J.files[f];
-    uint64_t off[3], len[3], np[3];
+  const auto pieces = [&](const FileOut& F, uint64_t* off, uint64_t* len, uint64_t* np) -> uint64_t {
+#pragma unroll
     for (uint32_t r = 0; r < 3; r++) {
       meta_region(F, r, &off[r], &len[r]);
       np[r] = (r == 0 && J.bits_per_key <= 0) ? 0 : (len[r] + kMetaPiece - 1) / kMetaPiece;
     }
-    const uint8_t* fbase = J.out + F.out_off;
-    const uint64_t total = np[0] + np[1] + np[2];
+    return np[0] + np[1] + np[2];
+  };
+  for (uint32_t f0 = 0; f0 < nf; f0 += 32) {
+    uint64_t off[3], len[3], np[3];
+    const uint64_t mine = f0 + lane < nf ? pieces(J.files[f0 + lane], off, len, np) : 0;
+    uint64_t total;
+    const uint64_t first = warp_excl<uint64_t>(mine, &total);
     for (; turn < total; turn += warps) {
+      const int l = 31 - __clz(__ballot_sync(0xffffffffu, first <= turn && mine));
+      const uint32_t f = f0 + l;
+      const FileOut& F = J.files[f];
+      const uint8_t* fbase = J.out + F.out_off;
+      pieces(F, off, len, np);
       uint32_t r = 0;
-      uint64_t q = turn;
+      uint64_t q = turn - __shfl_sync(0xffffffffu, first, l);
       while (q >= np[r]) q -= np[r++];
       const uint64_t a = q * kMetaPiece, e = min(len[r], a + kMetaPiece);
       const uint8_t* pa = fbase + off[r] + a;
@@ -1667,24 +1677,20 @@ void encode_kernel_attributes() {
 }
 
 void launch_encode_blocks(const Batch& bt, cudaStream_t st) {
-  // grid-stride over the device-side counts of blocks and windows: 3 CTAs per
-  // SM x 4 waves, shared out among the jobs (a job of few entries may have as
-  // many windows as its output bytes allow)
-  launch(k_encode_blocks, dim3(grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide), kEncWarps, bt.per_job(148 * 2 * 4)), bt.B), kEncWarps * 32, kEncSmem, st, bt.d);
+  // grid-stride over the device-side counts of blocks and windows: 2 CTAs per
+  // SM x 4 waves (a job of few entries may have as many windows as its output
+  // bytes allow), after the CTAs for everything else
+  const uint32_t side = grid_x(bt.max_entries, 2048, bt.per_job(148));
+  const uint32_t enc =
+      grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide), kEncWarps, bt.per_job(148 * 2 * 4));
+  launch(k_encode_blocks, dim3(side + enc, bt.B), kEncWarps * 32, kEncSmem, st, bt.d, side);
 }
 void launch_emit_decoded(const Batch& bt, cudaStream_t st) {
   if (!bt.any_keep_decoded) return;
   scan_batch(kScanDecKey, bt, bt.max_entries, st);
   launch(k_emit_decoded, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
-void launch_encode_filters(const Batch& bt, cudaStream_t st) {
-  launch(k_encode_filters, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
-}
-void launch_encode_index(const Batch& bt, cudaStream_t st) {
-  launch(k_encode_index, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 16)), bt.B), 256, 0, st, bt.d);
-}
 void launch_encode_meta(const Batch& bt, cudaStream_t st) {
-  launch(k_encode_meta, dim3(bt.max_cap_files, bt.B), 256, 0, st, bt.d);
   launch(k_meta_crc, dim3(grid_x(bt.max_entries, 4096, bt.per_job(148 * 4)), bt.B), 256, 0, st, bt.d);
   // (the wide blocks are at most the entries)
   launch(k_meta_trailers, dim3(std::max((3 * bt.max_cap_files + 255) / 256, grid_x(bt.max_entries, 2048, bt.per_job(148 * 2))), bt.B), 256, 0, st, bt.d);

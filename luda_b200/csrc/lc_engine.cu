@@ -622,8 +622,6 @@ void launch_tail(const Batch& bt, bool decode_merge, cudaStream_t st, PhaseTimer
   launch_encode_blocks(bt, st);
   launch_emit_decoded(bt, st);
   T.mark(kEncodeBlocks);
-  launch_encode_filters(bt, st);
-  launch_encode_index(bt, st);
   launch_encode_meta(bt, st);
   if (decode_merge) launch_results(bt, st);
   T.mark(kEncodeMeta);

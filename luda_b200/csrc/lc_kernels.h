@@ -151,13 +151,11 @@ void launch_block_sizes(const Batch& bt, cudaStream_t st);
 void launch_files(const Batch& bt, cudaStream_t st);
 void launch_block_layout(const Batch& bt, cudaStream_t st);
 void launch_file_layout(const Batch& bt, cudaStream_t st);
-// after the layout, blocks / filters / index + file keys are independent
+// data, filter and index blocks, metaindex, footer and file keys
 void launch_encode_blocks(const Batch& bt, cudaStream_t st);
-void launch_encode_filters(const Batch& bt, cudaStream_t st);
 // the decoded form of the survivors, for jobs with keep_decoded
 void launch_emit_decoded(const Batch& bt, cudaStream_t st);
-void launch_encode_index(const Batch& bt, cudaStream_t st);
-// metaindex, footer, filter tails and the trailers of filter/meta/index
+// the trailers of the filter, metaindex and index blocks and of wide data blocks
 void launch_encode_meta(const Batch& bt, cudaStream_t st);
 // counters and per-file results to the jobs' host buffers (JobDev::res_*)
 void launch_results(const Batch& bt, cudaStream_t st);

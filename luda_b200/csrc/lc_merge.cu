@@ -754,8 +754,8 @@ void launch_drop(const Batch& bt, cudaStream_t st) {
 }
 
 void launch_triggers(const Batch& bt, cudaStream_t st) {
-  if (bt.max_gp)
-    launch(k_gp_first, dim3((bt.max_gp + 1 + 255) / 256, bt.B), 256, 0, st, bt.d);
+  if (!bt.max_gp) return;  // no job has grandparents: no cuts (the counters start at zero)
+  launch(k_gp_first, dim3((bt.max_gp + 1 + 255) / 256, bt.B), 256, 0, st, bt.d);
   const size_t smem = (size_t)(bt.max_gp + 1) * 12;
   const bool in_smem = smem + 64 <= 48 * 1024;  // with the kernel's static shared memory
   launch(k_triggers, dim3(1, bt.B), 256, in_smem ? smem : 0, st, bt.d, in_smem);
