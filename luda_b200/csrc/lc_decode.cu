@@ -156,8 +156,24 @@ __global__ void k_table_index_entries(const JobDev* __restrict__ jobs) {
   const TableDesc T = J.tables[t];
   const bool unit = J.tbl_unit[t] != 0;
   if (part != 0 && (T.cached || !unit)) return;
+  // the blocks of the tables before this one; kept for the kernels after (the
+  // total by the last table's CTA)
+  __shared__ unsigned long long s_base;
+  if (threadIdx.x == 0) s_base = 0;
+  __syncthreads();
+  uint32_t before = 0;
+  for (uint32_t x = threadIdx.x; x < t; x += blockDim.x) before += J.tbl_nblocks[x];
+  if (before) atomicAdd(&s_base, (unsigned long long)before);
+  __syncthreads();
+  const uint64_t out_base = s_base, out_end = out_base + J.tbl_nblocks[t];
+  if (part == 0 && threadIdx.x == 0) {
+    J.tbl_block_base[t] = out_base;
+    if (t + 1 == J.n_tables) {
+      J.tbl_block_base[t + 1] = out_end;
+      J.ctr->n_blocks_in = out_end;
+    }
+  }
   if (T.cached) {
-    const uint64_t out_base = J.tbl_block_base[t], out_end = J.tbl_block_base[t + 1];
     for (uint64_t o = out_base + threadIdx.x; o < out_end && o < J.cap_blocks_in; o += blockDim.x) {
       J.blk_off[o] = ((uint64_t)t << 32) | ((o - out_base) * kDecRunBlock);
       J.blk_size[o] = kPseudoBlock;
@@ -173,8 +189,6 @@ __global__ void k_table_index_entries(const JobDev* __restrict__ jobs) {
   const uint8_t* idx = base + io;
   const uint64_t ra_off = is - 4 - 4ull * nr;
   const uint8_t* ra = idx + ra_off;
-  const uint64_t out_base = J.tbl_block_base[t];
-  const uint64_t out_end = J.tbl_block_base[t + 1];
   if (unit) {
     const uint32_t r0 = (uint32_t)((uint64_t)nr * part / kIdxSplit);
     const uint32_t r1 = (uint32_t)((uint64_t)nr * (part + 1) / kIdxSplit);
@@ -539,9 +553,11 @@ __global__ void __launch_bounds__(256) k_verify_blocks(const JobDev* __restrict_
   }
 }
 
-// Entries of merge child r start at the first block of its first table: one
-// thread per table, the first table of each run writes the run's start.
-__global__ void k_run_bounds(const JobDev* __restrict__ jobs) {
+// The parse's last kernel.  Entries of merge child r start at the first block
+// of its first table: one thread per table, the first table of each run writes
+// the run's start.  Then the counters, final now, to the host (res_ctr: mapped
+// pinned memory).
+__global__ void k_parse_done(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   const bool bad = J.ctr->error != 0;  // the job fails; keep every read in bounds
@@ -552,7 +568,11 @@ __global__ void k_run_bounds(const JobDev* __restrict__ jobs) {
       J.run_entry_begin_w[run] =
           bad ? 0 : J.blk_ent_base[min(J.tbl_block_base[t], J.cap_blocks_in)];
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) J.run_entry_begin_w[J.n_runs] = J.ctr->n_entries_in;
+  if (blockIdx.x != 0) return;
+  if (threadIdx.x == 0) J.run_entry_begin_w[J.n_runs] = J.ctr->n_entries_in;
+  if (J.res_ctr)
+    for (uint32_t i = threadIdx.x; i < sizeof(Counters) / 8; i += blockDim.x)
+      reinterpret_cast<uint64_t*>(J.res_ctr)[i] = reinterpret_cast<const uint64_t*>(J.ctr)[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -1073,8 +1093,8 @@ void launch_verify_blocks(const Batch& bt, cudaStream_t st) {
   if (!bt.any_verify) return;
   launch(k_verify_blocks, dim3(grid_x(bt.max_blocks_in, 8, bt.per_job(148 * 4)), bt.B), 256, 0, st, bt.d);
 }
-void launch_run_bounds(const Batch& bt, cudaStream_t st) {
-  launch(k_run_bounds, dim3((bt.max_tables + 127) / 128 + 1, bt.B), 128, 0, st, bt.d);
+void launch_parse_done(const Batch& bt, cudaStream_t st) {
+  launch(k_parse_done, dim3((bt.max_tables + 127) / 128 + 1, bt.B), 128, 0, st, bt.d);
 }
 void launch_block_decode(const Batch& bt, cudaStream_t st) {
   // pass 1: one warp per group of blocks; pass 2: one warp per unit of

@@ -1072,45 +1072,30 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       o.bsl = S.put(sl.data(), nb);
       o.bll = S.put(ll.data(), nb);
     }
-    // pinned staging before the first sync: [stage | descriptors | counters]
-    const size_t o_hj = (S.h.size() + 255) & ~size_t(255);
+    // pinned staging before the first sync: [stage | zeroed counters |
+    // descriptors], which goes up in one piece, and room for the counters' way back
+    const size_t o_ctr = (S.h.size() + 255) & ~size_t(255);
+    const size_t o_hj = o_ctr + ((sizeof(Counters) * B + 255) & ~size_t(255));
     const size_t o_hc = o_hj + ((sizeof(JobDev) * B + 255) & ~size_t(255));
     uint8_t* pin1 = slot.pinned(o_hc + sizeof(Counters) * B);
     memcpy(pin1, S.h.data(), S.h.size());
-    uint8_t* d_stage = A.get<uint8_t>(S.h.size());
-    slot.to_device(d_stage, pin1, S.h.size());  // not behind other jobs' bulk copies
+    memset(pin1 + o_ctr, 0, o_hj - o_ctr);
+    uint8_t* d_stage = A.get<uint8_t>(o_hc);
     uint8_t* d_in_all = in_total ? A.get<uint8_t>(in_total) : nullptr;
-    Counters* d_ctr = A.get<Counters>(B);
-    CK(cudaMemsetAsync(d_ctr, 0, sizeof(Counters) * B, st));
+    Counters* d_ctr = reinterpret_cast<Counters*>(d_stage + o_ctr);
     Batch bt;
-    bt.d = slot.d_jobs;
+    bt.d = reinterpret_cast<const JobDev*>(d_stage + o_hj);
     bt.B = B;
     bt.chunk = kChunk;
     bt.ctas_per_job = tun.ctas_per_job;
     bt.merge_items = tun.merge_items;
     bt.merge_threads = tun.merge_threads;
-    bool host_up = false;
-    for (uint32_t i = 0; i < B; i++)
-      host_up = host_up || (!zero_copy[i] && !jobs[i]->inputs_on_device && !runs[i].failed);
-    std::unique_lock<std::mutex> up_lk(e->up_lane.mu, std::defer_lock);
-    if (host_up) {
-      up_lk.lock();
-      if (e->up_lane.any) CK(cudaStreamWaitEvent(st, e->up_lane.done, 0));
-    }
     for (uint32_t i = 0; i < B; i++) {
       JobRun& r = runs[i];
       JobDev& J = r.J;
       lc_job* j = jobs[i];
       const Offs& o = offs[i];
-      if (!zero_copy[i]) {
-        J.in = d_in_all + in_base[i];
-        for (uint32_t t = 0; t < J.n_tables && !r.failed; t++) {
-          if (!j->tables[t].size) continue;
-          copy_pieces((uint8_t*)J.in + tds[i][t].off, j->tables[t].data, j->tables[t].size,
-                      j->inputs_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st,
-                      piece_for(J.in_size));
-        }
-      }
+      if (!zero_copy[i]) J.in = d_in_all + in_base[i];
       J.in_end = J.in + J.in_size + (zero_copy[i] ? 0 : 16);
       J.tables = (const TableDesc*)(d_stage + o.td);
       J.dec_runs = (const DecRun*)(d_stage + o.dec);
@@ -1124,6 +1109,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       J.base_small_len = (const uint32_t*)(d_stage + o.bsl);
       J.base_large_len = (const uint32_t*)(d_stage + o.bll);
       J.ctr = d_ctr + i;
+      J.res_ctr = slot.pin_dev ? reinterpret_cast<Counters*>(slot.pin_dev + o_hc) + i : nullptr;
       if (r.failed) {
         J.n_tables = 0;
         J.n_runs = 0;
@@ -1149,14 +1135,32 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       // (blocks are closed at block_size bytes; the input's block size is not known)
       bt.max_blocks_in = std::max<uint64_t>(bt.max_blocks_in, r.in_bytes / 2048 + 1);
     }
+    JobDev* hj = reinterpret_cast<JobDev*>(pin1 + o_hj);
+    for (uint32_t i = 0; i < B; i++) hj[i] = runs[i].J;
+    slot.to_device(d_stage, pin1, o_hc);  // not behind other jobs' bulk copies
+    bool host_up = false;
+    for (uint32_t i = 0; i < B; i++)
+      host_up = host_up || (!zero_copy[i] && !jobs[i]->inputs_on_device && !runs[i].failed);
+    std::unique_lock<std::mutex> up_lk(e->up_lane.mu, std::defer_lock);
+    if (host_up) {
+      up_lk.lock();
+      if (e->up_lane.any) CK(cudaStreamWaitEvent(st, e->up_lane.done, 0));
+    }
+    for (uint32_t i = 0; i < B; i++) {
+      const JobDev& J = runs[i].J;
+      const lc_job* j = jobs[i];
+      for (uint32_t t = 0; t < J.n_tables && !zero_copy[i]; t++) {
+        if (!j->tables[t].size) continue;
+        copy_pieces((uint8_t*)J.in + tds[i][t].off, j->tables[t].data, j->tables[t].size,
+                    j->inputs_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st,
+                    piece_for(J.in_size));
+      }
+    }
     if (host_up) {
       CK(cudaEventRecord(e->up_lane.done, st));
       e->up_lane.any = true;
       up_lk.unlock();
     }
-    JobDev* hj = reinterpret_cast<JobDev*>(pin1 + o_hj);
-    for (uint32_t i = 0; i < B; i++) hj[i] = runs[i].J;
-    slot.to_device(slot.d_jobs, (const uint8_t*)hj, sizeof(JobDev) * B);
     T.mark(kUpload);
     e->note_setup(t_setup0);
     // ---- parse: index blocks, then entry counts -- exact: a walk of every
@@ -1172,7 +1176,6 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     }
     if (bt.max_tables) {
       launch_table_index_count(bt, st);
-      scan_batch(kScanTblBlocks, bt, bt.max_tables, st);
       launch_table_index_entries(bt, st);
       launch_verify_blocks(bt, st);
       if (exact) {
@@ -1184,11 +1187,11 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
         scan_batch(kScanBlkEnt, bt, bt.max_blocks_in, st);
       }
     }
-    launch_run_bounds(bt, st);
+    launch_parse_done(bt, st);  // (the counters, into mapped memory)
     CK(cudaGetLastError());
     T.mark(kParse);
     std::vector<Counters> hc(B);
-    slot.to_host(pin1 + o_hc, d_ctr, sizeof(Counters) * B);
+    if (!slot.pin_dev) slot.to_host(pin1 + o_hc, d_ctr, sizeof(Counters) * B);
     CK(cudaStreamSynchronize(st));
     memcpy(hc.data(), pin1 + o_hc, sizeof(Counters) * B);
     // ---- allocate the rest from the totals
@@ -1305,6 +1308,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       J.files = reinterpret_cast<FileOut*>(d_res + res_off[i]);
       J.fkoff = reinterpret_cast<uint64_t*>(d_res + klen);
       J.fkeys = d_res + keys;
+      J.res_ctr = nullptr;
       if (uint8_t* m = slot.pin_dev) {
         J.res_ctr = reinterpret_cast<Counters*>(m) + i;
         J.res_files = reinterpret_cast<FileOut*>(m + p_res + res_off[i]);
@@ -1312,6 +1316,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
         J.res_keys = m + p_res + keys;
       }
     }
+    bt.d = slot.d_jobs;  // the graphs' descriptors
     if (any_zeroed) {
       memcpy(pin2, hc.data(), sizeof(Counters) * B);
       slot.to_device(d_ctr, pin2, sizeof(Counters) * B);

@@ -100,8 +100,7 @@ struct Batch {
 
 // lc_scan.cu -- exclusive prefix sums over per-job arrays chosen by selector
 enum ScanSel : int {
-  kScanTblBlocks = 0,  // tbl_nblocks -> tbl_block_base      (total: n_blocks_in)
-  kScanBlkEnt,         // blk_nent -> blk_ent_base           (total: n_entries_in)
+  kScanBlkEnt = 0,             // blk_nent -> blk_ent_base           (total: n_entries_in)
   kScanBlkKey,         // blk_kbytes -> blk_key_base         (total: key_bytes_in)
   kScanBcum,           // tmp32 -> b_cum
   kScanGcum,           // b_gbytes -> b_gcum
@@ -124,7 +123,7 @@ void launch_table_index_count(const Batch& bt, cudaStream_t st);
 void launch_table_index_entries(const Batch& bt, cudaStream_t st);
 void launch_block_count(const Batch& bt, cudaStream_t st);     // exact key counts (full walk)
 void launch_block_restarts(const Batch& bt, cudaStream_t st);  // entry counts from restart words
-void launch_run_bounds(const Batch& bt, cudaStream_t st);
+void launch_parse_done(const Batch& bt, cudaStream_t st);  // merge children's entries; counters out
 // Checks the CRC32C trailer of every input data block of the jobs that ask
 // for it (verify_checksums), after the block list is known.
 void launch_verify_blocks(const Batch& bt, cudaStream_t st);

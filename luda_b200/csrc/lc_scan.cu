@@ -34,15 +34,6 @@ constexpr int kTile = kScanThreads * kScanItems;
 template <int S>
 struct ScanOf;
 template <>
-struct ScanOf<kScanTblBlocks> {
-  using TI = uint32_t;
-  using TO = uint64_t;
-  static __device__ const TI* in(const JobDev& J) { return J.tbl_nblocks; }
-  static __device__ TO* out(const JobDev& J) { return J.tbl_block_base; }
-  static __device__ uint64_t n(const JobDev& J) { return J.n_tables; }
-  static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->n_blocks_in; }
-};
-template <>
 struct ScanOf<kScanBlkEnt> {
   using TI = uint32_t;
   using TO = uint64_t;
@@ -307,7 +298,6 @@ void scan_sel(const Batch& bt, uint64_t n_est, cudaStream_t st) {
 
 void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st) {
   switch (sel) {
-    case kScanTblBlocks: scan_sel<kScanTblBlocks>(bt, n_est, st); break;
     case kScanBlkEnt: scan_sel<kScanBlkEnt>(bt, n_est, st); break;
     case kScanBlkKey: scan_sel<kScanBlkKey>(bt, n_est, st); break;
     case kScanBcum: scan_sel<kScanBcum>(bt, n_est, st); break;
