@@ -301,23 +301,21 @@ def make_desc(job: CompactionJob, keep: _Keep, device_tables: Optional[Sequence[
 def _result(out: LcJobOut, outputs_on_device) -> CompactionResult:
     """outputs_on_device: 0/False host bytes, 1/True device only, 2 both."""
     on_device = int(outputs_on_device) == 1
-    n = out.n_files
-    files, offs = [], []
-    if n:
-        # whole arrays at once: a job may have hundreds of files, and reading
-        # their fields one by one cost 6 us a file
-        offs, sizes = out.file_offset[:n], out.file_size[:n]
-        small, large = out.smallest_offset[:n], out.largest_offset[:n]
-        slen, llen = out.smallest_len[:n], out.largest_len[:n]
-        keys = C.string_at(out.key_bytes, max(large[-1] + llen[-1], small[-1] + slen[-1]))
-        dec = out.decoded[:n] if out.decoded else [None] * n
-        whole = None
-        if not on_device and out.bytes_out:
-            whole = memoryview(np.ctypeslib.as_array(C.cast(out.data, _u8p), shape=(out.bytes_out,)))
-        files = [OutputFile(whole[o:o + z] if whole is not None else b"", keys[a:a + la],
-                            keys[b:b + lb], e, d)
-                 for o, z, a, la, b, lb, e, d in zip(offs, sizes, small, slen, large, llen,
-                                                     out.file_entries[:n], dec)]
+    files = []
+    offs = []
+    whole = None
+    if not on_device and out.bytes_out:
+        whole = np.ctypeslib.as_array(C.cast(out.data, _u8p), shape=(out.bytes_out,))
+    for i in range(out.n_files):
+        off, size = out.file_offset[i], out.file_size[i]
+        offs.append(off)
+        data = b"" if on_device else memoryview(whole[off:off + size])
+        sm = C.string_at(C.addressof(out.key_bytes.contents) + out.smallest_offset[i],
+                         out.smallest_len[i])
+        lg = C.string_at(C.addressof(out.key_bytes.contents) + out.largest_offset[i],
+                         out.largest_len[i])
+        dec = out.decoded[i] if out.decoded else None
+        files.append(OutputFile(data, sm, lg, int(out.file_entries[i]), dec))
     phases = {out.phase_name[i].decode(): out.phase_ms[i] for i in range(out.n_phases)}
     return CompactionResult(files, out.bytes_in, out.bytes_out, out.entries_in, out.entries_out,
                             out.device_ms, out.device_data, offs,
