@@ -637,7 +637,7 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
     J.cap_key_bytes = r.K;
     J.cap_entries = N;
     J.e_rec = A.get<uint4>(N);
-    J.e_koff = A.get<uint32_t>(N + 1);  // + the total (the scan of the key lengths)
+    J.e_koff = A.get<uint32_t>(N);
     J.e_klen = A.get<uint32_t>(N);
     J.e_voff = A.get<uint32_t>(N);
     J.e_vlen = A.get<uint32_t>(N);

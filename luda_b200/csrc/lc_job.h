@@ -52,7 +52,7 @@ struct Counters {
   uint32_t pad;
   uint64_t kept_key_bytes;    // internal-key bytes of the survivors
   uint64_t kept_value_bytes;  // value bytes of the survivors
-  uint64_t key_cursor;        // arena bytes of the decoded keys (the scan of their slots)
+  uint64_t key_cursor;        // arena bytes the decode's units have taken
   uint32_t key_skip;          // user-key bytes every input key shares (prefixes start after them)
   uint32_t pad2;
   uint64_t key_total;         // decoded key bytes, summed by the decode's first pass

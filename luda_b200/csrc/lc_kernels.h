@@ -107,7 +107,6 @@ enum ScanSel : int {
   kScanIcum,           // b_isize -> b_icum
   kScanDecKey,         // k_klen -> dec_kcum (jobs that keep their decoded form)
   kScanKb,             // k_b -> k_pb (block size estimates)
-  kScanDecKlen,        // e_klen -> e_koff (decode: key places)  (total: key_cursor)
 };
 // n_est: about how many elements the longest job has (sizes the grid)
 void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st);

@@ -99,16 +99,6 @@ struct ScanOf<kScanKb> {
   static __device__ uint64_t* total(const JobDev&) { return nullptr; }
 };
 
-template <>
-struct ScanOf<kScanDecKlen> {
-  using TI = uint32_t;
-  using TO = uint32_t;
-  static __device__ const TI* in(const JobDev& J) { return J.e_klen; }
-  static __device__ TO* out(const JobDev& J) { return J.e_koff; }
-  static __device__ uint64_t n(const JobDev& J) { return J.ctr->n_entries_in; }
-  static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->key_cursor; }
-};
-
 template <typename T>
 __device__ __forceinline__ T warp_incl_scan(T v) {
   const int lane = threadIdx.x & 31;
@@ -144,19 +134,11 @@ __device__ __forceinline__ T block_excl_scan(T v, T* total) {
   return res;
 }
 
-// What a scan adds up of an element: itself, but a key's slot for its length.
-template <int S, typename TO>
-__device__ __forceinline__ TO scan_value(const JobDev& J, TO x) {
-  if constexpr (S == kScanDecKlen) return (x + J.key_pad) & ~(TO)J.key_pad;
-  return x;
-}
-
 // Eight consecutive elements from i (a multiple of 8) as 16-byte loads
 // (every scanned array starts on a 256-byte boundary); elements at or past n
 // read as zero.
-template <int S, typename TI, typename TO>
-__device__ __forceinline__ void load8(const JobDev& J, const TI* in, uint64_t i, uint64_t n,
-                                      TO (&v)[8]) {
+template <typename TI, typename TO>
+__device__ __forceinline__ void load8(const TI* in, uint64_t i, uint64_t n, TO (&v)[8]) {
   if (i + 8 <= n) {
     constexpr int kB = 8 * sizeof(TI);
     if constexpr (kB == 8) {
@@ -175,17 +157,15 @@ __device__ __forceinline__ void load8(const JobDev& J, const TI* in, uint64_t i,
 #pragma unroll
     for (int k = 0; k < 8; k++) v[k] = i + k < n ? (TO)in[i + k] : TO(0);
   }
-#pragma unroll
-  for (int k = 0; k < 8; k++) v[k] = scan_value<S, TO>(J, v[k]);  // (0 stays 0)
 }
 
 // Sum of in[lo, hi) over the CTA (every thread gets it); lo a multiple of 8.
-template <int S, typename TO, typename TI>
-__device__ __forceinline__ TO block_sum(const JobDev& J, const TI* in, uint64_t lo, uint64_t hi) {
+template <typename TO, typename TI>
+__device__ __forceinline__ TO block_sum(const TI* in, uint64_t lo, uint64_t hi) {
   TO s = 0;
   for (uint64_t i = lo + 8 * threadIdx.x; i < hi; i += 8 * blockDim.x) {
     TO v[8];
-    load8<S, TI, TO>(J, in, i, hi, v);
+    load8<TI, TO>(in, i, hi, v);
 #pragma unroll
     for (int k = 0; k < 8; k++) s += v[k];
   }
@@ -207,7 +187,7 @@ __global__ void k_tile_reduce(const JobDev* __restrict__ jobs) {
   const uint64_t n = SP::n(J);
   TO* tile_sums = reinterpret_cast<TO*>(J.scan_scratch);
   for (uint64_t t = blockIdx.x; t * kTile <= n; t += gridDim.x) {
-    const TO total = block_sum<S, TO>(J, SP::in(J), t * kTile, min(n, (t + 1) * kTile));
+    const TO total = block_sum<TO>(SP::in(J), t * kTile, min(n, (t + 1) * kTile));
     if (threadIdx.x == 0) tile_sums[t] = total;
   }
 }
@@ -233,7 +213,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_scan(const JobDev* __restrict
   // offset of this CTA's first tile; each step of the grid stride adds the
   // tiles it skips
   const auto before = [&](uint64_t t0, uint64_t t1) -> TO {  // tiles [t0, t1)
-    if constexpr (kDirect) return block_sum<S, TO>(J, in, t0 * kT, min(n, t1 * kT));
+    if constexpr (kDirect) return block_sum<TO>(in, t0 * kT, min(n, t1 * kT));
     TO x = 0, total;
     for (uint64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) x += tile_sums[i];
     block_excl_scan<TO>(x, &total);
@@ -243,7 +223,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_scan(const JobDev* __restrict
   for (uint64_t t = blockIdx.x; t * kT <= n; t += gridDim.x) {
     const uint64_t tb = t * kT + (uint64_t)threadIdx.x * kScanItems;
     alignas(16) TO v[8];
-    load8<S, typename SP::TI, TO>(J, in, tb, n, v);
+    load8<typename SP::TI, TO>(in, tb, n, v);
     TO s = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
@@ -305,7 +285,6 @@ void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st) {
     case kScanIcum: scan_sel<kScanIcum>(bt, n_est, st); break;
     case kScanDecKey: scan_sel<kScanDecKey>(bt, n_est, st); break;
     case kScanKb: scan_sel<kScanKb>(bt, n_est, st); break;
-    case kScanDecKlen: scan_sel<kScanDecKlen>(bt, n_est, st); break;
   }
 }
 
