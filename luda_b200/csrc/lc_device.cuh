@@ -28,6 +28,12 @@ __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;\ngriddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
+// Barrier over the cluster's threads: what they wrote before it is seen by all
+// of them after it.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t ld_le32(const uint8_t* p) {
   return (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
 }

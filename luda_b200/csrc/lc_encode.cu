@@ -35,6 +35,7 @@
 
 #include "lc_device.cuh"
 #include "lc_kernels.h"
+#include "lc_scan.cuh"
 
 namespace lc {
 
@@ -117,10 +118,18 @@ __global__ void __launch_bounds__(256, 8) k_sizes(const JobDev* __restrict__ job
 // restart s + mR, the difference between the entry's restart size and its
 // compressed size, plus the restart words.  `D` is that difference summed
 // over the restarts up to segment m (the segment holding e).
-__device__ __forceinline__ uint64_t block_est(const JobDev& J, uint64_t s, uint64_t e, uint64_t D,
-                                              uint64_t m) {
-  return J.k_pb[e + 1] - J.k_pb[s] + D + 4 * (m + 1) + 4;
-}
+struct BlockEst {
+  const uint64_t* pb;
+  const uint32_t *a, *b, *cuts;
+  uint32_t R, ncuts;
+  uint64_t bs;
+  __device__ __forceinline__ explicit BlockEst(const JobDev& J)
+      : pb(J.k_pb), a(J.k_a), b(J.k_b), cuts(J.t_kept), R(J.restart_interval),
+        ncuts(J.ctr->n_triggers), bs(J.block_size) {}
+  __device__ __forceinline__ uint64_t est(uint64_t s, uint64_t e, uint64_t D, uint64_t m) const {
+    return pb[e + 1] - pb[s] + D + 4 * (m + 1) + 4;
+  }
+};
 
 // next(s): the first survivor of the block after the one that starts at s.
 // The block ends after the first e whose estimate reaches block_size
@@ -128,27 +137,26 @@ __device__ __forceinline__ uint64_t block_est(const JobDev& J, uint64_t s, uint6
 // grandparent cut after s, or at the end.  Restart segments (R survivors)
 // are stepped through, then the segment that reaches block_size is binary
 // searched: O(block / R + log R) loads instead of a walk over the block.
-__device__ __forceinline__ uint64_t next_of(const JobDev& J, uint64_t s, uint64_t n) {
-  const uint32_t R = J.restart_interval;
-  const uint64_t bs = J.block_size;
-  uint32_t lo = 0, hi = J.ctr->n_triggers;
+__device__ __forceinline__ uint64_t next_of(const BlockEst& B, uint64_t s, uint64_t n) {
+  const uint32_t R = B.R;
+  uint32_t lo = 0, hi = B.ncuts;
   while (lo < hi) {
     const uint32_t mid = (lo + hi) >> 1;
-    if (J.t_kept[mid] <= s) lo = mid + 1;
+    if (B.cuts[mid] <= s) lo = mid + 1;
     else hi = mid;
   }
-  const uint64_t limit = lo < J.ctr->n_triggers ? min(n, (uint64_t)J.t_kept[lo]) : n;
+  const uint64_t limit = lo < B.ncuts ? min(n, (uint64_t)B.cuts[lo]) : n;
   uint64_t D = 0;
   for (uint64_t m = 0;; m++) {
     const uint64_t a = s + m * R;
     if (a >= limit) return limit;
-    D += J.k_a[a] - J.k_b[a];
+    D += B.a[a] - B.b[a];
     const uint64_t z = min(a + R, limit);  // segment [a, z)
-    if (block_est(J, s, z - 1, D, m) >= bs) {
+    if (B.est(s, z - 1, D, m) >= B.bs) {
       uint64_t l = a, h = z - 1;
       while (l < h) {
         const uint64_t mid = (l + h) >> 1;
-        if (block_est(J, s, mid, D, m) >= bs) h = mid;
+        if (B.est(s, mid, D, m) >= B.bs) h = mid;
         else l = mid + 1;
       }
       return l + 1;
@@ -156,26 +164,32 @@ __device__ __forceinline__ uint64_t next_of(const JobDev& J, uint64_t s, uint64_
   }
 }
 
-__global__ void __launch_bounds__(256, 6) k_next(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
+__device__ __forceinline__ void next(const JobDev& J, uint32_t cta, uint32_t ctas) {
   const uint64_t n = J.ctr->n_kept;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t s0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const BlockEst B(J);
+  uint32_t* const out = J.k_next;
+  const uint64_t stride = (uint64_t)ctas * blockDim.x;
+  const uint64_t s0 = (uint64_t)cta * blockDim.x + threadIdx.x;
   const uint64_t w0 = s0 - (threadIdx.x & 31);
   const uint64_t trips = n > w0 ? (n - w0 + stride - 1) / stride : 0;
   uint32_t jump = 0;
   for (uint64_t it = 0, s = s0; it < trips; it++, s += stride) {
     if (s < n) {
-      const uint64_t nxt = next_of(J, s, n);
-      J.k_next[s] = (uint32_t)nxt;
+      const uint64_t nxt = next_of(B, s, n);
+      out[s] = (uint32_t)nxt;
       jump = max(jump, (uint32_t)(nxt - s));
     }
   }
   // the longest block, one atomic per warp
   jump = __reduce_max_sync(0xffffffffu, jump);
   if ((threadIdx.x & 31) == 0 && jump) atomicMax(&J.ctr->max_jump, jump);
+}
+
+__global__ void __launch_bounds__(256, 6) k_next(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  if (J.ctr->error) return;  // a failed job does no more work
+  next(J, blockIdx.x, gridDim.x);
 }
 
 
@@ -206,29 +220,24 @@ __device__ __forceinline__ uint32_t chain_walk(const uint32_t* s_next, uint64_t 
   return chain_word(e - from, blocks);
 }
 
-__global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
-  if (threadIdx.x == 0) s_failed = J.ctr->error;
-  __syncthreads();
-  if (s_failed) return;
-  extern __shared__ uint32_t s_next[];  // chunk next() values, then sub-chunk words
+__device__ __forceinline__ void chain_tables(const JobDev& J, uint32_t cta, uint32_t ctas, uint32_t* s_next) {
+  const uint32_t* const knext = J.k_next;
+  uint32_t* const table = J.chunk_table;
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
   if (W > C) return;  // resolved sequentially instead
   const bool sub = W <= kChainSub;
   uint32_t* s_sub = s_next + C;  // (C / kChainSub) x W
-  for (uint64_t c = blockIdx.x; c * C < n; c += gridDim.x) {
+  for (uint64_t c = cta; c * C < n; c += ctas) {
     const uint64_t c0 = c * C;
     const uint64_t c1 = min(n, c0 + C);
     __syncthreads();
-    for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = J.k_next[c0 + i];
+    for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = knext[c0 + i];
     __syncthreads();
     if (!sub) {
       for (uint32_t i = threadIdx.x; i < W; i += blockDim.x)
-        J.chunk_table[c * C + i] = chain_walk(s_next, c0, c0 + i, c1, c0);
+        table[c * C + i] = chain_walk(s_next, c0, c0 + i, c1, c0);
       continue;
     }
     const uint32_t nsub = (uint32_t)((c1 - c0 + kChainSub - 1) / kChainSub);
@@ -247,19 +256,27 @@ __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
         e = s0 + (w & 0xffff);
         blocks += w >> 16;
       }
-      J.chunk_table[c * C + i] = chain_word(e - c0, blocks);
+      table[c * C + i] = chain_word(e - c0, blocks);
     }
   }
+}
+
+__global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
+  if (threadIdx.x == 0) s_failed = J.ctr->error;
+  __syncthreads();
+  if (s_failed) return;
+  extern __shared__ __align__(16) uint32_t s_dyn[];
+  chain_tables(J, blockIdx.x, gridDim.x, s_dyn);
 }
 
 // Exits (and blocks, in the high half) of groups of kChainGroup chunks for
 // every entry point in the first `window` survivors of the group's first
 // chunk, by following the chunk tables (one thread per entry point).  Only
 // when the chunk tables do not fit the resolving CTA's shared memory.
-__global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
+__device__ __forceinline__ void chain_groups(const JobDev& J, uint32_t cta, uint32_t ctas) {
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
@@ -267,8 +284,8 @@ __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
   const uint64_t M = (n + C - 1) / C;
   if (M * W <= J.chain_smem_words) return;  // resolved from the chunk tables directly
   const uint64_t G = (M + kChainGroup - 1) / kChainGroup;
-  for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < G * W;
-       x += (uint64_t)gridDim.x * blockDim.x) {
+  for (uint64_t x = (uint64_t)cta * blockDim.x + threadIdx.x; x < G * W;
+       x += (uint64_t)ctas * blockDim.x) {
     const uint64_t g = x / W, i = x % W;
     const uint64_t c0 = g * kChainGroup, c1 = min(M, c0 + kChainGroup);
     uint64_t e = c0 * C + i, blocks = 0;
@@ -281,19 +298,19 @@ __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
   }
 }
 
+__global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  if (J.ctr->error) return;  // a failed job does no more work
+  chain_groups(J, blockIdx.x, gridDim.x);
+}
+
 // Entry point and first block of every chunk: the chain from survivor 0
 // through the chunk tables.  Few chunks: one thread walks them over a
 // shared-memory copy of the tables.  Many: one thread walks the group tables
 // (in shared memory when they fit), then one thread per group walks its chunks
 // from the group's entry point.
-__global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
-  if (threadIdx.x == 0) s_failed = J.ctr->error;
-  __syncthreads();
-  if (s_failed) return;
-  extern __shared__ __align__(8) uint32_t s_tab[];
+__device__ __forceinline__ void chain_resolve(const JobDev& J, uint32_t* s_tab) {
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
@@ -372,19 +389,25 @@ __global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
   }
 }
 
-// First survivor of every block: each chunk's chain from its resolved entry
-// point.  With sub-chunks, one thread finds the sub-chunks' entry points from
-// their words (recomputed as k_chain_tables does) and every sub-chunk is
-// walked by its own thread.  (The block starts used to be flags that a scan
-// over the survivors turned into block numbers: 8M survivors, 47 us more.)
-__global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
+__global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
   if (threadIdx.x == 0) s_failed = J.ctr->error;
   __syncthreads();
   if (s_failed) return;
-  extern __shared__ uint32_t s_next[];
+  extern __shared__ __align__(16) uint32_t s_dyn[];
+  chain_resolve(J, s_dyn);
+}
+
+// First survivor of every block: each chunk's chain from its resolved entry
+// point.  With sub-chunks, one thread finds the sub-chunks' entry points from
+// their words (recomputed as k_chain_tables does) and every sub-chunk is
+// walked by its own thread.  (The block starts used to be flags that a scan
+// over the survivors turned into block numbers: 8M survivors, 47 us more.)
+__device__ __forceinline__ void chain_mark(const JobDev& J, uint32_t cta, uint32_t ctas, uint32_t* s_next) {
+  const uint32_t* const knext = J.k_next;
+  uint32_t* const first = J.b_first;
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
@@ -392,19 +415,19 @@ __global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
   const bool sub = W <= kChainSub;
   uint32_t* s_sub = s_next + C;
   __shared__ uint2 s_entry[32];  // sub-chunk entry points and first blocks (C / kChainSub of them)
-  for (uint64_t c = blockIdx.x; c * C < n; c += gridDim.x) {
+  for (uint64_t c = cta; c * C < n; c += ctas) {
     const uint64_t c0 = c * C;
     const uint64_t c1 = min(n, c0 + C);
     const uint2 at = J.chunk_entry[c];
     __syncthreads();
-    for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = J.k_next[c0 + i];
+    for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = knext[c0 + i];
     __syncthreads();
     if (!sub) {
       if (threadIdx.x == 0) {
         uint64_t e = at.x;
         uint32_t b = at.y;
         while (e < c1) {
-          J.b_first[b++] = (uint32_t)e;
+          first[b++] = (uint32_t)e;
           e = s_next[e - c0];
         }
       }
@@ -436,30 +459,48 @@ __global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
       uint64_t e = s_entry[sb].x;
       uint32_t b = s_entry[sb].y;
       while (e < send) {
-        J.b_first[b++] = (uint32_t)e;
+        first[b++] = (uint32_t)e;
         e = s_next[e - c0];
       }
     }
   }
 }
 
+__global__ void k_chain_mark(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
+  if (threadIdx.x == 0) s_failed = J.ctr->error;
+  __syncthreads();
+  if (s_failed) return;
+  extern __shared__ __align__(16) uint32_t s_dyn[];
+  chain_mark(J, blockIdx.x, gridDim.x, s_dyn);
+}
+
 // Sizes of the output blocks.
+__device__ __forceinline__ void block_sizes(const JobDev& J, uint32_t cta, uint32_t ctas) {
+  const uint32_t *const first = J.b_first, *const ka = J.k_a, *const kb = J.k_b;
+  const uint64_t* const pb = J.k_pb;
+  uint32_t *const sizes = J.b_size, *const flushed = J.tmp32;
+  const uint64_t nb = J.ctr->n_blocks_out;
+  const uint32_t R = J.restart_interval;
+  for (uint64_t b = (uint64_t)cta * blockDim.x + threadIdx.x; b < nb;
+       b += (uint64_t)ctas * blockDim.x) {
+    const uint64_t k = first[b], e = first[b + 1];
+    uint64_t D = 0;
+    for (uint64_t a = k; a < e; a += R) D += ka[a] - kb[a];
+    const uint64_t nrest = (e - k + R - 1) / R;
+    const uint32_t size = (uint32_t)(pb[e] - pb[k] + D + 4 * nrest + 4);
+    sizes[b] = size;
+    flushed[b] = size + kTrailer;
+  }
+}
+
 __global__ void k_block_sizes(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   if (J.ctr->error) return;  // a failed job does no more work
-  const uint64_t nb = J.ctr->n_blocks_out;
-  const uint32_t R = J.restart_interval;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = J.b_first[b], e = J.b_first[b + 1];
-    uint64_t D = 0;
-    for (uint64_t a = k; a < e; a += R) D += J.k_a[a] - J.k_b[a];
-    const uint64_t nrest = (e - k + R - 1) / R;
-    const uint32_t size = (uint32_t)(J.k_pb[e] - J.k_pb[k] + D + 4 * nrest + 4);
-    J.b_size[b] = size;
-    J.tmp32[b] = size + kTrailer;
-  }
+  block_sizes(J, blockIdx.x, gridDim.x);
 }
 
 // Like the block chain, a file's end depends on where it starts: every block
@@ -467,26 +508,27 @@ __global__ void k_block_sizes(const JobDev* __restrict__ jobs) {
 // binary search for the size cut, and the next forced block); one thread then
 // walks the few file starts.
 
-__global__ void k_file_next(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
+__device__ __forceinline__ void file_next(const JobDev& J, uint32_t cta, uint32_t ctas) {
+  const uint64_t* const cum = J.b_cum;
+  const uint32_t *const firsts = J.b_first, *const cuts = J.t_kept;
+  uint32_t* const out = J.b_fnext;
+  const uint64_t max_size = J.max_file_size;
   const uint64_t nb = J.ctr->n_blocks_out;
   const uint32_t nt = J.ctr->n_triggers;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (uint64_t)gridDim.x * blockDim.x) {
+  for (uint64_t b = (uint64_t)cta * blockDim.x + threadIdx.x; b < nb;
+       b += (uint64_t)ctas * blockDim.x) {
     // first block end where the file's flushed bytes reach max_file_size
-    const uint64_t cum0 = J.b_cum[b];
+    const uint64_t cum0 = cum[b];
     const uint64_t target =
-        J.max_file_size > ~0ull - cum0 ? ~0ull : cum0 + J.max_file_size;  // saturating
+        max_size > ~0ull - cum0 ? ~0ull : cum0 + max_size;  // saturating
     uint64_t sc;
-    if (J.b_cum[nb] < target) {
+    if (cum[nb] < target) {
       sc = nb - 1;
     } else {
       uint64_t l = b, h = nb - 1;
       while (l < h) {
         const uint64_t mid = (l + h) >> 1;
-        if (J.b_cum[mid + 1] >= target) h = mid;
+        if (cum[mid + 1] >= target) h = mid;
         else l = mid + 1;
       }
       sc = l;
@@ -494,24 +536,31 @@ __global__ void k_file_next(const JobDev* __restrict__ jobs) {
     // or before the first grandparent cut after the block's start, which is a
     // block's start too: the block that starts at cut survivor kp
     uint32_t lo = 0, hi = nt;
-    const uint32_t first = J.b_first[b];
+    const uint32_t first = firsts[b];
     while (lo < hi) {
       const uint32_t mid = (lo + hi) >> 1;
-      if (J.t_kept[mid] <= first) lo = mid + 1;
+      if (cuts[mid] <= first) lo = mid + 1;
       else hi = mid;
     }
-    if (lo < nt && J.t_kept[lo] <= J.b_first[sc]) {
-      const uint32_t kp = J.t_kept[lo];
+    if (lo < nt && cuts[lo] <= firsts[sc]) {
+      const uint32_t kp = cuts[lo];
       uint64_t l = b + 1, h = sc;
       while (l < h) {
         const uint64_t mid = (l + h) >> 1;
-        if (J.b_first[mid] >= kp) h = mid;
+        if (firsts[mid] >= kp) h = mid;
         else l = mid + 1;
       }
       sc = l - 1;
     }
-    J.b_fnext[b] = (uint32_t)(sc + 1);
+    out[b] = (uint32_t)(sc + 1);
   }
+}
+
+__global__ void k_file_next(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  if (J.ctr->error) return;  // a failed job does no more work
+  file_next(J, blockIdx.x, gridDim.x);
 }
 
 // The file starts are the orbit of block 0 under b_fnext, which only moves
@@ -522,13 +571,7 @@ __global__ void k_file_next(const JobDev* __restrict__ jobs) {
 // vector load stays inside its allocation.)
 constexpr uint32_t kFileTile = 4096;
 constexpr uint32_t kFileThreads = kFileTile / 4;
-__global__ void k_files(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
-  if (threadIdx.x == 0) s_failed = J.ctr->error;
-  __syncthreads();
-  if (s_failed) return;
+__device__ __forceinline__ void files(const JobDev& J) {
   __shared__ __align__(16) uint32_t tile[kFileTile];
   __shared__ uint64_t s_b;
   __shared__ uint32_t s_f;
@@ -570,6 +613,16 @@ __global__ void k_files(const JobDev* __restrict__ jobs) {
   if (threadIdx.x == 0) J.ctr->n_files = s_f;
 }
 
+__global__ void k_files(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
+  if (threadIdx.x == 0) s_failed = J.ctr->error;
+  __syncthreads();
+  if (s_failed) return;
+  files(J);
+}
+
 __device__ __forceinline__ uint32_t file_of_block(const JobDev& J, uint64_t b) {
   uint32_t lo = 0, hi = J.ctr->n_files;
   while (hi - lo > 1) {
@@ -582,64 +635,56 @@ __device__ __forceinline__ uint32_t file_of_block(const JobDev& J, uint64_t b) {
 
 __device__ void block_layout_one(const JobDev& J, uint64_t b);
 
-__global__ void __launch_bounds__(256, 6) k_block_layout(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  if (J.ctr->error) return;  // a failed job does no more work
+__device__ __forceinline__ void block_layout(const JobDev& J, uint32_t cta, uint32_t ctas) {
   const uint64_t nb = J.ctr->n_blocks_out;
-  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-       b += (uint64_t)gridDim.x * blockDim.x)
+  for (uint64_t b = (uint64_t)cta * blockDim.x + threadIdx.x; b < nb;
+       b += (uint64_t)ctas * blockDim.x)
     block_layout_one(J, b);
 }
 
+__global__ void __launch_bounds__(256, 5) k_block_layout(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  if (J.ctr->error) return;  // a failed job does no more work
+  block_layout(J, blockIdx.x, gridDim.x);
+}
+
 __device__ void block_layout_one(const JobDev& J, uint64_t b) {
+  // the loads that wait for nothing first
+  const uint64_t cum = J.b_cum[b], cum1 = J.b_cum[b + 1], cum_before = b ? J.b_cum[b - 1] : 0;
+  const uint32_t k0 = J.b_first[b], nx = J.b_first[b + 1], size = J.b_size[b];
   const uint32_t f = file_of_block(J, b);
   const uint32_t fb0 = J.files[f].first_block, fb1 = J.files[f].end_block;
-  if (b == fb0) J.files[f].first_kept = J.b_first[b];
-  if (b + 1 == fb1) J.files[f].end_kept = J.b_first[b + 1];
+  const bool last = b + 1 == fb1;
+  const uint32_t llen = J.k_klen[nx - 1], ulen = llen - 8;
+  const uint8_t* lkey = J.keys + J.k_koff[nx - 1];
+  const uint32_t nlen = last ? 8 : J.k_klen[nx], shared = last ? 0 : J.k_shared[nx];
+  const uint8_t* nkey = J.keys + (last ? 0 : J.k_koff[nx]);
   const uint64_t base = J.b_cum[fb0];
-  const uint64_t off = J.b_cum[b] - base;
-  J.b_file[b] = f;
-  J.b_off[b] = off;
-  if (J.b_size[b] > kEncNarrow) {  // windows for the longest 16-byte phase
-    const uint32_t n = (15 + J.b_size[b] + 1 + kEncWindow - 1) / kEncWindow;
-    const uint32_t at = atomicAdd(&J.ctr->n_wide, n);
-    // (past the capacity: the files outgrow the output, an error of the file layout)
-    for (uint32_t i = 0; i < n && at + i < J.cap_wide; i++) J.wide[at + i] = make_uint2((uint32_t)b, i);
-    J.b_crc[b] = 0;
-  }
+  const uint64_t off = cum - base;
   // filter group: blocks of this file whose start offsets share off >> 11
   uint32_t gbytes = 0, gkeys = 0;
   if (J.bits_per_key > 0) {
     const uint64_t j = off >> kFilterBaseLg;
-    const bool start = (b == fb0) || (((J.b_cum[b - 1] - base) >> kFilterBaseLg) != j);
+    const bool start = b == fb0 || ((cum_before - base) >> kFilterBaseLg) != j;
     if (start) {
-      uint64_t n = 0;
-      for (uint64_t bb = b; bb < fb1 && ((J.b_cum[bb] - base) >> kFilterBaseLg) == j; bb++)
-        n += J.b_first[bb + 1] - J.b_first[bb];
+      uint64_t n = nx - k0;
+      if (((cum1 - base) >> kFilterBaseLg) == j)
+        for (uint64_t bb = b + 1; bb < fb1 && ((J.b_cum[bb] - base) >> kFilterBaseLg) == j; bb++)
+          n += J.b_first[bb + 1] - J.b_first[bb];
       gkeys = (uint32_t)n;
       gbytes = bloom_bytes(n, J.bits_per_key) + 1;
     }
   }
-  J.b_gbytes[b] = gbytes;
-  J.b_gkeys[b] = gkeys;
   // index key for this block
-  uint32_t llen;
-  const uint8_t* lkey = kept_key(J, J.b_first[b + 1] - 1, &llen);
-  const uint32_t ulen = llen - 8;
   uint32_t sep = kNoSep, ilen = llen;
-  if (b + 1 < fb1) {
-    uint32_t nlen;
-    const uint8_t* nkey = kept_key(J, J.b_first[b + 1], &nlen);
-    const uint32_t nul = nlen - 8;
-    const uint32_t m = min(ulen, nul);
-    uint32_t d = 0;
-    while (d < m && lkey[d] == nkey[d]) d++;
-    if (d < m) {
-      const uint32_t db = lkey[d];
-      if (db < 0xff && db + 1 < nkey[d] && d + 1 < ulen) {
-        sep = d;
-        ilen = d + 1 + 8;
+  if (!last) {
+    // the prefix it shares with the next block's first key is known
+    if (shared < ulen && shared < nlen - 8) {
+      const uint32_t db = lkey[shared];
+      if (db < 0xff && db + 1 < nkey[shared] && shared + 1 < ulen) {
+        sep = shared;
+        ilen = shared + 1 + 8;
       }
     }
   } else {
@@ -650,19 +695,26 @@ __device__ void block_layout_one(const JobDev& J, uint64_t b) {
       ilen = i + 1 + 8;
     }
   }
-  const uint32_t hl = varint_len(off) + varint_len(J.b_size[b]);
+  const uint32_t hl = varint_len(off) + varint_len(size);
+  if (b == fb0) J.files[f].first_kept = k0;
+  if (last) J.files[f].end_kept = nx;
+  J.b_file[b] = f;
+  J.b_off[b] = off;
+  J.b_gbytes[b] = gbytes;
+  J.b_gkeys[b] = gkeys;
   J.b_sep[b] = sep;
   J.b_ilen[b] = ilen;
   J.b_isize[b] = 1 + varint_len(ilen) + varint_len(hl) + ilen + hl;
+  if (size > kEncNarrow) {  // windows for the longest 16-byte phase
+    const uint32_t n = (15 + size + 1 + kEncWindow - 1) / kEncWindow;
+    const uint32_t at = atomicAdd(&J.ctr->n_wide, n);
+    // (past the capacity: the files outgrow the output, an error of the file layout)
+    for (uint32_t i = 0; i < n && at + i < J.cap_wide; i++) J.wide[at + i] = make_uint2((uint32_t)b, i);
+    J.b_crc[b] = 0;
+  }
 }
 
-__global__ void k_file_layout(const JobDev* __restrict__ jobs) {
-  pdl_begin();
-  const JobDev& J = jobs[blockIdx.y];
-  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
-  if (threadIdx.x == 0) s_failed = J.ctr->error;
-  __syncthreads();
-  if (s_failed) return;
+__device__ __forceinline__ void file_layout(const JobDev& J) {
   const uint32_t nf = J.ctr->n_files;
   for (uint32_t f = threadIdx.x; f < nf; f += blockDim.x) {
     FileOut& F = J.files[f];
@@ -706,6 +758,72 @@ __global__ void k_file_layout(const JobDev* __restrict__ jobs) {
     // with exact counting instead of failing
     if (o > J.cap_out) set_error(J.ctr, J.reserve_keys ? kErrRetryExact : kErrLimit, 3);
   }
+}
+
+__global__ void k_file_layout(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
+  if (threadIdx.x == 0) s_failed = J.ctr->error;
+  __syncthreads();
+  if (s_failed) return;
+  file_layout(J);
+}
+
+// All of the above (kAll: a job of few entries) or all from the block sizes on
+// (a job of few blocks): one cluster of CTAs per job, a barrier where a launch
+// would end.  Each of these kernels has microseconds of work in a small job;
+// on B200 a launch of its own costs such a step about 3.5 us, a step in the
+// cluster 1.2 to 2.8 us (what is left is the steps' chains of dependent loads).
+// 512 threads a CTA: with 1024 the steps whose lanes each read a line of their
+// own waited for the L1 of half as many SMs (block sizes of 2000 blocks 5.6
+// instead of 4 us, block layout 14 instead of 5.6).
+// Measured (a call): 800 entries 204 -> 191 us; 80000 entries in 2070 blocks
+// 296 -> 283 us.  Above the limits below the kernels one by one are as fast or
+// faster (2070 blocks and all 80000 entries in the cluster: no gain, 13600
+// blocks: 20 us more), and many jobs at once fill the device with theirs.
+constexpr uint32_t kPartThreads = 512;
+constexpr uint32_t kPartMaxCtas = 8;
+constexpr uint64_t kPartEntries = 8192, kPartBlocks = 8192;
+template <bool kAll>
+__global__ void __launch_bounds__(kPartThreads, 1) k_partition(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  __shared__ JobDev s_job;
+  extern __shared__ __align__(16) uint32_t s_dyn[];
+  copy_job(jobs + blockIdx.y, &s_job);
+  __syncthreads();
+  const JobDev& J = s_job;
+  const uint32_t cta = blockIdx.x, ctas = gridDim.x;  // the grid's x is one cluster
+  if (*(volatile uint32_t*)&J.ctr->error) return;  // (the same in all CTAs: set before this kernel)
+  if constexpr (kAll) {
+    tile_scan<kScanKb, kPartThreads, true>(J, cta, ctas);
+    cluster_sync();
+    next(J, cta, ctas);
+    cluster_sync();
+    chain_tables(J, cta, ctas, s_dyn);
+    cluster_sync();
+    chain_groups(J, cta, ctas);
+    cluster_sync();
+    if (cta == 0) chain_resolve(J, s_dyn);
+    cluster_sync();
+    chain_mark(J, cta, ctas, s_dyn);
+    cluster_sync();
+  }
+  block_sizes(J, cta, ctas);
+  cluster_sync();
+  tile_scan<kScanBcum, kPartThreads, true>(J, cta, ctas);
+  cluster_sync();
+  file_next(J, cta, ctas);
+  cluster_sync();
+  if (cta == 0) files(J);
+  cluster_sync();
+  if (*(volatile uint32_t*)&J.ctr->error) return;  // too many files (the next to set it is file_layout)
+  block_layout(J, cta, ctas);
+  cluster_sync();
+  tile_scan<kScanIcum, kPartThreads, true>(J, cta, ctas);
+  tile_scan<kScanGcum, kPartThreads, true>(J, ctas - 1 - cta, ctas);  // few tiles: another CTA's
+  cluster_sync();
+  if (cta == 0) file_layout(J);
 }
 
 // Data blocks, assembled in shared memory: one warp per block of at most
@@ -1645,34 +1763,53 @@ __global__ void __launch_bounds__(256) k_results(const JobDev* __restrict__ jobs
 void launch_sizes(const Batch& bt, cudaStream_t st) {
   launch(k_sizes, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
-void launch_next(const Batch& bt, cudaStream_t st) {
-  launch(k_next, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
+
+namespace {
+// CTAs of a job's k_partition: a power of two, a thread for every item or kPartMaxCtas
+unsigned part_ctas(uint64_t items) {
+  unsigned c = 1;
+  while ((uint64_t)c * kPartThreads < items && c < kPartMaxCtas) c *= 2;
+  return c;
 }
-void launch_chain(const Batch& bt, cudaStream_t st) {
+}  // namespace
+
+void launch_partition(const Batch& bt, cudaStream_t st) {
   const uint64_t chunks = (bt.max_entries + bt.chunk - 1) / bt.chunk + 1;
   // next() values, sub-chunk words (windows up to kChainSub)
   const size_t smem = ((size_t)bt.chunk + (bt.chunk / kChainSub) * kChainSub) * sizeof(uint32_t);
-  const unsigned g = (unsigned)std::min<uint64_t>(chunks, bt.per_job(148 * 4));
-  launch(k_chain_tables, dim3(g, bt.B), 256, smem, st, bt.d);
+  const size_t resolve_smem = (size_t)bt.chain_smem_words * 4;
+  const unsigned all_ctas = part_ctas(bt.max_entries), blk_ctas = part_ctas(bt.max_blocks_out);
+  if (bt.max_entries <= kPartEntries && (uint64_t)all_ctas * bt.jobs_of_largest <= 148) {
+    launch_clusters(all_ctas, k_partition<true>, dim3(all_ctas, bt.B), kPartThreads,
+                    std::max(smem, resolve_smem), st, bt.d);
+    return;
+  }
+  const auto grid = [&](uint64_t per) {
+    return dim3(grid_x(bt.max_entries, (unsigned)per, bt.per_job(148 * 8)), bt.B);
+  };
+  scan_batch(kScanKb, bt, bt.max_entries, st);
+  launch(k_next, grid(256), 256, 0, st, bt.d);
+  const dim3 g((unsigned)std::min<uint64_t>(chunks, bt.per_job(148 * 4)), bt.B);
+  launch(k_chain_tables, g, 256, smem, st, bt.d);
   if (chunks > kChainGroup)
     launch(k_chain_groups, dim3(grid_x(chunks / kChainGroup * bt.chunk, 256, 148 * 4), bt.B), 256, 0, st, bt.d);
-  launch(k_chain_resolve, dim3(1, bt.B), 1024, (size_t)bt.chain_smem_words * 4, st, bt.d);
-  launch(k_chain_mark, dim3(g, bt.B), 128, smem, st, bt.d);
-}
-void launch_block_sizes(const Batch& bt, cudaStream_t st) {
-  launch(k_block_sizes, dim3(grid_x(bt.max_entries, 1024, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
-}
-void launch_files(const Batch& bt, cudaStream_t st) {
-  launch(k_file_next, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
+  launch(k_chain_resolve, dim3(1, bt.B), 1024, resolve_smem, st, bt.d);
+  launch(k_chain_mark, g, 128, smem, st, bt.d);
+  if (bt.max_blocks_out <= kPartBlocks && (uint64_t)blk_ctas * bt.jobs_of_largest <= 148) {
+    launch_clusters(blk_ctas, k_partition<false>, dim3(blk_ctas, bt.B), kPartThreads, 0, st, bt.d);
+    return;
+  }
+  launch(k_block_sizes, grid(1024), 256, 0, st, bt.d);
+  scan_batch(kScanBcum, bt, bt.max_entries, st);
+  launch(k_file_next, grid(256), 256, 0, st, bt.d);
   launch(k_files, dim3(1, bt.B), kFileThreads, 0, st, bt.d);
-}
-void launch_block_layout(const Batch& bt, cudaStream_t st) {
-  launch(k_block_layout, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
-}
-void launch_file_layout(const Batch& bt, cudaStream_t st) {
+  launch(k_block_layout, grid(256), 256, 0, st, bt.d);
+  scan_batch(kScanIcum, bt, bt.max_entries, st);
+  scan_batch(kScanGcum, bt, bt.max_entries, st);
   launch(k_file_layout, dim3(1, bt.B), 256, 0, st, bt.d);
 }
 void encode_kernel_attributes() {
+  cudaFuncSetAttribute(k_partition<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10);
   cudaFuncSetAttribute(k_encode_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEncSmem);
 }
 

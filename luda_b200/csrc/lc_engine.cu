@@ -548,6 +548,11 @@ uint64_t pow2_at_least(uint64_t x) {
   return p;
 }
 
+// About how many blocks n entries of `bytes` bytes together fill.
+uint64_t blocks_out(uint64_t n, uint64_t bytes, uint64_t block_size) {
+  return std::max<uint64_t>(1, std::min(n, bytes / std::max<uint64_t>(block_size, 1) + 1));
+}
+
 // Host-side state of one job inside a batch.
 struct JobRun {
   lc_job* j = nullptr;
@@ -608,16 +613,7 @@ void launch_tail(const Batch& bt, bool decode_merge, cudaStream_t st, PhaseTimer
   } else {
     launch_sizes(bt, st);
   }
-  scan_batch(kScanKb, bt, bt.max_entries, st);
-  launch_next(bt, st);
-  launch_chain(bt, st);
-  launch_block_sizes(bt, st);
-  scan_batch(kScanBcum, bt, bt.max_entries, st);
-  launch_files(bt, st);
-  launch_block_layout(bt, st);
-  scan_batch(kScanIcum, bt, bt.max_entries, st);
-  scan_batch(kScanGcum, bt, bt.max_entries, st);
-  launch_file_layout(bt, st);
+  launch_partition(bt, st);
   T.mark(kPartition);
   launch_encode_blocks(bt, st);
   launch_emit_decoded(bt, st);
@@ -832,10 +828,10 @@ struct lc_slot {
       return 0;
     }
     char key[256];
-    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%llu|%llu|%u|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
+    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%llu|%llu|%llu|%u|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
              (int)decode_merge, bt.B, bt.max_tables, bt.max_gp, bt.max_cap_triggers,
              bt.max_cap_files, (unsigned long long)bt.max_dec_groups,
-             (unsigned long long)bt.max_dec_units,
+             (unsigned long long)bt.max_dec_units, (unsigned long long)bt.max_blocks_out,
              (unsigned long long)bt.max_entries, (unsigned long long)bt.max_cap_wide, bt.merge_rounds, bt.chunk, bt.ctas_per_job,
              bt.merge_items, bt.merge_threads, bt.max_runs, bt.jobs_of_largest,
              (int)bt.any_keep_decoded);
@@ -1263,6 +1259,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       }
       max_runs = std::max<uint32_t>(max_runs, r.J.n_runs);
       bt.max_entries = std::max<uint64_t>(bt.max_entries, r.N);
+      bt.max_blocks_out = std::max(bt.max_blocks_out, blocks_out(r.N, r.in_bytes, r.j->opt.block_size));
       bt.max_cap_wide = std::max<uint64_t>(bt.max_cap_wide, r.J.cap_wide);
       bt.max_gp = std::max<uint32_t>(bt.max_gp, r.J.n_gp);
       bt.max_cap_triggers = std::max<uint32_t>(bt.max_cap_triggers, r.J.cap_triggers);
@@ -1274,6 +1271,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     // grid shapes in powers of two, so that batches of similar size share a
     // captured graph (the kernels loop over whatever the grid leaves)
     bt.max_entries = pow2_at_least(std::max<uint64_t>(bt.max_entries, 1));
+    bt.max_blocks_out = pow2_at_least(bt.max_blocks_out);
     bt.max_cap_wide = pow2_at_least(bt.max_cap_wide);
     bt.max_dec_groups = pow2_at_least(bt.max_dec_groups);
     bt.max_dec_units = pow2_at_least(bt.max_dec_units);
@@ -1572,6 +1570,7 @@ void run_build(lc_job* j, lc_slot& slot) {
     bt.d = slot.d_jobs;
     bt.B = 1;
     bt.max_entries = std::max<uint64_t>(N, 1);
+    bt.max_blocks_out = blocks_out(N, kb + vb, j->opt.block_size);
     bt.max_cap_wide = J.cap_wide;
     bt.max_cap_files = J.cap_files;
     bt.max_cap_triggers = J.cap_triggers;

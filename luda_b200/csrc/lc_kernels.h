@@ -29,21 +29,30 @@ uint32_t launches_on_this_thread();
 // when its predecessor has drained.  Every kernel launched so begins with
 // pdl_begin().  On B200: an 800-entry
 // job 288 -> 272 us a call, a 66 MiB job 756 -> 719 us.
+// launch_clusters: the same, in thread-block clusters of `cluster` CTAs along x.
 template <typename... P, typename... A>
-inline void launch(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
-                   A... args) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+inline void launch_clusters(unsigned cluster, void (*k)(P...), dim3 grid, unsigned threads,
+                            size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = dim3(threads);
   c.dynamicSmemBytes = smem;
   c.stream = st;
-  c.attrs = &at;
-  c.numAttrs = 1;
+  c.attrs = at;
+  c.numAttrs = cluster > 1 ? 2 : 1;
   cudaLaunchKernelEx(&c, k, P(args)...);
   note_launch();
+}
+template <typename... P, typename... A>
+inline void launch(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                   A... args) {
+  launch_clusters(1, k, grid, threads, smem, st, args...);
 }
 
 // Raise the dynamic shared-memory limits of the kernels that need more than
@@ -75,6 +84,7 @@ struct Batch {
   uint32_t max_tables = 0, max_gp = 0, max_cap_triggers = 0, max_cap_files = 0;
   uint64_t max_blocks_in = 0;  // data blocks, as the input's bytes suggest
   uint64_t max_entries = 0, max_cap_wide = 0;
+  uint64_t max_blocks_out = 0;  // data blocks, as the bytes and the block size suggest
   uint64_t max_dec_groups = 0, max_dec_units = 0;  // decode work units
   uint32_t merge_rounds = 0;
   uint32_t max_runs = 1;
@@ -143,12 +153,8 @@ void launch_kept_compact(const Batch& bt, cudaStream_t st);  // survivors and th
 
 // lc_encode.cu -- survivors -> output tables
 void launch_sizes(const Batch& bt, cudaStream_t st);       // flush encoder: entry sizes
-void launch_next(const Batch& bt, cudaStream_t st);
-void launch_chain(const Batch& bt, cudaStream_t st);
-void launch_block_sizes(const Batch& bt, cudaStream_t st);
-void launch_files(const Batch& bt, cudaStream_t st);
-void launch_block_layout(const Batch& bt, cudaStream_t st);
-void launch_file_layout(const Batch& bt, cudaStream_t st);
+// the survivors' blocks, files and index keys
+void launch_partition(const Batch& bt, cudaStream_t st);
 // data, filter and index blocks, metaindex, footer and file keys
 void launch_encode_blocks(const Batch& bt, cudaStream_t st);
 // the decoded form of the survivors, for jobs with keep_decoded
