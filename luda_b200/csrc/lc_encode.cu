@@ -974,26 +974,35 @@ __device__ __forceinline__ void enc_prefetch(const JobDev& J, const EncWarp& W, 
 // that holds block byte `at` starts, and that round: the prefix sums k_pb
 // give an entry's place but for the restarts before it, whose extra bytes are
 // summed here, a lane per round.
-__device__ __forceinline__ void enc_seek(const JobDev& J, const EncBlock& B, uint32_t R, uint32_t at,
-                                         uint32_t lane, uint32_t* j0, uint32_t* pos) {
+__device__ __forceinline__ void enc_seek(const JobDev& J, const EncBlock& B, const RestartDiv& rd,
+                                         uint32_t at, uint32_t lane, uint32_t* j0, uint32_t* pos) {
   const uint64_t pb0 = J.k_pb[B.s];
-  uint32_t extra0 = 0;  // extra bytes of the restarts before the group of 32 rounds
-  *j0 = 0, *pos = 0;
-  for (uint32_t g = 0; g < B.n; g += 1024) {
-    const uint32_t a = g + 32 * lane, z = min(a + 32, B.n);  // the lane's round
+  uint32_t group = 0, extra = 0;  // extra bytes of the restarts before the group, before j0
+  *j0 = 0;
+  for (uint32_t g = 0; B.n > 32 && g < B.n; g += 1024) {
+    const uint32_t a = g + 32 * lane, z = min(a + 32, B.n);  // the lane's entries
     uint32_t x = 0;
-    for (uint32_t j = (a + R - 1) / R * R; j < z; j += R) x += J.k_a[B.s + j] - J.k_b[B.s + j];
+    for (uint32_t j = rd.div(a + rd.R - 1) * rd.R; j < z; j += rd.R) x += J.k_a[B.s + j] - J.k_b[B.s + j];
     uint32_t tot;
-    const uint32_t before = warp_excl<uint32_t>(x, &tot) + extra0;
-    extra0 += tot;
+    const uint32_t before = warp_excl<uint32_t>(x, &tot) + group;
+    group += tot;
     const uint32_t p = a < B.n ? (uint32_t)(J.k_pb[B.s + a] - pb0) + before : 0xffffffffu;
     const unsigned m = __ballot_sync(0xffffffffu, p <= at);
-    if (!m) return;  // the group starts past `at`: the last round of the one before
+    if (!m) break;  // the group starts past `at`: among the last 32 of the one before
     const int l = 31 - __clz(m);
     *j0 = g + 32 * l;
-    *pos = __shfl_sync(0xffffffffu, p, l);
-    if (l < 31) return;
+    extra = __shfl_sync(0xffffffffu, before, l);
+    if (l < 31) break;
   }
+  const uint32_t j = *j0 + lane;
+  const bool in = j < B.n;
+  uint32_t tot;
+  const uint32_t x = in && rd.div(j) * rd.R == j ? J.k_a[B.s + j] - J.k_b[B.s + j] : 0u;
+  const uint32_t before = warp_excl<uint32_t>(x, &tot) + extra;
+  const uint32_t p = in ? (uint32_t)(J.k_pb[B.s + j] - pb0) + before : 0xffffffffu;
+  const int l = 31 - __clz(__ballot_sync(0xffffffffu, p <= at));
+  *j0 += l;
+  *pos = __shfl_sync(0xffffffffu, p, l);
 }
 
 // Grid positions [p0, p1) of the block into the warp's stage (kWide: a
@@ -1029,7 +1038,7 @@ __device__ __forceinline__ void enc_assemble(const JobDev& J, EncWarp& W, const 
         }
       }
     }
-    if (p0 && n > 32) enc_seek(J, B, R, p0 - ph, lane, &j0, &carry);
+    if (p0 && n > 1) enc_seek(J, B, rd, p0 - ph, lane, &j0, &carry);
   }
   for (; j0 < n; j0 += 32) {
     if (kWide && ph + carry >= p1) break;
@@ -1091,6 +1100,14 @@ __device__ __forceinline__ void enc_assemble(const JobDev& J, EncWarp& W, const 
       kd = kz - ka, vl = ve - va;
       kpos = ka, vpos = va;
     }
+    if (kWide && vl) {  // (a narrow block's were brought in before it was begun)
+      if (vl >= 256) {
+        bulk_prefetch_l2(val, vl);
+      } else {
+        prefetch_l2(val);
+        prefetch_l2(val + vl - 1);
+      }
+    }
     kpos -= p0, vpos -= p0;  // stage positions
     __syncwarp();  // every header of the round is written: the words may be ored now
     const bool lng = vl >= kEncLong;
@@ -1146,28 +1163,53 @@ __device__ __forceinline__ void enc_assemble(const JobDev& J, EncWarp& W, const 
           }
         }
       } else {
-        const uint32_t li = lane & 7, cnt = min(32u, n - j0);
-        for (uint32_t e0 = 0; e0 < cnt; e0 += 4) {
-          const uint32_t e = e0 + (lane >> 3);
+        constexpr uint32_t kU = 4;
+        const uint32_t li = lane & 7;
+        // words i, i + 8, .. (kU of them) of the value at d / q with efw words
+        const auto step = [&](uint32_t* d, const uint32_t* q, uint32_t efw, uint32_t fsh, uint32_t i) {
+          uint32_t lo[kU], hi[kU];
+#pragma unroll
+          for (uint32_t x = 0; x < kU; x++) {
+            const bool on = i + x * 8 < efw;
+            lo[x] = on ? __ldg(q + i + x * 8) : 0u;
+            hi[x] = on && fsh ? __ldg(q + i + x * 8 + 1) : 0u;
+          }
+#pragma unroll
+          for (uint32_t x = 0; x < kU; x++)
+            if (i + x * 8 < efw) d[i + x * 8] = __funnelshift_r(lo[x], hi[x], fsh);
+        };
+        const auto value = [&](uint32_t e, uint32_t i) {
           const uint32_t ew0 = __shfl_sync(0xffffffffu, w0, e);
           const uint32_t efw = __shfl_sync(0xffffffffu, fw, e);
           const uint32_t eso = __shfl_sync(0xffffffffu, so, e);
           const uintptr_t a = reinterpret_cast<uintptr_t>(J.in + eso);
-          const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3)) + li;
-          const uint32_t fsh = 8 * (uint32_t)(a & 3);
-          uint32_t* d = reinterpret_cast<uint32_t*>(st) + ew0 + li;
-          constexpr uint32_t kU = 4;
-          for (uint32_t i = li; i < efw; i += 8 * kU, q += 8 * kU, d += 8 * kU) {
-            uint32_t lo[kU], hi[kU];
-#pragma unroll
-            for (uint32_t x = 0; x < kU; x++) {
-              const bool on = i + x * 8 < efw;
-              lo[x] = on ? __ldg(q + x * 8) : 0u;
-              hi[x] = on && fsh ? __ldg(q + x * 8 + 1) : 0u;
+          step(reinterpret_cast<uint32_t*>(st) + ew0, reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3)),
+               efw, 8 * (uint32_t)(a & 3), i);
+        };
+        if (!__any_sync(0xffffffffu, fw > 8 * kU)) {  // one step each
+          const uint32_t cnt = min(32u, n - j0);
+          for (uint32_t e0 = 0; e0 < cnt; e0 += 4) value(e0 + (lane >> 3), li);
+        } else {
+          // the values' steps in one list, four at a time: of four values at a
+          // time the shorter ones' lanes wait for the longest.  An entry has at
+          // least one step, so that a step's entry is the number of entries that
+          // start at or before it: those of the steps before, and those of a
+          // mask of the starts among the next 32 steps.  (66 MiB of
+          // lognormal values, median 128: the kernel 109 -> 93 us.)
+          const uint32_t steps = valid ? max(1u, (fw + 8 * kU - 1) / (8 * kU)) : 0u;
+          uint32_t all;
+          const uint32_t at = warp_excl<uint32_t>(steps, &all);
+          uint32_t before = 0;  // entries that start before step t0
+          for (uint32_t t0 = 0; t0 < all; t0 += 32) {
+            const unsigned starts =
+                __reduce_or_sync(0xffffffffu, at - t0 < 32 ? 1u << (at - t0) : 0u);
+            for (uint32_t t = t0; t < min(t0 + 32, all); t += 4) {
+              const uint32_t r = t - t0 + (lane >> 3);  // this lane group's step
+              const uint32_t e = before + __popc(starts & (0xffffffffu >> (31 - r))) - 1;
+              const uint32_t first = __shfl_sync(0xffffffffu, at, e);
+              value(e, (t0 + r - first) * 8 * kU + li);  // (past the last step: past the value's end)
             }
-#pragma unroll
-            for (uint32_t x = 0; x < kU; x++)
-              if (i + x * 8 < efw) d[x * 8] = __funnelshift_r(lo[x], hi[x], fsh);
+            before += __popc(starts);
           }
         }
       }
