@@ -192,6 +192,150 @@ __global__ void __launch_bounds__(256, 6) k_next(const JobDev* __restrict__ jobs
   next(J, blockIdx.x, gridDim.x);
 }
 
+// k_pb and next() in one: a CTA scans a tile of k_b (the second launch of the
+// long scan), keeps the sums of the tile and of the
+// kNextHalo survivors after it in shared memory and finds next() from them.  A
+// block that reaches beyond is walked entry by entry over k_a and k_b.
+//
+// The searches read k_pb (8 bytes a survivor) and k_a, k_b from memory before,
+// about 14 dependent loads a survivor: 8M survivors in blocks of 66, the scan's
+// second launch 33 and k_next 140 us, this kernel 76; 4M survivors in 32 jobs, 64
+// and 38 us.  For up to kDirectMax survivors a scan of one launch and k_next
+// take 13 us, a form of this kernel that summed the survivors before its tile
+// itself 22.  Blocks of more than kNextHalo / 2 entries on average (many would
+// reach past the halo) stay with k_next too.
+__device__ __forceinline__ uint64_t next_walk(const JobDev& J, uint64_t s, uint64_t limit) {
+  const uint32_t R = J.restart_interval;
+  uint64_t est = 4;
+  uint32_t r = 0;  // entries since the last restart
+  for (uint64_t e = s; e < limit; e++) {
+    est += r == 0 ? J.k_a[e] + 4ull : J.k_b[e];
+    if (est >= J.block_size) return e + 1;
+    if (++r == R) r = 0;
+  }
+  return limit;
+}
+__global__ void __launch_bounds__(kScanThreads, 5) k_scan_next(const JobDev* __restrict__ jobs) {
+  pdl_begin();
+  const JobDev& J = jobs[blockIdx.y];
+  constexpr uint32_t kSpan = kTile + kNextHalo, kHaloItems = kNextHalo / kScanThreads;
+  __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
+  // sums of k_b from the tile's first survivor (if an entry of the span has more
+  // than kNextBig bytes the tile's survivors walk instead), restarts' extra bytes
+  __shared__ __align__(16) uint32_t s_pb[kSpan + 1], s_d[kSpan];
+  static_assert((uint64_t)kSpan * kNextBig + 2 * kNextBig < 1ull << 31);
+  if (threadIdx.x == 0) s_failed = J.ctr->error;
+  __syncthreads();
+  if (s_failed) return;
+  const uint64_t n = J.ctr->n_kept;
+  if ((uint64_t)blockIdx.x * kTile > n) return;
+  const uint64_t* tile_sums = reinterpret_cast<const uint64_t*>(J.scan_scratch);
+  const uint32_t *const ka = J.k_a, *const kb = J.k_b, *const cuts = J.t_kept;
+  uint64_t* const pb = J.k_pb;
+  uint32_t* const out = J.k_next;
+  const uint32_t R = J.restart_interval, ncuts = J.ctr->n_triggers;
+  const uint32_t bs = (uint32_t)J.block_size;
+  uint64_t carry = tiles_sum<uint64_t, false>(kb, tile_sums, 0, blockIdx.x, kTile, n);
+  uint32_t jump = 0;
+  for (uint64_t t = blockIdx.x; t * kTile <= n; t += gridDim.x) {
+    const uint64_t t0 = t * kTile;
+    const uint32_t avail = (uint32_t)min(n - t0, (uint64_t)kSpan);
+    const uint32_t i0 = threadIdx.x * kScanItems;
+    bool big = false;
+    uint32_t v[kScanItems], h[kHaloItems], hs = 0;
+    uint64_t s = 0;
+    {
+      uint32_t a[kScanItems];
+      load8<uint32_t, uint32_t>(kb, t0 + i0, n, v);
+      load8<uint32_t, uint32_t>(ka, t0 + i0, n, a);
+#pragma unroll
+      for (uint32_t k = 0; k < kHaloItems; k++) {
+        const uint32_t i = kTile + threadIdx.x * kHaloItems + k;
+        const uint32_t x = i < avail ? ka[t0 + i] : 0;
+        h[k] = i < avail ? kb[t0 + i] : 0;
+        s_d[i] = x - h[k];
+        big |= x > kNextBig;
+        hs += h[k];
+      }
+#pragma unroll
+      for (int k = 0; k < kScanItems; k++) {
+        s_d[i0 + k] = a[k] - v[k];
+        big |= a[k] > kNextBig;
+        s += v[k];
+      }
+    }
+    uint64_t total;
+    uint32_t htotal;
+    uint64_t ex = block_excl_scan<uint64_t>(s, &total);
+    uint32_t hx = block_excl_scan<uint32_t>(hs, &htotal) + (uint32_t)total;
+#pragma unroll
+    for (uint32_t k = 0; k < kHaloItems; k++) {
+      s_pb[kTile + threadIdx.x * kHaloItems + k] = hx;
+      hx += h[k];
+    }
+    if (threadIdx.x == 0) s_pb[kSpan] = (uint32_t)total + htotal;
+    const uint64_t tb = t0 + i0;
+    {
+      uint32_t r = (uint32_t)ex;
+#pragma unroll
+      for (int k = 0; k < kScanItems; k++) {
+        s_pb[i0 + k] = r;
+        r += v[k];
+      }
+    }
+    ex += carry;
+    if (tb <= n && n < tb + kScanItems) pb[n] = ex + s;  // (survivors past n add nothing)
+#pragma unroll
+    for (int k = 0; k < kScanItems; k += 2) {
+      const uint64_t e1 = ex + v[k];
+      if (tb + k + 2 <= n)
+        *reinterpret_cast<ulonglong2*>(pb + tb + k) = make_ulonglong2(ex, e1);
+      else if (tb + k < n)
+        pb[tb + k] = ex;
+      ex = e1 + v[k + 1];
+    }
+    const bool walk = __syncthreads_or(big);
+    const uint32_t here = (uint32_t)min(n - t0, (uint64_t)kTile);
+    for (uint32_t i = threadIdx.x; i < here; i += kScanThreads) {
+      uint32_t lo = 0, hi = ncuts;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (cuts[mid] <= t0 + i) lo = mid + 1;
+        else hi = mid;
+      }
+      const uint64_t limit = lo < ncuts ? min(n, (uint64_t)cuts[lo]) : n;
+      const uint32_t last = walk ? 0 : (uint32_t)min(limit - t0, (uint64_t)avail);  // searched up to here
+      // as next_of: the restart segment that reaches the block size, then the entry
+      uint32_t nxt = 0;                // from the tile's first survivor
+      uint32_t need = bs + s_pb[i] - 4;  // less the restarts' extra bytes and words, and the count's
+      for (uint32_t x = i; x < last; x += R) {
+        need -= s_d[x] + 4;
+        const uint32_t z = min(x + R, last);
+        if ((int32_t)(s_pb[z] - need) >= 0) {
+          uint32_t l = x, r = z - 1;
+          while (l < r) {
+            const uint32_t mid = (l + r) >> 1;
+            if ((int32_t)(s_pb[mid + 1] - need) >= 0) r = mid;
+            else l = mid + 1;
+          }
+          nxt = l + 1;
+          break;
+        }
+      }
+      if (!nxt)
+        nxt = (uint32_t)((t0 + last == limit ? limit : next_walk(J, t0 + i, limit)) - t0);
+      out[t0 + i] = (uint32_t)t0 + nxt;
+      jump = max(jump, nxt - i);
+    }
+    __syncthreads();  // the tile's sums have been read
+    if ((t + gridDim.x) * kTile <= n)
+      carry += tiles_sum<uint64_t, false>(kb, tile_sums, t, t + gridDim.x, kTile, n);
+  }
+  // the longest block, one atomic per warp
+  jump = __reduce_max_sync(0xffffffffu, jump);
+  if ((threadIdx.x & 31) == 0 && jump) atomicMax(&J.ctr->max_jump, jump);
+}
+
 
 // Per chunk: exits of the chain for every entry point in the first `window`
 // survivors of the chunk.  The chunk's next() values are staged in shared
@@ -1829,8 +1973,14 @@ void launch_partition(const Batch& bt, cudaStream_t st) {
   const auto grid = [&](uint64_t per) {
     return dim3(grid_x(bt.max_entries, (unsigned)per, bt.per_job(148 * 8)), bt.B);
   };
-  scan_batch(kScanKb, bt, bt.max_entries, st);
-  launch(k_next, grid(256), 256, 0, st, bt.d);
+  if (bt.max_entries > kDirectMax && bt.max_block_entries <= kNextHalo / 2) {
+    tile_sums_kb(bt, bt.max_entries, st);
+    launch(k_scan_next, dim3(grid_x(bt.max_entries + 1, kTile, bt.per_job(148 * 5)), bt.B), kScanThreads,
+           0, st, bt.d);
+  } else {
+    scan_batch(kScanKb, bt, bt.max_entries, st);
+    launch(k_next, grid(256), 256, 0, st, bt.d);
+  }
   const dim3 g((unsigned)std::min<uint64_t>(chunks, bt.per_job(148 * 4)), bt.B);
   launch(k_chain_tables, g, 256, smem, st, bt.d);
   if (chunks > kChainGroup)

@@ -828,10 +828,11 @@ struct lc_slot {
       return 0;
     }
     char key[256];
-    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%llu|%llu|%llu|%u|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
+    snprintf(key, sizeof(key), "%d|%d|%u|%u|%u|%u|%u|%llu|%llu|%llu|%llu|%llu|%llu|%u|%u|%u|%u|%u|%u|%u|%d", (int)T.on,
              (int)decode_merge, bt.B, bt.max_tables, bt.max_gp, bt.max_cap_triggers,
              bt.max_cap_files, (unsigned long long)bt.max_dec_groups,
              (unsigned long long)bt.max_dec_units, (unsigned long long)bt.max_blocks_out,
+             (unsigned long long)bt.max_block_entries,
              (unsigned long long)bt.max_entries, (unsigned long long)bt.max_cap_wide, bt.merge_rounds, bt.chunk, bt.ctas_per_job,
              bt.merge_items, bt.merge_threads, bt.max_runs, bt.jobs_of_largest,
              (int)bt.any_keep_decoded);
@@ -1259,7 +1260,10 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       }
       max_runs = std::max<uint32_t>(max_runs, r.J.n_runs);
       bt.max_entries = std::max<uint64_t>(bt.max_entries, r.N);
-      bt.max_blocks_out = std::max(bt.max_blocks_out, blocks_out(r.N, r.in_bytes, r.j->opt.block_size));
+      const uint64_t blocks = blocks_out(r.N, r.in_bytes, r.j->opt.block_size);
+      bt.max_blocks_out = std::max(bt.max_blocks_out, blocks);
+      bt.max_block_entries = std::max(bt.max_block_entries,
+                                      r.j->opt.block_size > kNextBig ? uint64_t(1) << 30 : r.N / blocks);
       bt.max_cap_wide = std::max<uint64_t>(bt.max_cap_wide, r.J.cap_wide);
       bt.max_gp = std::max<uint32_t>(bt.max_gp, r.J.n_gp);
       bt.max_cap_triggers = std::max<uint32_t>(bt.max_cap_triggers, r.J.cap_triggers);
@@ -1272,6 +1276,7 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
     // captured graph (the kernels loop over whatever the grid leaves)
     bt.max_entries = pow2_at_least(std::max<uint64_t>(bt.max_entries, 1));
     bt.max_blocks_out = pow2_at_least(bt.max_blocks_out);
+    bt.max_block_entries = pow2_at_least(std::max<uint64_t>(bt.max_block_entries, 1));
     bt.max_cap_wide = pow2_at_least(bt.max_cap_wide);
     bt.max_dec_groups = pow2_at_least(bt.max_dec_groups);
     bt.max_dec_units = pow2_at_least(bt.max_dec_units);
@@ -1571,6 +1576,7 @@ void run_build(lc_job* j, lc_slot& slot) {
     bt.B = 1;
     bt.max_entries = std::max<uint64_t>(N, 1);
     bt.max_blocks_out = blocks_out(N, kb + vb, j->opt.block_size);
+    bt.max_block_entries = j->opt.block_size > kNextBig ? uint64_t(1) << 30 : N / bt.max_blocks_out;
     bt.max_cap_wide = J.cap_wide;
     bt.max_cap_files = J.cap_files;
     bt.max_cap_triggers = J.cap_triggers;

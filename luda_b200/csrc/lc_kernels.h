@@ -77,6 +77,10 @@ constexpr uint32_t kEncWindow = 4608;  // 9 full CRC rows
 constexpr uint32_t kMergeMaxTile = 4096;
 constexpr uint32_t kMergeSmemPerPos = 14;
 
+// k_scan_next: survivors after its tile that it keeps, and the largest entry
+// and block size its 32-bit sums are for.
+constexpr uint32_t kNextHalo = 512, kNextBig = 1u << 19;
+
 struct Batch {
   const JobDev* d = nullptr;  // device array of B job descriptors
   uint32_t B = 0;
@@ -85,6 +89,7 @@ struct Batch {
   uint64_t max_blocks_in = 0;  // data blocks, as the input's bytes suggest
   uint64_t max_entries = 0, max_cap_wide = 0;
   uint64_t max_blocks_out = 0;  // data blocks, as the bytes and the block size suggest
+  uint64_t max_block_entries = 0;  // a block's entries, likewise (2^30: a block size past kNextBig)
   uint64_t max_dec_groups = 0, max_dec_units = 0;  // decode work units
   uint32_t merge_rounds = 0;
   uint32_t max_runs = 1;
@@ -121,6 +126,8 @@ enum ScanSel : int {
 // n_est: about how many elements the longest job has (sizes the grid)
 void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st);
 uint64_t scan_scratch_elems(uint64_t n_cap);
+// the first of a long scan's two launches, for k_b (k_scan_next is the second)
+void tile_sums_kb(const Batch& bt, uint64_t n_est, cudaStream_t st);
 
 // lc_crc.cu -- masked CRC32C of one buffer; the kCrcScratchWords words of
 // `scratch` must be zero at launch and are zero again when the kernel is done

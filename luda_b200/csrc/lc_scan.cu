@@ -62,7 +62,13 @@ __global__ void __launch_bounds__(kThreads) k_tile_scan(const JobDev* __restrict
 // before its tile, at most 16 tiles.  More: tile sums first.  At 80k elements
 // one launch takes 4 us, two take 7.
 constexpr uint64_t kDirectThreads = 1024;
-constexpr uint64_t kDirectMax = 16 * kDirectThreads * kScanItems;
+static_assert(kDirectMax == 16 * kDirectThreads * kScanItems);
+
+template <int S>
+void launch_tile_sums(const Batch& bt, uint64_t n_est, cudaStream_t st) {
+  launch(k_tile_reduce<S>, dim3(grid_x(n_est + 1, kTile, bt.per_job(148 * 8)), bt.B), kScanThreads, 0,
+         st, bt.d);
+}
 
 template <int S>
 void scan_sel(const Batch& bt, uint64_t n_est, cudaStream_t st) {
@@ -72,7 +78,7 @@ void scan_sel(const Batch& bt, uint64_t n_est, cudaStream_t st) {
     return;
   }
   const unsigned tiles = grid_x(n_est + 1, kTile, bt.per_job(148 * 8));
-  launch(k_tile_reduce<S>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
+  launch_tile_sums<S>(bt, n_est, st);
   launch(k_tile_scan<S, kScanThreads, false>, dim3(tiles, bt.B), kScanThreads, 0, st, bt.d);
 }
 
@@ -88,6 +94,10 @@ void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st) {
     case kScanDecKey: scan_sel<kScanDecKey>(bt, n_est, st); break;
     case kScanKb: scan_sel<kScanKb>(bt, n_est, st); break;
   }
+}
+
+void tile_sums_kb(const Batch& bt, uint64_t n_est, cudaStream_t st) {
+  launch_tile_sums<kScanKb>(bt, n_est, st);
 }
 
 // tile sums for arrays of up to n_cap elements: 8 bytes for every kTile of them

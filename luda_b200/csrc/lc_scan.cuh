@@ -12,6 +12,7 @@ namespace {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kTile = kScanThreads * kScanItems;
+constexpr uint64_t kDirectMax = 131072;  // elements scanned without tile sums (lc_scan.cu)
 
 template <int S>
 struct ScanOf;
@@ -156,6 +157,19 @@ __device__ __forceinline__ TO block_sum(const TI* in, uint64_t lo, uint64_t hi) 
   return total;
 }
 
+// Sum over the CTA of the elements in tiles [t0, t1) of kT elements: from the
+// elements (kDirect) or the tile sums.
+template <typename TO, bool kDirect, typename TI>
+__device__ __forceinline__ TO tiles_sum(const TI* in, const TO* tile_sums, uint64_t t0, uint64_t t1,
+                                        uint64_t kT, uint64_t n) {
+  if (t0 == t1) return 0;
+  if constexpr (kDirect) return block_sum<TO>(in, t0 * kT, min(n, t1 * kT));
+  TO x = 0, total;
+  for (uint64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) x += tile_sums[i];
+  block_excl_scan<TO>(x, &total);
+  return total;
+}
+
 // CTA `cta` of `ctas` (of kThreads threads) of the scan of one job's array.
 // kDirect: no tile sums; a CTA sums the elements before its tile itself.
 template <int S, int kThreads, bool kDirect>
@@ -171,13 +185,8 @@ __device__ __forceinline__ void tile_scan(const JobDev& J, uint32_t cta, uint32_
   uint64_t* total_out = SP::total(J);
   // offset of this CTA's first tile; each step of the grid stride adds the
   // tiles it skips
-  const auto before = [&](uint64_t t0, uint64_t t1) -> TO {  // tiles [t0, t1)
-    if (t0 == t1) return 0;
-    if constexpr (kDirect) return block_sum<TO>(in, t0 * kT, min(n, t1 * kT));
-    TO x = 0, total;
-    for (uint64_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) x += tile_sums[i];
-    block_excl_scan<TO>(x, &total);
-    return total;
+  const auto before = [&](uint64_t t0, uint64_t t1) -> TO {
+    return tiles_sum<TO, kDirect>(in, tile_sums, t0, t1, kT, n);
   };
   TO carry = before(0, cta);
   for (uint64_t t = cta; t * kT <= n; t += ctas) {

@@ -82,3 +82,42 @@ def test_index_keys(engine, oracle_lib, kind, n, block):
 @pytest.mark.parametrize("n", [600, 5000, 9000, 30000])
 def test_grandparent_cuts(engine, oracle_lib, n):
     _run(engine, n, TableOptions(512, 16, 10, 8192), "digits", 40, gp_every=max(4, n // 60))
+
+
+def _long_job(lens, opts, gp_every=0):
+    rng = np.random.default_rng(len(lens))
+    n = len(lens)
+    data = rng.bytes(1 << 20)
+    files = []
+    for lv in (0, 1):
+        ids = range(lv, n, 2)
+        e = Entries.from_lists([internal_key(b"%08d" % i, 1 + i, 1) for i in ids],
+                               [data[i % 1000:i % 1000 + int(lens[i])] for i in ids])
+        files.append(FileMeta(lv, lv + 1, e.key(0), e.key(e.n - 1), entries=e))
+    for g in range(0, n - gp_every, gp_every) if gp_every else ():
+        files.append(FileMeta(2, 100 + g, internal_key(b"%08d" % g, 5, 1),
+                              internal_key(b"%08d" % (g + gp_every // 2), 5, 1),
+                              file_size=4 * opts.max_file_size))
+    return CompactionJob(0, files, [], 1 << 30, opts).materialize(
+        lambda e, o: oracle.build_table(e, o, "oracle"))
+
+
+@pytest.mark.parametrize("restart", [1, 16, 255])
+@pytest.mark.parametrize("kind", ["dense_runs", "big_entries", "plain", "cuts"])
+def test_block_starts_of_long_jobs(engine, oracle_lib, kind, restart):
+    """More than 131072 survivors: the block starts are searched for in tiles of
+    2048 survivors and the 512 after them.  Runs of empty values make blocks
+    that reach further, entries of more than 512 KiB leave the 32-bit sums."""
+    n, block, gp = 140000, 4096, 0
+    lens = np.random.default_rng(7).integers(0, 60, n)
+    if kind == "dense_runs":
+        block = 8192
+        lens = np.where(np.arange(n) // 5000 % 3 < 2, 0, 300)
+    elif kind == "big_entries":
+        lens[[5, 2047, 2048, 70000, 70001, 139999]] = [600000, 524288, 524270, 530000, 900000, 700000]
+    elif kind == "cuts":
+        gp = 900
+    job = _long_job(lens, TableOptions(block, restart, 10, 1 << 18 if gp else 1 << 22), gp)
+    res = engine.run(engine.prepare(job))
+    assert res.file_bytes() == [w[0] for w in oracle.compact(job, "oracle")]
+    res.release()
