@@ -860,8 +860,6 @@ __device__ __forceinline__ void decode_round_regs(const JobDev& J, uint8_t* last
   const uint32_t t0 = (t & 1) ? z[1] : z[0], t1 = (t & 1) ? z[2] : z[1], t2 = (t & 1) ? z[3] : z[2];
   const uint32_t ts = 8 * (u & 3);
   const uint64_t tag = (uint64_t)__funnelshift_r(t0, t1, ts) | ((uint64_t)__funnelshift_r(t1, t2, ts) << 32);
-  J.e_voff[e] = rec.w;
-  J.e_vlen[e] = rec.z;
   J.e_pfx[e] = p;
   J.e_tag[e] = tag;
   if (J.bits_per_key > 0) {  // bloom_hash
@@ -928,8 +926,7 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
       uint32_t tot;
       const uint32_t ko = warp_excl<uint32_t>((kl + pad) & ~pad, &tot);  // offset within the round
       if (valid) {
-        J.e_koff[e] = (uint32_t)(kpos + ko);
-        J.e_klen[e] = kl;
+        J.e_loc[e] = make_uint4((uint32_t)(kpos + ko), kl, rec.w, rec.z);
       }
       if (mk <= 4 * kDecRegWords && pad && (sh0 == 0 || last_staged)) {
         decode_round_regs(J, W.last, e, valid, rec, src, (uint32_t)(kpos + ko), kl, sh, cnt, lane);
@@ -1006,8 +1003,6 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
         const uint32_t t0 = h + body;
         if (t0 + lane < tot) gdst[t0 + lane] = kb[t0 + lane];
         if (valid) {
-          J.e_voff[e] = rec.w;
-          J.e_vlen[e] = rec.z;
           J.e_pfx[e] = user_prefix(kb + ko, kl);
           J.e_tag[e] = ld_le64(kb + ko + kl - 8);
           if (J.bits_per_key > 0) J.e_hash[e] = bloom_hash(kb + ko, kl);
@@ -1032,8 +1027,6 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
         if (last_staged)
           for (uint32_t t = lane; t < lkl; t += 32) W.last[t] = gdst[lko + t];
         if (valid) {
-          J.e_voff[e] = rec.w;
-          J.e_vlen[e] = rec.z;
           J.e_pfx[e] = user_prefix(gdst + ko, kl);
           J.e_tag[e] = ld_le64(gdst + ko + kl - 8);
           if (J.bits_per_key > 0) J.e_hash[e] = bloom_hash(gdst + ko, kl);
@@ -1056,12 +1049,6 @@ __global__ void k_entries_from_offsets(const JobDev* __restrict__ jobs) {
       set_error(J.ctr, kErrShortKey, (uint32_t)i);
       continue;
     }
-    J.e_koff[i] = (uint32_t)ko;
-    J.e_klen[i] = (uint32_t)kl;
-    J.e_voff[i] = (uint32_t)J.src_voffs[i];
-    J.e_vlen[i] = (uint32_t)(J.src_voffs[i + 1] - J.src_voffs[i]);
-    J.e_pfx[i] = user_prefix(J.keys + ko, (uint32_t)kl);
-    J.e_tag[i] = ld_le64(J.keys + ko + kl - 8);
     J.k_koff[i] = (uint32_t)ko;
     J.k_klen[i] = (uint32_t)kl;
     J.k_voff[i] = (uint32_t)J.src_voffs[i];

@@ -151,10 +151,11 @@ __device__ __forceinline__ uint64_t user_prefix_after(const uint8_t* k, uint32_t
 // or above zero.  Their first key_skip + 8 bytes are equal as far as both user
 // keys have them, so that only what follows is compared.
 __device__ __forceinline__ int user_key_rest_cmp(const JobDev& J, uint32_t a, uint32_t b) {
-  const uint32_t al = J.e_klen[a] - 8, bl = J.e_klen[b] - 8, m = al < bl ? al : bl;
+  const uint2 la = *reinterpret_cast<const uint2*>(J.e_loc + a), lb = *reinterpret_cast<const uint2*>(J.e_loc + b);
+  const uint32_t al = la.y - 8, bl = lb.y - 8, m = al < bl ? al : bl;
   uint32_t i = J.ctr->key_skip + 8;
   if (i < m) {
-    const uint8_t *x = J.keys + J.e_koff[a], *y = J.keys + J.e_koff[b];
+    const uint8_t *x = J.keys + la.x, *y = J.keys + lb.x;
     for (; i < m; i++)
       if (x[i] != y[i]) return x[i] < y[i] ? -1 : 1;
   }

@@ -633,10 +633,7 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
     J.cap_key_bytes = r.K;
     J.cap_entries = N;
     J.e_rec = A.get<uint4>(N);
-    J.e_koff = A.get<uint32_t>(N);
-    J.e_klen = A.get<uint32_t>(N);
-    J.e_voff = A.get<uint32_t>(N);
-    J.e_vlen = A.get<uint32_t>(N);
+    J.e_loc = A.get<uint4>(N);
     J.e_pfx = A.get<uint64_t>(N);
     J.e_tag = A.get<uint64_t>(N);
     J.e_hash = A.get<uint32_t>(J.bits_per_key > 0 ? N : 1);
@@ -1561,12 +1558,6 @@ void run_build(lc_job* j, lc_slot& slot) {
     init.n_kept = N;
     init.n_entries_in = N;
     CK(cudaMemcpyAsync(J.ctr, &init, sizeof(Counters), cudaMemcpyHostToDevice, st));
-    J.e_koff = A.get<uint32_t>(N);
-    J.e_klen = A.get<uint32_t>(N);
-    J.e_voff = A.get<uint32_t>(N);
-    J.e_vlen = A.get<uint32_t>(N);
-    J.e_pfx = A.get<uint64_t>(N);
-    J.e_tag = A.get<uint64_t>(N);
     r.N = N;
     r.K = kb;
     alloc_tail(r, A, false);

@@ -162,10 +162,7 @@ struct JobDev {
   uint4* e_rec;              // per entry: decode record (pass 1 -> pass 2)
   uint32_t dec_group;        // data blocks per warp in the decode's first pass
   uint32_t dec_unit;         // entries per warp in its second pass
-  uint32_t* e_koff;
-  uint32_t* e_klen;
-  uint32_t* e_voff;
-  uint32_t* e_vlen;
+  uint4* e_loc;               // key offset in the arena, key length, value offset in `in`, value length
   uint64_t* e_pfx;           // 8 user-key bytes after the key_skip common bytes, big endian
   uint64_t* e_tag;           // the key's last 8 bytes: (sequence << 8) | type
   uint32_t* e_hash;          // the bloom hash of the user key (jobs with a filter)

@@ -52,8 +52,8 @@ __global__ void k_key_skip(const JobDev* __restrict__ jobs) {
   uint32_t u0 = 0;
   const uint8_t* k0 = nullptr;
   if (n > 0) {
-    k0 = J.keys + J.e_koff[0];
-    u0 = J.e_klen[0] - 8;
+    k0 = J.keys + J.e_loc[0].x;
+    u0 = J.e_loc[0].y - 8;
   }
   // boundary keys: 2 per child
   for (uint32_t x = threadIdx.x; x < 2 * J.n_runs && n > 0; x += blockDim.x) {
@@ -61,8 +61,8 @@ __global__ void k_key_skip(const JobDev* __restrict__ jobs) {
     const uint64_t a = J.run_entry_begin[r], z = J.run_entry_begin[r + 1];
     if (a == z) continue;
     const uint64_t e = (x & 1) ? z - 1 : a;
-    const uint8_t* k = J.keys + J.e_koff[e];
-    const uint32_t u = J.e_klen[e] - 8, m = min(u, u0);
+    const uint8_t* k = J.keys + J.e_loc[e].x;
+    const uint32_t u = J.e_loc[e].y - 8, m = min(u, u0);
     uint32_t l = 0;
     while (l < m && k[l] == k0[l]) l++;
     atomicMin(&s_skip, l);
@@ -113,11 +113,11 @@ __global__ void __launch_bounds__(256, 8) k_prefix(const JobDev* __restrict__ jo
   const uint32_t L = J.ctr->key_skip;
   const uint64_t n = J.ctr->n_entries_in;
   if (n == 0) return;
-  const uint8_t* k0 = J.keys + J.e_koff[0];
+  const uint8_t* k0 = J.keys + J.e_loc[0].x;
   for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (uint64_t)gridDim.x * blockDim.x) {
-    const uint8_t* k = J.keys + J.e_koff[e];
-    const uint32_t kl = J.e_klen[e];  // >= 8: shorter keys failed the decode
+    const uint8_t* k = J.keys + J.e_loc[e].x;
+    const uint32_t kl = J.e_loc[e].y;  // >= 8: shorter keys failed the decode
     bool bad = false;
     uint64_t p;
     if (L) {
@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(256, 8) k_prefix(const JobDev* __restrict__ jo
       p = J.e_pfx[e];
     }
     if (!bad && e > 0 && !run_first(J, e)) {
-      const uint8_t* kp = J.keys + J.e_koff[e - 1];
-      const uint32_t klp = J.e_klen[e - 1];
+      const uint8_t* kp = J.keys + J.e_loc[e - 1].x;
+      const uint32_t klp = J.e_loc[e - 1].y;
       const uint64_t pp = L ? (klp - 8 < L ? 0 : user_prefix_after(kp, klp, L)) : J.e_pfx[e - 1];
       bad = pp > p || (pp == p && ikey_cmp(kp, klp, k, kl) > 0);
     }
@@ -351,7 +351,7 @@ __device__ __forceinline__ bool keep_entry(const JobDev& J, uint64_t p, uint64_t
     return false;
   if (type == 0 && (tag >> 8) <= J.smallest_snapshot) {
     const uint32_t id = J.m_ids[p];
-    if (is_base_level(J, J.keys + J.e_koff[id], J.e_klen[id] - 8)) return false;
+    if (is_base_level(J, J.keys + J.e_loc[id].x, J.e_loc[id].y - 8)) return false;
   }
   return true;
 }
@@ -373,7 +373,7 @@ __device__ __forceinline__ uint32_t grandparents_passed(const JobDev& J, uint64_
       const uint32_t id = J.m_ids[p];
       const uint64_t go = J.gp_key_off[mid];
       const uint32_t gl = (uint32_t)(J.gp_key_off[mid + 1] - go);
-      after = ikey_cmp(J.keys + J.e_koff[id], J.e_klen[id], J.gp_keys + go, gl) > 0;
+      after = ikey_cmp(J.keys + J.e_loc[id].x, J.e_loc[id].y, J.gp_keys + go, gl) > 0;
     }
     if (after) lo = mid + 1;
     else hi = mid;
@@ -592,12 +592,12 @@ __device__ __forceinline__ void gather_kept(const JobDev& J, const uint16_t* s_l
     // the survivor before the warp's first
     const bool any_prev = base + j0 != 0;
     const uint64_t pp = j0 ? t0 + s_list[j0 - 1] : prev;
-    uint32_t lid = any_prev ? J.m_ids[pp] : 0u, lkl = any_prev ? J.e_klen[lid] : 8u;
+    uint32_t lid = any_prev ? J.m_ids[pp] : 0u, lkl = any_prev ? J.e_loc[lid].y : 8u;
     uint64_t lpx = any_prev ? J.m_pfx[pp] : 0u;
 #pragma unroll
     for (uint32_t i = 0; i < kTwo; i++) {
-      koff[i] = J.e_koff[id[i]], kl[i] = J.e_klen[id[i]];
-      voff[i] = J.e_voff[id[i]], vl[i] = J.e_vlen[id[i]];
+      const uint4 loc = J.e_loc[id[i]];
+      koff[i] = loc.x, kl[i] = loc.y, voff[i] = loc.z, vl[i] = loc.w;
       hash[i] = J.bits_per_key > 0 ? J.e_hash[id[i]] : 0u;
     }
 #pragma unroll
@@ -618,7 +618,7 @@ __device__ __forceinline__ void gather_kept(const JobDev& J, const uint16_t* s_l
         const uint64_t d = px[i] ^ ppx;
         shared = min(L + (d ? (uint32_t)__clzll(d) >> 3 : 8u), mu);
         if (!d || shared == mu) {
-          const uint8_t *x = J.keys + koff[i], *y = J.keys + J.e_koff[pid];
+          const uint8_t *x = J.keys + koff[i], *y = J.keys + J.e_loc[pid].x;
           while (shared < m && x[shared] == y[shared]) shared++;
         }
       }
