@@ -566,7 +566,6 @@ struct JobRun {
   Counters hc{};
   std::vector<FileOut> files;
   std::vector<uint32_t> klen;  // lengths of the files' smallest and largest keys
-  std::vector<uint64_t> koff;  // (run_build: the same, as copied from the device)
   uint8_t* dec_block = nullptr;  // keep_decoded: the decoded buffer (device output slab)
   uint64_t dec_cap = 0;
 };
@@ -1554,14 +1553,32 @@ void run_build(lc_job* j, lc_slot& slot) {
     J.cap_key_bytes = kb;
     J.cap_entries = N;
     J.ctr = A.get<Counters>(1);
-    Counters init{};
-    init.n_kept = N;
-    init.n_entries_in = N;
-    CK(cudaMemcpyAsync(J.ctr, &init, sizeof(Counters), cudaMemcpyHostToDevice, st));
     r.N = N;
     r.K = kb;
     alloc_tail(r, A, false);
-    CK(cudaMemcpyAsync(slot.d_jobs, &J, sizeof(JobDev), cudaMemcpyHostToDevice, st));
+    // pinned staging, as a batch's: [counters | files | key lengths | keys |
+    // descriptor].  (Six copies of pageable memory, a wait each, took 60 us of
+    // a 4 MiB flush.)
+    const auto up16 = [](size_t x) { return (x + 15) & ~size_t(15); };
+    const size_t p_files = up16(sizeof(Counters));
+    const size_t p_klen = p_files + up16(sizeof(FileOut) * J.cap_files);
+    const size_t p_keys = p_klen + up16(8 * (2ull * J.cap_files + 1));
+    const size_t keys_cap = 2ull * J.cap_files * r.max_klen + 1;
+    const size_t p_job = p_keys + up16(keys_cap);
+    uint8_t* pin = slot.pinned(p_job + up16(sizeof(JobDev)));
+    if (uint8_t* m = slot.pin_dev) {
+      J.res_ctr = reinterpret_cast<Counters*>(m);
+      J.res_files = reinterpret_cast<FileOut*>(m + p_files);
+      J.res_klen = reinterpret_cast<uint32_t*>(m + p_klen);
+      J.res_keys = m + p_keys;
+    }
+    Counters init{};
+    init.n_kept = N;
+    init.n_entries_in = N;
+    memcpy(pin, &init, sizeof(Counters));
+    memcpy(pin + p_job, &J, sizeof(JobDev));
+    slot.to_device(J.ctr, pin, sizeof(Counters));
+    slot.to_device(slot.d_jobs, pin + p_job, sizeof(JobDev));
     Batch bt;
     bt.d = slot.d_jobs;
     bt.B = 1;
@@ -1576,26 +1593,33 @@ void run_build(lc_job* j, lc_slot& slot) {
     CK(cudaGetLastError());
     launch_tail(bt, false, st, T);
     CK(cudaGetLastError());
-    Counters hc;
-    r.files.resize(J.cap_files);
-    r.koff.resize(2ull * J.cap_files + 1);
-    j->key_bytes.resize(2ull * J.cap_files * r.max_klen + 1);
-    CK(cudaMemcpyAsync(&hc, J.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(r.files.data(), J.files, J.cap_files * sizeof(FileOut), cudaMemcpyDeviceToHost,
-                       st));
-    CK(cudaMemcpyAsync(r.koff.data(), J.fkoff, r.koff.size() * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(j->key_bytes.data(), J.fkeys, j->key_bytes.size(), cudaMemcpyDeviceToHost, st));
+    launch_results(bt, st);
+    if (!slot.pin_dev) {
+      slot.to_host(pin, J.ctr, sizeof(Counters));
+      slot.to_host(pin + p_files, J.files, J.cap_files * sizeof(FileOut));
+      slot.to_host(pin + p_klen, J.fkoff, 8 * (2ull * J.cap_files + 1));
+      slot.to_host(pin + p_keys, J.fkeys, keys_cap);
+    }
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(st));
+    Counters hc;
+    memcpy(&hc, pin, sizeof(Counters));
     std::string m;
     lc_status s = counters_status(hc, &m);
     if (s != LC_OK) throw StatusError{s, m};
+    const uint32_t nf = hc.n_files;
+    const FileOut* files = reinterpret_cast<const FileOut*>(pin + p_files);
+    const auto key_len = [&](uint32_t x) -> uint32_t {
+      return slot.pin_dev ? reinterpret_cast<const uint32_t*>(pin + p_klen)[x]
+                          : (uint32_t)reinterpret_cast<const uint64_t*>(pin + p_klen)[x];
+    };
+    j->key_bytes.assign(pin + p_keys, pin + p_keys + keys_cap);
     const uint64_t nbytes = hc.bytes_out;
     if (nbytes) {
       j->h_out = e->pinned.take(nbytes, &j->h_out_cap);
       if (!j->h_out) throw StatusError{LC_ERR_NO_MEMORY, "pinned host buffer"};
       copy_pieces(j->h_out, J.out, nbytes, cudaMemcpyDeviceToHost, st, piece_for(nbytes));
     }
-    const uint32_t nf = hc.n_files;
     j->file_offset.resize(nf);
     j->file_size.resize(nf);
     j->file_entries.resize(nf);
@@ -1604,13 +1628,13 @@ void run_build(lc_job* j, lc_slot& slot) {
     j->small_len.resize(nf);
     j->large_len.resize(nf);
     for (uint32_t f = 0; f < nf; f++) {
-      j->file_offset[f] = r.files[f].out_off;
-      j->file_size[f] = r.files[f].size;
-      j->file_entries[f] = r.files[f].end_kept - r.files[f].first_kept;
+      j->file_offset[f] = files[f].out_off;
+      j->file_size[f] = files[f].size;
+      j->file_entries[f] = files[f].end_kept - files[f].first_kept;
       j->small_off[f] = 2ull * f * r.max_klen;
-      j->small_len[f] = (uint32_t)r.koff[2 * f];
+      j->small_len[f] = key_len(2 * f);
       j->large_off[f] = (2ull * f + 1) * r.max_klen;
-      j->large_len[f] = (uint32_t)r.koff[2 * f + 1];
+      j->large_len[f] = key_len(2 * f + 1);
     }
     T.mark(kDownload);
     CK(cudaStreamSynchronize(st));
