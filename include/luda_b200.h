@@ -268,7 +268,9 @@ typedef struct {
   uint32_t ctas_per_job;  /* CTAs per job in the grid-stride kernels; 0 = from the sizes */
   uint32_t merge_items;   /* merge-path outputs per thread, 1..32 */
   uint32_t merge_threads; /* threads per merge CTA: 64..1024, a multiple of 32;
-                             the merge tile is merge_threads * merge_items outputs */
+                             the merge tile is at most merge_threads *
+                             merge_items outputs (fewer in small jobs, whose
+                             tiles would not fill the device) */
 } lc_tuning;
 
 lc_status lc_get_tuning(lc_engine* e, lc_tuning* out);

@@ -336,7 +336,6 @@ __global__ void __launch_bounds__(kScanThreads, 5) k_scan_next(const JobDev* __r
   if ((threadIdx.x & 31) == 0 && jump) atomicMax(&J.ctr->max_jump, jump);
 }
 
-
 // Per chunk: exits of the chain for every entry point in the first `window`
 // survivors of the chunk.  The chunk's next() values are staged in shared
 // memory and cut into sub-chunks of kChainSub survivors: every (sub-chunk,
@@ -1114,10 +1113,13 @@ __device__ __forceinline__ void enc_prefetch(const JobDev& J, const EncWarp& W, 
   }
 }
 
-// Where in its block (bytes from the block's start) the round of 32 entries
-// that holds block byte `at` starts, and that round: the prefix sums k_pb
-// give an entry's place but for the restarts before it, whose extra bytes are
-// summed here, a lane per round.
+// The entry that holds block byte `at`, and where in its block (bytes from the
+// block's start) it starts: the prefix sums k_pb give an entry's place but for
+// the restarts before it, whose extra bytes are summed here; first a lane per
+// 32 entries, then a lane per entry.  (Rounds that started at a multiple of 32
+// entries held the end of the window before too: 16 KiB blocks of 250-byte
+// entries, two rounds a window instead of one; with the values' lines brought
+// into L2 a round at a time the kernel took 239 instead of 283 us.)
 __device__ __forceinline__ void enc_seek(const JobDev& J, const EncBlock& B, const RestartDiv& rd,
                                          uint32_t at, uint32_t lane, uint32_t* j0, uint32_t* pos) {
   const uint64_t pb0 = J.k_pb[B.s];

@@ -1,17 +1,19 @@
 // Device-side state of one compaction job, shared by the host orchestration
-// (lc_engine.cu) and the kernels.  All arrays live in HBM; the struct itself is
-// passed to kernels by value.
+// (lc_engine.cu) and the kernels.  All arrays live in HBM; the kernels read the
+// struct from a device array of them, one per job.
 //
 // Data layout in HBM (one job):
 //   in        input tables back to back, each starting on a 16-byte boundary
 //   tables    per input table: offset in `in`, size, run index
 //   blocks    per input data block: offset in `in`, size, entry/key bases
-//   entries   per decoded entry (structure of arrays, input order):
-//               koff/klen  internal key in the key arena `keys`
-//               voff/vlen  value bytes, left in place inside `in`
-//               pfx        first 8 user-key bytes, big endian (compare fast path)
-//   merged    entry ids in merge order; kept ids after the drop rule
-//   per kept entry: restart/compressed sizes, shared prefix, block-start flag
+//   entries   per decoded entry (input order):
+//               loc   internal key's place in the key arena `keys`, value's
+//                     place inside `in`, where it is left
+//               pfx   8 user-key bytes, big endian (compare fast path)
+//               tag   sequence and type
+//               hash  the user key's filter hash
+//   merged    entry ids, prefixes and tags in merge order
+//   per kept entry: places, restart/compressed sizes, shared prefix, block end
 //   per output block / filter group / file: sizes, offsets, separators
 //   out       all output files back to back
 #pragma once

@@ -25,7 +25,7 @@ uint32_t launches_on_this_thread();
 
 // Launches k so that it may be set up (its blocks placed, up to pdl_begin)
 // while the kernel before it in the stream still runs: a job is a chain of
-// some 45 kernels, most of a few microseconds, and a plain launch starts only
+// some 20 to 40 kernels, most of a few microseconds, and a plain launch starts only
 // when its predecessor has drained.  Every kernel launched so begins with
 // pdl_begin().  On B200: an 800-entry
 // job 288 -> 272 us a call, a 66 MiB job 756 -> 719 us.
