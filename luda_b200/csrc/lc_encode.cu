@@ -925,8 +925,6 @@ __global__ void k_file_layout(const JobDev* __restrict__ jobs) {
 // 296 -> 283 us.  Above the limits below the kernels one by one are as fast or
 // faster (2070 blocks and all 80000 entries in the cluster: no gain, 13600
 // blocks: 20 us more), and many jobs at once fill the device with theirs.
-constexpr uint32_t kPartThreads = 512;
-constexpr uint32_t kPartMaxCtas = 8;
 constexpr uint64_t kPartEntries = 8192, kPartBlocks = 8192;
 template <bool kAll>
 __global__ void __launch_bounds__(kPartThreads, 1) k_partition(const JobDev* __restrict__ jobs) {
@@ -1951,15 +1949,6 @@ __global__ void __launch_bounds__(256) k_results(const JobDev* __restrict__ jobs
 void launch_sizes(const Batch& bt, cudaStream_t st) {
   launch(k_sizes, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
-
-namespace {
-// CTAs of a job's k_partition: a power of two, a thread for every item or kPartMaxCtas
-unsigned part_ctas(uint64_t items) {
-  unsigned c = 1;
-  while ((uint64_t)c * kPartThreads < items && c < kPartMaxCtas) c *= 2;
-  return c;
-}
-}  // namespace
 
 void launch_partition(const Batch& bt, cudaStream_t st) {
   const uint64_t chunks = (bt.max_entries + bt.chunk - 1) / bt.chunk + 1;

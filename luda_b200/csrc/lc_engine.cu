@@ -1175,12 +1175,13 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
         launch_block_count(bt, st);
         scan_batch(kScanBlkEnt, bt, bt.max_blocks_in, st);
         scan_batch(kScanBlkKey, bt, bt.max_blocks_in, st);
-      } else {
-        launch_block_restarts(bt, st);
-        scan_batch(kScanBlkEnt, bt, bt.max_blocks_in, st);
       }
     }
-    launch_parse_done(bt, st);  // (the counters, into mapped memory)
+    // (the counters, into mapped memory)
+    if (bt.max_tables && !exact)
+      launch_parse_blocks(bt, st);
+    else
+      launch_parse_done(bt, st);
     CK(cudaGetLastError());
     T.mark(kParse);
     std::vector<Counters> hc(B);

@@ -77,6 +77,16 @@ constexpr uint32_t kEncWindow = 4608;  // 9 full CRC rows
 constexpr uint32_t kMergeMaxTile = 4096;
 constexpr uint32_t kMergeSmemPerPos = 14;
 
+// Kernels that take a small job's steps in one launch: one cluster of CTAs per
+// job (k_parse_blocks, k_partition).
+constexpr uint32_t kPartThreads = 512, kPartMaxCtas = 8;
+// Their CTAs: a power of two, a thread for every item or kPartMaxCtas.
+inline unsigned part_ctas(uint64_t items) {
+  unsigned c = 1;
+  while ((uint64_t)c * kPartThreads < items && c < kPartMaxCtas) c *= 2;
+  return c;
+}
+
 // k_scan_next: survivors after its tile that it keeps, and the largest entry
 // and block size its 32-bit sums are for.
 constexpr uint32_t kNextHalo = 512, kNextBig = 1u << 19;
@@ -138,7 +148,8 @@ void launch_crc32c_chunks(const uint8_t* data, uint64_t n, uint32_t* scratch, ui
 void launch_table_index_count(const Batch& bt, cudaStream_t st);
 void launch_table_index_entries(const Batch& bt, cudaStream_t st);
 void launch_block_count(const Batch& bt, cudaStream_t st);     // exact key counts (full walk)
-void launch_block_restarts(const Batch& bt, cudaStream_t st);  // entry counts from restart words
+// entry counts from restart words and their sums, and what launch_parse_done does
+void launch_parse_blocks(const Batch& bt, cudaStream_t st);
 void launch_parse_done(const Batch& bt, cudaStream_t st);  // merge children's entries; counters out
 // Checks the CRC32C trailer of every input data block of the jobs that ask
 // for it (verify_checksums), after the block list is known.
