@@ -103,11 +103,11 @@ def parse_args():
 
 # DRAM bytes (read + write) per launch of each kernel, from one ncu capture
 # on each workload: (workload, kernel) -> bytes; None where none was taken.
-# large_A's capture ran at scale 0.25 (profiles/k_encode_blocks_large_A.md:
-# 276.8 + 222.3 MB); the kernel's traffic grows with the bytes it moves, so
+# large_A's capture ran at a quarter of its size (profiles/k_encode_blocks_large_A.md:
+# 285.4 + 227.8 MB); the kernel's traffic grows with the bytes it moves, so
 # the full-size figure is four times that.
 NCU_TRAFFIC = {
-    ("large_A", "encode_blocks"): 4 * (276.840960e6 + 223.603712e6),
+    ("large_A", "encode_blocks"): 4 * (285.409792e6 + 227.791360e6),
 }
 
 
