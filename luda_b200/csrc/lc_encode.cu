@@ -418,14 +418,16 @@ __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
 // Exits (and blocks, in the high half) of groups of kChainGroup chunks for
 // every entry point in the first `window` survivors of the group's first
 // chunk, by following the chunk tables (one thread per entry point).  Only
-// when the chunk tables do not fit the resolving CTA's shared memory.
+// for more chunks than a group has whose tables do not fit the resolving
+// CTA's shared memory (the host, which knows neither the survivors nor the
+// window, launches this for every job that may have more than a group's).
 __device__ __forceinline__ void chain_groups(const JobDev& J, uint32_t cta, uint32_t ctas) {
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
   if (W > C || n == 0) return;
   const uint64_t M = (n + C - 1) / C;
-  if (M * W <= J.chain_smem_words) return;  // resolved from the chunk tables directly
+  if (M <= kChainGroup || M * W <= J.chain_smem_words) return;  // resolved from the chunk tables
   const uint64_t G = (M + kChainGroup - 1) / kChainGroup;
   for (uint64_t x = (uint64_t)cta * blockDim.x + threadIdx.x; x < G * W;
        x += (uint64_t)ctas * blockDim.x) {
@@ -449,10 +451,11 @@ __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
 }
 
 // Entry point and first block of every chunk: the chain from survivor 0
-// through the chunk tables.  Few chunks: one thread walks them over a
-// shared-memory copy of the tables.  Many: one thread walks the group tables
-// (in shared memory when they fit), then one thread per group walks its chunks
-// from the group's entry point.
+// through the chunk tables.  Few chunks, or small tables: one thread walks
+// the tables, over a shared-memory copy where they fit (else a dependent load
+// a chunk, as a group's table would take to build).  Many: one thread walks
+// the group tables (in shared memory when they fit), then one thread per group
+// walks its chunks from the group's entry point.
 __device__ __forceinline__ void chain_resolve(const JobDev& J, uint32_t* s_tab) {
   const uint64_t n = J.ctr->n_kept;
   const uint32_t C = J.chunk;
@@ -477,16 +480,19 @@ __device__ __forceinline__ void chain_resolve(const JobDev& J, uint32_t* s_tab) 
     return;
   }
   const uint64_t M = (n + C - 1) / C;
-  if (M * W <= J.chain_smem_words) {
-    for (uint64_t i = threadIdx.x; i < M * W; i += blockDim.x)
-      s_tab[i] = J.chunk_table[(i / W) * C + (i % W)];
-    __syncthreads();
+  const bool fit = M * W <= J.chain_smem_words;
+  if (fit || M <= kChainGroup) {
+    if (fit) {
+      for (uint64_t i = threadIdx.x; i < M * W; i += blockDim.x)
+        s_tab[i] = J.chunk_table[(i / W) * C + (i % W)];
+      __syncthreads();
+    }
     if (threadIdx.x != 0) return;
     uint64_t e = 0, b = 0;
     for (uint64_t c = 0; c < M; c++) {
       J.chunk_entry[c] = make_uint2((uint32_t)e, (uint32_t)b);
       if (e < n) {
-        const uint32_t w = s_tab[c * W + (e - c * C)];
+        const uint32_t w = fit ? s_tab[c * W + (e - c * C)] : J.chunk_table[c * C + (e - c * C)];
         e = c * C + (w & 0xffff);
         b += w >> 16;
       }
@@ -1974,7 +1980,7 @@ void launch_partition(const Batch& bt, cudaStream_t st) {
   }
   const dim3 g((unsigned)std::min<uint64_t>(chunks, bt.per_job(148 * 4)), bt.B);
   launch(k_chain_tables, g, 256, smem, st, bt.d);
-  if (chunks > kChainGroup)
+  if (chunks > kChainGroup)  // (one more than the survivors can have)
     launch(k_chain_groups, dim3(grid_x(chunks / kChainGroup * bt.chunk, 256, 148 * 4), bt.B), 256, 0, st, bt.d);
   launch(k_chain_resolve, dim3(1, bt.B), 1024, resolve_smem, st, bt.d);
   launch(k_chain_mark, g, 128, smem, st, bt.d);
