@@ -81,7 +81,7 @@ __device__ __forceinline__ const uint8_t* entry_header(const uint8_t* p, const u
   return p;
 }
 
-__global__ void k_table_index_count(const JobDev* __restrict__ jobs) {
+__global__ void k_table_index_count(const JobDev* jobs) {  // may follow the upload
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   const uint32_t t = blockIdx.x;
@@ -578,7 +578,7 @@ __device__ __forceinline__ void parse_done(const JobDev& J, uint32_t cta, uint32
       reinterpret_cast<uint64_t*>(J.res_ctr)[i] = reinterpret_cast<const uint64_t*>(J.ctr)[i];
 }
 
-__global__ void k_parse_done(const JobDev* __restrict__ jobs) {
+__global__ void k_parse_done(const JobDev* jobs) {  // may follow the upload
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   parse_done(J, blockIdx.x, gridDim.x);
@@ -646,7 +646,7 @@ __device__ __forceinline__ uint4 dec_record(uint32_t src, uint32_t sh, uint32_t 
   return make_uint4(src, sh | (kl << 16), vl, voff);
 }
 
-__global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* __restrict__ jobs) {
+__global__ void __launch_bounds__(256, 5) k_decode_walk(const JobDev* jobs) {  // may follow the upload
   pdl_begin();
   __shared__ JobDev s_job;
   {  // the surplus CTAs of a small job leave at once
@@ -1066,7 +1066,7 @@ __global__ void __launch_bounds__(256, 4) k_decode_keys(const JobDev* __restrict
   }
 }
 
-__global__ void k_entries_from_offsets(const JobDev* __restrict__ jobs) {
+__global__ void k_entries_from_offsets(const JobDev* jobs) {  // may follow the upload
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
   const uint64_t n = J.cap_entries;

@@ -406,8 +406,8 @@ __global__ void __launch_bounds__(kKeepThreads, 12) k_drop(const JobDev* __restr
   if (s_failed) return;
   const uint64_t n = J.ctr->n_entries_in;
   uint32_t* counts = reinterpret_cast<uint32_t*>(J.scan_scratch);
-  const uint64_t* __restrict__ tags = J.m_tag;
-  const uint64_t* __restrict__ pfx = J.m_pfx;
+  const uint64_t* tags = J.m_tag;
+  const uint64_t* pfx = J.m_pfx;
   const bool gps = J.n_gp != 0;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (uint64_t t = blockIdx.x; t * kKeepTile < n; t += gridDim.x) {

@@ -113,7 +113,7 @@ namespace {
 // copies in turn, so with other jobs' bulk uploads and downloads in flight a
 // few-KB cudaMemcpyAsync waited behind megabytes of them and held up its
 // job's next kernels.  16-byte words, then the last bytes.
-__global__ void k_xfer(uint8_t* __restrict__ dst, const uint8_t* __restrict__ src, uint64_t n) {
+__global__ void k_xfer(uint8_t* dst, const uint8_t* src, uint64_t n) {
   pdl_begin();
   const uint64_t n16 = n / 16;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
