@@ -480,19 +480,31 @@ __device__ __forceinline__ void chain_resolve(const JobDev& J, uint32_t* s_tab) 
     return;
   }
   const uint64_t M = (n + C - 1) / C;
-  const bool fit = M * W <= J.chain_smem_words;
-  if (fit || M <= kChainGroup) {
-    if (fit) {
-      for (uint64_t i = threadIdx.x; i < M * W; i += blockDim.x)
-        s_tab[i] = J.chunk_table[(i / W) * C + (i % W)];
-      __syncthreads();
-    }
+  if (M * W <= J.chain_smem_words) {
+    for (uint64_t i = threadIdx.x; i < M * W; i += blockDim.x)
+      s_tab[i] = J.chunk_table[(i / W) * C + (i % W)];
+    __syncthreads();
     if (threadIdx.x != 0) return;
     uint64_t e = 0, b = 0;
     for (uint64_t c = 0; c < M; c++) {
       J.chunk_entry[c] = make_uint2((uint32_t)e, (uint32_t)b);
       if (e < n) {
-        const uint32_t w = fit ? s_tab[c * W + (e - c * C)] : J.chunk_table[c * C + (e - c * C)];
+        const uint32_t w = s_tab[c * W + (e - c * C)];
+        e = c * C + (w & 0xffff);
+        b += w >> 16;
+      }
+    }
+    finish(b);
+    return;
+  }
+  if (M <= kChainGroup) {
+    if (threadIdx.x != 0) return;
+    const uint32_t* const table = J.chunk_table;
+    uint32_t e = 0, b = 0;
+    for (uint32_t c = 0; c < (uint32_t)M; c++) {
+      J.chunk_entry[c] = make_uint2(e, b);
+      if (e < n) {
+        const uint32_t w = table[e];  // chunk c's table begins at its first survivor's place
         e = c * C + (w & 0xffff);
         b += w >> 16;
       }
