@@ -345,6 +345,16 @@ __global__ void __launch_bounds__(kScanThreads, 5) k_scan_next(const JobDev* __r
 // than a sub-chunk walk the chunk directly.
 constexpr uint32_t kChainSub = 256;
 
+// The chunk the chain is followed by, from the longest block W.  Where it is
+// longer than the one the job was launched for, next() is read from memory
+// instead of a stage: room for a long chunk in every launch cost the kernel
+// after k_chain_mark 7 us (k_partition of 80000 entries 21 -> 28.5 us).  60000
+// entries of 250 bytes with 3000 empty values in a row, in 16 KiB blocks, block
+// by block by one thread: 289 us for the partition phase, so 133.
+__device__ __forceinline__ uint32_t chain_chunk(const JobDev& J, uint32_t W) {
+  return W <= J.chunk ? J.chunk : kChunk;
+}
+
 // A chain table's word: how far past the (sub-)chunk's first survivor the
 // chain leaves it (below 2^14: a chunk and a window), and above bit 16 the
 // blocks started inside it.
@@ -352,7 +362,7 @@ __device__ __forceinline__ uint32_t chain_word(uint64_t exit_rel, uint32_t block
   return (uint32_t)exit_rel | (blocks << 16);
 }
 
-// The chain from survivor e of a staged chunk at c0 until it reaches `end`.
+// The chain from survivor e of a chunk at c0 (s_next: its next() values) until it reaches `end`.
 __device__ __forceinline__ uint32_t chain_walk(const uint32_t* s_next, uint64_t c0, uint64_t e,
                                                uint64_t end, uint64_t from) {
   uint32_t blocks = 0;
@@ -367,14 +377,19 @@ __device__ __forceinline__ void chain_tables(const JobDev& J, uint32_t cta, uint
   const uint32_t* const knext = J.k_next;
   uint32_t* const table = J.chunk_table;
   const uint64_t n = J.ctr->n_kept;
-  const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
+  const uint32_t C = chain_chunk(J, W);
   if (W > C) return;  // resolved sequentially instead
   const bool sub = W <= kChainSub;
   uint32_t* s_sub = s_next + C;  // (C / kChainSub) x W
   for (uint64_t c = cta; c * C < n; c += ctas) {
     const uint64_t c0 = c * C;
     const uint64_t c1 = min(n, c0 + C);
+    if (C != J.chunk) {
+      for (uint32_t i = threadIdx.x; i < W; i += blockDim.x)
+        table[c * C + i] = chain_walk(knext + c0, c0, c0 + i, c1, c0);
+      continue;
+    }
     __syncthreads();
     for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = knext[c0 + i];
     __syncthreads();
@@ -423,8 +438,8 @@ __global__ void k_chain_tables(const JobDev* __restrict__ jobs) {
 // window, launches this for every job that may have more than a group's).
 __device__ __forceinline__ void chain_groups(const JobDev& J, uint32_t cta, uint32_t ctas) {
   const uint64_t n = J.ctr->n_kept;
-  const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
+  const uint32_t C = chain_chunk(J, W);
   if (W > C || n == 0) return;
   const uint64_t M = (n + C - 1) / C;
   if (M <= kChainGroup || M * W <= J.chain_smem_words) return;  // resolved from the chunk tables
@@ -458,8 +473,8 @@ __global__ void k_chain_groups(const JobDev* __restrict__ jobs) {
 // walks its chunks from the group's entry point.
 __device__ __forceinline__ void chain_resolve(const JobDev& J, uint32_t* s_tab) {
   const uint64_t n = J.ctr->n_kept;
-  const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
+  const uint32_t C = chain_chunk(J, W);
   const auto finish = [&](uint64_t blocks) {
     J.b_first[blocks] = (uint32_t)n;
     J.ctr->n_blocks_out = blocks;
@@ -570,8 +585,8 @@ __device__ __forceinline__ void chain_mark(const JobDev& J, uint32_t cta, uint32
   const uint32_t* const knext = J.k_next;
   uint32_t* const first = J.b_first;
   const uint64_t n = J.ctr->n_kept;
-  const uint32_t C = J.chunk;
   const uint32_t W = J.ctr->max_jump;
+  const uint32_t C = chain_chunk(J, W);
   if (W > C) return;
   const bool sub = W <= kChainSub;
   uint32_t* s_sub = s_next + C;
@@ -580,6 +595,13 @@ __device__ __forceinline__ void chain_mark(const JobDev& J, uint32_t cta, uint32
     const uint64_t c0 = c * C;
     const uint64_t c1 = min(n, c0 + C);
     const uint2 at = J.chunk_entry[c];
+    if (C != J.chunk) {
+      if (threadIdx.x == 0) {
+        uint32_t e = at.x, b = at.y;
+        for (; e < c1; e = knext[e]) first[b++] = e;
+      }
+      continue;
+    }
     __syncthreads();
     for (uint64_t i = threadIdx.x; i < c1 - c0; i += blockDim.x) s_next[i] = knext[c0 + i];
     __syncthreads();

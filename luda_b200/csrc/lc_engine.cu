@@ -47,11 +47,6 @@ thread_local std::string g_last_error;
 
 const char* kVersion = "luda_b200 0.1 (sm_100a)";
 constexpr uint32_t kCrcXpowN = 8192;
-// Survivors per chunk of the block chain (a CTA each): short chunks for batches
-// too small to give every SM a long one, when blocks are expected (from the
-// block size and the mean entry) to hold at most a quarter as many; blocks of
-// more survivors than a chunk are resolved one after the other.
-constexpr uint32_t kChunk = 4096, kShortChunk = 1024;
 
 struct CudaError {
   cudaError_t e;
@@ -660,9 +655,9 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
   J.k_shared = A.get<uint32_t>(N);
   J.k_next = A.get<uint32_t>(N);
   const uint64_t chunks = (N + J.chunk - 1) / J.chunk + 1;
-  J.chunk_table = A.get<uint32_t>(chunks * J.chunk);
+  J.chunk_table = A.get<uint32_t>(((N + kChunk - 1) / kChunk + 1) * kChunk);  // chunks of either length
   J.chunk_entry = A.get<uint2>(chunks);
-  J.group_table = A.get<uint64_t>((chunks / kChainGroup + 1) * J.chunk);
+  J.group_table = A.get<uint64_t>((chunks / kChainGroup + 1) * kChunk);
   J.b_first = A.get<uint32_t>(N + 1);
   J.b_size = A.get<uint32_t>(N);
   J.tmp32 = A.get<uint32_t>(N);

@@ -202,7 +202,7 @@ struct JobDev {
   uint32_t* k_next;          // first entry of the next block if a block starts here
 
   // chain resolution
-  uint32_t chunk;            // entries per chunk
+  uint32_t chunk;            // entries per chunk (kChunk where a block is longer: chain_chunk)
   uint32_t* chunk_table;     // per chunk: exit and blocks for each window entry (chain_word)
   uint2* chunk_entry;        // per chunk: resolved entry point, first block
   uint64_t* group_table;     // per group of kChainGroup chunks: exit | blocks << 32

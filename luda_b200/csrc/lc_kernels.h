@@ -64,6 +64,13 @@ void decode_kernel_attributes();
 void encode_kernel_attributes();
 void merge_kernel_attributes();
 
+// Survivors per chunk of the block chain (a CTA each): short chunks for batches
+// too small to give every SM a long one, when blocks are expected (from the
+// block size and the mean entry) to hold at most a quarter as many.  A job in
+// which a block turns out longer than a short chunk goes by long ones
+// (chain_chunk); blocks of more survivors than those are resolved one after
+// the other.
+constexpr uint32_t kChunk = 4096, kShortChunk = 1024;
 // Chunks per group in the block-chain resolution.
 constexpr uint32_t kChainGroup = 64;
 
@@ -105,7 +112,7 @@ struct Batch {
   uint64_t max_dec_groups = 0, max_dec_units = 0;  // decode work units
   uint32_t merge_rounds = 0;
   uint32_t max_runs = 1;
-  uint32_t chunk = 4096;    // survivors per chunk of the block chain
+  uint32_t chunk = kChunk;  // survivors per chunk of the block chain
   uint32_t chain_smem_words = 11 * 1024;
   bool any_verify = false;  // some job checks its input blocks' CRCs
   bool any_keep_decoded = false;  // some job keeps its outputs' decoded form

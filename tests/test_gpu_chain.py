@@ -150,3 +150,39 @@ def test_flush_matches_restatement(engine, oracle_lib, other_job, name):
     want = oracle.build_table(entries, opts, "oracle")
     other_job()
     assert engine.build_table(entries, opts) == want
+
+
+# A block of more survivors than a short chunk among blocks of some 60: the job
+# goes by long chunks, and is not walked block by block.
+def stretch(count):
+    n, opts = 60000, TableOptions(16384, 16, 10, 1 << 21)
+    lens = value_lens(n, 240, 260, ((20000, count),))
+    keys = [internal_key(user_key(i, 16), 1 + i, 1) for i in range(n)]
+    e = Entries.from_lists(keys, [b"v" * int(v) for v in lens])
+    f = FileMeta(0, 1, e.key(0), e.key(n - 1), entries=e)
+    job = CompactionJob(0, [f], [], 1 << 30, opts)
+    job.materialize(lambda x, o: oracle.build_table(x, o, "oracle"))
+    return job, longest_block(keys, lens, opts)
+
+
+@pytest.mark.gpu
+def test_one_long_block_costs_no_serial_walk(oracle_lib):
+    """Of some 940 blocks.  Walked one after the other by a thread (a dependent
+    load of device memory each, half a microsecond or more) they take 500 us,
+    where the whole partition phase of the job without the stretch takes about
+    100: four times that is the limit."""
+    from luda_b200.engine import Engine
+    ms = []
+    with Engine(0, phase_timing=True) as eng:
+        for count in (0, 3000):
+            job, longest = stretch(count)
+            assert longest <= 256 if not count else 1024 < longest <= 4096
+            got = []
+            for _ in range(8):
+                res = eng.run(eng.prepare(job))
+                got.append(res.phase_ms["partition"])
+                files = res.file_bytes()
+                res.release()
+            assert files == [w[0] for w in oracle.compact(job, "oracle")]
+            ms.append(min(got))
+    assert ms[1] < 4 * ms[0], ms
