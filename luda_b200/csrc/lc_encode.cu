@@ -897,8 +897,13 @@ __device__ void block_layout_one(const JobDev& J, uint64_t b) {
   }
 }
 
+// Pieces of a filter, metaindex or index block, a warp each in k_meta_crc.
+constexpr uint32_t kMetaPiece = 4096;
+__device__ __forceinline__ uint64_t meta_pieces(uint64_t len) { return (len + kMetaPiece - 1) / kMetaPiece; }
+
 __device__ __forceinline__ void file_layout(const JobDev& J) {
   const uint32_t nf = J.ctr->n_files;
+  uint32_t pieces = 0;
   for (uint32_t f = threadIdx.x; f < nf; f += blockDim.x) {
     FileOut& F = J.files[f];
     const uint32_t fb0 = F.first_block, fb1 = F.end_block;
@@ -928,7 +933,10 @@ __device__ __forceinline__ void file_layout(const JobDev& J) {
     F.index_off = meta_off + F.meta_size + kTrailer;
     F.index_size = (J.b_icum[fb1] - J.b_icum[fb0]) + 4ull * (fb1 - fb0) + 4;
     F.size = F.index_off + F.index_size + kTrailer + kFooter;
+    pieces += (uint32_t)(meta_pieces(F.filter_size) + meta_pieces(F.meta_size) + meta_pieces(F.index_size));
   }
+  pieces = __reduce_add_sync(0xffffffffu, pieces);
+  if ((threadIdx.x & 31) == 0 && pieces) atomicAdd(&J.ctr->meta_pieces, pieces);
   __syncthreads();
   if (threadIdx.x == 0) {
     uint64_t o = 0;
@@ -1827,10 +1835,11 @@ __global__ void k_emit_decoded(const JobDev* __restrict__ jobs) {
 // piece's 16-byte chunks); a piece's raw register, moved to the region's end
 // past its type byte, is xored into the file's accumulator (the xor of every
 // byte's share is the register of the whole), and k_meta_trailers writes the
-// finished CRCs.  The grid follows the job's entries (the filter and index
-// blocks grow with them); a grid of CTAs per file and file slot spent 446 us of
-// a 32-job batch on CTAs that loaded their tables and had no file.
-constexpr uint32_t kMetaPiece = 4096;
+// finished CRCs.  As many CTAs work as there are pieces for (a grid of CTAs per
+// file and file slot spent 446 us of a 32-job batch on CTAs that loaded their
+// tables and had no file; one by the entries alone left the filter offsets of
+// large values, 4 bytes per 2 KiB of data, to a few warps: 240 MiB of 4-64 KiB
+// values 55 us, and 66 us for the trailers of their 61000 windows; now 12 and 5).
 
 __device__ __forceinline__ void meta_region(const FileOut& F, uint32_t r, uint64_t* off,
                                             uint64_t* len) {
@@ -1853,7 +1862,7 @@ __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ job
   __shared__ uint32_t s_xinv[kCrcXinvSmem];
   __shared__ uint32_t s_tab8[256];
   if (J.ctr->error) return;
-  const uint32_t ctas = (uint32_t)min((uint64_t)gridDim.x, J.ctr->n_kept / 4096 + 1);  // at work
+  const uint32_t ctas = min(gridDim.x, (J.ctr->meta_pieces + 7) / 8);  // at work: 8 warps each
   if (blockIdx.x >= ctas) return;
   for (uint32_t i = threadIdx.x; i < kCrcH5Words; i += blockDim.x) s_h5[i] = J.crc_h5[i];
   for (uint32_t i = threadIdx.x; i < kCrcXinvN; i += blockDim.x) s_xinv[xinv_slot(i)] = J.crc_xinv[i];
@@ -1869,7 +1878,7 @@ __global__ void __launch_bounds__(256) k_meta_crc(const JobDev* __restrict__ job
 #pragma unroll
     for (uint32_t r = 0; r < 3; r++) {
       meta_region(F, r, &off[r], &len[r]);
-      np[r] = (r == 0 && J.bits_per_key <= 0) ? 0 : (len[r] + kMetaPiece - 1) / kMetaPiece;
+      np[r] = meta_pieces(len[r]);  // (no filter: no bytes)
     }
     return np[0] + np[1] + np[2];
   };
@@ -2051,9 +2060,14 @@ void launch_emit_decoded(const Batch& bt, cudaStream_t st) {
   launch(k_emit_decoded, dim3(grid_x(bt.max_entries, 256, bt.per_job(148 * 8)), bt.B), 256, 0, st, bt.d);
 }
 void launch_encode_meta(const Batch& bt, cudaStream_t st) {
-  launch(k_meta_crc, dim3(grid_x(bt.max_entries, 4096, bt.per_job(148 * 4)), bt.B), 256, 0, st, bt.d);
-  // (the wide blocks are at most the entries)
-  launch(k_meta_trailers, dim3(std::max((3 * bt.max_cap_files + 255) / 256, grid_x(bt.max_entries, 2048, bt.per_job(148 * 2))), bt.B), 256, 0, st, bt.d);
+  // a CTA for 32 KiB of filter and index: an entry has at most some 64 bytes of
+  // them (when it is a block by itself), 16 MiB of data (6600 units of max_cap_wide)
+  // have 32 KiB of filter offsets
+  launch(k_meta_crc, dim3(grid_x(bt.max_entries + bt.max_cap_wide / 8, 512, bt.per_job(148 * 4)), bt.B),
+         256, 0, st, bt.d);
+  launch(k_meta_trailers,
+         dim3(std::max((3 * bt.max_cap_files + 255) / 256, grid_x(bt.max_cap_wide, 512, bt.per_job(148 * 2))), bt.B),
+         256, 0, st, bt.d);
 }
 
 void launch_results(const Batch& bt, cudaStream_t st) {

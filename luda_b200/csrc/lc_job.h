@@ -51,7 +51,7 @@ struct Counters {
   uint32_t n_triggers;
   uint32_t n_files;
   uint32_t n_wide;  // windows of the output blocks too wide for the encoder's stage
-  uint32_t pad;
+  uint32_t meta_pieces;       // pieces of the files' filter, metaindex and index blocks (k_meta_crc)
   uint64_t kept_key_bytes;    // internal-key bytes of the survivors
   uint64_t kept_value_bytes;  // value bytes of the survivors
   uint64_t key_cursor;        // arena bytes the decode's units have taken
