@@ -265,7 +265,9 @@ lc_status lc_engine_get_stats(lc_engine* e, lc_engine_stats* out);
 
 /* Launch parameters the autotuner chooses (no counterpart in the reference). */
 typedef struct {
-  uint32_t ctas_per_job;  /* CTAs per job in the grid-stride kernels; 0 = from the sizes */
+  uint32_t ctas_per_job;  /* CTAs per job in the grid-stride kernels; 0 = from the sizes (the
+                             kernels that take a small job's steps in one launch have their
+                             own number) */
   uint32_t merge_items;   /* merge-path outputs per thread, 1..32 */
   uint32_t merge_threads; /* threads per merge CTA: 64..1024, a multiple of 32;
                              the merge tile is at most merge_threads *

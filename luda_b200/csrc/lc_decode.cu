@@ -415,7 +415,7 @@ __device__ void block_count_one(const JobDev& J, uint64_t b, uint32_t lane, cons
     if (!all_ok) set_error(J.ctr, kErrBadBlock, (uint32_t)b);
     else if (any_short) set_error(J.ctr, kErrShortKey, (uint32_t)b);
     J.blk_nent[b] = all_ok ? (uint32_t)ent : 0;
-    J.blk_kbytes[b] = all_ok ? kb : 0;
+    if (all_ok) atomicAdd((unsigned long long*)&J.ctr->key_bytes_in, (unsigned long long)kb);
     atomicMax(&J.ctr->max_klen, maxk);
   }
 }
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kDecWarps * 32) k_block_count(const JobDev* __
       for (int o = 16; o > 0; o >>= 1) mk = max(mk, __shfl_xor_sync(0xffffffffu, mk, o));
       if (lane == 0) {
         J.blk_nent[b] = (uint32_t)(j1 - j0);
-        J.blk_kbytes[b] = R.kcum[j1] - R.kcum[j0];
+        atomicAdd((unsigned long long*)&J.ctr->key_bytes_in, (unsigned long long)(R.kcum[j1] - R.kcum[j0]));
         atomicMax(&J.ctr->max_klen, mk);
       }
       continue;

@@ -84,17 +84,9 @@ __host__ __device__ __forceinline__ uint32_t varint_len(uint64_t v) {
   }
   return n;
 }
-// 32-bit forms of the two above (no 64-bit shifts or compares).
+// Its 32-bit form (no 64-bit shifts or compares).
 __device__ __forceinline__ uint32_t varint_len32(uint32_t v) {
   return 1u + (v >= (1u << 7)) + (v >= (1u << 14)) + (v >= (1u << 21)) + (v >= (1u << 28));
-}
-__device__ __forceinline__ uint8_t* put_varint32(uint8_t* p, uint32_t v) {
-  while (v >= 128) {
-    *p++ = (uint8_t)(v | 128);
-    v >>= 7;
-  }
-  *p++ = (uint8_t)v;
-  return p;
 }
 __device__ __forceinline__ uint8_t* put_varint(uint8_t* p, uint64_t v) {
   while (v >= 128) {

@@ -719,7 +719,6 @@ void alloc_tail(JobRun& r, DevAlloc& A, bool with_merge) {
   J.fkeys = A.get<uint8_t>(2ull * J.cap_files * r.max_klen + 1);
   J.fkey_stride = r.max_klen;
   J.fkoff = A.get<uint64_t>(2ull * J.cap_files + 1);
-  J.cap_scan = N + 1;
   J.scan_scratch = A.get<uint64_t>(scan_scratch_elems(N + 1));
 }
 
@@ -1112,8 +1111,6 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       J.blk_run = A.get<uint32_t>(cap_blk);
       J.blk_nent = A.get<uint32_t>(cap_blk);
       J.blk_ent_base = A.get<uint64_t>(cap_blk + 1);
-      J.blk_kbytes = A.get<uint64_t>(cap_blk);
-      J.blk_key_base = A.get<uint64_t>(cap_blk + 1);
       J.scan_scratch = A.get<uint64_t>(scan_scratch_elems(cap_blk + J.n_tables + 1));
       J.run_entry_begin_w = A.get<uint64_t>(J.n_runs + 1);
       J.run_entry_begin = J.run_entry_begin_w;
@@ -1169,7 +1166,6 @@ void run_batch(std::vector<lc_job*>& jobs, lc_slot& slot, const Tunables& tun,
       if (exact) {
         launch_block_count(bt, st);
         scan_batch(kScanBlkEnt, bt, bt.max_blocks_in, st);
-        scan_batch(kScanBlkKey, bt, bt.max_blocks_in, st);
       }
     }
     // (the counters, into mapped memory)
@@ -2343,6 +2339,7 @@ lc_status lc_autotune(lc_engine* e, int32_t n, const lc_job_desc* descs, int32_t
   for (uint32_t th : threads)
     for (uint32_t it : items) {
       if (s != LC_OK) break;
+      if (th * it > kMergeMaxTile) continue;  // launched as a smaller one
       Tunables t = best;
       t.merge_threads = th;
       t.merge_items = it;

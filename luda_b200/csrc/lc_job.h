@@ -152,8 +152,6 @@ struct JobDev {
   uint32_t* blk_run;         // merge child of the block
   uint32_t* blk_nent;        // entries per block
   uint64_t* blk_ent_base;    // cap_blocks_in + 1
-  uint64_t* blk_kbytes;      // key bytes per block
-  uint64_t* blk_key_base;    // cap_blocks_in + 1
   uint64_t cap_blocks_in;
 
   // entries (input order)
@@ -206,16 +204,16 @@ struct JobDev {
   uint32_t* chunk_table;     // per chunk: exit and blocks for each window entry (chain_word)
   uint2* chunk_entry;        // per chunk: resolved entry point, first block
   uint64_t* group_table;     // per group of kChainGroup chunks: exit | blocks << 32
-  uint32_t window;           // table width
   uint32_t chain_smem_words; // shared-memory words for staging the chunk tables
-  uint32_t reserve_keys;     // 1: decode reserves key-arena space per block (single
-                             // pass, restart counts only); 0: blk_key_base from counting
-  uint32_t max_key_len;      // 1: longest key the single-pass layout allows
+  uint32_t reserve_keys;     // 1: single pass, capacities from the input's bytes (what outgrows
+                             // one is rerun with exact counting: kErrRetryExact); 0: the key
+                             // bytes were counted
+  uint32_t max_key_len;      // longest key the single pass allows
 
   // output blocks
-  uint32_t* b_first;         // first kept entry of block (cap_blocks_out + 1)
+  uint32_t* b_first;         // first kept entry of block, and the end of the last
   uint32_t* b_size;          // block contents size (without trailer)
-  uint64_t* b_cum;           // prefix of (b_size + 5), cap_blocks_out + 1
+  uint64_t* b_cum;           // prefix of (b_size + 5), and the total
   uint32_t* b_file;          // file of block
   uint64_t* b_off;           // block offset within its file
   uint32_t* b_isize;         // index entry size
@@ -234,7 +232,6 @@ struct JobDev {
   uint32_t cap_wide;
   uint32_t* b_crc;           // wide blocks: raw CRC32C registers xored from their windows
                              // (k_next's memory, which the layout no longer needs)
-  uint64_t cap_blocks_out;
 
   // files
   FileOut* files;
@@ -256,7 +253,6 @@ struct JobDev {
   const uint64_t* src_koffs; // flush encoder: key offsets (n + 1)
   const uint64_t* src_voffs; // flush encoder: value offsets (n + 1)
   uint64_t* scan_scratch;    // tile sums of the prefix sums
-  uint64_t cap_scan;         // capacity of the arrays scanned (for the tile sums)
 
   // CRC32C shift table: x^(8m) mod P for m in [0, crc_tab_n)
   const uint32_t* crc_xpow;

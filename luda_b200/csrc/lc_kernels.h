@@ -135,7 +135,6 @@ struct Batch {
 // lc_scan.cu -- exclusive prefix sums over per-job arrays chosen by selector
 enum ScanSel : int {
   kScanBlkEnt = 0,             // blk_nent -> blk_ent_base           (total: n_entries_in)
-  kScanBlkKey,         // blk_kbytes -> blk_key_base         (total: key_bytes_in)
   kScanBcum,           // tmp32 -> b_cum
   kScanGcum,           // b_gbytes -> b_gcum
   kScanIcum,           // b_isize -> b_icum

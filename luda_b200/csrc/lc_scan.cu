@@ -87,7 +87,6 @@ void scan_sel(const Batch& bt, uint64_t n_est, cudaStream_t st) {
 void scan_batch(ScanSel sel, const Batch& bt, uint64_t n_est, cudaStream_t st) {
   switch (sel) {
     case kScanBlkEnt: scan_sel<kScanBlkEnt>(bt, n_est, st); break;
-    case kScanBlkKey: scan_sel<kScanBlkKey>(bt, n_est, st); break;
     case kScanBcum: scan_sel<kScanBcum>(bt, n_est, st); break;
     case kScanGcum: scan_sel<kScanGcum>(bt, n_est, st); break;
     case kScanIcum: scan_sel<kScanIcum>(bt, n_est, st); break;

@@ -26,15 +26,6 @@ struct ScanOf<kScanBlkEnt> {
   static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->n_entries_in; }
 };
 template <>
-struct ScanOf<kScanBlkKey> {
-  using TI = uint64_t;
-  using TO = uint64_t;
-  static __device__ const TI* in(const JobDev& J) { return J.blk_kbytes; }
-  static __device__ TO* out(const JobDev& J) { return J.blk_key_base; }
-  static __device__ uint64_t n(const JobDev& J) { return min(J.ctr->n_blocks_in, J.cap_blocks_in); }
-  static __device__ uint64_t* total(const JobDev& J) { return &J.ctr->key_bytes_in; }
-};
-template <>
 struct ScanOf<kScanBcum> {
   using TI = uint32_t;
   using TO = uint64_t;
