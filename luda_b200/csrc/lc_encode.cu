@@ -194,8 +194,10 @@ __global__ void __launch_bounds__(256, 6) k_next(const JobDev* __restrict__ jobs
 
 // k_pb and next() in one: a CTA scans a tile of k_b (the second launch of the
 // long scan), keeps the sums of the tile and of the
-// kNextHalo survivors after it in shared memory and finds next() from them.  A
-// block that reaches beyond is walked entry by entry over k_a and k_b.
+// kNextHalo survivors after it in shared memory and finds next() from them.
+// Blocks that reach beyond are followed a span at a time (next_beyond; walked
+// entry by entry, 1M entries of which nine tenths were empty values in 32 KiB
+// blocks of 2730 took 7319 us for the partition phase, so 510).
 //
 // The searches read k_pb (8 bytes a survivor) and k_a, k_b from memory before,
 // about 14 dependent loads a survivor: 8M survivors in blocks of 66, the scan's
@@ -204,26 +206,98 @@ __global__ void __launch_bounds__(256, 6) k_next(const JobDev* __restrict__ jobs
 // take 13 us, a form of this kernel that summed the survivors before its tile
 // itself 22.  Blocks of more than kNextHalo / 2 entries on average (many would
 // reach past the halo) stay with k_next too.
-__device__ __forceinline__ uint64_t next_walk(const JobDev& J, uint64_t s, uint64_t limit) {
-  const uint32_t R = J.restart_interval;
-  uint64_t est = 4;
-  uint32_t r = 0;  // entries since the last restart
-  for (uint64_t e = s; e < limit; e++) {
-    est += r == 0 ? J.k_a[e] + 4ull : J.k_b[e];
-    if (est >= J.block_size) return e + 1;
-    if (++r == R) r = 0;
+constexpr uint32_t kNextSpan = kTile + kNextHalo;
+static_assert((uint64_t)kNextSpan * kNextBig + 2 * kNextBig < 1ull << 31);
+
+// The end of the range that a block from survivor s may cover: the first
+// grandparent cut after s, or n.
+__device__ __forceinline__ uint64_t next_limit(const uint32_t* cuts, uint32_t ncuts, uint64_t s, uint64_t n) {
+  uint32_t lo = 0, hi = ncuts;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (cuts[mid] <= s) lo = mid + 1;
+    else hi = mid;
   }
-  return limit;
+  return lo < ncuts ? min(n, (uint64_t)cuts[lo]) : n;
 }
+
+// next() of the survivors of the tile at t0 that have none yet (0), those whose
+// block reaches past what k_scan_next holds.  The CTA takes the survivors from
+// t0 on a span at a time and keeps where each search stands, the next restart
+// (from t0) in tmp32 and the bytes still missing in b_size, both free until the
+// blocks are sized.  Entries count as at most kNextBig bytes, which ends any
+// block that reaches them (block sizes are at most that).
+__device__ __forceinline__ void next_beyond(const JobDev& J, uint64_t t0, uint32_t* s_pb, uint32_t* s_d) {
+  constexpr uint32_t kPer = kNextSpan / kScanThreads;
+  const uint64_t n = J.ctr->n_kept;
+  const uint32_t here = (uint32_t)min(n - t0, (uint64_t)kTile);
+  const uint32_t R = J.restart_interval, ncuts = J.ctr->n_triggers;
+  const uint32_t *const ka = J.k_a, *const kb = J.k_b, *const cuts = J.t_kept;
+  uint32_t *const out = J.k_next, *const at = J.tmp32, *const rem = J.b_size;
+  uint32_t jump = 0;
+  bool left = false;
+  for (uint32_t i = threadIdx.x; i < here; i += kScanThreads) left |= out[t0 + i] == 0;
+  for (uint32_t w = 0; __syncthreads_or(left); w += kNextSpan) {
+    const uint64_t w0 = t0 + w;
+    const uint32_t len = (uint32_t)min(n - w0, (uint64_t)kNextSpan);
+    uint32_t sum = 0, total;
+    for (uint32_t k = kPer * threadIdx.x; k < kPer * (threadIdx.x + 1); k++) {
+      const uint32_t b = k < len ? min(kb[w0 + k], kNextBig) : 0;
+      s_d[k] = (k < len ? min(ka[w0 + k], kNextBig) : 0) - b;
+      s_pb[k] = sum;
+      sum += b;
+    }
+    const uint32_t ex = block_excl_scan<uint32_t>(sum, &total);
+    for (uint32_t k = kPer * threadIdx.x; k < kPer * (threadIdx.x + 1); k++) s_pb[k] += ex;
+    if (threadIdx.x == 0) s_pb[kNextSpan] = total;
+    __syncthreads();
+    left = false;
+    for (uint32_t i = threadIdx.x; i < here; i += kScanThreads) {
+      if (out[t0 + i]) continue;
+      const uint64_t limit = next_limit(cuts, ncuts, t0 + i, n);
+      const uint32_t end = (uint32_t)min(limit - t0, (uint64_t)w + len);  // searched up to here
+      uint32_t cur = w ? w : i, x = w ? at[t0 + i] : i, nxt = 0;
+      uint32_t need = (w ? rem[t0 + i] : (uint32_t)J.block_size - 4) + s_pb[cur - w];
+      while (cur < end) {
+        if (cur == x) {
+          need -= s_d[cur - w] + 4;
+          x += R;
+        }
+        const uint32_t z = min(x, end);
+        if ((int32_t)(s_pb[z - w] - need) >= 0) {
+          uint32_t l = cur, r = z - 1;
+          while (l < r) {
+            const uint32_t mid = (l + r) >> 1;
+            if ((int32_t)(s_pb[mid + 1 - w] - need) >= 0) r = mid;
+            else l = mid + 1;
+          }
+          nxt = l + 1;
+          break;
+        }
+        cur = z;
+      }
+      if (!nxt && t0 + end == limit) nxt = end;
+      if (nxt) {
+        out[t0 + i] = (uint32_t)t0 + nxt;
+        jump = max(jump, nxt - i);
+      } else {
+        at[t0 + i] = x;
+        rem[t0 + i] = need - s_pb[end - w];
+        left = true;
+      }
+    }
+  }
+  if (jump) atomicMax(&J.ctr->max_jump, jump);
+}
+
 __global__ void __launch_bounds__(kScanThreads, 5) k_scan_next(const JobDev* __restrict__ jobs) {
   pdl_begin();
   const JobDev& J = jobs[blockIdx.y];
-  constexpr uint32_t kSpan = kTile + kNextHalo, kHaloItems = kNextHalo / kScanThreads;
+  constexpr uint32_t kSpan = kNextSpan, kHaloItems = kNextHalo / kScanThreads;
   __shared__ uint32_t s_failed;  // read once per CTA: the CTA's barriers stay uniform
-  // sums of k_b from the tile's first survivor (if an entry of the span has more
-  // than kNextBig bytes the tile's survivors walk instead), restarts' extra bytes
+  // sums of k_b from the tile's first survivor (not used if an entry of the span
+  // has more than kNextBig bytes), restarts' extra bytes
   __shared__ __align__(16) uint32_t s_pb[kSpan + 1], s_d[kSpan];
-  static_assert((uint64_t)kSpan * kNextBig + 2 * kNextBig < 1ull << 31);
   if (threadIdx.x == 0) s_failed = J.ctr->error;
   __syncthreads();
   if (s_failed) return;
@@ -237,6 +311,7 @@ __global__ void __launch_bounds__(kScanThreads, 5) k_scan_next(const JobDev* __r
   const uint32_t bs = (uint32_t)J.block_size;
   uint64_t carry = tiles_sum<uint64_t, false>(kb, tile_sums, 0, blockIdx.x, kTile, n);
   uint32_t jump = 0;
+  bool left = false;
   for (uint64_t t = blockIdx.x; t * kTile <= n; t += gridDim.x) {
     const uint64_t t0 = t * kTile;
     const uint32_t avail = (uint32_t)min(n - t0, (uint64_t)kSpan);
@@ -294,17 +369,11 @@ __global__ void __launch_bounds__(kScanThreads, 5) k_scan_next(const JobDev* __r
         pb[tb + k] = ex;
       ex = e1 + v[k + 1];
     }
-    const bool walk = __syncthreads_or(big);
+    const bool over = __syncthreads_or(big);
     const uint32_t here = (uint32_t)min(n - t0, (uint64_t)kTile);
     for (uint32_t i = threadIdx.x; i < here; i += kScanThreads) {
-      uint32_t lo = 0, hi = ncuts;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (cuts[mid] <= t0 + i) lo = mid + 1;
-        else hi = mid;
-      }
-      const uint64_t limit = lo < ncuts ? min(n, (uint64_t)cuts[lo]) : n;
-      const uint32_t last = walk ? 0 : (uint32_t)min(limit - t0, (uint64_t)avail);  // searched up to here
+      const uint64_t limit = next_limit(cuts, ncuts, t0 + i, n);
+      const uint32_t last = over ? 0 : (uint32_t)min(limit - t0, (uint64_t)avail);  // searched up to here
       // as next_of: the restart segment that reaches the block size, then the entry
       uint32_t nxt = 0;                // from the tile's first survivor
       uint32_t need = bs + s_pb[i] - 4;  // less the restarts' extra bytes and words, and the count's
@@ -322,15 +391,17 @@ __global__ void __launch_bounds__(kScanThreads, 5) k_scan_next(const JobDev* __r
           break;
         }
       }
-      if (!nxt)
-        nxt = (uint32_t)((t0 + last == limit ? limit : next_walk(J, t0 + i, limit)) - t0);
-      out[t0 + i] = (uint32_t)t0 + nxt;
-      jump = max(jump, nxt - i);
+      if (!nxt && t0 + last == limit) nxt = last;
+      out[t0 + i] = nxt ? (uint32_t)t0 + nxt : 0;
+      if (nxt) jump = max(jump, nxt - i);
+      else left = true;
     }
     __syncthreads();  // the tile's sums have been read
     if ((t + gridDim.x) * kTile <= n)
       carry += tiles_sum<uint64_t, false>(kb, tile_sums, t, t + gridDim.x, kTile, n);
   }
+  if (__syncthreads_or(left))
+    for (uint64_t t = blockIdx.x; t * kTile < n; t += gridDim.x) next_beyond(J, t * kTile, s_pb, s_d);
   // the longest block, one atomic per warp
   jump = __reduce_max_sync(0xffffffffu, jump);
   if ((threadIdx.x & 31) == 0 && jump) atomicMax(&J.ctr->max_jump, jump);
