@@ -1661,34 +1661,64 @@ __device__ __forceinline__ void encode_filters(const JobDev& J, uint32_t* sbuf, 
   }
 }
 
-__device__ __forceinline__ void encode_index_entry(const JobDev& J, uint64_t b) {
-  const FileOut& F = J.files[J.b_file[b]];
-  const uint32_t fb0 = F.first_block, fb1 = F.end_block;
-  uint8_t* ib = J.out + F.out_off + F.index_off;
-  const uint64_t eoff = J.b_icum[b] - J.b_icum[fb0];
-  uint8_t* p = ib + eoff;
-  const uint32_t ilen = J.b_ilen[b], sep = J.b_sep[b];
-  const uint64_t off = J.b_off[b];
-  const uint32_t bsz = J.b_size[b];
-  *p++ = 0;
-  p = put_varint(p, ilen);
-  p = put_varint(p, varint_len(off) + varint_len(bsz));
-  uint32_t llen;
-  const uint8_t* lkey = kept_key(J, J.b_first[b + 1] - 1, &llen);
-  // (copy_small loads a piece's bytes before it stores any)
-  const uint32_t from_key = sep == kNoSep ? ilen : sep;
-  for (uint32_t i = 0; i < from_key; i += 32) copy_small<32>(p + i, lkey + i, min(32u, from_key - i));
-  if (sep != kNoSep) {
-    p[sep] = (uint8_t)(lkey[sep] + 1);
-    uint64_t t = kSeekTag;
-    for (int i = 0; i < 8; i++) p[sep + 1 + i] = (uint8_t)(t >> (8 * i));
+// Index entries: a warp takes a run of up to 32 blocks, a lane each; keys of
+// more than kIndexLong bytes are copied by the warp, one after the other (by
+// their lanes, 1500 keys of 9 KB took 15 ms on B200).
+constexpr uint32_t kIndexLong = 64;
+__device__ __forceinline__ void encode_index(const JobDev& J, uint64_t warp, uint64_t warps, uint32_t lane) {
+  const uint64_t nb = J.ctr->n_blocks_out;
+  const uint64_t run = min((uint64_t)32, (nb + warps - 1) / warps);  // blocks per warp and turn
+  for (uint64_t b0 = warp * run; b0 < nb; b0 += warps * run) {
+    const uint64_t b = b0 + lane;
+    uint32_t from_key = 0;
+    uint8_t* p = nullptr;
+    const uint8_t* lkey = nullptr;
+    if (lane < run && b < nb) {
+      const FileOut& F = J.files[J.b_file[b]];
+      const uint32_t fb0 = F.first_block, fb1 = F.end_block;
+      uint8_t* ib = J.out + F.out_off + F.index_off;
+      const uint64_t eoff = J.b_icum[b] - J.b_icum[fb0];
+      p = ib + eoff;
+      const uint32_t ilen = J.b_ilen[b], sep = J.b_sep[b];
+      const uint64_t off = J.b_off[b];
+      const uint32_t bsz = J.b_size[b];
+      *p++ = 0;
+      p = put_varint(p, ilen);
+      p = put_varint(p, varint_len(off) + varint_len(bsz));
+      uint32_t llen;
+      lkey = kept_key(J, J.b_first[b + 1] - 1, &llen);
+      // (copy_small loads a piece's bytes before it stores any)
+      from_key = sep == kNoSep ? ilen : sep;
+      if (from_key <= kIndexLong)
+        for (uint32_t i = 0; i < from_key; i += 32) copy_small<32>(p + i, lkey + i, min(32u, from_key - i));
+      if (sep != kNoSep) {
+        p[sep] = (uint8_t)(lkey[sep] + 1);
+        uint64_t t = kSeekTag;
+        for (int i = 0; i < 8; i++) p[sep + 1 + i] = (uint8_t)(t >> (8 * i));
+      }
+      uint8_t* q = put_varint(p + ilen, off);
+      put_varint(q, bsz);
+      uint8_t* ra = ib + (J.b_icum[fb1] - J.b_icum[fb0]) + 4 * (b - fb0);
+      st_le32(ra, ((uint32_t)eoff << 8) | 1u);
+      if (b + 1 == fb1) st_le32(ra + 4, fb1 - fb0);
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, from_key > kIndexLong); m; m &= m - 1) {
+      const int e = __ffs(m) - 1;
+      const auto of = [&](const uint8_t* x) {
+        return __shfl_sync(0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(x), e);
+      };
+      uint8_t* d = reinterpret_cast<uint8_t*>(of(p));
+      const uint8_t* k = reinterpret_cast<const uint8_t*>(of(lkey));
+      const uint32_t n = __shfl_sync(0xffffffffu, from_key, e);
+      const uint32_t head = (uint32_t)(-reinterpret_cast<uintptr_t>(d)) & 3, words = (n - head) / 4;
+      const uint32_t tail = head + 4 * words;
+      if (lane < head) d[lane] = k[lane];
+#pragma unroll 4
+      for (uint32_t i = lane; i < words; i += 32)
+        reinterpret_cast<uint32_t*>(d + head)[i] = enc_word(k + head + 4 * i, k + n);
+      if (tail + lane < n) d[tail + lane] = k[tail + lane];
+    }
   }
-  p += ilen;
-  p = put_varint(p, off);
-  p = put_varint(p, bsz);
-  uint8_t* ra = ib + (J.b_icum[fb1] - J.b_icum[fb0]) + 4 * (b - fb0);
-  st_le32(ra, ((uint32_t)eoff << 8) | 1u);
-  if (b + 1 == fb1) st_le32(ra + 4, fb1 - fb0);
 }
 
 // File f's metaindex block, footer and the tail of its filter block's offset
@@ -1751,11 +1781,16 @@ __device__ __forceinline__ void encode_meta_file(const JobDev& J, uint32_t f, ui
 __device__ __forceinline__ void encode_side(const JobDev& J, uint32_t* sbuf, uint32_t cta,
                                             uint32_t ctas) {
   const uint32_t lane = threadIdx.x & 31;
-  const uint64_t thread = (uint64_t)cta * blockDim.x + threadIdx.x, threads = (uint64_t)ctas * blockDim.x;
-  const uint64_t warp = thread >> 5, warps = threads >> 5;
+  // Less than a full turn of blocks: consecutive warps on different CTAs, so that
+  // a few large filters or long index keys spread over the SMs (side by side on
+  // one they wait for its L1: 100000 entries in 64 KiB blocks at 20 bits a key, a
+  // flush 1911 -> 886 us).  More: neighbours in one CTA (8M entries, 126k blocks:
+  // the kernel 537 instead of 555 us).
+  const uint32_t own = threadIdx.x >> 5, per = blockDim.x >> 5;
+  const uint64_t warps = (uint64_t)ctas * per;
+  const uint64_t warp = J.ctr->n_blocks_out < 32 * warps ? (uint64_t)own * ctas + cta : (uint64_t)cta * per + own;
   encode_filters(J, sbuf, warp, warps, lane);
-  const uint64_t nb = J.ctr->n_blocks_out;
-  for (uint64_t b = thread; b < nb; b += threads) encode_index_entry(J, b);
+  encode_index(J, warp, warps, lane);
   for (uint64_t f = warps - 1 - warp; f < J.ctr->n_files; f += warps) encode_meta_file(J, (uint32_t)f, lane);
 }
 
@@ -2119,8 +2154,9 @@ void encode_kernel_attributes() {
 void launch_encode_blocks(const Batch& bt, cudaStream_t st) {
   // grid-stride over the device-side counts of blocks and windows: 2 CTAs per
   // SM x 4 waves (a job of few entries may have as many windows as its output
-  // bytes allow), after the CTAs for everything else
-  const uint32_t side = grid_x(bt.max_entries, 2048, bt.per_job(148));
+  // bytes allow), after the CTAs for everything else: filters and index keys go by
+  // the entries, filter offsets and long keys by the bytes
+  const uint32_t side = grid_x(bt.max_entries + bt.max_cap_wide / 2, 2048, bt.per_job(148));
   const uint32_t enc =
       grid_x(std::max<uint64_t>(bt.max_entries, bt.max_cap_wide), kEncWarps, bt.per_job(148 * 2 * 4));
   launch(k_encode_blocks, dim3(side + enc, bt.B), kEncWarps * 32, kEncSmem, st, bt.d, side);
