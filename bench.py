@@ -869,6 +869,45 @@ def reduce_over_ranks(dist, device, total_ms, e2e_total, in_bytes):
     return float(t[0]), float(t[1]), float(b[0])
 
 
+def summary_line(line):
+    """The record with its legs cut to their figures (28 KB in full, most of it
+    the served loop's slowest jobs) and floats to seven digits."""
+    def num(x):
+        if isinstance(x, float):
+            return float("%.7g" % x)
+        if isinstance(x, dict):
+            return {k: num(v) for k, v in x.items()}
+        return [num(v) for v in x] if isinstance(x, (list, tuple)) else x
+
+    def pick(d, *keys):
+        return None if d is None else {k: d[k] for k in keys if k in d}
+
+    out = dict(line)
+    out["pcie"] = pick(line.get("pcie"), "h2d_gbs", "d2h_gbs", "engine_upload_gbs", "engine_download_gbs")
+    out["legs"] = {}
+    for name, leg in (line.get("legs") or {}).items():
+        cut = pick(leg, "input_mib", "entries_in", "value", "unit", "ms_per_step", "latency_ms", "phase_ms",
+                   "gpu_launches")
+        cut["e2e"] = pick(leg.get("e2e"), "value", "unit", "ms_per_step", "sequential_value")
+        cut["parity"] = pick(leg.get("parity"), "checked", "files")
+        cut["roofline"] = pick(leg.get("roofline"), "kernel", "achieved", "unit", "frac")
+        cut["cpu_baseline"] = pick(leg.get("cpu_baseline"), "value", "unit", "cores", "kind")
+        out["legs"][name] = cut
+    b = line.get("batched")
+    if b:
+        out["batched"] = pick(b, "jobs", "input_mib", "speedup_batched_vs_plain", "speedup_batched_vs_plain_e2e")
+        for k in ("plain", "batched", "plain_e2e", "batched_e2e"):
+            out["batched"][k] = pick(b.get(k), "value", "unit", "ms_per_step", "p50_ms", "p99_ms")
+    sv = line.get("served")
+    if sv:
+        def load(d):
+            return {k: pick(v, "value", "unit", "p50_ms", "p99_ms", "mean_ms", "jobs", "batch_jobs_mean")
+                    if isinstance(v, dict) else v for k, v in d.items()}
+        out["served"] = dict(pick(sv, "flushes", "flush_mib"), capacity=load(sv["capacity"]),
+                             loads={k: load(v) for k, v in sv["loads"].items()})
+    return num(out)
+
+
 def main():
     args = parse_args()
     rank = int(os.environ.get("RANK", "0"))
@@ -954,7 +993,9 @@ def main():
             "gpu_launches": head["gpu_launches"],
             "host": {"cpus": os.cpu_count()},
         }
-        print(json.dumps(line))
+        # the whole record to stderr; the line is for programs that keep a few KB of it
+        print(json.dumps(line), file=sys.stderr)
+        print(json.dumps(summary_line(line)))
     eng.close()
     if dist is not None:
         dist.barrier()
