@@ -650,8 +650,8 @@ __global__ void k_chain_resolve(const JobDev* __restrict__ jobs) {
 // First survivor of every block: each chunk's chain from its resolved entry
 // point.  With sub-chunks, one thread finds the sub-chunks' entry points from
 // their words (recomputed as k_chain_tables does) and every sub-chunk is
-// walked by its own thread.  (The block starts used to be flags that a scan
-// over the survivors turned into block numbers: 8M survivors, 47 us more.)
+// walked by its own thread.  (Block starts as flags that a scan over the
+// survivors turns into block numbers: 8M survivors, 47 us more.)
 __device__ __forceinline__ void chain_mark(const JobDev& J, uint32_t cta, uint32_t ctas, uint32_t* s_next) {
   const uint32_t* const knext = J.k_next;
   uint32_t* const first = J.b_first;
@@ -1101,24 +1101,26 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_partition(const JobDev* __r
 //     stored, so no byte is stored twice and nothing is written bytewise but
 //     headers.
 //  2. The whole 16-byte chunks go out with one bulk copy from shared memory,
-//     and meanwhile every lane feeds its chunks (l, l + 32, ...) to the row
-//     CRC (crc_h5).  The grid bytes outside the message are zero, so every
-//     chunk takes the same step; the initial all-ones register enters at the
-//     end, as its register carried over the message's length (crc_ones).
+//     and meanwhile every lane folds a run of consecutive chunks into its last
+//     32 bytes and looks those up (enc_out).  The grid bytes outside the message
+//     are zero, so every chunk takes the same step; the initial all-ones
+//     register enters at the end, as its register carried over the message's
+//     length (crc_ones).
 //  3. The lanes' registers combined, the trailer, and the partial chunks at
 //     both ends with byte stores.  A window's register is moved over the
 //     bytes after it and xored into its block's (k_meta_trailers finishes
 //     wide blocks).
 //
-// Bound by its serial chain per block (about 2000 instructions and six waits
-// on memory) at the warps an SM holds: 32 of them (64 registers, 5.8 KB of
+// Bound by issue, the integer pipe first (1 KiB values: ALU 62% of its cycles,
+// issue 73%), at the warps an SM holds: 32 of them (64 registers, 5.8 KB of
 // shared memory each) where 24 warps with a 6 KB stage took a third longer.
-// Measured on B200, one launch: 1 GiB of 1 KiB values 866 -> 623 us, 480 MiB of
-// 32-byte values 712 -> 447 us, 66 MiB of lognormal values 224 -> 98 us (before:
-// values as 16-byte chunks straight from global to global memory through the
-// row CRC, short pieces bytewise into the stage); 200 MiB in 16 KiB blocks 2753
-// -> 282 us and 240 MiB of 4-64 KiB values 6759 -> 229 us (before: a lane per
-// entry, byte by byte, for any block beyond the stage).
+// Measured on B200, one launch, filters and index blocks included: 1 GiB of 1 KiB
+// values 677 us, 512 MiB of 32-byte values 537, 66 MiB of lognormal values 88,
+// 210 MiB in 16 KiB blocks 238, 280 MiB of 4-64 KiB values 225.  (The data blocks
+// alone took 866, 712 and 224 us with values as 16-byte chunks straight from
+// global to global memory through the row CRC and short pieces bytewise into the
+// stage, and 2753 and 6759 us by a lane per entry, byte by byte, for any block
+// beyond the stage.)
 struct EncWarp {
   uint32_t ahead[5][kEncAhead];  // next block's entries: key length, shared, value length, key
                                  // offset, value offset
@@ -1570,7 +1572,7 @@ __device__ __forceinline__ void enc_drain(uint32_t lane) {
 //
 // Bound by latency: a warp per group that loaded its group's places and keys
 // itself took 279 us for 8M keys in 126k groups on B200 (70 registers), and 54
-// us for 1M keys in 256k groups; this form 86 and 19 us.
+// us for 1M keys in 256k groups; this form, as a kernel of its own, 86 and 19.
 constexpr uint32_t kFilterSmem = 1024;
 constexpr uint32_t kFilterFew = 8;    // keys, and at most 16 filter bytes: by one lane
 __device__ __forceinline__ void encode_filters(const JobDev& J, uint32_t* sbuf, uint64_t warp,

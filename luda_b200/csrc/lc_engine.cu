@@ -98,9 +98,9 @@ uint64_t piece_for(uint64_t job_bytes) {
 // the next job at once, on any stream: the engine returns scratch and outputs
 // only after the batch that used them has completed, and a caller returns an
 // output (lc_job_release) only after its own reads of it have completed.
-// (Scratch used to come from the stream-ordered pool: a batch bigger than any
-// before made the pool map fresh memory in the middle of the batch, ~0.4 s
-// for a few GB, holding up every other thread's CUDA calls meanwhile.)
+// (With scratch from the stream-ordered pool, a batch bigger than any before makes
+// the pool map fresh memory in the middle of the batch, ~0.4 s for a few GB,
+// holding up every other thread's CUDA calls meanwhile.)
 struct SlabCache {
   static constexpr uint64_t kAlign = 4096;
   const bool device;      // device memory (cudaMalloc) rather than pinned host memory

@@ -25,12 +25,12 @@ uint32_t launches_on_this_thread();
 
 // Launches k so that it may be set up (its blocks placed, up to pdl_begin)
 // while the kernel before it in the stream still runs: a job is a chain of
-// some 20 to 40 kernels, most of a few microseconds, and a plain launch starts only
+// some 20 to 35 kernels, most of a few microseconds, and a plain launch starts only
 // when its predecessor has drained.  Every kernel launched so begins with
 // pdl_begin(), and has no __restrict__ pointer to what its predecessor may still
 // be writing (loads through one may be moved above the wait): the descriptors
-// are one only where their upload cannot be the predecessor.  On B200: an 800-entry
-// job 288 -> 272 us a call, a 66 MiB job 756 -> 719 us.
+// are one only where their upload cannot be the predecessor.  On B200, with chains
+// of 49 kernels: an 800-entry job 288 -> 272 us a call, a 66 MiB job 756 -> 719 us.
 // launch_clusters: the same, in thread-block clusters of `cluster` CTAs along x.
 template <typename... P, typename... A>
 inline void launch_clusters(unsigned cluster, void (*k)(P...), dim3 grid, unsigned threads,
@@ -79,7 +79,7 @@ constexpr uint32_t kChainGroup = 64;
 // kEncNarrow bytes has at most z / (kEncNarrow / 2) windows.
 constexpr uint32_t kEncStage = 5120;
 constexpr uint32_t kEncNarrow = kEncStage - 64;
-constexpr uint32_t kEncWindow = 4608;  // 9 full CRC rows
+constexpr uint32_t kEncWindow = 4608;  // whole 16-byte chunks, inside the stage
 
 // Largest merge tile (threads x items) and the shared memory the tile takes
 // per position.

@@ -247,9 +247,12 @@ __device__ __forceinline__ uint64_t merge_split(const JobDev& J, const MergeRoun
 // finds its own diagonal there and merges `items` outputs as source positions,
 // and the tile is written back with coalesced stores, ids and prefixes from
 // shared memory and the tags from memory by source position (two ascending
-// streams).  Only equal prefixes read key bytes.  Bound by the latency of the
-// serial merge: 14 bytes of shared memory a position instead of 28 and 40
-// registers give an SM 48 warps instead of 24 (8M entries on B200: 221 -> 166 us).
+// streams).  Only equal prefixes read key bytes.  Bound by latency, the tile's
+// loads and the barriers behind them before the serial merge in shared memory
+// (of 2M entries 12.6, 8.1 and 2.3 cycles a warp and instruction issued; DRAM at
+// 8%): 14 bytes of shared memory a position instead of 28 and 40 registers (28
+// bytes of them spilled) give an SM 48 warps instead of 24 (8M entries on B200:
+// 221 -> 166 us).
 __global__ void __maxnreg__(40) k_merge_tile(const JobDev* __restrict__ jobs, uint32_t r,
                                                      uint32_t rounds, uint32_t items) {
   pdl_begin();
@@ -386,9 +389,11 @@ __device__ __forceinline__ uint32_t grandparents_passed(const JobDev& J, uint64_
 // its place (the counts before it) and gathers.  A warp of k_drop loads four
 // strips of its positions ahead (tag and prefix; the position before a lane's
 // is its neighbour's, by shuffle); entry ids only where two prefixes are equal.
-// Bound by the two streams' latency: with the flags' scan and the gather as
-// kernels of their own, 8M entries took 117 + 26 + 91 us on B200 and the
-// entry sizes 108 more; k_drop and k_kept_compact take 71 + 181.
+// Bound by latency: k_drop by its two streams' loads (40 registers for 48 warps an
+// SM; the rare paths' 40 bytes are spilled), k_kept_compact by the gathers from
+// the entry arrays (issue at 38%).  With the flags' scan and the gather as kernels
+// of their own, 8M entries took 117 + 26 + 91 us on B200 and the entry sizes 108
+// more; k_drop and k_kept_compact take 68 + 187.
 constexpr uint32_t kKeepTile = 512;
 constexpr uint32_t kKeepThreads = 128;
 constexpr uint32_t kKeepStrips = kKeepTile / kKeepThreads;
