@@ -343,20 +343,33 @@ __device__ __forceinline__ bool is_base_level(const JobDev& J, const uint8_t* uk
   return true;
 }
 
+// Two entries of equal prefixes: the same user key?  (Lengths first: keys that
+// are prefixes of one another would be walked to the shorter one's end.)
+__device__ __forceinline__ bool same_user_key_rest(const JobDev& J, uint32_t a, uint32_t b) {
+  return J.e_loc[a].y == J.e_loc[b].y && user_key_rest_cmp(J, a, b) == 0;
+}
+
 // The drop rule for merged position p (tag, prefix), after position p - 1
-// (ptag, ppfx).
-__device__ __forceinline__ bool keep_entry(const JobDev& J, uint64_t p, uint64_t tag, uint64_t upfx,
-                                           uint64_t ptag, uint64_t ppfx) {
+// (ptag, ppfx); `in`: there is such a position.  Every lane of the warp takes part:
+// they meet again after each of the two rare searches.
+__device__ __forceinline__ bool keep_entry(const JobDev& J, uint64_t p, bool in, uint64_t tag,
+                                           uint64_t upfx, uint64_t ptag, uint64_t ppfx) {
   const uint32_t type = (uint32_t)(tag & 0xff);
-  if (type > 1) return true;
-  if (p > 0 && ppfx == upfx && (ptag & 0xff) <= 1 && (ptag >> 8) <= J.smallest_snapshot &&
-      user_key_rest_cmp(J, J.m_ids[p - 1], J.m_ids[p]) == 0)
-    return false;
-  if (type == 0 && (tag >> 8) <= J.smallest_snapshot) {
-    const uint32_t id = J.m_ids[p];
-    if (is_base_level(J, J.keys + J.e_loc[id].x, J.e_loc[id].y - 8)) return false;
+  bool hidden = in && type <= 1 && p > 0 && ppfx == upfx && (ptag & 0xff) <= 1 &&
+                (ptag >> 8) <= J.smallest_snapshot;
+  if (__any_sync(0xffffffffu, hidden)) {
+    if (hidden) hidden = same_user_key_rest(J, J.m_ids[p - 1], J.m_ids[p]);
+    __syncwarp();
   }
-  return true;
+  bool dead = in && !hidden && type == 0 && (tag >> 8) <= J.smallest_snapshot;
+  if (__any_sync(0xffffffffu, dead)) {
+    if (dead) {
+      const uint32_t id = J.m_ids[p];
+      dead = is_base_level(J, J.keys + J.e_loc[id].x, J.e_loc[id].y - 8);
+    }
+    __syncwarp();
+  }
+  return in && !hidden && !dead;
 }
 
 // Grandparents passed at merged position p: the count of g with key >
@@ -394,13 +407,20 @@ __device__ __forceinline__ uint32_t grandparents_passed(const JobDev& J, uint64_
 // the entry arrays (issue at 38%).  With the flags' scan and the gather as kernels
 // of their own, 8M entries took 117 + 26 + 91 us on B200 and the entry sizes 108
 // more; k_drop and k_kept_compact take 68 + 187.
-constexpr uint32_t kKeepTile = 512;
+//
+// A tile is kStrips positions a thread: four, or one in jobs whose tiles of four
+// would leave SMs with less than eight.  There the time is that of the rare paths'
+// key comparisons in one warp, strip after strip: 232 deletions of keys with 40
+// bytes in common, looked up in 60 files below, 238 us for both kernels with
+// four, 90 with one; 80000 entries without long comparisons 18 and 16, 267000 55
+// and 51.
 constexpr uint32_t kKeepThreads = 128;
-constexpr uint32_t kKeepStrips = kKeepTile / kKeepThreads;
-static_assert(kKeepTile >= 512, "the counts fit scan_scratch (scan_scratch_elems)");
+static_assert(kKeepThreads >= 128, "the counts fit scan_scratch (scan_scratch_elems)");
 
+template <uint32_t kStrips>
 __global__ void __launch_bounds__(kKeepThreads, 12) k_drop(const JobDev* __restrict__ jobs) {
   pdl_begin();
+  constexpr uint32_t kKeepTile = kStrips * kKeepThreads, kKeepStrips = kStrips;
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed, s_count;
   if (threadIdx.x == 0) {
@@ -431,9 +451,8 @@ __global__ void __launch_bounds__(kKeepThreads, 12) k_drop(const JobDev* __restr
       const uint64_t p = w0 + 32 * i + lane;
       const uint64_t ut = __shfl_up_sync(0xffffffffu, tg[i], 1);
       const uint64_t up = __shfl_up_sync(0xffffffffu, px[i], 1);
-      bool keep = false;
+      const bool keep = keep_entry(J, p, p < n, tg[i], px[i], lane ? ut : lt, lane ? up : lp);
       if (p < n) {
-        keep = keep_entry(J, p, tg[i], px[i], lane ? ut : lt, lane ? up : lp);
         J.keep[p] = keep ? 1 : 0;
         if (gps) J.gp_idx[p] = grandparents_passed(J, p, px[i]);
       }
@@ -550,6 +569,7 @@ __device__ __forceinline__ uint32_t keep_scan(uint32_t v, uint32_t* s_warp, uint
 }
 
 // The last survivor before tile t (which has some before it), by one warp.
+template <uint32_t kKeepTile>
 __device__ __forceinline__ uint64_t last_kept_before(const JobDev& J, const uint32_t* counts,
                                                      uint64_t t) {
   const uint32_t lane = threadIdx.x & 31;
@@ -576,19 +596,19 @@ __device__ __forceinline__ uint64_t last_kept_before(const JobDev& J, const uint
 // with the survivor before it (its neighbour's id, key length and prefix come by
 // shuffle).  The two prefixes (the 8 user-key bytes after the job's common
 // ones) give the shared length when they differ inside both user keys; key
-// bytes are read only otherwise.  Two survivors per thread at a time, so that
+// bytes are read only otherwise.  kPer survivors per thread at a time, so that
 // their loads overlap.
+template <uint32_t kPer>
 __device__ __forceinline__ void gather_kept(const JobDev& J, const uint16_t* s_list, uint32_t total,
                                             uint64_t t0, uint32_t base, uint64_t prev,
                                             unsigned long long* kb, unsigned long long* vb) {
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t L = J.ctr->key_skip;
-  constexpr uint32_t kTwo = 2;
-  for (uint32_t j0 = 32 * kTwo * warp; j0 < total; j0 += kTwo * kKeepThreads) {
-    uint32_t id[kTwo], koff[kTwo], kl[kTwo], voff[kTwo], vl[kTwo], hash[kTwo];
-    uint64_t px[kTwo];
+  for (uint32_t j0 = 32 * kPer * warp; j0 < total; j0 += kPer * kKeepThreads) {
+    uint32_t id[kPer], koff[kPer], kl[kPer], voff[kPer], vl[kPer], hash[kPer];
+    uint64_t px[kPer];
 #pragma unroll
-    for (uint32_t i = 0; i < kTwo; i++) {
+    for (uint32_t i = 0; i < kPer; i++) {
       const uint32_t j = j0 + 32 * i + lane;
       const uint64_t p = t0 + s_list[j < total ? j : 0];
       id[i] = J.m_ids[p];
@@ -600,13 +620,13 @@ __device__ __forceinline__ void gather_kept(const JobDev& J, const uint16_t* s_l
     uint32_t lid = any_prev ? J.m_ids[pp] : 0u, lkl = any_prev ? J.e_loc[lid].y : 8u;
     uint64_t lpx = any_prev ? J.m_pfx[pp] : 0u;
 #pragma unroll
-    for (uint32_t i = 0; i < kTwo; i++) {
+    for (uint32_t i = 0; i < kPer; i++) {
       const uint4 loc = J.e_loc[id[i]];
       koff[i] = loc.x, kl[i] = loc.y, voff[i] = loc.z, vl[i] = loc.w;
       hash[i] = J.bits_per_key > 0 ? J.e_hash[id[i]] : 0u;
     }
 #pragma unroll
-    for (uint32_t i = 0; i < kTwo; i++) {
+    for (uint32_t i = 0; i < kPer; i++) {
       const uint32_t j = j0 + 32 * i + lane;
       uint32_t pid = __shfl_up_sync(0xffffffffu, id[i], 1);
       uint32_t pl = __shfl_up_sync(0xffffffffu, kl[i], 1);
@@ -642,8 +662,10 @@ __device__ __forceinline__ void gather_kept(const JobDev& J, const uint16_t* s_l
   }
 }
 
+template <uint32_t kStrips>
 __global__ void __launch_bounds__(kKeepThreads, 8) k_kept_compact(const JobDev* __restrict__ jobs) {
   pdl_begin();
+  constexpr uint32_t kKeepTile = kStrips * kKeepThreads;
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed, s_warp[kKeepThreads / 32];
   __shared__ uint16_t s_list[kKeepTile];  // the tile's survivors
@@ -663,18 +685,24 @@ __global__ void __launch_bounds__(kKeepThreads, 8) k_kept_compact(const JobDev* 
   uint32_t base = before(0, blockIdx.x);
   unsigned long long kb = 0, vb = 0;
   for (uint64_t t = blockIdx.x; t * kKeepTile < n; t += gridDim.x) {
-    const uint64_t t0 = t * kKeepTile, tb = t0 + 4 * threadIdx.x;
-    uint32_t w = tb < n ? *reinterpret_cast<const uint32_t*>(J.keep + tb) : 0;  // four flags
-    if (tb < n && n - tb < 4) w &= (1u << (8 * (uint32_t)(n - tb))) - 1;
+    const uint64_t t0 = t * kKeepTile, tb = t0 + kStrips * threadIdx.x;
+    uint32_t w = 0;  // the thread's flags
+    if constexpr (kStrips == 4) {
+      w = tb < n ? *reinterpret_cast<const uint32_t*>(J.keep + tb) : 0;
+      if (tb < n && n - tb < 4) w &= (1u << (8 * (uint32_t)(n - tb))) - 1;
+    } else {
+      static_assert(kStrips == 1);
+      w = tb < n ? J.keep[tb] : 0;
+    }
     uint32_t at;
     const uint32_t total = keep_scan((uint32_t)__popc(w), s_warp, &at);
-    for (uint32_t m = w; m; m &= m - 1) s_list[at++] = (uint16_t)(4 * threadIdx.x + ((__ffs(m) - 1) >> 3));
+    for (uint32_t m = w; m; m &= m - 1) s_list[at++] = (uint16_t)(kStrips * threadIdx.x + ((__ffs(m) - 1) >> 3));
     if (base && threadIdx.x < 32) {
-      const uint64_t x = last_kept_before(J, counts, t);
+      const uint64_t x = last_kept_before<kKeepTile>(J, counts, t);
       if (threadIdx.x == 0) s_prev = x;
     }
     __syncthreads();
-    gather_kept(J, s_list, total, t0, base, s_prev, &kb, &vb);
+    gather_kept<kStrips == 1 ? 1 : 2>(J, s_list, total, t0, base, s_prev, &kb, &vb);
     // the survivors before each grandparent cut in the tile
     if (nt) {
       uint32_t lo = 0, hi = nt;
@@ -753,9 +781,16 @@ void launch_merge(const Batch& bt, cudaStream_t st) {
   }
 }
 
+// Positions a thread of k_drop and k_kept_compact: four when the batch has eight
+// tiles of four for every SM.
+static uint32_t keep_strips(const Batch& bt) {
+  return bt.max_entries * bt.jobs_of_largest < 148ull * 8 * 4 * kKeepThreads ? 1 : 4;
+}
+
 void launch_drop(const Batch& bt, cudaStream_t st) {
-  launch(k_drop, dim3(grid_x(bt.max_entries, kKeepTile, bt.per_job(148 * 12)), bt.B), kKeepThreads, 0,
-         st, bt.d);
+  const uint32_t strips = keep_strips(bt);
+  const dim3 g(grid_x(bt.max_entries, strips * kKeepThreads, bt.per_job(148 * 12)), bt.B);
+  launch(strips == 1 ? k_drop<1> : k_drop<4>, g, kKeepThreads, 0, st, bt.d);
 }
 
 void launch_triggers(const Batch& bt, cudaStream_t st) {
@@ -767,8 +802,9 @@ void launch_triggers(const Batch& bt, cudaStream_t st) {
 }
 
 void launch_kept_compact(const Batch& bt, cudaStream_t st) {
-  launch(k_kept_compact, dim3(grid_x(bt.max_entries, kKeepTile, bt.per_job(148 * 12)), bt.B), kKeepThreads,
-         0, st, bt.d);
+  const uint32_t strips = keep_strips(bt);
+  const dim3 g(grid_x(bt.max_entries, strips * kKeepThreads, bt.per_job(148 * 12)), bt.B);
+  launch(strips == 1 ? k_kept_compact<1> : k_kept_compact<4>, g, kKeepThreads, 0, st, bt.d);
 }
 
 }  // namespace lc

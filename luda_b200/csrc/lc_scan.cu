@@ -100,9 +100,9 @@ void tile_sums_kb(const Batch& bt, uint64_t n_est, cudaStream_t st) {
 }
 
 // tile sums for arrays of up to n_cap elements: 8 bytes for every kTile of them
-// here, 4 bytes for every 512 in the drop rule's counts
-uint64_t scan_scratch_elems(uint64_t n_cap) { return (n_cap + 1) / 1024 + 4; }
-static_assert(kTile >= 1024, "scan_scratch_elems");
+// here, 4 bytes for every 128 in the drop rule's counts
+uint64_t scan_scratch_elems(uint64_t n_cap) { return (n_cap + 1) / 256 + 4; }
+static_assert(kTile >= 256, "scan_scratch_elems");
 
 namespace {
 
