@@ -67,6 +67,36 @@ def test_both_tiles_at_the_limit(engine, oracle_lib, past):
     _check(engine, job)
 
 
+def test_nested_keys(engine, oracle_lib):
+    """Keys that are heads of one another, several versions each."""
+    for byte in (b"\xff", b"a", b"\0"):
+        _check(engine, _job([byte * k for k in range(1, 400, 3)], 3, 0.3, [], 4))
+
+
+@pytest.mark.parametrize("skip", [0, 5])
+def test_differing_byte_behind_the_prefix(engine, oracle_lib, skip):
+    """Neighbours that differ first at every place from the prefix's last byte to
+    40 bytes on, with both lengths: word by word from any alignment."""
+    keys = set()
+    for at in range(7, 48):
+        for c in b"\x01\x7f\x80\xff":
+            for more in range(5):
+                keys.add(b"p" * (skip + at) + bytes([c]) + b"z" * more)
+        keys.add(b"p" * (skip + at))
+    _check(engine, _job(sorted(keys), 2, 0.2, [], 6))
+
+
+
+def test_long_equal_keys(oracle_lib):
+    """Two versions of each of four keys of 5 KB in two runs.  Compared byte by byte
+    the merge's rounds (a tile's cuts, a thread's place in it, the merge itself)
+    take 1.5 times the decode phase of these keys, word by word two thirds."""
+    job = _job([b"k%d" % i * 2500 for i in range(4)], 2, 0.0)
+    with Engine(0, phase_timing=True) as eng:
+        res = [eng.run(eng.prepare(job)) for _ in range(6)]
+        assert min(r.phase_ms["merge"] for r in res) < min(r.phase_ms["decode"] for r in res)
+
+
 def _drop_us(job):
     best = None
     with Engine(0, phase_timing=True) as eng:
