@@ -247,11 +247,11 @@ __device__ __forceinline__ uint64_t merge_split(const JobDev& J, const MergeRoun
 // finds its own diagonal there and merges `items` outputs as source positions,
 // and the tile is written back with coalesced stores, ids and prefixes from
 // shared memory and the tags from memory by source position (two ascending
-// streams).  Only equal prefixes read key bytes.  Bound by latency, the tile's
+// streams).  Only equal prefixes read key bytes, word by word.  Bound by latency, the tile's
 // loads and the barriers behind them before the serial merge in shared memory
-// (of 2M entries 12.6, 8.1 and 2.3 cycles a warp and instruction issued; DRAM at
-// 8%): 14 bytes of shared memory a position instead of 28 and 40 registers (28
-// bytes of them spilled) give an SM 48 warps instead of 24 (8M entries on B200:
+// (of 2M entries 13.3, 7.6 and 2.2 cycles a warp and instruction issued; DRAM at
+// 9%): 14 bytes of shared memory a position instead of 28 and 40 registers (the
+// comparison's 48 bytes are spilled) give an SM 48 warps instead of 24 (8M entries on B200:
 // 221 -> 166 us).
 __global__ void __maxnreg__(40) k_merge_tile(const JobDev* __restrict__ jobs, uint32_t r,
                                                      uint32_t rounds, uint32_t items) {
@@ -399,15 +399,14 @@ __device__ __forceinline__ uint32_t grandparents_passed(const JobDev& J, uint64_
 
 // Survivors are found and gathered in tiles of kKeepTile merged positions:
 // k_drop marks them and counts each tile's, k_kept_compact gives every tile
-// its place (the counts before it) and gathers.  A warp of k_drop loads four
-// strips of its positions ahead (tag and prefix; the position before a lane's
+// its place (the counts before it) and gathers.  A warp of k_drop loads its
+// strips of 32 positions ahead (tag and prefix; the position before a lane's
 // is its neighbour's, by shuffle); entry ids only where two prefixes are equal.
 // Bound by latency: k_drop by its two streams' loads (40 registers for 48 warps an
 // SM; the rare paths' 40 bytes are spilled), k_kept_compact by the gathers from
 // the entry arrays (issue at 38%).  With the flags' scan and the gather as kernels
 // of their own, 8M entries took 117 + 26 + 91 us on B200 and the entry sizes 108
 // more; k_drop and k_kept_compact take 68 + 187.
-//
 // A tile is kStrips positions a thread: four, or one in jobs whose tiles of four
 // would leave SMs with less than eight.  There the time is that of the rare paths'
 // key comparisons in one warp, strip after strip: 232 deletions of keys with 40
@@ -420,7 +419,7 @@ static_assert(kKeepThreads >= 128, "the counts fit scan_scratch (scan_scratch_el
 template <uint32_t kStrips>
 __global__ void __launch_bounds__(kKeepThreads, 12) k_drop(const JobDev* __restrict__ jobs) {
   pdl_begin();
-  constexpr uint32_t kKeepTile = kStrips * kKeepThreads, kKeepStrips = kStrips;
+  constexpr uint32_t kKeepTile = kStrips * kKeepThreads;
   const JobDev& J = jobs[blockIdx.y];
   __shared__ uint32_t s_failed, s_count;
   if (threadIdx.x == 0) {
@@ -436,10 +435,10 @@ __global__ void __launch_bounds__(kKeepThreads, 12) k_drop(const JobDev* __restr
   const bool gps = J.n_gp != 0;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (uint64_t t = blockIdx.x; t * kKeepTile < n; t += gridDim.x) {
-    const uint64_t w0 = t * kKeepTile + 32 * kKeepStrips * warp;  // the warp's positions
-    uint64_t tg[kKeepStrips], px[kKeepStrips];
+    const uint64_t w0 = t * kKeepTile + 32 * kStrips * warp;  // the warp's positions
+    uint64_t tg[kStrips], px[kStrips];
 #pragma unroll
-    for (uint32_t i = 0; i < kKeepStrips; i++) {
+    for (uint32_t i = 0; i < kStrips; i++) {
       const uint64_t p = w0 + 32 * i + lane;
       tg[i] = p < n ? tags[p] : 0xff;
       px[i] = p < n ? pfx[p] : 0;
@@ -447,7 +446,7 @@ __global__ void __launch_bounds__(kKeepThreads, 12) k_drop(const JobDev* __restr
     uint64_t lt = w0 > 0 && w0 < n ? tags[w0 - 1] : 0, lp = w0 > 0 && w0 < n ? pfx[w0 - 1] : 0;
     uint32_t cnt = 0;
 #pragma unroll
-    for (uint32_t i = 0; i < kKeepStrips; i++) {
+    for (uint32_t i = 0; i < kStrips; i++) {
       const uint64_t p = w0 + 32 * i + lane;
       const uint64_t ut = __shfl_up_sync(0xffffffffu, tg[i], 1);
       const uint64_t up = __shfl_up_sync(0xffffffffu, px[i], 1);
